@@ -144,6 +144,9 @@ __global__ void __launch_bounds__(kSetupThreads, 3)
     k_f4_lineinit(const LayerPlan* plans, int layer0, const ShrunkLine* sh, int64_t stride,
                               const int64_t* nsh, F4Rec* rec, F4RecD* recd, int64_t rstride, int64_t* nrec,
                               int64_t* nmirror, unsigned long long* stats, double* cpl);
+__global__ void __launch_bounds__(kSetupThreads)
+    k_f4_mirror(const LayerPlan* plans, int layer0, const ShrunkLine* sh, int64_t stride, const int64_t* nsh,
+                F4Rec* rec, F4RecD* recd, int64_t rstride, int64_t* nmirror, unsigned long long* stats, double* cpl);
 // layer averages and amounts of a nadir path (ALAYER + FPACK)
 constexpr int kMaxLayerMol = 64;
 __global__ void k_layer_amounts(int nlev, int nmol, const double* z, const double* p, const double* t,

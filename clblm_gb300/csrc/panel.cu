@@ -1251,7 +1251,7 @@ __global__ void __launch_bounds__(kF4Threads, Plain ? 1 : 16) k_f4_conv(F4Args a
   using Rec = typename std::conditional<Plain, F4RecD, F4Rec>::type;
   __shared__ __align__(128) Rec stage[2][CHUNK];
   __shared__ __align__(8) uint64_t bar[2];
-  __shared__ int64_t rng[2];
+  __shared__ int64_t rng[3];
 
   const int layer = blockIdx.y;
   const LayerPlan& P = a.plans[layer + a.layer0];
@@ -1286,16 +1286,27 @@ __global__ void __launch_bounds__(kF4Threads, Plain ? 1 : 16) k_f4_conv(F4Args a
     }
     rng[0] = lo;
     rng[1] = (m0 >= P.nptr4) ? lo : l;  // tiles past NPTR4 need no records
+    // mirror records lie below 0 cm-1: none reaches a point past 25 cm-1 (with
+    // a step to spare for JMAX's rounding)
+    rng[2] = (m0 >= P.nptr4 || P.v1r4 + P.dvr4 * (double)(m0 - 2) > P.bound4) ? 0 : nm;
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
     mbar_fence_init();
   }
   __syncthreads();
   const int64_t lo = rng[0], hi = rng[1];
-  const int64_t nchunk = (hi - lo + CHUNK - 1) / CHUNK;
+  // chunks of the direct records, then of the mirror records that follow them
+  // in the record list (CNVF4Q adds a line's mirror after the direct lines)
+  const int64_t nchunk_d = (hi - lo + CHUNK - 1) / CHUNK;
+  const int64_t nchunk = nchunk_d + (rng[2] + CHUNK - 1) / CHUNK;
+  auto first_of = [&](int64_t c) { return c < nchunk_d ? lo + c * CHUNK : n + (c - nchunk_d) * CHUNK; };
+  auto count_of = [&](int64_t c) {
+    const int64_t left = (c < nchunk_d ? hi : n + nm) - first_of(c);
+    return left < CHUNK ? left : (int64_t)CHUNK;
+  };
   auto issue = [&](int64_t c) {  // thread 0: chunk c into stage c&1
-    const int64_t r0 = lo + c * CHUNK;
-    const int64_t nr = hi - r0 < CHUNK ? hi - r0 : (int64_t)CHUNK;
+    const int64_t r0 = first_of(c);
+    const int64_t nr = count_of(c);
     const uint32_t bytes = (uint32_t)(nr * (int64_t)sizeof(Rec));
     mbar_arrive_expect_tx(&bar[c & 1], bytes);
     bulk_g2s(&stage[c & 1][0], recs + r0, bytes, &bar[c & 1]);
@@ -1340,8 +1351,7 @@ __global__ void __launch_bounds__(kF4Threads, Plain ? 1 : 16) k_f4_conv(F4Args a
       break;
     }
     const Rec* S = stage[c & 1];
-    const int64_t left = hi - (lo + c * CHUNK);
-    const int cnt = (int)(left < CHUNK ? left : CHUNK);
+    const int cnt = (int)count_of(c);
     if (liveA) {
       if constexpr (Plain) {
         for (int k = 0; k < cnt; ++k) {
@@ -1397,36 +1407,13 @@ __global__ void __launch_bounds__(kF4Threads, Plain ? 1 : 16) k_f4_conv(F4Args a
     mbar_inval(&bar[1]);
   }
   if (failed) return;
-  // the reference's R4 is zero past NPTR4 (LBLF4Q :91-94); mirror records of
-  // lines below 25 cm-1 follow the direct ones
+  // the reference's R4 is zero past NPTR4 (LBLF4Q :91-94)
 #pragma unroll
   for (int q = 0; q < kF4Pts; ++q) {
     const int64_t m = ms[q];
     if (m >= P.nptr4 + 2) continue;
-    if (m >= P.nptr4) {
-      R4[m] = (Real)0;
-      continue;
-    }
-    const int J = (int)m + 1;
-    if constexpr (Plain) {
-      double s = acc[q];
-      for (int64_t i = n; i < n + nm; ++i) {
-        const F4RecD& d = recs[i];
-        if (J >= d.jmin && J <= d.jmax) s += term_d(d, m);
-      }
-      R4[m] = s;
-    } else {
-      KahanF& s = kacc[q];
-      const float2 Jm = q < 2 ? JmAB : JmCD;
-      const int J0 = q < 2 ? JA : JC, J1 = q < 2 ? JB : JD;
-      for (int64_t i = n; i < n + nm; ++i) {
-        const F4Rec& r = recs[i];
-        if (J < r.jmin || J > r.jmax) continue;
-        const float2 t = f4_term<true, true>(r, Jm, dvr4, J0, J1);  // lane x is the pair's first point
-        s.add((q & 1) == 0 ? t.x : t.y);
-      }
-      R4[m] = s.value();
-    }
+    if constexpr (Plain) R4[m] = m < P.nptr4 ? acc[q] : 0.;
+    else R4[m] = m < P.nptr4 ? kacc[q].value() : 0.f;
   }
 }
 

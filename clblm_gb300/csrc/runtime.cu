@@ -1025,6 +1025,20 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
       dplans, first, h->f4sh.as<ShrunkLine>(), f4stride, h->f4nout.as<int64_t>(), h->f4rec.as<F4Rec>(),
       h->f4recd.as<F4RecD>(), rstride, h->f4nrec.as<int64_t>(), h->f4nmir.as<int64_t>(),
       h->stats.as<unsigned long long>(), h->has_cpl ? h->f4cpl.as<double>() : nullptr);
+  {
+    // mirror records: only where a far-wing line may lie at or below 25 cm-1
+    bool low = false;
+    for (int k = 0; k < count; ++k)
+      low |= !(hps[first + k].P.v1l4 - h->shiftmax * hps[first + k].P.rhorat > 26.);
+    if (low) {
+      h->launches++;
+      k_f4_mirror<<<count, kSetupThreads, 0, st>>>(dplans, first, h->f4sh.as<ShrunkLine>(), f4stride,
+                                                   h->f4nout.as<int64_t>(), h->f4rec.as<F4Rec>(),
+                                                   h->f4recd.as<F4RecD>(), rstride, h->f4nmir.as<int64_t>(),
+                                                   h->stats.as<unsigned long long>(),
+                                                   h->has_cpl ? h->f4cpl.as<double>() : nullptr);
+    }
+  }
   h->launches++;
   k_f4_bounds<<<count, 1024, 0, st>>>(h->f4rec.as<F4Rec>(), rstride, h->f4nrec.as<int64_t>(), first,
                                       h->f4pm.as<int>(), h->f4sm.as<int>());
