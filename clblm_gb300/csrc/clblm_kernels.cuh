@@ -136,7 +136,9 @@ __global__ void k_f4_walk(const LayerPlan* __restrict__ plans, int layer0, int n
                           const long long* __restrict__ lbits, const int* __restrict__ gnxt,
                           const unsigned char* __restrict__ flags, const int64_t* __restrict__ ntot,
                           const int64_t* __restrict__ cut, int4* __restrict__ groups, int64_t* __restrict__ ngroups);
-__global__ void k_f4_groupsum(const LayerPlan* plans, int layer0, const F4Prep* prep, int64_t stride,
+constexpr int kGroupSumThreads = 256;
+__global__ void __launch_bounds__(kGroupSumThreads)
+    k_f4_groupsum(const LayerPlan* plans, int layer0, const F4Prep* prep, int64_t stride,
                               const int64_t* src, const int4* groups, const int64_t* ngroups, ShrunkLine* out);
 struct F4Rec;
 struct F4RecD;

@@ -1722,129 +1722,182 @@ template __global__ void k_f4_walk<2>(CLBLM_WALK_ARGS);
 template __global__ void k_f4_walk<kWalkPer>(CLBLM_WALK_ARGS);
 #undef CLBLM_WALK_ARGS
 
+// a coupled line as a pseudo-line of its own (SHRINQ :1566-1578)
+__device__ __forceinline__ ShrunkLine shrunk_coupled(const F4Prep& r, bool mixed) {
+  ShrunkLine L;
+  L.vnu = r.vnu;
+  L.sp = r.sp;
+  if (mixed) {
+    L.w.f[0] = r.w.f[0];
+    L.w.f[1] = r.w.f[1];
+    L.w.f[2] = r.w.f[2];
+    L.w.f[3] = (float)r.spp;
+    L.w.f[4] = L.w.f[5] = 0.f;
+  } else {
+    L.w.d[0] = r.w.d[0];
+    L.w.d[1] = r.w.d[1];
+    L.w.d[2] = r.spp;
+  }
+  L.mol = r.mol == 2 ? 2 : 0;
+  L.pad = 0;
+  return L;
+}
+
+// the pseudo-line of a group's members of kind k (1: CO2) from its sums; the
+// centre sets the record's point range (binary64), the mixed path's widths and
+// strength set none
+__device__ __forceinline__ ShrunkLine shrunk_line(int k, bool mixed, double SUMV, double SUMS, double SUMAL,
+                                                  double SUMAD, float SAL, float SAD) {
+  ShrunkLine L;
+  L.vnu = SUMV / SUMS;
+  L.sp = SUMS;
+  if (mixed) {
+    const float sf = (float)SUMS;
+    L.w.f[0] = SAL / sf;
+    L.w.f[1] = SAD / sf;
+    L.w.f[2] = sf;
+    L.w.f[3] = 0.f;  // SUMC: zero
+    L.w.f[4] = L.w.f[5] = 0.f;
+  } else {
+    L.w.d[0] = SUMAL / SUMS;
+    L.w.d[1] = SUMAD / SUMS;
+    L.w.d[2] = 0.;  // SUMC
+  }
+  L.mol = k ? 2 : 0;
+  L.pad = 0;
+  return L;
+}
+
 // Sums of each group in the reference's order (SHRINQ :1563-1637): non-CO2
 // members into one pseudo-line, CO2 members into another, written to the
 // group's output slots.
-__global__ void k_f4_groupsum(const LayerPlan* __restrict__ plans, int layer0, const F4Prep* __restrict__ prep,
-                              int64_t stride, const int64_t* __restrict__ src, const int4* __restrict__ groups,
-                              const int64_t* __restrict__ ngroups, ShrunkLine* __restrict__ out) {
+//
+// The sums set line centres (SUMV/SUMS), so they are added one by one in the
+// reference's order; what bounds the kernel is the chain of a group's member
+// loads and binary64 additions.  A warp takes a group: its lanes load 32
+// members at once and form their products, and lanes 0..7 then add one sum
+// each (the kinds' SUMV, SUMS, SUMAL, SUMAD) from shared memory, one member a
+// step.  Zero products stand in for the members of the other kind (x + 0 = x).
+// A surface layer's groups hold 64 lines and more (DVR4/2 = 0.32 cm-1 at 200
+// lines per cm-1): 170 us for one such layer with a thread per group, whose
+// loads followed one another.  Layers with fewer than kGroupWarpMin lines
+// per group keep a thread per group: their chains are short and there are
+// many of them (a warp each would leave most lanes idle).
+constexpr int kGroupWarps = kGroupSumThreads / 32;
+constexpr int kGroupWarpMin = 6;  // mean lines per group from which a warp takes a group
+
+// one group by one thread
+__device__ __forceinline__ void group_sum_thread(const F4Prep* __restrict__ pr, const int64_t* __restrict__ S,
+                                                 const int4 gr, bool mixed, ShrunkLine* __restrict__ O) {
+  int slot = gr.z;
+  double SUMS[2] = {0., 0.}, SUMV[2] = {0., 0.}, AL[2] = {0., 0.}, AD[2] = {0., 0.};
+  float ALf[2] = {0.f, 0.f}, ADf[2] = {0.f, 0.f};
+  for (int u = gr.x; u <= gr.y; ++u) {
+    const F4Prep& r = pr[S[u]];
+    const bool weak = r.sp < 1.0e-35;
+    if (!weak && r.spp != 0.) {  // a coupled line is not shrunk (SHRINQ :1566-1578)
+      O[slot++] = shrunk_coupled(r, mixed);
+      continue;
+    }
+    const double sp = weak ? 0.0 : r.sp;
+    auto add = [&](int k) {
+      SUMV[k] = SUMV[k] + r.vnu * sp;
+      SUMS[k] = SUMS[k] + sp;
+      if (mixed) {  // widths set no index: FP32
+        const float spf = weak ? 0.f : r.w.f[2];
+        ALf[k] = ALf[k] + spf * r.w.f[0];
+        ADf[k] = ADf[k] + spf * r.w.f[1];
+      } else {
+        AL[k] = AL[k] + sp * r.w.d[0];
+        AD[k] = AD[k] + sp * r.w.d[1];
+      }
+    };
+    if (r.mol != 2) add(0);
+    else add(1);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    if (SUMS[k] > 0.) O[slot++] = shrunk_line(k, mixed, SUMV[k], SUMS[k], AL[k], AD[k], ALf[k], ADf[k]);
+}
+
+__global__ void __launch_bounds__(kGroupSumThreads)
+    k_f4_groupsum(const LayerPlan* __restrict__ plans, int layer0, const F4Prep* __restrict__ prep, int64_t stride,
+                  const int64_t* __restrict__ src, const int4* __restrict__ groups,
+                  const int64_t* __restrict__ ngroups, ShrunkLine* __restrict__ out) {
+  __shared__ double sd[kGroupWarps][8][33];
+  __shared__ float sf[kGroupWarps][4][33];
   const int layer = blockIdx.y;
   const int64_t ng = ngroups[2 * (layer + layer0)];
+  if (ng <= 0) return;
   const int4* G = groups + (int64_t)layer * stride;
   const int64_t* S = src + (int64_t)layer * stride;
   const F4Prep* pr = prep + (int64_t)layer * stride;
   ShrunkLine* O = out + (int64_t)layer * stride;
   const bool mixed = plans[layer + layer0].mixed != 0;
-  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ng; g += (int64_t)gridDim.x * blockDim.x) {
+  if ((int64_t)G[ng - 1].y + 1 < kGroupWarpMin * ng) {  // (groups cover the stream from its start)
+    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ng; g += (int64_t)gridDim.x * blockDim.x)
+      group_sum_thread(pr, S, G[g], mixed, O);
+    return;
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double(*D)[33] = sd[warp];
+  float(*F)[33] = sf[warp];
+  for (int64_t g = (int64_t)blockIdx.x * kGroupWarps + warp; g < ng; g += (int64_t)gridDim.x * kGroupWarps) {
     const int4 gr = G[g];
     int slot = gr.z;
-    if (mixed) {
-      // the centre VNU = SUMV/SUMS sets the record's point range: binary64 in
-      // the reference's order; the widths and the FP32 strength set no index
-      double SUMS = 0., SUMV = 0., SUMS2 = 0., SUMV2 = 0.;
-      float SAL = 0.f, SAD = 0.f, SAL2 = 0.f, SAD2 = 0.f;
-      for (int u = gr.x; u <= gr.y; ++u) {
-        const F4Prep& r = pr[S[u]];
+    double sum = 0.;   // lanes 0..7: SUMV, SUMS, SUMAL, SUMAD of kind 0, then of kind 1
+    float sumf = 0.f;  // lanes 0..3 (mixed): SUMAL, SUMAD of kind 0, then of kind 1
+    for (int u0 = gr.x; u0 <= gr.y; u0 += 32) {
+      const int cnt = min(32, gr.y - u0 + 1);
+      bool coupled = false;
+      F4Prep r;
+      if (lane < cnt) {
+        r = pr[S[u0 + lane]];
         const bool weak = r.sp < 1.0e-35;
-        if (!weak && r.spp != 0.) {  // a coupled line is not shrunk (SHRINQ :1566-1578)
-          ShrunkLine L;
-          L.vnu = r.vnu;
-          L.sp = r.sp;
-          L.w.f[0] = r.w.f[0];
-          L.w.f[1] = r.w.f[1];
-          L.w.f[2] = r.w.f[2];
-          L.w.f[3] = (float)r.spp;
-          L.w.f[4] = L.w.f[5] = 0.f;
-          L.mol = r.mol == 2 ? 2 : 0;
-          L.pad = 0;
-          O[slot++] = L;
-          continue;
-        }
-        const double sp = weak ? 0.0 : r.sp;
-        const float spf = weak ? 0.f : r.w.f[2];
-        if (r.mol != 2) {
-          SUMV = SUMV + r.vnu * sp;
-          SUMS = SUMS + sp;
-          SAL = SAL + spf * r.w.f[0];
-          SAD = SAD + spf * r.w.f[1];
+        coupled = !weak && r.spp != 0.;  // a coupled line is not shrunk (SHRINQ :1566-1578)
+        const double sp = weak || coupled ? 0.0 : r.sp;
+        const int k = r.mol != 2 ? 0 : 1;
+        D[4 * k][lane] = coupled ? 0. : r.vnu * sp;
+        D[4 * k + 1][lane] = sp;
+        D[4 * (1 - k)][lane] = D[4 * (1 - k) + 1][lane] = 0.;
+        if (mixed) {
+          const float spf = weak || coupled ? 0.f : r.w.f[2];
+          F[2 * k][lane] = spf * r.w.f[0];
+          F[2 * k + 1][lane] = spf * r.w.f[1];
+          F[2 * (1 - k)][lane] = F[2 * (1 - k) + 1][lane] = 0.f;
         } else {
-          SUMV2 = SUMV2 + r.vnu * sp;
-          SUMS2 = SUMS2 + sp;
-          SAL2 = SAL2 + spf * r.w.f[0];
-          SAD2 = SAD2 + spf * r.w.f[1];
+          D[4 * k + 2][lane] = sp * r.w.d[0];
+          D[4 * k + 3][lane] = sp * r.w.d[1];
+          D[4 * (1 - k) + 2][lane] = D[4 * (1 - k) + 3][lane] = 0.;
         }
       }
-      for (int k = 0; k < 2; ++k) {
-        const double ss = k ? SUMS2 : SUMS;
-        if (!(ss > 0.)) continue;
-        ShrunkLine L;
-        L.vnu = (k ? SUMV2 : SUMV) / ss;
-        L.sp = ss;
-        const float sf = (float)ss;
-        L.w.f[0] = (k ? SAL2 : SAL) / sf;
-        L.w.f[1] = (k ? SAD2 : SAD) / sf;
-        L.w.f[2] = sf;
-        L.w.f[3] = 0.f;  // SUMC: zero
-        L.w.f[4] = L.w.f[5] = 0.f;
-        L.mol = k ? 2 : 0;
-        L.pad = 0;
-        O[slot++] = L;
+      const unsigned cb = __ballot_sync(0xffffffffu, coupled);
+      if (coupled) O[slot + __popc(cb & ((1u << lane) - 1u))] = shrunk_coupled(r, mixed);
+      slot += __popc(cb);
+      __syncwarp();
+      const int row = lane & 7, rowf = lane & 3;
+      if (mixed) {
+        if (lane < 8 && (lane & 3) < 2) {  // SUMV, SUMS of both kinds
+          for (int i = 0; i < cnt; ++i) sum = sum + D[row][i];
+        } else if (lane >= 8 && lane < 12) {
+          for (int i = 0; i < cnt; ++i) sumf = sumf + F[rowf][i];
+        }
+      } else if (lane < 8) {
+        for (int i = 0; i < cnt; ++i) sum = sum + D[row][i];
       }
-      continue;
+      __syncwarp();  // the rows are written again
     }
-    double SUMAL = 0., SUMAD = 0., SUMS = 0., SUMV = 0., SUMC = 0.;
-    double SUMAL2 = 0., SUMAD2 = 0., SUMS2 = 0., SUMV2 = 0., SUMC2 = 0.;
-    for (int u = gr.x; u <= gr.y; ++u) {
-      const F4Prep& r = pr[S[u]];
-      if (!(r.sp < 1.0e-35) && r.spp != 0.) {  // a coupled line is not shrunk (SHRINQ :1566-1578)
-        ShrunkLine L;
-        L.vnu = r.vnu;
-        L.sp = r.sp;
-        L.w.d[0] = r.w.d[0];
-        L.w.d[1] = r.w.d[1];
-        L.w.d[2] = r.spp;
-        L.mol = r.mol == 2 ? 2 : 0;
-        L.pad = 0;
-        O[slot++] = L;
-        continue;
-      }
-      double sp = r.sp < 1.0e-35 ? 0.0 : r.sp;
-      if (r.mol != 2) {
-        SUMV = SUMV + r.vnu * sp;
-        SUMS = SUMS + sp;
-        SUMAL = SUMAL + sp * r.w.d[0];
-        SUMAD = SUMAD + sp * r.w.d[1];
-        SUMC = SUMC + 0.;
-      } else {
-        SUMV2 = SUMV2 + r.vnu * sp;
-        SUMS2 = SUMS2 + sp;
-        SUMAL2 = SUMAL2 + sp * r.w.d[0];
-        SUMAD2 = SUMAD2 + sp * r.w.d[1];
-        SUMC2 = SUMC2 + 0.;
-      }
-    }
-    if (SUMS > 0.) {
-      ShrunkLine L;
-      L.sp = SUMS;
-      L.w.d[0] = SUMAL / SUMS;
-      L.w.d[1] = SUMAD / SUMS;
-      L.vnu = SUMV / SUMS;
-      L.w.d[2] = SUMC;
-      L.mol = 0;
-      L.pad = 0;
-      O[slot++] = L;
-    }
-    if (SUMS2 > 0.) {
-      ShrunkLine L;
-      L.sp = SUMS2;
-      L.w.d[0] = SUMAL2 / SUMS2;
-      L.w.d[1] = SUMAD2 / SUMS2;
-      L.vnu = SUMV2 / SUMS2;
-      L.w.d[2] = SUMC2;
-      L.mol = 2;
-      L.pad = 0;
-      O[slot++] = L;
-    }
+    double q[4];
+    float qf[2];
+    const int k = lane & 1;  // lane 0 writes kind 0, lane 1 kind 1
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[i] = __shfl_sync(0xffffffffu, sum, 4 * k + i);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) qf[i] = __shfl_sync(0xffffffffu, sumf, 8 + 2 * k + i);
+    const bool emit = lane < 2 && q[1] > 0.;
+    const unsigned eb = __ballot_sync(0xffffffffu, emit);
+    if (emit)
+      O[slot + __popc(eb & ((1u << lane) - 1u))] = shrunk_line(k, mixed, q[0], q[1], q[2], q[3], qf[0], qf[1]);
   }
 }
 

@@ -1015,7 +1015,7 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
                                          h->f4flag.as<unsigned char>(), h->f4ntot.as<int64_t>(),
                                          h->f4cut.as<int64_t>(), h->f4grp.as<int4>(), h->f4nout.as<int64_t>());
     h->launches++;
-    k_f4_groupsum<<<dim3((unsigned)std::min<int64_t>((f4stride + 255) / 256, 4096), count), 256, 0, st>>>(
+    k_f4_groupsum<<<dim3((unsigned)std::min<int64_t>((f4stride + 255) / 256, 4096), count), kGroupSumThreads, 0, st>>>(
         dplans, first, h->f4prep.as<F4Prep>(), f4stride, h->f4src.as<int64_t>(), h->f4grp.as<int4>(),
         h->f4nout.as<int64_t>(), h->f4sh.as<ShrunkLine>());
   }
