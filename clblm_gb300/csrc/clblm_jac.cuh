@@ -4,6 +4,7 @@
 
 #include <cstdint>
 
+#include "clblm_interpmap.cuh"
 #include "clblm_rt.cuh"
 
 namespace clblm {
@@ -50,7 +51,7 @@ constexpr int kJacMaxWarps = 4;  // warps of the largest k_jac block (128 thread
 // derivatives [nlay + 1, 2 nlay + 1], then dR/dTskin and dR/demis
 __host__ __device__ constexpr int jac_vjp_slots(int nlay) { return 2 * (nlay + 1) + 2; }
 
-__global__ void k_interp_map_jobs(const JacJob* jobs, int njob);
+__global__ void __launch_bounds__(kMapThreads) k_interp_map_jobs(const JacJob* jobs, int njob);
 // k_od_jobs: threads per CTA and output points per CTA
 constexpr int kOdJobThreads = 256;
 constexpr int kOdJobPoints = 2048;

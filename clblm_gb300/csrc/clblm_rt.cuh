@@ -4,6 +4,8 @@
 
 #include <cstdint>
 
+#include "clblm_interpmap.cuh"
+
 namespace clblm {
 
 // How one spectrum grid maps onto another under interpSpectrum
@@ -144,8 +146,8 @@ __device__ __forceinline__ Stencil<W> interp_stencil(const InterpSpec& s, int64_
 }
 
 cudaError_t rt_upload_interp_coef(cudaStream_t st);
-__global__ void k_interp_map(InterpSpec s, const int64_t* blk_j1, const double* blk_vo, int nblk, int64_t nout,
-                             int2* map);
+__global__ void __launch_bounds__(kMapThreads)
+    k_interp_map(InterpSpec s, const int64_t* blk_j1, const double* blk_vo, int nblk, int64_t nout, int2* map);
 constexpr int kRtMaxThreads = 512;  // largest k_rt_segment block the autotuner times
 template <bool Plain>
 __global__ void __launch_bounds__(kRtMaxThreads) k_rt_segment(const __grid_constant__ RtSegArgs a);

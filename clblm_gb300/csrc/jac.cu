@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include "clblm_common.cuh"
+#include "clblm_interpmap.cuh"
 #include "clblm_jac.cuh"
 #include "clblm_kernels.cuh"
 #include "clblm_panel.cuh"
@@ -24,47 +25,14 @@
 
 namespace clblm {
 
-// grid (blocks of 64 interpolation blocks, jobs); each job its own block list
-__global__ void k_interp_map_jobs(const JacJob* __restrict__ jobs, int njob) {
-  const int j = blockIdx.y;
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= njob || b >= jobs[j].nblk) return;
-  const InterpSpec& s = jobs[j].spec;
-  if (!jobs[j].build_map) return;
-  int2* map = jobs[j].map;
-  const int64_t* blk_j1 = jobs[j].blk_j1;
-  const int64_t nout = jobs[j].nout;
-  const double Vo = jobs[j].blk_vo[b];
-  int64_t iIn = (int64_t)__dadd_rn(__ddiv_rn(__dadd_rn(Vo, -s.v1), s.dvin), 1.00001);
-  double Vi = __dadd_rn(s.v1, __dmul_rn((double)(iIn - 1), s.dvin));
-  double P = __ddiv_rn(__dadd_rn(Vo, -Vi), s.dvin);
-  const int64_t J1 = blk_j1[b];
-  if (J1 < 1 || J1 > nout) return;  // a block start off the output grid writes nothing
-  const int64_t J2 = min(nout, J1 + 2400 - 1);
-  if (s.ratio < 0.999) {
-    // P < 1 on entry to every step, so P + RATIO < 1.999: a carry is INT(P)
-    // = 1 and INT(iIn + P) = iIn + 1, and P - 1 is exact (the same values,
-    // with a shorter chain of dependent binary64 operations per step)
-    for (int64_t J = J1; J <= J2; ++J) {
-      int IP = (int)__dadd_rn(__dmul_rn(P, 201.), 1.00001);
-      map[J - 1] = make_int2((int)iIn, IP < 0 ? 0 : (IP > 202 ? 202 : IP));
-      P = __dadd_rn(P, s.ratio);
-      if (P >= 1.0) {
-        iIn += 1;
-        P = __dadd_rn(P, -1.0);
-      }
-    }
-    return;
-  }
-  for (int64_t J = J1; J <= J2; ++J) {
-    int IP = (int)__dadd_rn(__dmul_rn(P, 201.), 1.00001);
-    map[J - 1] = make_int2((int)iIn, IP < 0 ? 0 : (IP > 202 ? 202 : IP));
-    P = __dadd_rn(P, s.ratio);
-    if (P >= 1.0) {
-      iIn = (int64_t)__dadd_rn((double)iIn, P);
-      P = __dadd_rn(P, -(double)((int64_t)P));
-    }
-  }
+// grid (interpolation blocks, jobs); each job its own block list
+__global__ void __launch_bounds__(kMapThreads) k_interp_map_jobs(const JacJob* __restrict__ jobs, int njob) {
+  const int j = blockIdx.y, b = blockIdx.x;
+  if (j >= njob || b >= jobs[j].nblk || !jobs[j].build_map) return;
+  const JacJob& jb = jobs[j];
+  const int64_t J1 = jb.blk_j1[b];
+  if (J1 < 1 || J1 > jb.nout) return;  // a block start off the output grid writes nothing
+  interp_map_block(jb.spec.v1, jb.spec.dvin, jb.spec.ratio, J1, jb.blk_vo[b], jb.nout, jb.map);
 }
 
 // interpSpectrum's linear extension by two points past either end

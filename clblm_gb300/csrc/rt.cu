@@ -17,6 +17,7 @@
 #include <climits>
 
 #include "clblm_common.cuh"
+#include "clblm_interpmap.cuh"
 #include "clblm_kernels.cuh"
 #include "clblm_panel.cuh"
 #include "clblm_rt.cuh"
@@ -30,46 +31,20 @@ __constant__ float c_IAf[4][203];
 
 // The general-ratio branch of interpSpectrum (clblm_Spectrum.f90:528-565)
 // steps the phase P by DVout/DVin with a carry into iIn and restarts it from
-// the exact wavenumber every 2400 output points.  One thread per such block
-// replays the steps, so that the table index IP at grid coincidences (P just
-// below 1 or just past the carry) is the reference's.
-__global__ void k_interp_map(InterpSpec s, const int64_t* __restrict__ blk_j1, const double* __restrict__ blk_vo,
-                             int nblk, int64_t nout, int2* __restrict__ map) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
+// the exact wavenumber every 2400 output points: one CTA per such block forms
+// its points' (iIn, IP), the reference's also at grid coincidences (P just
+// below 1 or just past the carry).  Without block tables (blk_j1 null) block b
+// starts at point 2400 b + 1, as the reference's restarts do while DVout is
+// well above the rounding of the wavenumbers.
+__global__ void __launch_bounds__(kMapThreads)
+    k_interp_map(InterpSpec s, const int64_t* __restrict__ blk_j1, const double* __restrict__ blk_vo, int nblk,
+                 int64_t nout, int2* __restrict__ map) {
+  const int b = blockIdx.x;
   if (b >= nblk) return;
-  // every product and sum rounded on its own (no FMA contraction): a fused
-  // v1 + (iIn-1)*dvin moves P by ~1e-10 and flips the carry at coincidences
-  const double Vo = blk_vo[b];
-  int64_t iIn = (int64_t)__dadd_rn(__ddiv_rn(__dadd_rn(Vo, -s.v1), s.dvin), 1.00001);
-  double Vi = __dadd_rn(s.v1, __dmul_rn((double)(iIn - 1), s.dvin));
-  double P = __ddiv_rn(__dadd_rn(Vo, -Vi), s.dvin);
-  const int64_t J1 = blk_j1[b];
+  const int64_t J1 = blk_j1 ? blk_j1[b] : (int64_t)b * kMapBlock + 1;
+  const double Vo = blk_j1 ? blk_vo[b] : (b == 0 ? s.v1 : __dadd_rn(s.v1, __dmul_rn((double)(J1 - 1), s.dvout)));
   if (J1 < 1 || J1 > nout) return;  // a block start off the output grid writes nothing
-  const int64_t J2 = min(nout, J1 + 2400 - 1);
-  if (s.ratio < 0.999) {
-    // P < 1 on entry to every step, so P + RATIO < 1.999: a carry is INT(P)
-    // = 1 and INT(iIn + P) = iIn + 1, and P - 1 is exact (the same values,
-    // with a shorter chain of dependent binary64 operations per step)
-    for (int64_t J = J1; J <= J2; ++J) {
-      int IP = (int)__dadd_rn(__dmul_rn(P, 201.), 1.00001);
-      map[J - 1] = make_int2((int)iIn, IP < 0 ? 0 : (IP > 202 ? 202 : IP));
-      P = __dadd_rn(P, s.ratio);
-      if (P >= 1.0) {
-        iIn += 1;
-        P = __dadd_rn(P, -1.0);
-      }
-    }
-    return;
-  }
-  for (int64_t J = J1; J <= J2; ++J) {
-    int IP = (int)__dadd_rn(__dmul_rn(P, 201.), 1.00001);
-    map[J - 1] = make_int2((int)iIn, IP < 0 ? 0 : (IP > 202 ? 202 : IP));
-    P = __dadd_rn(P, s.ratio);
-    if (P >= 1.0) {
-      iIn = (int64_t)__dadd_rn((double)iIn, P);
-      P = __dadd_rn(P, -(double)((int64_t)P));
-    }
-  }
+  interp_map_block(s.v1, s.dvin, s.ratio, J1, Vo, nout, map);
 }
 
 // value of spInExt(i) (1-based, extended by two points each side)

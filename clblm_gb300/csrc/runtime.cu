@@ -834,15 +834,28 @@ InterpSpec interp_spec(double v1in, double dvin, int64_t nin, double v1out, doub
   return s;
 }
 
-// For a general-ratio spec: the block starts of interpSpectrum's outer loop
-// (exact FP64 replay on the host, a few thousand blocks at most) and the
-// per-point (iIn, IP) map built on the device into `buf`.
+// For a general-ratio spec: the per-point (iIn, IP) map, built on the device
+// into `buf`.  interpSpectrum's outer loop restarts at J1 = INT((Vo - V1)/DVout
+// + 1.001), Vo = V1 + J2*DVout: every 2400 points while the rounding of Vo
+// stays below a thousandth of DVout, and then no table goes to the device (a
+// host wait in the middle of the call's launches); for finer grids the host
+// replays the loop.
 int build_interp_map(clblm_handle* h, InterpSpec* s, int64_t nout, DevBuf* buf) {
   if (s->kind == 0 || s->itype >= 0) return CLBLM_OK;
+  const double V2out = s->v1 + (double)(nout - 1) * s->dvout;
+  if (std::max(std::fabs(s->v1), std::fabs(V2out)) * 1.e-12 < s->dvout && s->dvout > 1.e-7) {
+    const size_t nb = (size_t)((nout + kMapBlock - 1) / kMapBlock);
+    CUDA_TRY(h, buf->ensure(sizeof(int2) * nout + 16 * (nb + 1) + 512));
+    int2* map = buf->as<int2>();
+    h->launches++;
+    k_interp_map<<<(unsigned)nb, kMapThreads, 0, h->stream>>>(*s, nullptr, nullptr, (int)nb, nout, map);
+    CUDA_TRY(h, cudaGetLastError());
+    s->map = map;
+    return CLBLM_OK;
+  }
   std::vector<int64_t> j1;
   std::vector<double> vo;
   const double TOL = 1.e-8;
-  double V2out = s->v1 + (double)(nout - 1) * s->dvout;
   double Vo = s->v1;
   while (Vo < V2out + TOL) {
     int64_t J1 = (int64_t)((Vo - s->v1) / s->dvout + 1.001);
@@ -863,7 +876,7 @@ int build_interp_map(clblm_handle* h, InterpSpec* s, int64_t nout, DevBuf* buf) 
   CUDA_TRY(h, cudaMemcpyAsync(dj1, j1.data(), 8 * nb, cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(h, cudaMemcpyAsync(dvo, vo.data(), 8 * nb, cudaMemcpyHostToDevice, h->stream));
   h->launches++;
-  k_interp_map<<<(unsigned)((nb + 63) / 64), 64, 0, h->stream>>>(*s, dj1, dvo, (int)nb, nout, map);
+  k_interp_map<<<(unsigned)nb, kMapThreads, 0, h->stream>>>(*s, dj1, dvo, (int)nb, nout, map);
   CUDA_TRY(h, cudaGetLastError());
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));  // host block tables go out of scope
   s->map = map;
@@ -2325,7 +2338,7 @@ extern "C" int clblm_gpu_interp_spectrum_noalloc(const double* d_in, int64_t nin
     double* dvo = reinterpret_cast<double*>(base + kNoAllocMapBytes + 8 * (size_t)kNoAllocBlocks);
     k_noalloc_blocks<<<1, 32, 0, st>>>(v1, dvout, nout, nb, dj1, dvo);
     if (cudaGetLastError() != cudaSuccess) return CLBLM_ERR_CUDA;
-    k_interp_map<<<(unsigned)((nb + 63) / 64), 64, 0, st>>>(s, dj1, dvo, nb, nout, map);
+    k_interp_map<<<(unsigned)nb, kMapThreads, 0, st>>>(s, dj1, dvo, nb, nout, map);
     if (cudaGetLastError() != cudaSuccess) return CLBLM_ERR_CUDA;
     s.map = map;
   }
@@ -2801,7 +2814,7 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
       CUDA_TRY(h, cudaMemcpyAsync(h->jjobs.p, jobs.data(), sizeof(JacJob) * count, cudaMemcpyHostToDevice,
                                   h->stream));
       h->launches += 2;
-      k_interp_map_jobs<<<dim3((unsigned)((nbt + 63) / 64), count), 64, 0, h->stream>>>(h->jjobs.as<JacJob>(), count);
+      k_interp_map_jobs<<<dim3((unsigned)nbt, count), kMapThreads, 0, h->stream>>>(h->jjobs.as<JacJob>(), count);
       {
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return set_err(h, CLBLM_ERR_CUDA, "k_interp_map_jobs: %s", cudaGetErrorString(e));
@@ -3229,7 +3242,7 @@ int batch_enqueue(clblm_handle* h, BatchPlan& bp, const clblm_profile_t* prof, c
     const int64_t nmax = c.nmax;
     const int bmax = c.bmax;
     h->launches += 2;
-    k_interp_map_jobs<<<dim3((unsigned)((bmax + 63) / 64), c.count), 64, 0, h->stream>>>(jobs, c.count);
+    k_interp_map_jobs<<<dim3((unsigned)bmax, c.count), kMapThreads, 0, h->stream>>>(jobs, c.count);
     if (plain)
       k_od_jobs<true><<<dim3((unsigned)((nmax + kOdJobPoints - 1) / kOdJobPoints), c.count), kOdJobThreads, 0,
                         h->stream>>>(jobs, c.count, h->od.p, h->jod.p);
