@@ -44,6 +44,8 @@ struct IsoRow {
   float scor_f, alfd1_f, rhoslf_f, pad;
 };
 
+constexpr int kMaxSlices = 32;
+
 // Per-layer plan, filled on the host (exact FP64 restatement of the scalar
 // set-up of ODLAY_nonStruct, OPDPTH and HIRACQ) and read by the kernels.
 struct LayerPlan {
@@ -70,6 +72,7 @@ struct LayerPlan {
   double lc_rectlc, lc_tmpdif, lc4_rectlc, lc4_tmpdif;
   int jrad, ilnflg, max1, max2, max3, nalfmax, nbound;
   int npanels, nhi_last;          // panels and NHI of the last panel
+  int nslice;                     // CTAs of the line pass per panel (panel_slices)
   int64_t nsamp;                  // R1 points output
   // processed line range [line_lo, line_hi] (global indices, inclusive)
   int64_t line_lo, line_hi;
@@ -101,7 +104,9 @@ struct LayerPlan {
   int64_t iso_off;
   // offsets of this layer's slices inside the shared per-call buffers
   int64_t vft_off;     // VFT of panel p at vft_off + p
-  int64_t od_off;      // OD output
+  int64_t od_off;      // OD output; the line pass writes slice z of a panel's records at
+  int64_t od_pts;      // od_off + z od_pts, the far-wing pass the OD at od_off
+  int64_t cta0;        // first entry of this layer in the line pass's list of CTAs
   int64_t r4_off;      // R4 grid
   int64_t abs_off;     // ABSRB (N_ABSRB + 8 per layer)
 };

@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
                                GridRecLo* reclo, double* cpl, unsigned long long* stats,
                                double* alfvmax, int* aggmax, int* aggmin, int nagg);
 __global__ void k_panel_ranges(const LayerPlan* plans, int layer0, const double* vnu_raw, const double* alfvmax,
-                               double shiftmax, int64_t* ranges, int64_t panel_stride);
+                               double shiftmax, int64_t* ranges, int64_t panel_stride, int2* work);
 __global__ void k_continuum(const LayerPlan* plans, int layer0, ContIn cont, double* absrb_all);
 template <bool Cpl>
 __global__ void __launch_bounds__(kSetupThreads, 4)

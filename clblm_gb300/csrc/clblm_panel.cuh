@@ -25,6 +25,7 @@ struct PanelArgs {
   int64_t stride;
   const int64_t* ranges;     // per panel: candidate record windows of R1, R2, R3
   int64_t panel_stride;
+  const int2* work;          // line pass: (layer * kMaxSlices + slice, panel) of each CTA
   const void* r4_all;
   const double* absrb_all;
   void* od_all;
@@ -100,9 +101,9 @@ size_t panel_smem_bytes(bool plain, bool wings = false);  // wings: the mixed fa
 __global__ void k_r4_radfac(const LayerPlan* plans, int layer0, const double* blk_v1, const int* blk_n,
                             double* blk_fac);
 
-// k_panel in one pass (kPanelAll), or the line sums (kPanelLines) and the far
-// wings, continuum, combine and radiation term (kPanelWings) in two
-constexpr int kPanelAll = 0, kPanelLines = 1, kPanelWings = 2;
+// the passes of k_panel: the line sums (kPanelLines), then the far wings, the
+// continuum and the radiation term (kPanelWings)
+constexpr int kPanelLines = 1, kPanelWings = 2;
 // Cpl: the line list holds coupled lines, whose grid records carry kCplBit
 // (the branch-free sums of the mixed path skip them; they are added with
 // their dispersion term); without it the line sums stay as lean as before

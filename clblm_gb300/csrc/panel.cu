@@ -6,10 +6,10 @@
 //                    clblm_ODLAY.f90:2067-2258), far-wing and continuum
 //                    interpolation into R3 (XINT, clblm_Spectrum.f90:874-915),
 //                    the R3->R2->R1 4-point interpolation and the radiation
-//                    term (panelOut, clblm_ODLAY.f90:2289-2493).  The FP64
-//                    path runs it in one launch (kPanelAll); the mixed path
-//                    in two: the line sums (kPanelLines) beside the far-wing
-//                    chain, then R4 and the continuum (kPanelWings).
+//                    term (panelOut, clblm_ODLAY.f90:2289-2493).  Two
+//                    launches: the line sums (kPanelLines) beside the far-wing
+//                    chain, a CTA per slice of a panel's records, then R4,
+//                    the continuum and the radiation term (kPanelWings).
 //   k_f4_conv<Plain> far-wing function 4 on the DVR4 grid (CNVF4Q,
 //                    clblm_ODLAY_LineF4.f90:187-494): two points per thread
 //                    (packed FP32x2 in the mixed path), records streamed
@@ -58,7 +58,7 @@ struct SumD {
 // that, in FP64 with ZFL and ZSLOPE formed again from the line record `rec`
 // of this CTA's layer, as CNVFNQ's set-up forms them.
 __device__ __noinline__ int table_index_near_boundary(int k, float zfl, float zs, GridRecLo lo, const PanelArgs* pa,
-                                                      int64_t rec, int q, int grid) {
+                                                      int64_t rec, int q, int grid, int layer) {
   const float kf = (float)k;
   const float p = kf * zs;
   const float pe = fmaf(kf, zs, -p);                // kf*zs = p + pe exactly
@@ -71,8 +71,8 @@ __device__ __noinline__ int table_index_near_boundary(int k, float zfl, float zs
   const float dd = (a - n) + al;                    // |ZF| - n
   if (fabsf(fabsf(dd) - 0.5f) < 1e-7f) {
     // ZFkL and ZSLOPE in FP64 from the line, as the record set-up forms them
-    const LayerPlan& P = pa->plans[blockIdx.y + pa->layer0];
-    const LinePrep L = pa->prep[(int64_t)blockIdx.y * pa->stride + rec];
+    const LayerPlan& P = pa->plans[layer + pa->layer0];
+    const LinePrep L = pa->prep[(int64_t)layer * pa->stride + rec];
     const CnvfnqSetup cs = cnvfnq_setup(P, pa->vft_all[P.vft_off + q], L.vnu, L.recalf, L.bhwdxf);
     const double zf64 = fma((double)k, cs.zslope, cs.zf[grid - 1]);
     return (int)(fabs(zf64) + 1.5);
@@ -110,6 +110,7 @@ struct PanelTiles {
   int lo1[2 * kTiles1], hi1[2 * kTiles1], lo2[2 * kTiles2], hi2[2 * kTiles2], lo3[2 * kTiles3], hi3[2 * kTiles3];
   GridRec wrec[kPanelWarps][kBatch];
   XintPanel X;
+  int layer;
 };
 
 // mixed path: under 74 KB, so that three CTAs of the line pass share an SM.
@@ -133,23 +134,25 @@ constexpr size_t kWingsSmem = sizeof(PanelSmem<false>) - sizeof(MixedTables);
 static_assert(kWingsSmem % 16 == 0, "the tables start on a 16-byte boundary");
 template <>
 struct PanelSmem<true> : PanelTiles {
-  GridRecD wrecd[kPanelWarps][kBatch];
-  double t1[3 * kNFMX];
-  double t2[kNFMX];
-  double t3[kNFMX];
   double r3n[kR3Pts];
   double r3o[8];
   double r2[kR2Pts];
   int seg_start[kMaxSeg + 1];
   double seg_v[kMaxSeg], seg_d[kMaxSeg];
   int nseg, seg_slot;
+  GridRecD wrecd[kPanelWarps][kBatch];  // the line pass alone, from here on
+  double t1[3 * kNFMX];
+  double t2[kNFMX];
+  double t3[kNFMX];
 };
+constexpr size_t kWingsSmemD =
+    sizeof(PanelSmem<true>) - sizeof(double) * 5 * kNFMX - sizeof(GridRecD) * kPanelWarps * kBatch;
 
 // three CTAs of the mixed path per SM (228 KB, 1 KB reserved per CTA)
 static_assert(3 * (sizeof(PanelSmem<false>) + 1024) <= 228 * 1024, "mixed k_panel: three CTAs per SM");
 
 size_t panel_smem_bytes(bool plain, bool wings) {
-  return plain ? sizeof(PanelSmem<true>) : (wings ? kWingsSmem : sizeof(PanelSmem<false>));
+  return plain ? (wings ? kWingsSmemD : sizeof(PanelSmem<true>)) : (wings ? kWingsSmem : sizeof(PanelSmem<false>));
 }
 
 // RADFNI, clblm_ODLAY_CommonSub.f90:379-508 (FP64).  *VINEW carries the end
@@ -287,6 +290,29 @@ __device__ __forceinline__ long long floordiv16(long long x) { return x >> 4; } 
 __device__ __forceinline__ void tile_ranges(const int* __restrict__ pm, const int* __restrict__ sm, int64_t w0,
                                             int64_t w1, int G0, int T, int* lo, int* hi) {
   const long long g0 = G0;
+  if (w1 - w0 > 2048) {
+    // a long window (wide lines): two searches per half tile instead of a pass
+    // over it, which every slice of the panel would repeat
+    for (int t = threadIdx.x; t < T; t += blockDim.x) {
+      const long long b = g0 + 16 * t;
+      int64_t l = w0, h = w1;
+      while (l < h) {
+        const int64_t m = (l + h) >> 1;
+        if (pm[m] < b) l = m + 1;
+        else h = m;
+      }
+      lo[t] = (int)l;
+      h = w1;
+      l = w0;
+      while (l < h) {
+        const int64_t m = (l + h) >> 1;
+        if (sm[m] <= b + 15) l = m + 1;
+        else h = m;
+      }
+      hi[t] = (int)l;
+    }
+    return;
+  }
   for (int64_t i = w0 + threadIdx.x; i < w1; i += blockDim.x) {
     // lo: tiles t with prev < G0 + 16 t <= cur
     const long long cur = pm[i];
@@ -359,7 +385,7 @@ __device__ __forceinline__ float fix_terms(const PanelSmem<false>& S, const Grid
     const int izf = fast_index(kk, r, &d);
     const float vf = table_term<GRID>(S, r, min(izf, kNFMX));
     const int iz = fabsf(d) > 0.499f
-                       ? table_index_near_boundary(kk, r.zfl, r.zs, reclo[base + k], &a, base + k, r.q, GRID)
+                       ? table_index_near_boundary(kk, r.zfl, r.zs, reclo[base + k], &a, base + k, r.q, GRID, S.layer)
                        : izf;
     if (iz > kNFMX) {
       atomicOr(a.err, 2);
@@ -389,14 +415,14 @@ __device__ __forceinline__ float cpl_terms(const PanelSmem<false>& S, const Grid
     if (kk < 1 || g > r.g_hi || q > qmax) continue;
     float d;
     int iz = fast_index(kk, r, &d);
-    if (fabsf(d) > 0.499f) iz = table_index_near_boundary(kk, r.zfl, r.zs, reclo[base + k], &a, base + k, q, GRID);
+    if (fabsf(d) > 0.499f) iz = table_index_near_boundary(kk, r.zfl, r.zs, reclo[base + k], &a, base + k, q, GRID, S.layer);
     if (iz > kNFMX) {
       atomicOr(a.err, 2);
       continue;
     }
     const float v = table_term<GRID>(S, r, iz);
     const float zf = fmaf((float)kk, r.zs, r.zfl);
-    const float dpt = (float)a.cpl[(int64_t)blockIdx.y * a.stride + base + k];
+    const float dpt = (float)a.cpl[(int64_t)S.layer * a.stride + base + k];
     c += v + (v * (clc * dpt)) * zf;
   }
   return c;
@@ -452,7 +478,7 @@ __device__ __forceinline__ void gather_grid(PanelSmem<Plain>& S, const PanelArgs
         }
         // a coupled line adds its dispersion term: the strengths times CLCk
         // times DPTRAT, the shape times ZF (clblm_ODLAY.f90:2195-2239)
-        const double dpt = (Cpl && (r.q & kCplBit)) ? a.cpl[(int64_t)blockIdx.y * a.stride + base + k] : 0.;
+        const double dpt = (Cpl && (r.q & kCplBit)) ? a.cpl[(int64_t)S.layer * a.stride + base + k] : 0.;
         if constexpr (GRID == 1) {
           const double* T = S.t1 + 3 * (iz - 1);
           acc.add(d.a0 * T[0] + d.a1 * T[1] + d.a2 * T[2]);
@@ -519,25 +545,40 @@ __device__ __forceinline__ void gather_grid(PanelSmem<Plain>& S, const PanelArgs
 }
 
 template <bool Plain, int Part, bool Cpl>
-__global__ void __launch_bounds__(kPanelThreads, Plain ? 1 : (Part == kPanelWings ? 6 : 3))
+__global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 2 : 1) : (Part == kPanelWings ? 6 : 3))
     k_panel(const __grid_constant__ PanelArgs a) {
-  // Part: kPanelAll, or the line sums alone (kPanelLines: the far wings and
-  // the continuum are not yet known), or the rest alone (kPanelWings: R4 and
-  // ABSRB through XINT, the R3->R2->R1 combine and the radiation term, added
-  // to the OD the line pass wrote).  Every step is linear in R3, R2 and R1,
-  // so the two passes give the one-pass OD up to FP32 rounding.
+  // Part: the line sums alone (kPanelLines: the far wings and the continuum
+  // are not yet known), or the rest (kPanelWings: R4 and ABSRB through XINT
+  // and the R3->R2->R1 combine, added to what the line pass wrote, and the
+  // radiation term).  Every step is linear in R3, R2 and R1, so the passes,
+  // and the slices of the line pass, give the one-pass OD up to rounding.
+  //
+  // Slices: the line pass of a panel is a chain of record batches per warp,
+  // and a surface panel has thousands of records on every R3 tile (wide lines:
+  // 768 DV of them, 2400 at 200 lines per cm-1): one CTA took 700 us for it
+  // whatever else the GPU had to do.  A layer's panels are cut into nslice
+  // CTAs (panel_slices), each adding its share of every tile's records, in
+  // record order, and carrying it through the combine into its own row of the
+  // OD buffer; the far-wing pass adds the rows, compensated.
   constexpr bool kLines = Part != kPanelWings, kWings = Part != kPanelLines;
   using Real = typename std::conditional<Plain, double, float>::type;
   using Acc = typename std::conditional<Plain, SumD, KahanF>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PanelSmem<Plain>& S = *reinterpret_cast<PanelSmem<Plain>*>(smem_raw);
 
-  const int layer = blockIdx.y;
+  int layer = blockIdx.y, p = blockIdx.x, slice = 0;
+  if constexpr (kLines) {  // (k_panel_ranges lists the CTAs of every layer)
+    const int2 w = a.work[blockIdx.x];
+    layer = w.x / kMaxSlices;
+    slice = w.x % kMaxSlices;
+    p = w.y;
+  }
   const LayerPlan& P = a.plans[layer + a.layer0];
-  const int p = blockIdx.x;
   if (p >= P.npanels) return;
+  const int nslice = P.nslice;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) S.layer = layer;
   const double dv = P.dv;
   const double* vft = a.vft_all + P.vft_off;
   const double VFT = vft[p];
@@ -546,12 +587,13 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? 1 : (Part == kPanelWing
 
   // ---- shape tables into shared memory ----
   if constexpr (Plain) {
-    for (int i = tid; i < 3 * kNFMX; i += blockDim.x) S.t1[i] = a.tabs.t1d[i];
-    for (int i = tid; i < kNFMX; i += blockDim.x) {
-      S.t2[i] = a.tabs.t2d[i];
-      S.t3[i] = a.tabs.t3d[i];
+    if constexpr (kLines) {
+      for (int i = tid; i < 3 * kNFMX; i += blockDim.x) S.t1[i] = a.tabs.t1d[i];
+      for (int i = tid; i < kNFMX; i += blockDim.x) {
+        S.t2[i] = a.tabs.t2d[i];
+        S.t3[i] = a.tabs.t3d[i];
+      }
     }
-    __syncthreads();
   } else {
     // one bulk copy of the table image; the CTA waits for it just before its
     // first gather
@@ -589,20 +631,30 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? 1 : (Part == kPanelWing
   // the far-wing pass adds to the OD the line pass wrote: its loads are
   // issued here, ahead of the R3 and R2 phases
   constexpr int kT1PerWarp = (kTiles1 + kPanelWarps - 1) / kPanelWarps;
-  float od_pre[Part == kPanelWings ? kT1PerWarp : 1];
+  Real od_pre[Part == kPanelWings ? kT1PerWarp : 1];
   if constexpr (Part == kPanelWings) {
-    const float* od = reinterpret_cast<const float*>(a.od_all) + P.od_off + (int64_t)kPanelPts * p;
+    const Real* od = reinterpret_cast<const Real*>(a.od_all) + P.od_off + (int64_t)kPanelPts * p;
 #pragma unroll
     for (int i = 0; i < kT1PerWarp; ++i) {
       const int J = kNSHIFT + 1 + (warp + i * kPanelWarps) * 32 + lane;
-      od_pre[i] = (warp + i * kPanelWarps < nT1 && J <= NHI) ? od[J - kNSHIFT - 1] : 0.f;
+      od_pre[i] = (warp + i * kPanelWarps < nT1 && J <= NHI) ? od[J - kNSHIFT - 1] : (Real)0;
     }
   }
+  // a slice's share of the records [lo, hi) of a tile
+  auto share = [&](int64_t* lo, int64_t* hi) {
+    if (nslice > 1) {
+      const int n = (int)(*hi - *lo), q = n / nslice, r = n - q * nslice;
+      *lo += q * slice + min(slice, r);
+      *hi = *lo + q + (slice < r ? 1 : 0);
+    }
+  };
   const int G01 = kPanelPts * p + kNSHIFT, G02 = kPanelR2 * p - 1, G03 = kPanelR3 * p - 1;
-  for (int t = tid; t < 2 * kTiles1; t += blockDim.x) S.lo1[t] = S.hi1[t] = (int)rg[1];
-  for (int t = tid; t < 2 * kTiles2; t += blockDim.x) S.lo2[t] = S.hi2[t] = (int)rg[3];
-  for (int t = tid; t < 2 * kTiles3; t += blockDim.x) S.lo3[t] = S.hi3[t] = (int)rg[5];
-  if (tid == 0) {  // XINT set-up of the panel (once, in FP64)
+  if constexpr (kLines) {
+    for (int t = tid; t < 2 * kTiles1; t += blockDim.x) S.lo1[t] = S.hi1[t] = (int)rg[1];
+    for (int t = tid; t < 2 * kTiles2; t += blockDim.x) S.lo2[t] = S.hi2[t] = (int)rg[3];
+    for (int t = tid; t < 2 * kTiles3; t += blockDim.x) S.lo3[t] = S.hi3[t] = (int)rg[5];
+  }
+  if (kWings && tid == 0) {  // XINT set-up of the panel (once, in FP64)
     XintPanel& X = S.X;
     const double DVR3 = 16. * dv;
     if (P.nptr4 > 0) {
@@ -639,7 +691,7 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? 1 : (Part == kPanelWing
     }
   }
   __syncthreads();
-  if constexpr (!Plain) {  // ABSRB of the panel as FP32
+  if constexpr (!Plain && kWings) {  // ABSRB of the panel as FP32
     const double* AB = a.absrb_all + P.abs_off;  // 1-based
     for (int i = tid; i < S.X.nab; i += blockDim.x) S.absf[i] = (float)AB[S.X.ab0 + i];
   }
@@ -663,7 +715,7 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? 1 : (Part == kPanelWing
   // ---- R3: line sums on p-frame points 0..160 (new) and 0..7 (old) ----
   // units 0..kTiles3-1: 32 new points each; unit kTiles3: the 8 old points
   static_assert(kTiles3 + 1 < kPanelWarps, "the last warp has no R3 unit");
-  if (warp == kPanelWarps - 1 && lane == 0) {  // idle in the R3 phase: radiation-term segments (panelOut, JRAD = 0)
+  if (kWings && warp == kPanelWarps - 1 && lane == 0) {  // idle in the R3 phase: radiation-term segments (panelOut, JRAD = 0)
     int ns = 0, slot = -1;
     if (P.jrad == 0) {
       const int NLO = kNSHIFT + 1;
@@ -742,9 +794,12 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? 1 : (Part == kPanelWing
     const int t = old ? 0 : u;
     // the FP64 path: the 32-point tile's range; mixed: the lane's half tile's
     const int h0 = 2 * t + (Plain ? 0 : (lane >> 4)), h1 = Plain ? 2 * t + 1 : h0;
-    const int64_t lo = S.lo3[h0], hi = max(S.lo3[h0], S.hi3[h1]);
     Acc acc;
-    if (kLines) gather_grid<Plain, 3, Cpl>(S, a, rec3, rd3, rl3, lo, hi, g, active, qmax, acc);
+    if constexpr (kLines) {
+      int64_t lo = S.lo3[h0], hi = max(S.lo3[h0], S.hi3[h1]);
+      share(&lo, &hi);
+      gather_grid<Plain, 3, Cpl>(S, a, rec3, rd3, rl3, lo, hi, g, active, qmax, acc);
+    }
     if (active && kWings) {
       // far wings (R4) and continuum (ABSRB) interpolated into R3 (XINT).
       // The R4 block LBLF4Q held when XINT reached the point: this panel's
@@ -828,8 +883,11 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? 1 : (Part == kPanelWing
       int g = kPanelR2 * p + J - 1;
       Acc acc;
       const int h0 = 2 * tile + (Plain ? 0 : (lane >> 4)), h1 = Plain ? 2 * tile + 1 : h0;
-      if (kLines)
-        gather_grid<Plain, 2, Cpl>(S, a, rec2, rd2, rl2, S.lo2[h0], max(S.lo2[h0], S.hi2[h1]), g, active, p, acc);
+      if constexpr (kLines) {
+        int64_t lo = S.lo2[h0], hi = max(S.lo2[h0], S.hi2[h1]);
+        share(&lo, &hi);
+        gather_grid<Plain, 2, Cpl>(S, a, rec2, rd2, rl2, lo, hi, g, active, p, acc);
+      }
       if (active) {
         int off = (J - 1) & 3;
         int Jg = J - off;
@@ -861,16 +919,19 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? 1 : (Part == kPanelWing
   {
     const Real X00 = -7. / 128., X01 = 105. / 128., X02 = 35. / 128., X03 = -5. / 128.;
     const Real X10 = -1. / 16., X11 = 9. / 16.;
-    Real* od = reinterpret_cast<Real*>(a.od_all) + P.od_off;
-    // one 32-point tile; `prev`: the OD the line pass wrote (far-wing pass)
-    auto r1_tile = [&](int tile, float prev) {
+    Real* od = reinterpret_cast<Real*>(a.od_all) + P.od_off + (int64_t)slice * P.od_pts;
+    // one 32-point tile; `prev`: the line sums of the first slice (far-wing pass)
+    auto r1_tile = [&](int tile, Real prev) {
       int J = kNSHIFT + 1 + tile * 32 + lane;  // p-frame R1 index, 33..
       bool active = J <= NHI;
       int g = kPanelPts * p + J - 1;
       Acc acc;
       const int h0 = 2 * tile + (Plain ? 0 : (lane >> 4)), h1 = Plain ? 2 * tile + 1 : h0;
-      if (kLines)
-        gather_grid<Plain, 1, Cpl>(S, a, rec1, rd1, rl1, S.lo1[h0], max(S.lo1[h0], S.hi1[h1]), g, active, p, acc);
+      if constexpr (kLines) {
+        int64_t lo = S.lo1[h0], hi = max(S.lo1[h0], S.hi1[h1]);
+        share(&lo, &hi);
+        gather_grid<Plain, 1, Cpl>(S, a, rec1, rd1, rl1, lo, hi, g, active, p, acc);
+      }
       if (active) {
         int off = (J - 33) & 3;
         int Jg = J - off;
@@ -888,36 +949,44 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? 1 : (Part == kPanelWing
         }
         acc.add(v);
         Real val = acc.value();
-        if (P.jrad == 0 && S.nseg > 0) {
-          // segment of J: largest s with seg_start[s] <= J
-          const int slot = S.seg_slot;
-          const int* ss = slot < 0 ? S.seg_start : a.seg_pool_start + (int64_t)slot * (kSegSlot + 1);
-          int s0 = 0, s1 = S.nseg;
-          while (s1 - s0 > 1) {
-            int m = (s0 + s1) >> 1;
-            if (ss[m] <= J) s0 = m;
-            else s1 = m;
-          }
-          if (slot < 0) {
-            if constexpr (Plain) {
-              double f = S.seg_v[s0] + (double)(J - S.seg_start[s0]) * S.seg_d[s0];
-              val = val * f;
-            } else {
-              val *= fmaf((float)(J - S.seg_start[s0]), S.segf_d[s0], S.segf_v[s0]);
-            }
-          } else {
-            const double gv = a.seg_pool_v[(int64_t)slot * kSegSlot + s0];
-            const double gd = a.seg_pool_d[(int64_t)slot * kSegSlot + s0];
-            if constexpr (Plain) {
-              val = val * (gv + (double)(J - ss[s0]) * gd);
-            } else {
-              val *= fmaf((float)(J - ss[s0]), (float)gd, (float)gv);
-            }
-          }
-        }
         Real* o = od + (int64_t)kPanelPts * p + (J - kNSHIFT - 1);
-        if constexpr (Part == kPanelWings) *o = prev + val;
-        else *o = val;
+        if constexpr (kWings) {  // the slices' line sums and the wings, each times the radiation term
+          Acc lines;
+          lines.add(prev);
+          for (int z = 1; z < nslice; ++z) lines.add(o[(int64_t)z * P.od_pts]);
+          Real sum = lines.value();
+          if (P.jrad == 0 && S.nseg > 0) {
+            // segment of J: largest s with seg_start[s] <= J
+            const int slot = S.seg_slot;
+            const int* ss = slot < 0 ? S.seg_start : a.seg_pool_start + (int64_t)slot * (kSegSlot + 1);
+            int s0 = 0, s1 = S.nseg;
+            while (s1 - s0 > 1) {
+              int m = (s0 + s1) >> 1;
+              if (ss[m] <= J) s0 = m;
+              else s1 = m;
+            }
+            Real f;
+            if (slot < 0) {
+              if constexpr (Plain) f = S.seg_v[s0] + (double)(J - S.seg_start[s0]) * S.seg_d[s0];
+              else f = fmaf((float)(J - S.seg_start[s0]), S.segf_d[s0], S.segf_v[s0]);
+            } else {
+              const double gv = a.seg_pool_v[(int64_t)slot * kSegSlot + s0];
+              const double gd = a.seg_pool_d[(int64_t)slot * kSegSlot + s0];
+              if constexpr (Plain) f = gv + (double)(J - ss[s0]) * gd;
+              else f = fmaf((float)(J - ss[s0]), (float)gd, (float)gv);
+            }
+            if constexpr (Plain) {
+              sum = sum * f;
+              val = val * f;
+            } else {  // (rounded on their own)
+              sum = __fmul_rn(sum, f);
+              val = __fmul_rn(val, f);
+            }
+          }
+          if constexpr (Plain) val = sum + val;
+          else val = __fadd_rn(sum, val);
+        }
+        *o = val;
       }
     };
     if constexpr (Part == kPanelWings) {
@@ -925,7 +994,7 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? 1 : (Part == kPanelWing
       for (int i = 0; i < kT1PerWarp; ++i)
         if (warp + i * kPanelWarps < nT1) r1_tile(warp + i * kPanelWarps, od_pre[i]);
     } else {
-      for (int tile = warp; tile < nT1; tile += kPanelWarps) r1_tile(tile, 0.f);
+      for (int tile = warp; tile < nT1; tile += kPanelWarps) r1_tile(tile, (Real)0);
     }
   }
 }
@@ -933,8 +1002,9 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? 1 : (Part == kPanelWing
 template __global__ void k_panel<false, kPanelLines, false>(const __grid_constant__ PanelArgs);
 template __global__ void k_panel<false, kPanelLines, true>(const __grid_constant__ PanelArgs);
 template __global__ void k_panel<false, kPanelWings, false>(const __grid_constant__ PanelArgs);
-template __global__ void k_panel<true, kPanelAll, false>(const __grid_constant__ PanelArgs);
-template __global__ void k_panel<true, kPanelAll, true>(const __grid_constant__ PanelArgs);
+template __global__ void k_panel<true, kPanelLines, false>(const __grid_constant__ PanelArgs);
+template __global__ void k_panel<true, kPanelLines, true>(const __grid_constant__ PanelArgs);
+template __global__ void k_panel<true, kPanelWings, false>(const __grid_constant__ PanelArgs);
 
 // ---------------------------------------------------------------------------
 // RSYM (clblm_ODLAY.f90:3020-3085): when a layer's first panel starts at or

@@ -574,11 +574,14 @@ __device__ __forceinline__ int64_t lower_bound_d(const double* a, int64_t lo, in
 
 __global__ void k_panel_ranges(const LayerPlan* __restrict__ plans, int layer0, const double* __restrict__ vnu_raw,
                                const double* __restrict__ alfvmax, double shiftmax, int64_t* __restrict__ ranges,
-                               int64_t panel_stride) {
+                               int64_t panel_stride, int2* __restrict__ work) {
   int layer = blockIdx.y;
   const LayerPlan& P = plans[layer + layer0];
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= P.npanels) return;
+  // the line pass's CTAs of this panel
+  for (int z = 0; z < P.nslice; ++z)
+    work[P.cta0 + (int64_t)p * P.nslice + z] = make_int2(layer * kMaxSlices + z, p);
   double a = alfvmax[layer + layer0];
   double dv = P.dv;
   double s = shiftmax * P.rhorat + 1e-9;

@@ -116,6 +116,7 @@ struct clblm_handle {
   DevBuf f4prep, f4sh, f4nout, f4rec, f4recd, f4nrec, f4nmir, f4pm, f4sm, err;
   DevBuf pblk, bv1, bn, bm0, bfac;
   DevBuf gpm, gsm;  // per grid record bounds of the panel kernel
+  DevBuf pwork;     // CTAs of the panel kernel's line pass
   DevBuf reclo;     // low parts of the records' ZFL/ZSLOPE
   DevBuf jprof, jod, jmap, jjobs, jblk;  // Jacobians: profiles, block ODs, maps, jobs, grid blocks
   DevBuf jvjp;                          // vector-Jacobian product: CTA partial sums and the totals
@@ -139,7 +140,7 @@ struct clblm_handle {
                               &bm0,       &bfac,     &f4blk,     &f4ntot,  &f4cidx,  &f4vb,   &f4lb,    &f4src,
                               &f4flag,    &f4cut,    &f4grp,     &f4nxt,   &ragg,    &segpool, &gpm,    &gsm,
                               &reclo,     &jprof,    &jod,       &jmap,    &jjobs,   &jblk,    &jvjp,   &isotab,
-                              &linecpl,   &f4cpl,    &f4cpll,    &f4ncpl};
+                              &linecpl,   &f4cpl,    &f4cpll,    &f4ncpl,   &pwork};
     for (auto& b : rt) v.push_back(&b);
     for (auto& b : imap) v.push_back(&b);
     v.push_back(&rtseg);
@@ -536,6 +537,26 @@ int jrad_step(int jrad_state, bool first_pass, int jrad_ctrl, double V1, double 
   return JRAD;
 }
 
+// CTAs of the line pass per panel of a layer: one for each `per` lines that
+// reach a 16-point R3 half tile, whose 256 DV and 64 ALFV to either side are
+// 768 DV at the usual ALFV = 4 DV.  A layer's own numbers decide, not the
+// launch's size, so that its OD does not depend on what it shares a launch
+// with; a call for one layer, which has the GPU to itself, cuts finer.  (A
+// surface layer of 20,000 lines on 100 cm-1, 2400 lines on a half tile: 1032
+// us in one CTA per panel, 634, 526, 532, 540 at 512, 256, 128, 64 lines a slice;
+// 3000 lines on 15 cm-1: 910, 547, 448, 395, 397.  In a launch that fills the
+// GPU the slices cost their set-up: the 60-layer 2000 cm-1 column took 45.3 ms
+// uncut, 45.6, 45.9, 47.3, 50.4.)  The Jacobians' ODs are not cut: they gain
+// nothing (117.9 ms uncut, 117.6 at 512), and their differences of two ODs
+// amplify the rounding of a sum formed in another order.
+constexpr int kSliceLinesLayer = 128, kSliceLines = 512;
+int panel_slices(const LayerPlan& P, int per) {
+  const int64_t n = P.line_hi - P.line_lo + 1;
+  if (n <= 0) return 1;
+  const double z = (double)n / (P.vtop - P.vbot) * 768. * P.dv / (double)per;
+  return z < 1. ? 1 : (z > (double)kMaxSlices ? kMaxSlices : (int)z);
+}
+
 int plan_layer(clblm_handle* h, const clblm_layer_t* lay, const clblm_grid_t* g, const clblm_od_ctrl_t* c,
                int jrad_state, bool first_pass, HostPlan* hp, int* jrad_after) {
   if (!lay || !g || !c) return set_err(h, CLBLM_ERR_ARG, "null argument");
@@ -686,6 +707,7 @@ int plan_layer(clblm_handle* h, const clblm_layer_t* lay, const clblm_grid_t* g,
   P.npanels = (int)hp->vft.size();
   P.nsamp = nsamp;
   line_range(h, P.vbot, P.vtop, &P.line_lo, &P.line_hi, &P.first_rec_end);
+  P.nslice = 1;  // (clblm_gpu_od and clblm_gpu_rt_mode2 cut the panels)
   // far wings, OPDPTH :899-931
   double ALFAV4 = 64. * g->sample * DV;
   P.dvr4 = ALFAV4 / g->sample;
@@ -902,7 +924,7 @@ size_t od_job_bytes(const LayerPlan& P, bool plain) {
                         sizeof(F4Rec) + 2 * sizeof(int) + (plain ? sizeof(F4RecD) : 0);
   const size_t real = plain ? 8 : 4;
   return (size_t)(P.line_hi - P.line_lo + 1) * per_line + (size_t)(P.f4_hi - P.f4_lo) * per_f4 +
-         (size_t)(P.nsamp + P.nptr4) * real;
+         (size_t)(P.nsamp * P.nslice + P.nptr4) * real;
 }
 
 // Bytes of OD-pipeline workspace one batch of layers may take: 60 % of the
@@ -1139,11 +1161,16 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
                                                             h->ragg.as<int>() + (int64_t)3 * count * nagg, nagg,
                                                             h->gpm.as<int>(), h->gsm.as<int>());
   int maxp = 0;
-  for (int k = 0; k < count; ++k) maxp = std::max(maxp, hps[first + k].P.npanels);
+  int64_t ctas = 0;  // of the line pass
+  for (int k = 0; k < count; ++k) {
+    maxp = std::max(maxp, hps[first + k].P.npanels);
+    ctas += (int64_t)hps[first + k].P.npanels * hps[first + k].P.nslice;
+  }
   h->launches++;
   k_panel_ranges<<<dim3((maxp + 127) / 128, count), 128, 0, st>>>(dplans, first, h->vkey.as<double>(),
                                                                    h->alfvmax.as<double>(), h->shiftmax,
-                                                                   h->ranges.as<int64_t>(), pstride);
+                                                                   h->ranges.as<int64_t>(), pstride,
+                                                                   h->pwork.as<int2>());
   PanelArgs pa;
   pa.plans = dplans;
   pa.layer0 = first;
@@ -1156,6 +1183,7 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
   pa.stride = lstride;
   pa.ranges = h->ranges.as<int64_t>();
   pa.panel_stride = pstride;
+  pa.work = h->pwork.as<int2>();
   pa.r4_all = h->r4.p;
   pa.absrb_all = h->absrb.as<double>();
   pa.od_all = h->od.p;
@@ -1188,50 +1216,41 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
                                                             h->bfac.as<double>());
   }
   CUDA_TRY(h, cudaEventRecord(h->ev[5], st));
-  size_t smem = panel_smem_bytes(plain);
-  if (plain) {
-    // FP64: one pass once R4 and ABSRB are ready
-    CUDA_TRY(h, cudaStreamWaitEvent(st, h->join_ev, 0));
-    if (!h->panel_attr_set[1]) {
-      CUDA_TRY(h, cudaFuncSetAttribute(k_panel<true, kPanelAll, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
-      CUDA_TRY(h, cudaFuncSetAttribute(k_panel<true, kPanelAll, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
-      h->panel_attr_set[1] = true;
+  // the line sums run beside the far-wing chain, then, once R4 and ABSRB are
+  // ready, a second pass adds the far wings and the continuum through XINT and
+  // the combine (the OD is linear in R3, R2 and R1)
+  const size_t smem = panel_smem_bytes(plain), smem_w = panel_smem_bytes(plain, true);
+  if (!h->panel_attr_set[plain ? 1 : 0]) {
+    const auto attr = [](auto* f, size_t b) {
+      return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+    };
+    if (plain) {
+      CUDA_TRY(h, attr(k_panel<true, kPanelLines, false>, smem));
+      CUDA_TRY(h, attr(k_panel<true, kPanelLines, true>, smem));
+      CUDA_TRY(h, attr(k_panel<true, kPanelWings, false>, smem_w));
+    } else {
+      CUDA_TRY(h, attr(k_panel<false, kPanelLines, false>, smem));
+      CUDA_TRY(h, attr(k_panel<false, kPanelLines, true>, smem));
+      CUDA_TRY(h, attr(k_panel<false, kPanelWings, false>, smem_w));
     }
-    h->launches++;
-    CUDA_TRY(h, cudaEventRecord(h->ev[2], st));
-    if (h->has_cpl) k_panel<true, kPanelAll, true><<<dim3(maxp, count), kPanelThreads, smem, st>>>(pa);
-    else k_panel<true, kPanelAll, false><<<dim3(maxp, count), kPanelThreads, smem, st>>>(pa);
-    CUDA_TRY(h, cudaEventRecord(h->ev[3], st));
-    CUDA_TRY(h, cudaEventRecord(h->ev[8], st));
-    CUDA_TRY(h, cudaEventRecord(h->ev[9], st));
-  } else {
-    // mixed: the line sums run beside the far-wing chain, then, once R4 and
-    // ABSRB are ready, a second pass adds the far wings and the continuum
-    // through XINT and the combine (the OD is linear in R3, R2 and R1)
-    if (!h->panel_attr_set[0]) {
-      CUDA_TRY(h, cudaFuncSetAttribute(k_panel<false, kPanelLines, false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      CUDA_TRY(h, cudaFuncSetAttribute(k_panel<false, kPanelLines, true>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      CUDA_TRY(h, cudaFuncSetAttribute(k_panel<false, kPanelWings, false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)panel_smem_bytes(false, true)));
-      h->panel_attr_set[0] = true;
-    }
-    h->launches += 2;
-    CUDA_TRY(h, cudaEventRecord(h->ev[2], st));
-    if (h->has_cpl) k_panel<false, kPanelLines, true><<<dim3(maxp, count), kPanelThreads, smem, st>>>(pa);
-    else k_panel<false, kPanelLines, false><<<dim3(maxp, count), kPanelThreads, smem, st>>>(pa);
-    CUDA_TRY(h, cudaEventRecord(h->ev[3], st));
-    CUDA_TRY(h, cudaStreamWaitEvent(st, h->join_ev, 0));  // R4 and ABSRB are ready
-    // the radiation-term pool is claimed again by the second pass
-    CUDA_TRY(h, cudaMemsetAsync(pa.seg_next, 0, sizeof(int), st));
-    CUDA_TRY(h, cudaEventRecord(h->ev[8], st));
-    // without the shape tables: six CTAs of the far-wing pass share an SM
-    k_panel<false, kPanelWings, false><<<dim3(maxp, count), kPanelThreads, panel_smem_bytes(false, true), st>>>(pa);
-    CUDA_TRY(h, cudaEventRecord(h->ev[9], st));
+    h->panel_attr_set[plain ? 1 : 0] = true;
   }
+  h->launches += 2;
+  CUDA_TRY(h, cudaEventRecord(h->ev[2], st));
+  if (plain) {
+    if (h->has_cpl) k_panel<true, kPanelLines, true><<<(unsigned)ctas, kPanelThreads, smem, st>>>(pa);
+    else k_panel<true, kPanelLines, false><<<(unsigned)ctas, kPanelThreads, smem, st>>>(pa);
+  } else {
+    if (h->has_cpl) k_panel<false, kPanelLines, true><<<(unsigned)ctas, kPanelThreads, smem, st>>>(pa);
+    else k_panel<false, kPanelLines, false><<<(unsigned)ctas, kPanelThreads, smem, st>>>(pa);
+  }
+  CUDA_TRY(h, cudaEventRecord(h->ev[3], st));
+  CUDA_TRY(h, cudaStreamWaitEvent(st, h->join_ev, 0));  // R4 and ABSRB are ready
+  CUDA_TRY(h, cudaEventRecord(h->ev[8], st));
+  // without the shape tables: six CTAs of the mixed far-wing pass share an SM
+  if (plain) k_panel<true, kPanelWings, false><<<dim3(maxp, count), kPanelThreads, smem_w, st>>>(pa);
+  else k_panel<false, kPanelWings, false><<<dim3(maxp, count), kPanelThreads, smem_w, st>>>(pa);
+  CUDA_TRY(h, cudaEventRecord(h->ev[9], st));
   // RSYM: the first panel of a layer whose panel origin is at or below 0 cm-1
   bool fold = false;
   for (int k = 0; k < count; ++k) fold |= !(hps[first + k].P.vft0 > 0.);
@@ -1251,6 +1270,7 @@ struct WsDims {
   int64_t psc = 0;     // panels x layers
   int64_t cnt = 0;     // layers
   int64_t odt = 0;     // OD points (padded)
+  int64_t ctas = 0;    // CTAs of the panel kernel's line pass
   int64_t r4t = 0;     // R4 points (padded)
   int64_t nblk4c = 0;  // far-wing scan blocks x layers
   int64_t smaxc = 0;   // first-fit scan blocks x layers
@@ -1261,6 +1281,7 @@ struct WsDims {
     psc = std::max(psc, o.psc);
     cnt = std::max(cnt, o.cnt);
     odt = std::max(odt, o.odt);
+    ctas = std::max(ctas, o.ctas);
     r4t = std::max(r4t, o.r4t);
     nblk4c = std::max(nblk4c, o.nblk4c);
     smaxc = std::max(smaxc, o.smaxc);
@@ -1272,7 +1293,7 @@ struct WsDims {
 // per-batch buffers (OD, R4, ABSRB).
 WsDims batch_dims(std::vector<HostPlan>& hps, int first, int count, int64_t* lstride, int64_t* f4stride,
                   int64_t* pstride) {
-  int64_t ls = 1, fs = 1, ps = 1, odt = 0, r4t = 0;
+  int64_t ls = 1, fs = 1, ps = 1, odt = 0, r4t = 0, ctas = 0;
   for (int k = 0; k < count; ++k) {
     LayerPlan& P = hps[first + k].P;
     ls = std::max<int64_t>(ls, P.line_hi - P.line_lo + 1);
@@ -1284,7 +1305,10 @@ WsDims batch_dims(std::vector<HostPlan>& hps, int first, int count, int64_t* lst
   for (int k = 0; k < count; ++k) {
     LayerPlan& P = hps[first + k].P;
     P.od_off = odt;
-    odt += pad256(P.nsamp + 8);
+    P.od_pts = pad256(P.nsamp + 8);
+    odt += P.od_pts * P.nslice;
+    P.cta0 = ctas;
+    ctas += (int64_t)P.npanels * P.nslice;
     P.r4_off = r4t;
     r4t += pad256(P.nptr4 + 8);
     P.abs_off = (int64_t)k * (kNABSRB + 8);
@@ -1295,6 +1319,7 @@ WsDims batch_dims(std::vector<HostPlan>& hps, int first, int count, int64_t* lst
   d.psc = ps * count;
   d.cnt = count;
   d.odt = odt;
+  d.ctas = ctas;
   d.r4t = r4t;
   d.nblk4c = ((fs + 1 + 1023) / 1024) * count;
   d.smaxc = ((ls + 1023) / 1024) * count;
@@ -1333,6 +1358,7 @@ cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int
   WS_ENSURE(h->ragg.ensure(sizeof(int) * d.raggc));
   WS_ENSURE(h->ranges.ensure(sizeof(int64_t) * 6 * d.psc));
   WS_ENSURE(h->od.ensure(real * d.odt));
+  WS_ENSURE(h->pwork.ensure(sizeof(int2) * (size_t)d.ctas));
   WS_ENSURE(h->r4.ensure(real * d.r4t));
   WS_ENSURE(h->absrb.ensure(sizeof(double) * (kNABSRB + 8) * d.cnt));
   WS_ENSURE(h->stats.ensure(sizeof(unsigned long long) * kStatsPerLayer * nL));
@@ -1378,7 +1404,7 @@ std::vector<DevBuf*> ws_buffers(clblm_handle* h) {
           &h->f4vb,   &h->f4lb,   &h->f4src,  &h->f4flag,   &h->f4nxt,  &h->f4cut,  &h->f4grp,  &h->f4rec,
           &h->f4recd, &h->f4nrec, &h->f4nmir, &h->f4pm,     &h->f4sm,   &h->err,    &h->segpool, &h->pblk,
           &h->bv1,    &h->bn,     &h->bm0,    &h->bfac,   &h->isotab, &h->linecpl, &h->f4cpl, &h->f4cpll,
-          &h->f4ncpl};
+          &h->f4ncpl, &h->pwork};
 }
 
 // Frees every work buffer of the handle (all but the line list, the shape
@@ -1835,6 +1861,7 @@ int clblm_gpu_od(clblm_handle_t* h, const clblm_layer_t* layer, const clblm_grid
   }
   if (rc) return rc;
   if (!out || cap < hps[0].n_out) return set_err(h, CLBLM_ERR_CAPACITY, "output needs %lld points", (long long)hps[0].n_out);
+  hps[0].P.nslice = panel_slices(hps[0].P, kSliceLinesLayer);
   bool plain = ctrl->precision == CLBLM_PREC_PLAIN;
   h->reset_call();
   int64_t ls, fs, ps, odt;
@@ -2056,6 +2083,7 @@ int clblm_gpu_rt_mode2(clblm_handle_t* h, const clblm_column_t* col, const clblm
   }
   if (rc) return rc;
   const int n = col->nlay;
+  for (HostPlan& hp : rp.hps) hp.P.nslice = panel_slices(hp.P, kSliceLines);
   int64_t nfinal = rp.grid_n.back();
   if (!rad || cap < nfinal) return set_err(h, CLBLM_ERR_CAPACITY, "radiance needs %lld points", (long long)nfinal);
   bool plain = ctrl->od.precision == CLBLM_PREC_PLAIN;
