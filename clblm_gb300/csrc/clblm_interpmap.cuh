@@ -162,6 +162,29 @@ struct MapReplay {
       fixed = (double)q * (1. / 2305843009213693952.) == P ? 1 : 0;
     }
   }
+  // n steps.  At 0.5 <= RATIO < 0.999 a sum below 1 is exact on multiples of
+  // 2^-53 and one above 1 rounds to a multiple of 2^-52: a chain of a few
+  // integer operations.
+  CLBLM_HD void steps(int n) {
+    int k = 0;
+    while (k < n && !(fixed && ratio >= 0.5 && ratio < 0.999 && (q & 255) == 0)) {
+      step();
+      ++k;
+    }
+    if (k == n) return;
+    uint64_t p = q >> 8;
+    const uint64_t r = rq >> 8;
+    int carries = 0;
+    for (; k < n; ++k) {
+      const uint64_t s = p + r;
+      const uint64_t c = s >> 53;  // 1: a carry
+      p = (s + (c & (s >> 1))) & ~c & (((uint64_t)1 << 53) - 1);
+      carries += (int)c;
+    }
+    // (a sum of exactly 2 cannot occur: P < 1 and RATIO < 1)
+    q = p << 8;
+    iIn += carries;
+  }
 };
 
 #ifdef __CUDACC__
@@ -203,14 +226,21 @@ __device__ __forceinline__ void interp_map_block(double v1, double dvin, double 
   }
   __syncthreads();
   if (threadIdx.x != 0 || last < 0) return;
-  const int stop = lin.sticky ? n - 1 : last;
+  // from one undecided point to the next
   MapReplay r;
   r.start(lin.i0, p0, ratio);
-  for (int k = 0;; ++k) {
-    if ((flags[k >> 5] >> (k & 31) & 1u) || (lin.sticky && k >= first))
+  int k = 0;
+  for (int w = first >> 5; w < (n + 31) / 32 && (lin.sticky || w <= last >> 5); ++w) {
+    unsigned f = flags[w];
+    if (lin.sticky) f = 32 * w >= first ? 0xffffffffu : f | (0xffffffffu << (first & 31));
+    while (f) {
+      const int t = 32 * w + __ffs(f) - 1;
+      f &= f - 1;
+      if (t >= n) break;
+      r.steps(t - k);
+      k = t;
       out[k] = make_int2((int)r.iIn, map_ip(r.phase()));
-    if (k >= stop) break;
-    r.step();
+    }
   }
 }
 #endif

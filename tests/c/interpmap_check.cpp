@@ -13,8 +13,10 @@ static long long bad = 0, points = 0, undecided = 0;
 
 static void block(int64_t i0, double P0, double r) {
   const MapLin m = map_lin(i0, P0, r);
-  MapReplay rep;
+  MapReplay rep, far;  // step by step, and in strides as a block's undecided points take them
   rep.start(i0, P0, r);
+  far.start(i0, P0, r);
+  int at = 0, stride = 1;
   int64_t iIn = i0;
   double P = P0;
   bool from = false;
@@ -30,6 +32,14 @@ static void block(int64_t i0, double P0, double r) {
       gi = rep.iIn;
       gp = map_ip(rep.phase());
       undecided++;
+    }
+    if (k == at + stride || k == kMapBlock - 1) {
+      far.steps(k - at);
+      at = k;
+      stride = stride % 97 + 1;
+      if (far.iIn != rep.iIn || far.phase() != rep.phase()) {
+        if (bad++ < 5) printf("strides: i0 %lld P0 %.17g r %.17g k %d\n", (long long)i0, P0, r, k);
+      }
     }
     points++;
     if (gi != iIn || gp != IP) {
