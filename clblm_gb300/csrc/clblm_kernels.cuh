@@ -126,16 +126,18 @@ __global__ void k_f4_compact(const F4Prep* prep, int64_t stride, const LayerPlan
                              int64_t* src, unsigned char* flags, int64_t* cut);
 __global__ void k_f4_next(const long long* vbits, const long long* lbits, const int64_t* ntot, int64_t stride,
                           int* gnxt);
-// PF: lines per thread of the next SHRINQ call loaded ahead (5: all; for a
-// batch of at most one CTA per SM, where each layer's walk is latency-bound)
-// (declared with the definition's __restrict__ qualifiers: a template's
-// declaration and definition must agree for the launch to find the kernel)
-template <int PF>
-__global__ void k_f4_walk(const LayerPlan* __restrict__ plans, int layer0, int nlayers, int64_t nlines_total,
-                          int64_t stride, const int64_t* __restrict__ cidx, const long long* __restrict__ vbits,
-                          const long long* __restrict__ lbits, const int* __restrict__ gnxt,
-                          const unsigned char* __restrict__ flags, const int64_t* __restrict__ ntot,
-                          const int64_t* __restrict__ cut, int4* __restrict__ groups, int64_t* __restrict__ ngroups);
+constexpr int kCallEnds = 32;    // records a tabulated SHRINQ call may span
+constexpr int kCallStarts = 12;  // records that calls start at, per CTA of k_f4_calls
+__global__ void k_f4_calls(const LayerPlan* plans, int layer0, int64_t stride, const int64_t* cidx,
+                           const long long* vbits, const long long* lbits, const int* gnxt,
+                           const unsigned char* flags, const int64_t* ntot, int64_t tab_records, unsigned* tab);
+__global__ void k_f4_walk(const LayerPlan* plans, int layer0, int nlayers, int64_t nlines_total, int64_t stride,
+                          const int64_t* cidx, const long long* vbits, const long long* lbits, const int* gnxt,
+                          const unsigned char* flags, const int64_t* ntot, const int64_t* cut, int64_t tab_records,
+                          const unsigned* tab, int4* calls, int2* ncalls, int64_t* ngroups);
+__global__ void k_f4_groups(int layer0, int64_t stride, const long long* vbits, const long long* lbits,
+                            const int* gnxt, const unsigned char* flags, int64_t tab_records, const int4* calls,
+                            const int2* ncalls, int4* groups, int64_t* ngroups);
 constexpr int kGroupSumThreads = 256;
 __global__ void __launch_bounds__(kGroupSumThreads)
     k_f4_groupsum(const LayerPlan* plans, int layer0, const F4Prep* prep, int64_t stride,
@@ -161,7 +163,12 @@ constexpr int kRecNone = 0x7fffffff;
 __global__ void k_rec_carry(const LayerPlan* plans, int layer0, int* aggmax, int* aggmin, int nagg);
 __global__ void k_rec_bounds(const LayerPlan* plans, int layer0, const GridRec* rec, int64_t stride,
                              const int* aggmax, const int* aggmin, int nagg, int* pmax, int* smin);
-__global__ void k_f4_bounds(const F4Rec* rec, int64_t rstride, const int64_t* nrec, int layer0, int* pmax,
-                            int* smin);
+// running bounds of the far-wing records, in blocks of kF4Blk records
+constexpr int kF4Blk = 1024, kF4BlkThreads = 256;
+__global__ void __launch_bounds__(kF4BlkThreads)
+    k_f4_agg(const F4Rec* rec, int64_t rstride, const int64_t* nrec, int layer0, int nblk, int* aggmax, int* aggmin);
+__global__ void __launch_bounds__(kF4BlkThreads)
+    k_f4_bounds(const F4Rec* rec, int64_t rstride, const int64_t* nrec, int layer0, int nblk, const int* aggmax,
+                const int* aggmin, int* pmax, int* smin);
 
 }  // namespace clblm

@@ -14,7 +14,7 @@
 //   k_continuum      mt_ckd_h2o_absco + CONTNM H2O block onto ABSRB
 //                    (mt_ckd_h2o_module.f90:72-170, clblm_ODLAY_Continuum.f90:355-405)
 //   k_f4_prep        LINF4Q per-line corrections (clblm_ODLAY_LineF4.f90:872-1171)
-//   k_f4_count/compact/walk/groupsum  the LINF4Q record loop with SHRINQ
+//   k_f4_count/compact/next/calls/walk/groups/groupsum  the LINF4Q record loop with SHRINQ
 //                    (:959-1234, :1516-1647)
 #include "clblm_common.cuh"
 #include "clblm_fpconv.cuh"
@@ -1315,9 +1315,10 @@ template __global__ void k_f4_prep<true>(const LayerPlan* __restrict__, int, Lin
 //
 // Pieces: (1) prefix count of the lines that enter the buffer, (2) compaction
 // with the integer image of each centre and of centre + DVR4/2 (positive
-// doubles order like their bit patterns), (3) one warp per layer replays the
-// record loop and finds group ends with ballots, (4) one thread per group
-// forms the group's sums in the reference's order.
+// doubles order like their bit patterns), (3) the group that follows a group
+// ending at each line, (4) the counts of every call that may occur, the record
+// loop over them and the groups of its calls, (5) the groups' sums in the
+// reference's order.
 
 __global__ void k_f4_count(const F4Prep* __restrict__ prep, int64_t stride, const LayerPlan* __restrict__ plans,
                            int layer0, int64_t* __restrict__ blocksum, int nblk) {
@@ -1436,25 +1437,31 @@ __global__ void k_f4_next(const long long* __restrict__ vbits, const long long* 
   }
 }
 
-// Group list of one layer: one CTA replays LINF4Q's record loop (records of
-// 250 lines appended to a buffer until it holds 1000, then SHRINQ over the
-// lines not yet shrunk, clblm_ODLAY_LineF4.f90:1355-1476 and :1516-1647).
+// Group list of one layer.  LINF4Q's record loop appends records of 250 lines
+// to a buffer until it holds 1000, then SHRINQ shrinks the lines not yet
+// shrunk (clblm_ODLAY_LineF4.f90:1355-1476 and :1516-1647); how many records
+// the next call takes depends on the pseudo-lines that the call emits, so the
+// calls form one serial chain per layer.  A CTA that shrank the calls one
+// after another took 5.6 us a call, 1.8 ms for a layer of 250,000 lines.
+// Three kernels instead:
+//   k_f4_calls   for every record that a call may start at and every record
+//                that it may end at, the groups and pseudo-lines of that call
+//                (all starts at once),
+//   k_f4_walk    the record loop, a table look-up per call: the list of calls
+//                with their first output slot and group,
+//   k_f4_groups  the groups of every call of the list (all calls at once).
 //
 // One SHRINQ call over m lines: the group ends form the chain e0, nxt(e0),
-// nxt(nxt(e0)), ... up to the call's last line, with nxt the capped
-// next-group map and e0 the end of the first group (VLMT = VNU(first) +
-// DVR4/2).  The chain is found in parallel: binary-lifting tables nxt^(2^k)
-// in shared memory, then every line v >= e0 descends greedily from e0 to the
-// last chain node <= v and is a group end when it lands on itself.  A block
-// scan ranks the ends and counts each line's non-CO2 / CO2 flags; a group
-// emits a non-CO2 line when one of its members has a non-CO2 line with
-// SP >= 1e-35, a CO2 line likewise, and a second scan gives the output slots
-// that the record loop's buffer arithmetic counts.
+// nxt(nxt(e0)), ... up to the call's last line, with nxt the next-group map
+// capped at that line and e0 the end of the first group (VLMT = VNU(first) +
+// DVR4/2).  A group emits a non-CO2 line when one of its members has a
+// non-CO2 line with SP >= 1e-35, a CO2 line likewise, and each of its coupled
+// lines.
 constexpr int kWalkThreads = 256;
 constexpr int kWalkMax = 1280;  // lines of one SHRINQ call: < 1000 + one 250-line record
 constexpr int kWalkPer = kWalkMax / kWalkThreads;
 constexpr int kLift = 11;       // 2^11 > kWalkMax
-constexpr int kRecWin = 256;    // records whose stream offsets are staged at a time
+constexpr int kRecWin = 256;    // records whose stream offsets and calls are staged at a time
 
 // exclusive block scan of one value per thread; returns the block total
 template <typename T>
@@ -1484,23 +1491,250 @@ __device__ __forceinline__ T block_scan_excl(T v, T* warp_tot, T* out_excl) {
   return total;
 }
 
-template <int kWalkPf>
+
+// stream offset of the first line of record `rec` (lines of the layer's
+// prepared range before it that entered the stream)
+__device__ __forceinline__ int64_t rec_offset(const int64_t* __restrict__ ci, int64_t rec, int64_t f4_lo, int64_t n) {
+  const int64_t t = rec * 250 - f4_lo;
+  return ci[t < 0 ? 0 : (t > n ? n : t)];
+}
+
+// Groups and pseudo-lines of the calls that start at each record of a
+// layer: tab[(record - first) * kCallEnds + k - 1] for the call that ends
+// before record start + k, pseudo-lines in the low 16 bits and groups above.  Ends
+// past the first 1000 lines are never a call's, those past kCallEnds records
+// (streams of few lines per record) are left to k_f4_walk.  A CTA stages the
+// lines that calls from its kCallStarts records reach; one thread a start
+// follows the chain and notes the counts at every record boundary, the last
+// group cut there.  What bounds it is the chain: the next group end and the
+// flag counts up to it, two shared-memory reads side by side a group.
+constexpr int kCallSpan = kCallStarts * 250 + kWalkMax;
+constexpr int kCallPer = (kCallSpan + kWalkThreads - 1) / kWalkThreads;
+__global__ void __launch_bounds__(kWalkThreads, 4)
+    k_f4_calls(const LayerPlan* __restrict__ plans, int layer0, int64_t stride, const int64_t* __restrict__ cidx,
+               const long long* __restrict__ vbits, const long long* __restrict__ lbits,
+               const int* __restrict__ gnxt, const unsigned char* __restrict__ flags,
+               const int64_t* __restrict__ ntot, int64_t tab_records, unsigned* __restrict__ tab) {
+  // flag counts before each staged line, 16 bits each: non-CO2, CO2, coupled
+  __shared__ unsigned long long pc[kCallSpan + 1];
+  __shared__ short nx[kCallSpan];
+  __shared__ int64_t civ[kCallStarts + kCallEnds + 1];
+  __shared__ unsigned long long wt64[kWalkThreads / 32 + 1];
+  const int layer = blockIdx.y;
+  const LayerPlan& P = plans[layer + layer0];
+  const int64_t n = P.f4_hi - P.f4_lo;
+  const int64_t first = P.f4_lo / 250, r0 = first + (int64_t)blockIdx.x * kCallStarts;
+  if (r0 * 250 - P.f4_lo >= n) return;  // whole CTA
+  const int tid = threadIdx.x;
+  const int64_t* ci = cidx + (int64_t)layer * (stride + 1);
+  for (int k = tid; k <= kCallStarts + kCallEnds; k += kWalkThreads) civ[k] = rec_offset(ci, r0 + k, P.f4_lo, n);
+  __syncthreads();
+  const int64_t total = ntot[layer], b0 = civ[0];
+  const int cnt = (int)min(total - b0, (int64_t)kCallSpan);  // staged lines
+  const int64_t off = (int64_t)layer * stride + b0;
+  for (int i = tid; i < cnt; i += kWalkThreads) {
+    nx[i] = (short)min((int64_t)gnxt[off + i] - b0, (int64_t)cnt - 1);
+    const unsigned f = flags[off + i];
+    pc[i + 1] = (unsigned long long)(f & 1u) + ((unsigned long long)((f >> 1) & 1u) << 16) +
+                ((unsigned long long)((f >> 2) & 1u) << 32);
+  }
+  if (tid == 0) pc[0] = 0;
+  __syncthreads();
+  {  // inclusive sums over pc[1 .. cnt], thread t's share tid*kCallPer + 1 ..
+    const int i0 = tid * kCallPer + 1, i1 = min(i0 + kCallPer, cnt + 1);
+    unsigned long long mine = 0, run;
+    for (int i = i0; i < i1; ++i) mine += pc[i];
+    block_scan_excl<unsigned long long>(mine, wt64, &run);
+    for (int i = i0; i < i1; ++i) {
+      run += pc[i];
+      pc[i] = run;
+    }
+  }
+  __syncthreads();
+  constexpr int kEvery = kWalkThreads / kCallStarts;
+  const int s = tid / kEvery;
+  if (tid % kEvery || s >= kCallStarts) return;
+  const int64_t rs = r0 + s;
+  if (rs * 250 - P.f4_lo >= n || rs - first >= tab_records) return;
+  unsigned* T = tab + ((int64_t)layer * tab_records + (rs - first)) * kCallEnds;
+  const int u0 = (int)(civ[s] - b0);
+  auto emits = [](unsigned long long d) {  // pseudo-lines of a group with the flag counts d
+    return ((d & 0xFFFF) ? 1 : 0) + ((d & 0xFFFF0000ull) ? 1 : 0) + (int)(d >> 32);
+  };
+  int e = u0, E = 0, g = 0;
+  // the first group: its first line alone when the second lies past VLMT =
+  // VNU(first) + DVR4/2, else up to the next-group map's end
+  if (u0 + 1 < cnt && !(vbits[off + u0 + 1] > lbits[off + u0])) e = nx[u0];
+  unsigned long long c0 = pc[u0];  // counts before the group that ends at e
+  for (int k = 1; k <= kCallEnds; ++k) {
+    const int u1 = (int)min(civ[s + k] - b0, (int64_t)cnt);
+    unsigned v = 0;
+    if (u1 > u0) {
+      while (e < u1 - 1) {
+        const unsigned long long c1 = pc[e + 1];
+        e = nx[e];
+        E += emits(c1 - c0);
+        ++g;
+        c0 = c1;
+      }
+      v = (unsigned)(E + emits(pc[u1] - c0)) | ((unsigned)(g + 1) << 16);
+    }
+    T[k - 1] = v;
+    if (u1 - u0 >= 1000) break;
+  }
+}
+
+// The groups of one SHRINQ call over the stream lines [u0, u0 + m) by a CTA:
+// binary-lifting tables nxt^(2^k) in shared memory, then every line v >= e0
+// descends greedily from e0 to the last chain node <= v and is a group end
+// when it lands on itself.  A block scan ranks the ends and counts each
+// line's flags, a second one gives the output slots that the record loop's
+// buffer arithmetic counts.  G (when not null) receives the groups: first and
+// last line, first slot, kinds.
+struct CallShared {
+  short up[kLift][kWalkMax];     // up[k][b]: nxt applied 2^k times
+  short ends[kWalkMax];          // group ends of the call, in order
+  short pc1[kWalkMax + 1], pc2[kWalkMax + 1];  // flag counts before each line
+  short pc4[kWalkMax + 1];                     // coupled lines before each line
+  unsigned char sf[kWalkMax];
+  unsigned long long wt64[kWalkThreads / 32 + 1];
+  int wt32[kWalkThreads / 32 + 1];
+  int e0;
+};
+__device__ void shrink_call(CallShared& W, int64_t u0, int m, const long long* __restrict__ V,
+                            const long long* __restrict__ Lm, const int* __restrict__ GN,
+                            const unsigned char* __restrict__ F, int slot, int4* __restrict__ G, int64_t room,
+                            int* gcount, int* emitted) {
+  const int tid = threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < kWalkPer; ++k) {
+    const int i = tid + k * kWalkThreads;
+    if (i < m) {
+      const int64_t e = (int64_t)GN[u0 + i] - u0;
+      W.up[0][i] = (short)(e < m - 1 ? e : m - 1);
+      W.sf[i] = F[u0 + i];
+    }
+  }
+  // the first group: VLMT = VNU(first) + DVR4/2
+  if (tid == 0) W.e0 = (m == 1 || V[u0 + 1] > Lm[u0]) ? 0 : -1;
+  __syncthreads();
+  if (tid == 0 && W.e0 < 0) W.e0 = W.up[0][0];
+  __syncthreads();
+  const int e0 = W.e0;
+  // lifting tables until 2^K steps from e0 reach the last line
+  int K = 0;
+  while (K < kLift - 1 && W.up[K][e0] != m - 1) {
+    for (int i = tid; i < m; i += kWalkThreads) W.up[K + 1][i] = W.up[K][W.up[K][i]];
+    ++K;
+    __syncthreads();
+  }
+  // group ends: lines v >= e0 on the chain; thread t owns lines t*kWalkPer + q
+  bool on[kWalkPer];
+  {
+    int x[kWalkPer];
+#pragma unroll
+    for (int q = 0; q < kWalkPer; ++q) x[q] = e0;
+    for (int k = K; k >= 0; --k) {
+#pragma unroll
+      for (int q = 0; q < kWalkPer; ++q) {
+        const int v = tid * kWalkPer + q;
+        const int y = W.up[k][x[q]];
+        if (y <= v) x[q] = y;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kWalkPer; ++q) {
+      const int v = tid * kWalkPer + q;
+      on[q] = v < m && v >= e0 && x[q] == v;
+    }
+  }
+  // one scan, 16 bits a count (m <= kWalkMax < 2^16): ends, non-CO2
+  // flags, CO2 flags, coupled lines
+  auto packed = [](bool e, unsigned f) {
+    return (unsigned long long)e + ((unsigned long long)(f & 1u) << 16) + ((unsigned long long)((f >> 1) & 1u) << 32) +
+           ((unsigned long long)((f >> 2) & 1u) << 48);
+  };
+  unsigned long long mine = 0;
+#pragma unroll
+  for (int q = 0; q < kWalkPer; ++q) {
+    const int v = tid * kWalkPer + q;
+    const unsigned f = v < m ? W.sf[v] : 0u;
+    mine += packed(on[q], f);
+  }
+  unsigned long long ex;
+  const unsigned long long tot = block_scan_excl<unsigned long long>(mine, W.wt64, &ex);
+  {
+    unsigned long long run = ex;
+#pragma unroll
+    for (int q = 0; q < kWalkPer; ++q) {
+      const int v = tid * kWalkPer + q;
+      if (v < m) {
+        W.pc1[v] = (short)((run >> 16) & 0xFFFF);
+        W.pc2[v] = (short)((run >> 32) & 0xFFFF);
+        W.pc4[v] = (short)((run >> 48) & 0xFFFF);
+        if (on[q]) W.ends[run & 0xFFFF] = (short)v;
+        run += packed(on[q], W.sf[v]);
+      }
+    }
+  }
+  if (tid == 0) {
+    W.pc1[m] = (short)((tot >> 16) & 0xFFFF);
+    W.pc2[m] = (short)((tot >> 32) & 0xFFFF);
+    W.pc4[m] = (short)((tot >> 48) & 0xFFFF);
+  }
+  __syncthreads();
+  const int ng = (int)(tot & 0xFFFF);
+  // which kinds each group emits, then the output slots (its coupled
+  // lines first, then its sums); thread t owns groups t*kWalkPer + q
+  int kind[kWalkPer], ncp[kWalkPer], cnt = 0;
+#pragma unroll
+  for (int q = 0; q < kWalkPer; ++q) {
+    const int g = tid * kWalkPer + q;
+    kind[q] = 0;
+    ncp[q] = 0;
+    if (g < ng) {
+      const int s0 = g == 0 ? 0 : W.ends[g - 1] + 1, s1 = W.ends[g] + 1;
+      kind[q] = (W.pc1[s1] > W.pc1[s0] ? 1 : 0) | (W.pc2[s1] > W.pc2[s0] ? 2 : 0);
+      ncp[q] = W.pc4[s1] - W.pc4[s0];
+      cnt += (kind[q] & 1) + (kind[q] >> 1) + ncp[q];
+    }
+  }
+  int excl;
+  *emitted = block_scan_excl<int>(cnt, W.wt32, &excl);
+  *gcount = ng;
+  if (G) {
+    int run = slot + excl;
+#pragma unroll
+    for (int q = 0; q < kWalkPer; ++q) {
+      const int g = tid * kWalkPer + q;
+      if (g < ng) {
+        const int s0 = g == 0 ? 0 : W.ends[g - 1] + 1, s1 = W.ends[g];
+        if (g < room) G[g] = make_int4((int)(u0 + s0), (int)(u0 + s1), run, kind[q]);
+        run += (kind[q] & 1) + (kind[q] >> 1) + ncp[q];
+      }
+    }
+  }
+  __syncthreads();  // the shared arrays are reused by the next call
+}
+
+// LINF4Q's record loop of one layer: the list of its SHRINQ calls (first and
+// end line of the stream, first output slot, first group) from k_f4_calls'
+// table, whose rows are staged a window of records at a time.  A call of
+// more records than the table holds is counted by the CTA.  The last call (at the end of
+// the stream) may end inside a record: its counts are k_f4_groups'.
 __global__ void __launch_bounds__(kWalkThreads)
     k_f4_walk(const LayerPlan* __restrict__ plans, int layer0, int nlayers, int64_t nlines_total, int64_t stride,
               const int64_t* __restrict__ cidx, const long long* __restrict__ vbits,
               const long long* __restrict__ lbits, const int* __restrict__ gnxt,
               const unsigned char* __restrict__ flags, const int64_t* __restrict__ ntot,
-              const int64_t* __restrict__ cut, int4* __restrict__ groups, int64_t* __restrict__ ngroups) {
-  // (a template: declared with the same qualifiers in clblm_kernels.cuh)
-  __shared__ short up[kLift][kWalkMax];     // up[k][b]: nxt applied 2^k times
-  __shared__ short ends[kWalkMax];          // group ends of the call, in order
-  __shared__ short pc1[kWalkMax + 1], pc2[kWalkMax + 1];  // flag counts before each line
-  __shared__ short pc4[kWalkMax + 1];                      // coupled lines before each line
-  __shared__ unsigned char sf[kWalkMax];
+              const int64_t* __restrict__ cut, int64_t tab_records, const unsigned* __restrict__ tab,
+              int4* __restrict__ calls, int2* __restrict__ ncalls, int64_t* __restrict__ ngroups) {
+  union Sh {
+    unsigned tab[kRecWin][kCallEnds];
+    CallShared call;
+  };
+  __shared__ Sh sh;
   __shared__ int64_t civ[kRecWin + 1];      // stream offsets of records wbase .. wbase+kRecWin
-  __shared__ unsigned long long wt64[kWalkThreads / 32 + 1];
-  __shared__ int wt32[kWalkThreads / 32 + 1];
-  __shared__ int sh_e0;
 
   const int layer = blockIdx.x;
   if (layer >= nlayers) return;
@@ -1512,38 +1746,79 @@ __global__ void __launch_bounds__(kWalkThreads)
   const long long* Lm = lbits + (int64_t)layer * stride;
   const int* GN = gnxt + (int64_t)layer * stride;
   const unsigned char* F = flags + (int64_t)layer * stride;
-  int4* G = groups + (int64_t)layer * stride;
+  const unsigned* T = tab + (int64_t)layer * tab_records * kCallEnds;
+  int4* C = calls + (int64_t)layer * (tab_records + 2);
   const int64_t total = ntot[layer];
   const unsigned long long cutv = (unsigned long long)cut[layer];
   const bool has_cut = cutv < (unsigned long long)total;
   const int64_t send = has_cut ? (int64_t)cutv + 1 : total;  // stream ends after the first line above V2L4
   const int64_t R = 250;
   const int64_t nrec_total = (nlines_total + R - 1) / R;
-  int64_t rec = P.f4_lo / R;
+  const int64_t rec_first = P.f4_lo / R;
+  int64_t rec = rec_first, rs = rec_first;  // next record; first record of the next call
   int64_t wbase = -(kRecWin + 2);  // no record staged yet
   int64_t IJ = 0, ILO = 1;  // 1-based buffer positions, as in LINF4Q
   int64_t u0 = 0;           // stream index of the first unshrunk line
-  int64_t ng = 0, slot = 0;
+  int64_t ng = 0, slot = 0, nc = 0;
   int status = 0;
-  bool IEOF = false;
-  // prefetched map, flags and first-group test operands of the call at pf_base
-  int pf_gn[kWalkPf];
-  unsigned char pf_f[kWalkPf];
-  long long pf_v1 = 0, pf_lm = 0;
-  int64_t pf_base = -1;
+  bool IEOF = false, last = false;
+  // stage the offsets of the records from `from` on and their rows of the table
+  auto stage = [&](int64_t from) {
+    wbase = from;
+    __syncthreads();
+    for (int k = tid; k <= kRecWin; k += kWalkThreads) civ[k] = rec_offset(ci, wbase + k, P.f4_lo, n);
+    const int64_t row0 = wbase - rec_first;
+    for (int k = tid; k < kRecWin * kCallEnds; k += kWalkThreads) {
+      const int64_t row = row0 + k / kCallEnds;
+      (&sh.tab[0][0])[k] = row < tab_records ? T[row * kCallEnds + k % kCallEnds] : 0u;
+    }
+    __syncthreads();
+  };
   for (;;) {  // every thread runs the (uniform) record loop
+    // Calls whose records lie inside the staged window and before the end of
+    // the stream, in 32-bit arithmetic: they are nearly all of them
+    if (rec == rs && rec >= wbase && rec < wbase + kRecWin && IJ == ILO - 1) {
+      // records up to which the window, the prepared range and the stream allow it
+      const int64_t safe = min(min(wbase + kRecWin, nrec_total), (n + P.f4_lo) / R);
+      const int rmax = (int)(safe - wbase);  // civ[r] for r <= rmax
+      int r = (int)(rec - wbase), buf = (int)IJ, un = (int)(u0 - civ[0]);
+      const int sendr = (int)min(send - civ[0], (int64_t)0x7fffffff);
+      for (;;) {
+        const int r0 = r;
+        int ce = un;
+        bool ok = false;
+        while (r < rmax && r - r0 < kCallEnds) {
+          ++r;
+          ce = (int)(civ[r] - civ[0]);
+          if (ce >= sendr) break;
+          if (buf + ce - un >= 1000) {
+            ok = true;
+            break;
+          }
+        }
+        if (!ok || ce - un > kWalkMax) {
+          r = r0;
+          break;
+        }
+        if (tid == 0)
+          C[nc] = make_int4((int)(civ[0] + un), (int)(civ[0] + ce), (int)slot, (int)ng);
+        nc++;
+        const unsigned v = sh.tab[r0][r - r0 - 1];
+        const int emitted = (int)(v & 0xFFFFu);
+        ng += (int)(v >> 16);
+        slot += emitted;
+        buf = buf + emitted < 1000 ? buf + emitted : 0;
+        un = ce;
+      }
+      rec = rs = wbase + r;
+      u0 = civ[0] + un;
+      IJ = buf;
+      ILO = buf + 1;
+    }
     if (rec >= nrec_total) {
       IEOF = true;
     } else {
-      if (rec + 1 > wbase + kRecWin) {  // stage the offsets of the next records
-        wbase = rec;
-        __syncthreads();
-        for (int k = tid; k <= kRecWin; k += kWalkThreads) {
-          int64_t t = (wbase + k) * R - P.f4_lo;
-          civ[k] = ci[t < 0 ? 0 : (t > n ? n : t)];
-        }
-        __syncthreads();
-      }
+      if (rec < wbase || rec + (rec == rs ? kCallEnds : 1) > wbase + kRecWin) stage(rec);
       int64_t tb = rec * R - P.f4_lo, te = tb + R;
       const int64_t cb = civ[rec - wbase];
       rec++;
@@ -1570,138 +1845,28 @@ __global__ void __launch_bounds__(kWalkThreads)
     }
     int64_t nemit = 0;
     if (m > 0) {
-      // this call's next-group map and flags: from the registers the previous
-      // call filled when it started here, else from memory
-      const bool have = (pf_base == u0);
-#pragma unroll
-      for (int k = 0; k < kWalkPer; ++k) {
-        const int i = tid + k * kWalkThreads;
-        if (i < m) {
-          const bool pf = have && k < kWalkPf;
-          const int64_t e = pf ? (int64_t)pf_gn[k < kWalkPf ? k : 0] : (int64_t)GN[u0 + i];
-          up[0][i] = (short)((e < u1 - 1 ? e : u1 - 1) - u0);
-          sf[i] = pf ? pf_f[k < kWalkPf ? k : 0] : F[u0 + i];
-        }
+      if (tid == 0) C[nc] = make_int4((int)u0, (int)u1, (int)slot, (int)ng);
+      nc++;
+      if (IEOF) {
+        last = true;
+        break;
       }
-      if (tid == 0) {
-        // the first group: VLMT = VNU(first) + DVR4/2
-        const bool split = m == 1 || (have ? pf_v1 > pf_lm : V[u0 + 1] > Lm[u0]);
-        sh_e0 = split ? 0 : -1;
-      }
-      // the next call starts at u1: its loads overlap this call's work
-      pf_base = u1;
-#pragma unroll
-      for (int k = 0; k < kWalkPf; ++k) {
-        const int64_t i = u1 + tid + k * kWalkThreads;
-        if (i < total) {
-          pf_gn[k] = GN[i];
-          pf_f[k] = F[i];
-        }
-      }
-      if (tid == 0) {
-        pf_v1 = u1 + 1 < total ? V[u1 + 1] : 0;
-        pf_lm = u1 < total ? Lm[u1] : 0;
-      }
-      __syncthreads();
-      if (tid == 0 && sh_e0 < 0) sh_e0 = up[0][0];
-      __syncthreads();
-      const int e0 = sh_e0;
-      // lifting tables until 2^K steps from e0 reach the last line
-      int K = 0;
-      while (K < kLift - 1 && up[K][e0] != m - 1) {
-        for (int i = tid; i < m; i += kWalkThreads) up[K + 1][i] = up[K][up[K][i]];
-        ++K;
-        __syncthreads();
-      }
-      // group ends: lines v >= e0 on the chain; thread t owns lines t*kWalkPer + q
-      bool on[kWalkPer];
-      {
-        int x[kWalkPer];
-#pragma unroll
-        for (int q = 0; q < kWalkPer; ++q) x[q] = e0;
-        for (int k = K; k >= 0; --k) {
-#pragma unroll
-          for (int q = 0; q < kWalkPer; ++q) {
-            const int v = tid * kWalkPer + q;
-            const int y = up[k][x[q]];
-            if (y <= v) x[q] = y;
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < kWalkPer; ++q) {
-          const int v = tid * kWalkPer + q;
-          on[q] = v < m && v >= e0 && x[q] == v;
-        }
-      }
-      // one scan, 16 bits a count (m <= kWalkMax < 2^16): ends, non-CO2
-      // flags, CO2 flags, coupled lines
-      auto packed = [](bool e, unsigned f) {
-        return (unsigned long long)e + ((unsigned long long)(f & 1u) << 16) +
-               ((unsigned long long)((f >> 1) & 1u) << 32) + ((unsigned long long)((f >> 2) & 1u) << 48);
-      };
-      unsigned long long mine = 0;
-#pragma unroll
-      for (int q = 0; q < kWalkPer; ++q) {
-        const int v = tid * kWalkPer + q;
-        const unsigned f = v < m ? sf[v] : 0u;
-        mine += packed(on[q], f);
-      }
-      unsigned long long ex;
-      const unsigned long long tot = block_scan_excl<unsigned long long>(mine, wt64, &ex);
-      {
-        unsigned long long run = ex;
-#pragma unroll
-        for (int q = 0; q < kWalkPer; ++q) {
-          const int v = tid * kWalkPer + q;
-          if (v < m) {
-            pc1[v] = (short)((run >> 16) & 0xFFFF);
-            pc2[v] = (short)((run >> 32) & 0xFFFF);
-            pc4[v] = (short)((run >> 48) & 0xFFFF);
-            if (on[q]) ends[run & 0xFFFF] = (short)v;
-            run += packed(on[q], sf[v]);
-          }
-        }
-      }
-      if (tid == 0) {
-        pc1[m] = (short)((tot >> 16) & 0xFFFF);
-        pc2[m] = (short)((tot >> 32) & 0xFFFF);
-        pc4[m] = (short)((tot >> 48) & 0xFFFF);
-      }
-      __syncthreads();
-      const int gcount = (int)(tot & 0xFFFF);
-      // which kinds each group emits, then the output slots (its coupled
-      // lines first, then its sums); thread t owns groups t*kWalkPer + q
-      int kind[kWalkPer], ncp[kWalkPer], cnt = 0;
-#pragma unroll
-      for (int q = 0; q < kWalkPer; ++q) {
-        const int g = tid * kWalkPer + q;
-        kind[q] = 0;
-        ncp[q] = 0;
-        if (g < gcount) {
-          const int s0 = g == 0 ? 0 : ends[g - 1] + 1, s1 = ends[g] + 1;
-          kind[q] = (pc1[s1] > pc1[s0] ? 1 : 0) | (pc2[s1] > pc2[s0] ? 2 : 0);
-          ncp[q] = pc4[s1] - pc4[s0];
-          cnt += (kind[q] & 1) + (kind[q] >> 1) + ncp[q];
-        }
-      }
-      int excl;
-      const int emitted = block_scan_excl<int>(cnt, wt32, &excl);
-      int run = (int)slot + excl;
-#pragma unroll
-      for (int q = 0; q < kWalkPer; ++q) {
-        const int g = tid * kWalkPer + q;
-        if (g < gcount) {
-          const int s0 = g == 0 ? 0 : ends[g - 1] + 1, s1 = ends[g];
-          if (ng + g < stride) G[ng + g] = make_int4((int)(u0 + s0), (int)(u0 + s1), run, kind[q]);
-          run += (kind[q] & 1) + (kind[q] >> 1) + ncp[q];
-        }
+      int gcount, emitted;
+      if (rec - rs <= kCallEnds && rs >= wbase) {
+        const unsigned v = sh.tab[rs - wbase][rec - rs - 1];
+        emitted = (int)(v & 0xFFFFu);
+        gcount = (int)(v >> 16);
+      } else {
+        __syncthreads();  // the window is overwritten
+        shrink_call(sh.call, u0, m, V, Lm, GN, F, 0, nullptr, 0, &gcount, &emitted);
+        wbase = -(kRecWin + 2);
       }
       ng += gcount;
       slot += emitted;
       nemit = emitted;
-      __syncthreads();  // shared arrays are reused by the next call
     }
     u0 = u1;
+    rs = rec;
     const int64_t J = ILO - 1 + nemit;
     ILO = J + 1;
     IJ = J;
@@ -1711,19 +1876,34 @@ __global__ void __launch_bounds__(kWalkThreads)
     if (IEOF) break;
   }
   if (tid == 0) {
+    ncalls[layer] = make_int2((int)nc, last && !status ? 1 : 0);
     ngroups[2 * (layer + layer0)] = status ? -status : ng;
     ngroups[2 * (layer + layer0) + 1] = slot;
   }
 }
 
-#define CLBLM_WALK_ARGS                                                                                       \
-  const LayerPlan* __restrict__, int, int, int64_t, int64_t, const int64_t* __restrict__,                     \
-      const long long* __restrict__, const long long* __restrict__, const int* __restrict__,                  \
-      const unsigned char* __restrict__, const int64_t* __restrict__, const int64_t* __restrict__,            \
-      int4* __restrict__, int64_t* __restrict__
-template __global__ void k_f4_walk<2>(CLBLM_WALK_ARGS);
-template __global__ void k_f4_walk<kWalkPer>(CLBLM_WALK_ARGS);
-#undef CLBLM_WALK_ARGS
+// The groups of the calls of every layer's list; the layer's totals when its
+// last call ended the stream.
+__global__ void __launch_bounds__(kWalkThreads)
+    k_f4_groups(int layer0, int64_t stride, const long long* __restrict__ vbits, const long long* __restrict__ lbits,
+                const int* __restrict__ gnxt, const unsigned char* __restrict__ flags, int64_t tab_records,
+                const int4* __restrict__ calls, const int2* __restrict__ ncalls, int4* __restrict__ groups,
+                int64_t* __restrict__ ngroups) {
+  __shared__ CallShared W;
+  const int layer = blockIdx.y;
+  const int2 nc = ncalls[layer];
+  const int64_t off = (int64_t)layer * stride;
+  for (int c = blockIdx.x; c < nc.x; c += gridDim.x) {
+    const int4 k = calls[(int64_t)layer * (tab_records + 2) + c];
+    int gcount, emitted;
+    shrink_call(W, k.x, k.y - k.x, vbits + off, lbits + off, gnxt + off, flags + off, k.z, groups + off + k.w,
+                stride - k.w, &gcount, &emitted);
+    if (nc.y && c == nc.x - 1 && threadIdx.x == 0) {
+      ngroups[2 * (layer + layer0)] = (int64_t)k.w + gcount;
+      ngroups[2 * (layer + layer0) + 1] = (int64_t)k.z + emitted;
+    }
+  }
+}
 
 // a coupled line as a pseudo-line of its own (SHRINQ :1566-1578)
 __device__ __forceinline__ ShrunkLine shrunk_coupled(const F4Prep& r, bool mixed) {
@@ -2109,52 +2289,105 @@ __global__ void __launch_bounds__(kSetupThreads)
   if (threadIdx.x == 0) nmirror[layer + layer0] = nm;
 }
 
-// Per layer (one 1024-thread block): running max of jmax from the left and
-// running min of jmin from the right over the direct records, so that the
-// records overlapping a point form the contiguous index range found by two
-// binary searches.
-__global__ void k_f4_bounds(const F4Rec* __restrict__ rec, int64_t rstride, const int64_t* __restrict__ nrec,
-                            int layer0, int* __restrict__ pmax, int* __restrict__ smin) {
-  const int layer = blockIdx.x;
-  const int64_t n = nrec[layer + layer0];
+// Running max of jmax from the left and running min of jmin from the right
+// over a layer's direct records, so that the records overlapping a point form
+// the contiguous index range found by two binary searches.  k_f4_agg: the
+// bounds of every kF4Blk records; k_f4_bounds: a CTA per kF4Blk records takes
+// its carries from all of those and scans its own.  (One CTA per layer walked
+// all its records twice: 350 us for a layer of 150,000.)
+__device__ __forceinline__ int block_max(int v, int* sh) {
+  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = sh[0];
+  for (int w = 1; w < kF4BlkThreads / 32; ++w) v = max(v, sh[w]);
+  __syncthreads();
+  return v;
+}
+
+__global__ void __launch_bounds__(kF4BlkThreads)
+    k_f4_agg(const F4Rec* __restrict__ rec, int64_t rstride, const int64_t* __restrict__ nrec, int layer0, int nblk,
+             int* __restrict__ aggmax, int* __restrict__ aggmin) {
+  __shared__ int sh[kF4BlkThreads / 32];
+  const int layer = blockIdx.y;
+  const int64_t n = nrec[layer + layer0], base = (int64_t)blockIdx.x * kF4Blk;
+  if (base >= n) return;
   const F4Rec* R = rec + (int64_t)layer * rstride;
-  int* pm = pmax + (int64_t)layer * rstride;
-  int* sm = smin + (int64_t)layer * rstride;
-  const int T = blockDim.x;
-  const int64_t chunk = (n + T - 1) / T;
-  const int64_t b = threadIdx.x * chunk, e = min(n, b + chunk);
-  __shared__ int shmax[1024], shmin[1024];
   int mx = -1, mn = 1 << 30;
-  for (int64_t i = b; i < e; ++i) mx = max(mx, R[i].jmax);
-  for (int64_t i = b; i < e; ++i) mn = min(mn, R[i].jmin);
-  shmax[threadIdx.x] = mx;
-  shmin[threadIdx.x] = mn;
-  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kF4Blk / kF4BlkThreads; ++q) {
+    const int64_t i = base + threadIdx.x + q * kF4BlkThreads;
+    if (i < n) {
+      mx = max(mx, R[i].jmax);
+      mn = min(mn, R[i].jmin);
+    }
+  }
+  mx = block_max(mx, sh);
+  mn = -block_max(-mn, sh);
   if (threadIdx.x == 0) {
-    int run = -1;
-    for (int t = 0; t < T; ++t) {
-      int v = shmax[t];
-      shmax[t] = run;  // exclusive prefix max
-      run = max(run, v);
-    }
-    run = 1 << 30;
-    for (int t = T - 1; t >= 0; --t) {
-      int v = shmin[t];
-      shmin[t] = run;  // exclusive suffix min
-      run = min(run, v);
-    }
+    aggmax[(int64_t)layer * nblk + blockIdx.x] = mx;
+    aggmin[(int64_t)layer * nblk + blockIdx.x] = mn;
   }
+}
+
+__global__ void __launch_bounds__(kF4BlkThreads)
+    k_f4_bounds(const F4Rec* __restrict__ rec, int64_t rstride, const int64_t* __restrict__ nrec, int layer0, int nblk,
+                const int* __restrict__ aggmax, const int* __restrict__ aggmin, int* __restrict__ pmax,
+                int* __restrict__ smin) {
+  constexpr int kPer = kF4Blk / kF4BlkThreads, kWarps = kF4BlkThreads / 32;
+  __shared__ int sh[kWarps], wmax[kWarps], wmin[kWarps];
+  __shared__ int jmx[kF4Blk], jmn[kF4Blk];
+  const int layer = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t n = nrec[layer + layer0], base = (int64_t)blockIdx.x * kF4Blk;
+  if (base >= n) return;
+  const F4Rec* R = rec + (int64_t)layer * rstride;
+  const int nb = (int)((n + kF4Blk - 1) / kF4Blk);
+  int cm = -1, cn = 1 << 30;  // carries: blocks before, blocks after
+  for (int b = tid; b < nb; b += kF4BlkThreads) {
+    if (b < (int)blockIdx.x) cm = max(cm, aggmax[(int64_t)layer * nblk + b]);
+    if (b > (int)blockIdx.x) cn = min(cn, aggmin[(int64_t)layer * nblk + b]);
+  }
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const int k = tid + q * kF4BlkThreads;
+    const int64_t i = base + k;
+    jmx[k] = i < n ? R[i].jmax : -1;
+    jmn[k] = i < n ? R[i].jmin : 1 << 30;
+  }
+  cm = block_max(cm, sh);
+  cn = -block_max(-cn, sh);  // (its barriers also close the staging)
+  // thread t: records t*kPer .. of the block; inclusive within the thread,
+  // then over the warp's and the block's threads
+  int x[kPer], y[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) x[q] = max(jmx[tid * kPer + q], q ? x[q > 0 ? q - 1 : 0] : -1);
+#pragma unroll
+  for (int q = kPer - 1; q >= 0; --q) y[q] = min(jmn[tid * kPer + q], q < kPer - 1 ? y[q < kPer - 1 ? q + 1 : q] : 1 << 30);
+  int tx = x[kPer - 1], ty = y[0];
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, tx, o), d = __shfl_down_sync(0xffffffffu, ty, o);
+    if (lane >= o) tx = max(tx, u);
+    if (lane + o < 32) ty = min(ty, d);
+  }
+  if (lane == 31) wmax[warp] = tx;
+  if (lane == 0) wmin[warp] = ty;
   __syncthreads();
-  int run = shmax[threadIdx.x];
-  for (int64_t i = b; i < e; ++i) {
-    run = max(run, R[i].jmax);
-    pm[i] = run;
+  int ex = __shfl_up_sync(0xffffffffu, tx, 1), ey = __shfl_down_sync(0xffffffffu, ty, 1);
+  if (lane == 0) ex = -1;
+  if (lane == 31) ey = 1 << 30;
+  ex = max(ex, cm);
+  ey = min(ey, cn);
+  for (int w = 0; w < kWarps; ++w) {
+    if (w < warp) ex = max(ex, wmax[w]);
+    if (w > warp) ey = min(ey, wmin[w]);
   }
-  run = shmin[threadIdx.x];
-  for (int64_t i = e - 1; i >= b; --i) {
-    run = min(run, R[i].jmin);
-    sm[i] = run;
-  }
+  const int64_t o = (int64_t)layer * rstride + base + tid * kPer;
+#pragma unroll
+  for (int q = 0; q < kPer; ++q)
+    if (base + tid * kPer + q < n) {
+      pmax[o + q] = max(x[q], ex);
+      smin[o + q] = min(y[q], ey);
+    }
 }
 
 // Per (layer, grid): running max of g_hi from the left and running min of

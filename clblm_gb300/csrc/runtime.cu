@@ -121,6 +121,8 @@ struct clblm_handle {
   DevBuf jprof, jod, jmap, jjobs, jblk;  // Jacobians: profiles, block ODs, maps, jobs, grid blocks
   DevBuf jvjp;                          // vector-Jacobian product: CTA partial sums and the totals
   DevBuf f4blk, f4ntot, f4cidx, f4vb, f4lb, f4src, f4flag, f4cut, f4grp, f4nxt, ragg;
+  DevBuf f4agg;                    // bounds of the far-wing records, per kF4Blk records
+  DevBuf f4tab, f4calls, f4ncall;  // SHRINQ calls: counts of the possible ones, the list, its length
   DevBuf segpool;  // radiation-term segments of panels with more than kMaxSeg
   DevBuf rt[4], outbuf, imap[2];
   DevBuf rtseg;                  // layer tables of the radiance runs (RtSegLayer)
@@ -140,7 +142,8 @@ struct clblm_handle {
                               &bm0,       &bfac,     &f4blk,     &f4ntot,  &f4cidx,  &f4vb,   &f4lb,    &f4src,
                               &f4flag,    &f4cut,    &f4grp,     &f4nxt,   &ragg,    &segpool, &gpm,    &gsm,
                               &reclo,     &jprof,    &jod,       &jmap,    &jjobs,   &jblk,    &jvjp,   &isotab,
-                              &linecpl,   &f4cpl,    &f4cpll,    &f4ncpl,   &pwork};
+                              &linecpl,   &f4cpl,    &f4cpll,    &f4ncpl,   &pwork,
+                              &f4tab,     &f4calls,  &f4ncall,  &f4agg};
     for (auto& b : rt) v.push_back(&b);
     for (auto& b : imap) v.push_back(&b);
     v.push_back(&rtseg);
@@ -921,7 +924,8 @@ size_t od_job_bytes(const LayerPlan& P, bool plain) {
   const size_t per_line = sizeof(LinePrep) + sizeof(int) + 3 * (sizeof(GridRec) + sizeof(GridRecLo) + 2 * sizeof(int)) +
                           (plain ? 3 * sizeof(GridRecD) : 0);
   const size_t per_f4 = sizeof(F4Prep) + sizeof(ShrunkLine) + 4 * sizeof(int64_t) + 1 + sizeof(int) + sizeof(int4) +
-                        sizeof(F4Rec) + 2 * sizeof(int) + (plain ? sizeof(F4RecD) : 0);
+                        sizeof(F4Rec) + 2 * sizeof(int) + (plain ? sizeof(F4RecD) : 0) +
+                        (sizeof(unsigned) * kCallEnds + sizeof(int4) + 249) / 250;
   const size_t real = plain ? 8 : 4;
   return (size_t)(P.line_hi - P.line_lo + 1) * per_line + (size_t)(P.f4_hi - P.f4_lo) * per_f4 +
          (size_t)(P.nsamp * P.nslice + P.nptr4) * real;
@@ -989,6 +993,9 @@ int tune_pick(clblm_handle* h, cudaStream_t st, int n, int def, F launch, int* s
   return CLBLM_OK;
 }
 
+// 250-line records that a layer's far-wing range of at most f4stride lines meets
+int64_t f4_records(int64_t f4stride) { return f4stride / 250 + 2; }
+
 // Runs the OD pipeline for `count` layers whose plans are already uploaded at
 // plans[first..]; OD of layer k lands at od + P.od_off (Real).
 int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int count, bool plain, int64_t lstride,
@@ -1037,20 +1044,26 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     k_f4_next<<<dim3((unsigned)std::min<int64_t>((f4stride + 255) / 256, 4096), count), 256, 0, st>>>(
         h->f4vb.as<long long>(), h->f4lb.as<long long>(), h->f4ntot.as<int64_t>(), f4stride, h->f4nxt.as<int>());
     h->launches++;
-    // one CTA per layer: with at most one per SM each walk is latency-bound and
-    // loads the whole next call ahead; with more, occupancy counts and it loads two lines per thread
-    if (count <= h->nsm)
-      k_f4_walk<5><<<count, 256, 0, st>>>(dplans, first, count, h->nlines, f4stride, h->f4cidx.as<int64_t>(),
-                                         h->f4vb.as<long long>(), h->f4lb.as<long long>(), h->f4nxt.as<int>(),
-                                         h->f4flag.as<unsigned char>(), h->f4ntot.as<int64_t>(),
-                                         h->f4cut.as<int64_t>(), h->f4grp.as<int4>(), h->f4nout.as<int64_t>());
-    else
-      k_f4_walk<2><<<count, 256, 0, st>>>(dplans, first, count, h->nlines, f4stride, h->f4cidx.as<int64_t>(),
-                                         h->f4vb.as<long long>(), h->f4lb.as<long long>(), h->f4nxt.as<int>(),
-                                         h->f4flag.as<unsigned char>(), h->f4ntot.as<int64_t>(),
-                                         h->f4cut.as<int64_t>(), h->f4grp.as<int4>(), h->f4nout.as<int64_t>());
+    const int64_t trec = f4_records(f4stride);
+    k_f4_calls<<<dim3((unsigned)((trec + kCallStarts - 1) / kCallStarts), count), 256, 0, st>>>(
+        dplans, first, f4stride, h->f4cidx.as<int64_t>(), h->f4vb.as<long long>(), h->f4lb.as<long long>(),
+        h->f4nxt.as<int>(), h->f4flag.as<unsigned char>(), h->f4ntot.as<int64_t>(), trec, h->f4tab.as<unsigned>());
     h->launches++;
-    k_f4_groupsum<<<dim3((unsigned)std::min<int64_t>((f4stride + 255) / 256, 4096), count), kGroupSumThreads, 0, st>>>(
+    k_f4_walk<<<count, 256, 0, st>>>(dplans, first, count, h->nlines, f4stride, h->f4cidx.as<int64_t>(),
+                                     h->f4vb.as<long long>(), h->f4lb.as<long long>(), h->f4nxt.as<int>(),
+                                     h->f4flag.as<unsigned char>(), h->f4ntot.as<int64_t>(), h->f4cut.as<int64_t>(),
+                                     trec, h->f4tab.as<unsigned>(), h->f4calls.as<int4>(), h->f4ncall.as<int2>(),
+                                     h->f4nout.as<int64_t>());
+    h->launches++;
+    // (a call takes 250 lines or more but for the last: a CTA for each)
+    k_f4_groups<<<dim3((unsigned)std::min<int64_t>(trec + 1, 2048), count), 256, 0, st>>>(
+        first, f4stride, h->f4vb.as<long long>(), h->f4lb.as<long long>(), h->f4nxt.as<int>(),
+        h->f4flag.as<unsigned char>(), trec, h->f4calls.as<int4>(), h->f4ncall.as<int2>(), h->f4grp.as<int4>(),
+        h->f4nout.as<int64_t>());
+    h->launches++;
+    // (about 16 CTAs per SM in all: a group is little work for a CTA's start)
+    const int64_t gsum = std::max<int64_t>((int64_t)16 * h->nsm / count, 1);
+    k_f4_groupsum<<<dim3((unsigned)std::min<int64_t>((f4stride + 255) / 256, gsum), count), kGroupSumThreads, 0, st>>>(
         dplans, first, h->f4prep.as<F4Prep>(), f4stride, h->f4src.as<int64_t>(), h->f4grp.as<int4>(),
         h->f4nout.as<int64_t>(), h->f4sh.as<ShrunkLine>());
   }
@@ -1074,9 +1087,17 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
                                                    h->has_cpl ? h->f4cpl.as<double>() : nullptr);
     }
   }
-  h->launches++;
-  k_f4_bounds<<<count, 1024, 0, st>>>(h->f4rec.as<F4Rec>(), rstride, h->f4nrec.as<int64_t>(), first,
-                                      h->f4pm.as<int>(), h->f4sm.as<int>());
+  {
+    const int nblk = (int)((f4stride + kF4Blk - 1) / kF4Blk);
+    int* amax = h->f4agg.as<int>();
+    int* amin = amax + (int64_t)count * nblk;
+    h->launches += 2;
+    k_f4_agg<<<dim3(nblk, count), kF4BlkThreads, 0, st>>>(h->f4rec.as<F4Rec>(), rstride, h->f4nrec.as<int64_t>(),
+                                                          first, nblk, amax, amin);
+    k_f4_bounds<<<dim3(nblk, count), kF4BlkThreads, 0, st>>>(h->f4rec.as<F4Rec>(), rstride, h->f4nrec.as<int64_t>(),
+                                                             first, nblk, amax, amin, h->f4pm.as<int>(),
+                                                             h->f4sm.as<int>());
+  }
   {
     int64_t maxr4 = 0;
     for (int k = 0; k < count; ++k) maxr4 = std::max(maxr4, hps[first + k].P.nptr4);
@@ -1267,6 +1288,8 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
 struct WsDims {
   int64_t lsc = 0;     // line stride x layers
   int64_t fsc = 0;     // far-wing line stride x layers
+  int64_t frecc = 0;   // far-wing records x layers
+  int64_t f4aggc = 0;  // blocks of far-wing pseudo-lines x layers
   int64_t psc = 0;     // panels x layers
   int64_t cnt = 0;     // layers
   int64_t odt = 0;     // OD points (padded)
@@ -1278,6 +1301,8 @@ struct WsDims {
   void max_with(const WsDims& o) {
     lsc = std::max(lsc, o.lsc);
     fsc = std::max(fsc, o.fsc);
+    frecc = std::max(frecc, o.frecc);
+    f4aggc = std::max(f4aggc, o.f4aggc);
     psc = std::max(psc, o.psc);
     cnt = std::max(cnt, o.cnt);
     odt = std::max(odt, o.odt);
@@ -1316,6 +1341,8 @@ WsDims batch_dims(std::vector<HostPlan>& hps, int first, int count, int64_t* lst
   WsDims d;
   d.lsc = ls * count;
   d.fsc = fs * count;
+  d.frecc = f4_records(fs) * count;
+  d.f4aggc = (fs + kF4Blk - 1) / kF4Blk * count;
   d.psc = ps * count;
   d.cnt = count;
   d.odt = odt;
@@ -1378,6 +1405,10 @@ cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int
   WS_ENSURE(h->f4nxt.ensure(sizeof(int) * d.fsc));
   WS_ENSURE(h->f4cut.ensure(sizeof(int64_t) * d.cnt));
   WS_ENSURE(h->f4grp.ensure(sizeof(int4) * d.fsc));
+  WS_ENSURE(h->f4tab.ensure(sizeof(unsigned) * kCallEnds * d.frecc));
+  WS_ENSURE(h->f4calls.ensure(sizeof(int4) * (d.frecc + 2 * d.cnt)));
+  WS_ENSURE(h->f4ncall.ensure(sizeof(int2) * d.cnt));
+  WS_ENSURE(h->f4agg.ensure(sizeof(int) * 2 * d.f4aggc));
   WS_ENSURE(h->f4rec.ensure(sizeof(F4Rec) * (d.fsc + 4096 * d.cnt)));
   WS_ENSURE(h->f4recd.ensure(plain ? sizeof(F4RecD) * (d.fsc + 4096 * d.cnt) : 256));
   WS_ENSURE(h->f4nrec.ensure(sizeof(int64_t) * nL));
@@ -1404,7 +1435,7 @@ std::vector<DevBuf*> ws_buffers(clblm_handle* h) {
           &h->f4vb,   &h->f4lb,   &h->f4src,  &h->f4flag,   &h->f4nxt,  &h->f4cut,  &h->f4grp,  &h->f4rec,
           &h->f4recd, &h->f4nrec, &h->f4nmir, &h->f4pm,     &h->f4sm,   &h->err,    &h->segpool, &h->pblk,
           &h->bv1,    &h->bn,     &h->bm0,    &h->bfac,   &h->isotab, &h->linecpl, &h->f4cpl, &h->f4cpll,
-          &h->f4ncpl, &h->pwork};
+          &h->f4ncpl, &h->pwork,  &h->f4tab,  &h->f4calls,  &h->f4ncall, &h->f4agg};
 }
 
 // Frees every work buffer of the handle (all but the line list, the shape
