@@ -21,6 +21,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 UNITS = {
     "prep.cu": ["--fmad=false"],
     "panel.cu": [],
+    "f4far.cu": [],
     "rt.cu": [],
     "jac.cu": [],
     "scan.cu": [],

@@ -131,10 +131,17 @@ constexpr int kCallStarts = 12;  // records that calls start at, per CTA of k_f4
 __global__ void k_f4_calls(const LayerPlan* plans, int layer0, int64_t stride, const int64_t* cidx,
                            const long long* vbits, const long long* lbits, const int* gnxt,
                            const unsigned char* flags, const int64_t* ntot, int64_t tab_records, unsigned* tab);
-__global__ void k_f4_walk(const LayerPlan* plans, int layer0, int nlayers, int64_t nlines_total, int64_t stride,
-                          const int64_t* cidx, const long long* vbits, const long long* lbits, const int* gnxt,
-                          const unsigned char* flags, const int64_t* ntot, const int64_t* cut, int64_t tab_records,
-                          const unsigned* tab, int4* calls, int2* ncalls, int64_t* ngroups);
+constexpr int kWalkThreads = 256;
+// (declared with the definition's qualifiers, as k_line_prep)
+template <bool Table>
+__global__ void __launch_bounds__(kWalkThreads)
+    k_f4_walk(const LayerPlan* __restrict__ plans, int layer0, int nlayers, int64_t nlines_total, int64_t stride,
+              const int64_t* __restrict__ cidx, const long long* __restrict__ vbits,
+              const long long* __restrict__ lbits, const int* __restrict__ gnxt,
+              const unsigned char* __restrict__ flags, const int64_t* __restrict__ ntot,
+              const int64_t* __restrict__ cut, int64_t tab_records, const unsigned* __restrict__ tab,
+              int4* __restrict__ calls, int2* __restrict__ ncalls, int4* __restrict__ groups,
+              int64_t* __restrict__ ngroups);
 __global__ void k_f4_groups(int layer0, int64_t stride, const long long* vbits, const long long* lbits,
                             const int* gnxt, const unsigned char* flags, int64_t tab_records, const int4* calls,
                             const int2* ncalls, int4* groups, int64_t* ngroups);
@@ -165,10 +172,16 @@ __global__ void k_rec_bounds(const LayerPlan* plans, int layer0, const GridRec* 
                              const int* aggmax, const int* aggmin, int nagg, int* pmax, int* smin);
 // running bounds of the far-wing records, in blocks of kF4Blk records
 constexpr int kF4Blk = 1024, kF4BlkThreads = 256;
+template <int Kind>
 __global__ void __launch_bounds__(kF4BlkThreads)
-    k_f4_agg(const F4Rec* rec, int64_t rstride, const int64_t* nrec, int layer0, int nblk, int* aggmax, int* aggmin);
+    k_f4_agg(const LayerPlan* __restrict__ plans, const F4Rec* __restrict__ rec, const F4RecD* __restrict__ recd,
+             int64_t rstride, const int64_t* __restrict__ nrec, int layer0, int nblk, int* __restrict__ aggmax,
+             int* __restrict__ aggmin, int* __restrict__ core);
+template <int Kind>
 __global__ void __launch_bounds__(kF4BlkThreads)
-    k_f4_bounds(const F4Rec* rec, int64_t rstride, const int64_t* nrec, int layer0, int nblk, const int* aggmax,
-                const int* aggmin, int* pmax, int* smin);
+    k_f4_bounds(const LayerPlan* __restrict__ plans, const F4Rec* __restrict__ rec, const F4RecD* __restrict__ recd,
+                int64_t rstride, const int64_t* __restrict__ nrec, int layer0, int nblk,
+                const int* __restrict__ aggmax, const int* __restrict__ aggmin, int* __restrict__ pmax,
+                int* __restrict__ smin);
 
 }  // namespace clblm

@@ -73,6 +73,7 @@ constexpr int kF4Tile = 256;     // R4 points per CTA of k_f4_conv
 constexpr int kF4Pts = 4;        // points per thread: a record read from shared memory serves four
 constexpr int kF4Threads = kF4Tile / kF4Pts;
 constexpr int kF4Group = 32;     // records per FP32 partial sum of the mixed path
+constexpr int kFarTile = 128, kFarThreads = 128;  // points and threads of a CTA of k_f4_far
 // records per shared-memory stage of k_f4_conv: the variants the autotuner
 // times (64, 128, 256)
 
@@ -84,8 +85,9 @@ struct F4Args {
   const F4Rec* rec;
   const F4RecD* recd;
   int64_t stride;
-  const int* pmax_jmax;     // running max of jmax
-  const int* smin_jmin;     // running min (from the right) of jmin
+  const int* pmax_jmax;     // running max of jmax (k_f4_far: of the centres)
+  const int* smin_jmin;     // running min (from the right) of jmin (of the centres)
+  const int* core;          // k_f4_far: points that no line's core reaches past, per layer
   void* r4_all;
   int* err;                 // bit 2: a shared-memory stage never arrived
   const double* cpl;        // DPTRAT of each record (line coupling; 0: uncoupled)
@@ -109,7 +111,12 @@ constexpr int kPanelLines = 1, kPanelWings = 2;
 // their dispersion term); without it the line sums stay as lean as before
 template <bool Plain, int Part, bool Cpl>
 __global__ void k_panel(const __grid_constant__ PanelArgs a);
-template <bool Plain, int CHUNK>
+// the far wings: distant records through nodes (k_f4_far), or every record at
+// every point in the order of the reference's sum (k_f4_conv: the ODs of the mixed path's
+// Jacobians)
+template <bool Plain>
+__global__ void k_f4_far(const __grid_constant__ F4Args a);
+template <int CHUNK>
 __global__ void k_f4_conv(F4Args a);
 // RSYM of the first panel of every layer whose panel origin is at or below
 // 0 cm-1, as a correction of the OD the panel kernel wrote (one CTA per layer

@@ -10,10 +10,11 @@
 //                    launches: the line sums (kPanelLines) beside the far-wing
 //                    chain, a CTA per slice of a panel's records, then R4,
 //                    the continuum and the radiation term (kPanelWings).
-//   k_f4_conv<Plain> far-wing function 4 on the DVR4 grid (CNVF4Q,
-//                    clblm_ODLAY_LineF4.f90:187-494): two points per thread
-//                    (packed FP32x2 in the mixed path), records streamed
-//                    through shared memory by bulk copies.
+//   k_f4_conv        far-wing function 4 on the DVR4 grid (CNVF4Q,
+//                    clblm_ODLAY_LineF4.f90:187-494) record by record, for the
+//                    ODs of the mixed path's Jacobians: packed FP32x2, records
+//                    streamed through shared memory by bulk copies (the
+//                    others: k_f4_far, f4far.cu).
 //   k_rsym<Plain>    RSYM's fold about 0 cm-1 of the first panel of a window
 //                    starting within 32 DV of zero (clblm_ODLAY.f90:3020-3085),
 //                    applied as a binary64 correction after k_panel.
@@ -1253,12 +1254,16 @@ template __global__ void k_rsym<true>(const __grid_constant__ PanelArgs);
 // range streams through shared memory in chunks of CHUNK records, one bulk
 // copy per chunk into two alternating stages; every thread then evaluates all
 // records of the chunk at its kF4Pts points (m0 + t + i kF4Threads), each
-// record's fields loaded once for all of them.  The FP64 path adds the terms in
-// the reference's order (record order); the mixed path sums groups of
-// kF4Group records (two packed partial sums over alternate records) and adds
-// each group's total into a Kahan sum.  Groups start at the tile's first
+// record's fields loaded once for all of them.  Groups of
+// kF4Group records are summed (two packed partial sums over alternate records)
+// and each group's total added into a Kahan sum.  Groups start at the tile's first
 // record, so the records per stage (CHUNK, a multiple of kF4Group, chosen by
 // the autotuner) do not change the result.
+//
+// Only the ODs of the mixed path's Jacobians come through here: they are
+// differenced (T + 1 K, Wtot * 1.01), which amplifies the last bits of a sum
+// formed another way by some thousands; k_f4_far, with a quarter of the
+// evaluations, serves every other call.
 
 // FP32 terms of far-wing record r at a thread's two points (packed FP32x2):
 // Core: the point may lie within 64 ALFV of the line (the polynomial core of
@@ -1313,12 +1318,11 @@ __device__ __forceinline__ void f4_chunk(const F4Rec* S, int cnt, float2 JmAB, f
   *tCD = __fadd2_rn(q0, q1);
 }
 
-template <bool Plain, int CHUNK>
-__global__ void __launch_bounds__(kF4Threads, Plain ? 1 : 16) k_f4_conv(F4Args a) {
+template <int CHUNK>
+__global__ void __launch_bounds__(kF4Threads, 16) k_f4_conv(F4Args a) {
   static_assert(kF4Pts == 4, "the thread's points are the pairs AB and CD");
   static_assert(CHUNK % kF4Group == 0, "groups of the FP32 sums lie within a chunk");
-  using Real = typename std::conditional<Plain, double, float>::type;
-  using Rec = typename std::conditional<Plain, F4RecD, F4Rec>::type;
+  using Rec = F4Rec;
   __shared__ __align__(128) Rec stage[2][CHUNK];
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ int64_t rng[3];
@@ -1330,11 +1334,10 @@ __global__ void __launch_bounds__(kF4Threads, Plain ? 1 : 16) k_f4_conv(F4Args a
   // the thread's four points: m0 + t + i kF4Threads, i = 0..3
   const int64_t mA = m0 + threadIdx.x, mB = mA + kF4Threads, mC = mB + kF4Threads, mD = mC + kF4Threads;
   const int JA = (int)mA + 1, JB = (int)mB + 1, JC = (int)mC + 1, JD = (int)mD + 1;
-  Real* R4 = reinterpret_cast<Real*>(a.r4_all) + P.r4_off;
+  float* R4 = reinterpret_cast<float*>(a.r4_all) + P.r4_off;
   const int64_t n = a.nrec[layer + a.layer0];
   const int64_t nm = a.nmirror[layer + a.layer0];
-  const Rec* recs = reinterpret_cast<const Rec*>(Plain ? (const void*)a.recd : (const void*)a.rec) +
-                    (int64_t)layer * a.stride;
+  const Rec* recs = a.rec + (int64_t)layer * a.stride;
 
   if (threadIdx.x == 0) {
     const int* pm = a.pmax_jmax + (int64_t)layer * a.stride;
@@ -1389,22 +1392,8 @@ __global__ void __launch_bounds__(kF4Threads, Plain ? 1 : 16) k_f4_conv(F4Args a
   const float2 JmCD = make_float2((float)(JC - 1), (float)(JD - 1));
   const float dvr4f = (float)P.dvr4;
   const float2 dvr4 = make_float2(dvr4f, dvr4f);
-  const double ZSQBND = 64. * 64.;
-  const double A3 = (1. + 2. * ZSQBND) / ((1. + ZSQBND) * (1. + ZSQBND));
-  const double B3 = -1. / ((1. + ZSQBND) * (1. + ZSQBND));
-  const double bnd2 = P.bound4 * P.bound4;
-  double acc[kF4Pts] = {0., 0., 0., 0.};  // FP64 path
-  KahanF kacc[kF4Pts];                     // mixed path: chunk totals
+  KahanF kacc[kF4Pts];  // group totals
   bool failed = false;
-  // FP64 term of record d at point m, in the reference's operations
-  auto term_d = [&](const F4RecD& d, int64_t m) -> double {
-    double XM = (double)m * P.dvr4 - d.xnui;
-    double XMSQ = XM * XM;
-    double ZVSQ = XMSQ / d.alv2;
-    double fb = d.co2 ? (2. - XMSQ / bnd2) * d.fbnd : d.fbnd;
-    if (ZVSQ <= ZSQBND) return (d.siv * A3 + ZVSQ * (d.siv * B3)) - fb;
-    return d.sil / (d.al2 + XMSQ) - fb;
-  };
   const int tJlo = (int)m0 + 1;
   const int tJhi = (int)(m0 + kF4Tile < P.nptr4 ? m0 + kF4Tile : P.nptr4);
   for (int64_t c = 0; c < nchunk; ++c) {
@@ -1422,19 +1411,7 @@ __global__ void __launch_bounds__(kF4Threads, Plain ? 1 : 16) k_f4_conv(F4Args a
     }
     const Rec* S = stage[c & 1];
     const int cnt = (int)count_of(c);
-    if (liveA) {
-      if constexpr (Plain) {
-        for (int k = 0; k < cnt; ++k) {
-          const F4RecD& d = S[k];
-#pragma unroll
-          for (int q = 0; q < kF4Pts; ++q) {
-            const int J = (int)ms[q] + 1;
-            if (ms[q] < P.nptr4 && J >= d.jmin && J <= d.jmax) acc[q] += term_d(d, ms[q]);
-          }
-        }
-      }
-    }
-    if constexpr (!Plain) {
+    {
       // A chunk whose records all span the tile's live points needs no range
       // test.  One whose records all keep the tile beyond 64.064 ALFV (the
       // tile's offsets from each line are monotone in J, so its end points
@@ -1482,8 +1459,7 @@ __global__ void __launch_bounds__(kF4Threads, Plain ? 1 : 16) k_f4_conv(F4Args a
   for (int q = 0; q < kF4Pts; ++q) {
     const int64_t m = ms[q];
     if (m >= P.nptr4 + 2) continue;
-    if constexpr (Plain) R4[m] = m < P.nptr4 ? acc[q] : 0.;
-    else R4[m] = m < P.nptr4 ? kacc[q].value() : 0.f;
+    R4[m] = m < P.nptr4 ? kacc[q].value() : 0.f;
   }
 }
 
@@ -1585,11 +1561,8 @@ __global__ void k_f4_cpl(const F4Args a, const int64_t* list, const int64_t* nli
 template __global__ void k_f4_cpl<false>(const F4Args, const int64_t*, const int64_t*);
 template __global__ void k_f4_cpl<true>(const F4Args, const int64_t*, const int64_t*);
 
-template __global__ void k_f4_conv<false, 64>(F4Args);
-template __global__ void k_f4_conv<false, 128>(F4Args);
-template __global__ void k_f4_conv<false, 256>(F4Args);
-template __global__ void k_f4_conv<true, 64>(F4Args);
-template __global__ void k_f4_conv<true, 128>(F4Args);
-template __global__ void k_f4_conv<true, 256>(F4Args);
+template __global__ void k_f4_conv<64>(F4Args);
+template __global__ void k_f4_conv<128>(F4Args);
+template __global__ void k_f4_conv<256>(F4Args);
 
 }  // namespace clblm

@@ -1457,7 +1457,6 @@ __global__ void k_f4_next(const long long* __restrict__ vbits, const long long* 
 // DVR4/2).  A group emits a non-CO2 line when one of its members has a
 // non-CO2 line with SP >= 1e-35, a CO2 line likewise, and each of its coupled
 // lines.
-constexpr int kWalkThreads = 256;
 constexpr int kWalkMax = 1280;  // lines of one SHRINQ call: < 1000 + one 250-line record
 constexpr int kWalkPer = kWalkMax / kWalkThreads;
 constexpr int kLift = 11;       // 2^11 > kWalkMax
@@ -1717,18 +1716,31 @@ __device__ void shrink_call(CallShared& W, int64_t u0, int m, const long long* _
   __syncthreads();  // the shared arrays are reused by the next call
 }
 
-// LINF4Q's record loop of one layer: the list of its SHRINQ calls (first and
+// LINF4Q's record loop of one layer.
+// Table: the list of its SHRINQ calls (first and
 // end line of the stream, first output slot, first group) from k_f4_calls'
 // table, whose rows are staged a window of records at a time.  A call of
 // more records than the table holds is counted by the CTA.  The last call (at the end of
 // the stream) may end inside a record: its counts are k_f4_groups'.
+// Without: the CTA shrinks the calls one after another.  With more layers in
+// the launch than SMs the chains run side by side, and the table's work, which
+// visits every line from each start that reaches it, costs more than it saves
+// (240 layers of 17,000 lines: 159 us against 187 for the three kernels).
+#define CLBLM_WALK_ARGS                                                                                       \
+  const LayerPlan* __restrict__, int, int, int64_t, int64_t, const int64_t* __restrict__,                     \
+      const long long* __restrict__, const long long* __restrict__, const int* __restrict__,                  \
+      const unsigned char* __restrict__, const int64_t* __restrict__, const int64_t* __restrict__, int64_t,   \
+      const unsigned* __restrict__, int4* __restrict__, int2* __restrict__, int4* __restrict__,               \
+      int64_t* __restrict__
+template <bool Table>
 __global__ void __launch_bounds__(kWalkThreads)
     k_f4_walk(const LayerPlan* __restrict__ plans, int layer0, int nlayers, int64_t nlines_total, int64_t stride,
               const int64_t* __restrict__ cidx, const long long* __restrict__ vbits,
               const long long* __restrict__ lbits, const int* __restrict__ gnxt,
               const unsigned char* __restrict__ flags, const int64_t* __restrict__ ntot,
               const int64_t* __restrict__ cut, int64_t tab_records, const unsigned* __restrict__ tab,
-              int4* __restrict__ calls, int2* __restrict__ ncalls, int64_t* __restrict__ ngroups) {
+              int4* __restrict__ calls, int2* __restrict__ ncalls, int4* __restrict__ groups,
+              int64_t* __restrict__ ngroups) {
   union Sh {
     unsigned tab[kRecWin][kCallEnds];
     CallShared call;
@@ -1768,7 +1780,7 @@ __global__ void __launch_bounds__(kWalkThreads)
     __syncthreads();
     for (int k = tid; k <= kRecWin; k += kWalkThreads) civ[k] = rec_offset(ci, wbase + k, P.f4_lo, n);
     const int64_t row0 = wbase - rec_first;
-    for (int k = tid; k < kRecWin * kCallEnds; k += kWalkThreads) {
+    for (int k = tid; Table && k < kRecWin * kCallEnds; k += kWalkThreads) {
       const int64_t row = row0 + k / kCallEnds;
       (&sh.tab[0][0])[k] = row < tab_records ? T[row * kCallEnds + k % kCallEnds] : 0u;
     }
@@ -1777,7 +1789,7 @@ __global__ void __launch_bounds__(kWalkThreads)
   for (;;) {  // every thread runs the (uniform) record loop
     // Calls whose records lie inside the staged window and before the end of
     // the stream, in 32-bit arithmetic: they are nearly all of them
-    if (rec == rs && rec >= wbase && rec < wbase + kRecWin && IJ == ILO - 1) {
+    if (Table && rec == rs && rec >= wbase && rec < wbase + kRecWin && IJ == ILO - 1) {
       // records up to which the window, the prepared range and the stream allow it
       const int64_t safe = min(min(wbase + kRecWin, nrec_total), (n + P.f4_lo) / R);
       const int rmax = (int)(safe - wbase);  // civ[r] for r <= rmax
@@ -1845,14 +1857,19 @@ __global__ void __launch_bounds__(kWalkThreads)
     }
     int64_t nemit = 0;
     if (m > 0) {
-      if (tid == 0) C[nc] = make_int4((int)u0, (int)u1, (int)slot, (int)ng);
-      nc++;
-      if (IEOF) {
-        last = true;
-        break;
-      }
       int gcount, emitted;
-      if (rec - rs <= kCallEnds && rs >= wbase) {
+      if constexpr (Table) {
+        if (tid == 0) C[nc] = make_int4((int)u0, (int)u1, (int)slot, (int)ng);
+        nc++;
+        if (IEOF) {
+          last = true;
+          break;
+        }
+      }
+      if constexpr (!Table) {
+        shrink_call(sh.call, u0, m, V, Lm, GN, F, (int)slot, groups + (int64_t)layer * stride + ng, stride - ng, &gcount,
+                    &emitted);
+      } else if (rec - rs <= kCallEnds && rs >= wbase) {
         const unsigned v = sh.tab[rs - wbase][rec - rs - 1];
         emitted = (int)(v & 0xFFFFu);
         gcount = (int)(v >> 16);
@@ -1876,11 +1893,15 @@ __global__ void __launch_bounds__(kWalkThreads)
     if (IEOF) break;
   }
   if (tid == 0) {
-    ncalls[layer] = make_int2((int)nc, last && !status ? 1 : 0);
+    if (Table) ncalls[layer] = make_int2((int)nc, last && !status ? 1 : 0);
     ngroups[2 * (layer + layer0)] = status ? -status : ng;
     ngroups[2 * (layer + layer0) + 1] = slot;
   }
 }
+
+template __global__ void k_f4_walk<false>(CLBLM_WALK_ARGS);
+template __global__ void k_f4_walk<true>(CLBLM_WALK_ARGS);
+#undef CLBLM_WALK_ARGS
 
 // The groups of the calls of every layer's list; the layer's totals when its
 // last call ended the stream.
@@ -2142,9 +2163,6 @@ __device__ void f4_record(const LayerPlan& P, const ShrunkLine& L, double VNUI, 
     const float spp = VNUI == L.vnu ? L.w.f[3] : -L.w.f[3];
     *dpt = spp != 0.f ? (double)(spp / (SP * ALFAVI)) : 0.;
   } else {
-    const int mc = (int)floor(XNUI / P.dvr4 + 0.5);
-    r->nmc = pair(-(double)mc);
-    r->x0 = pair((double)mc * P.dvr4 - XNUI);
     const double BNDSQ = P.bound4 * P.bound4;
     const double ALFALI = L.w.d[0], ALFADI = L.w.d[1];
     const double ZETAI = ALFALI / (ALFALI + ALFADI);
@@ -2157,13 +2175,6 @@ __device__ void f4_record(const LayerPlan& P, const ShrunkLine& L, double VNUI, 
     const double ALFLI2 = ALFALI * ALFALI;
     const double ALFVI2 = ALFAVI * ALFAVI;
     const double F4BND = SIL / (ALFLI2 + BNDSQ);
-    r->sil = pair(SIL);
-    r->al2 = pair(ALFLI2);
-    r->ralv2 = pair(1. / ALFVI2);
-    r->sa3 = pair(SIV * A3);
-    r->sb3 = pair(SIV * B3);
-    r->nfb0 = pair(co2 ? -2. * F4BND : -F4BND);
-    r->fb2 = pair(co2 ? F4BND / BNDSQ : 0.);
     d->jmin = JMIN;
     d->jmax = JMAX;
     d->co2 = co2;
@@ -2207,8 +2218,8 @@ __global__ void __launch_bounds__(kSetupThreads, 3)
       r.jmax = d.jmax = -1;
     }
     if (r.jmax >= r.jmin) steps += (unsigned long long)(r.jmax - r.jmin + 1);
-    R[i] = r;
-    if (!P.mixed) D[i] = d;
+    if (P.mixed) R[i] = r;
+    else D[i] = d;
   }
   for (int o = 16; o > 0; o >>= 1) steps += __shfl_down_sync(0xffffffffu, steps, o);
   if ((threadIdx.x & 31) == 0 && steps) atomicAdd(&stats[(layer + layer0) * kStatsPerLayer + 6], steps);
@@ -2275,8 +2286,8 @@ __global__ void __launch_bounds__(kSetupThreads)
     }
     const int64_t slot = n + nm + before + __popc(bal & ((1u << lane) - 1u));
     if (ok && slot < rstride) {
-      R[slot] = r;
-      if (!P.mixed) D[slot] = d;
+      if (P.mixed) R[slot] = r;
+      else D[slot] = d;
       if (cpl) cpl[(int64_t)layer * rstride + slot] = dpt;
       steps += (unsigned long long)(r.jmax - r.jmin + 1);
     }
@@ -2305,21 +2316,51 @@ __device__ __forceinline__ int block_max(int v, int* sh) {
   return v;
 }
 
+#define CLBLM_F4_AGG_ARGS                                                                                      \
+  const LayerPlan* __restrict__, const F4Rec* __restrict__, const F4RecD* __restrict__, int64_t,               \
+      const int64_t* __restrict__, int, int, int* __restrict__, int* __restrict__, int* __restrict__
+#define CLBLM_F4_BOUNDS_ARGS                                                                                   \
+  const LayerPlan* __restrict__, const F4Rec* __restrict__, const F4RecD* __restrict__, int64_t,               \
+      const int64_t* __restrict__, int, int, const int* __restrict__, const int* __restrict__,                 \
+      int* __restrict__, int* __restrict__
+
+// What is bounded (Kind): 0 the records' point ranges JMAX and JMIN (mixed
+// records); 1, 2 their centres, the grid point nearest the line, of the mixed
+// and FP64 records (k_f4_far's searches).  With centres also the points that
+// no line's core (64 ALFV, a little more) reaches past.
+template <int Kind>
+__device__ __forceinline__ int2 f4_extent(const F4Rec* __restrict__ R, const F4RecD* __restrict__ D, double rdvr4,
+                                          int64_t i) {
+  if constexpr (Kind == 0) return make_int2(R[i].jmax, R[i].jmin);
+  int m;
+  if constexpr (Kind == 1) m = -(int)R[i].nmc.x;
+  else m = (int)floor(D[i].xnui * rdvr4 + 0.5);
+  return make_int2(m, m);
+}
+
+template <int Kind>
 __global__ void __launch_bounds__(kF4BlkThreads)
-    k_f4_agg(const F4Rec* __restrict__ rec, int64_t rstride, const int64_t* __restrict__ nrec, int layer0, int nblk,
-             int* __restrict__ aggmax, int* __restrict__ aggmin) {
+    k_f4_agg(const LayerPlan* __restrict__ plans, const F4Rec* __restrict__ rec, const F4RecD* __restrict__ recd,
+             int64_t rstride, const int64_t* __restrict__ nrec, int layer0, int nblk, int* __restrict__ aggmax,
+             int* __restrict__ aggmin, int* __restrict__ core) {
   __shared__ int sh[kF4BlkThreads / 32];
   const int layer = blockIdx.y;
   const int64_t n = nrec[layer + layer0], base = (int64_t)blockIdx.x * kF4Blk;
   if (base >= n) return;
   const F4Rec* R = rec + (int64_t)layer * rstride;
-  int mx = -1, mn = 1 << 30;
+  const F4RecD* D = recd + (int64_t)layer * rstride;
+  const double rdvr4 = plans[layer + layer0].rdvr4;
+  int mx = -(1 << 30), mn = 1 << 30;
+  float wide = 0.f;  // largest ALFV
 #pragma unroll
   for (int q = 0; q < kF4Blk / kF4BlkThreads; ++q) {
     const int64_t i = base + threadIdx.x + q * kF4BlkThreads;
     if (i < n) {
-      mx = max(mx, R[i].jmax);
-      mn = min(mn, R[i].jmin);
+      const int2 e = f4_extent<Kind>(R, D, rdvr4, i);
+      mx = max(mx, e.x);
+      mn = min(mn, e.y);
+      if constexpr (Kind == 1) wide = fmaxf(wide, rsqrtf(R[i].ralv2.x));
+      else if constexpr (Kind == 2) wide = fmaxf(wide, sqrtf((float)D[i].alv2));
     }
   }
   mx = block_max(mx, sh);
@@ -2328,10 +2369,20 @@ __global__ void __launch_bounds__(kF4BlkThreads)
     aggmax[(int64_t)layer * nblk + blockIdx.x] = mx;
     aggmin[(int64_t)layer * nblk + blockIdx.x] = mn;
   }
+  if constexpr (Kind != 0) {
+    const float reach = ceilf(64.064f * wide * (float)rdvr4) + 2.f;
+    const int c = block_max(reach < 1.e6f ? (int)reach : 1000000, sh);
+    if (threadIdx.x == 0) atomicMax(&core[layer + layer0], c);
+  }
 }
+template __global__ void k_f4_agg<0>(CLBLM_F4_AGG_ARGS);
+template __global__ void k_f4_agg<1>(CLBLM_F4_AGG_ARGS);
+template __global__ void k_f4_agg<2>(CLBLM_F4_AGG_ARGS);
 
+template <int Kind>
 __global__ void __launch_bounds__(kF4BlkThreads)
-    k_f4_bounds(const F4Rec* __restrict__ rec, int64_t rstride, const int64_t* __restrict__ nrec, int layer0, int nblk,
+    k_f4_bounds(const LayerPlan* __restrict__ plans, const F4Rec* __restrict__ rec, const F4RecD* __restrict__ recd,
+                int64_t rstride, const int64_t* __restrict__ nrec, int layer0, int nblk,
                 const int* __restrict__ aggmax, const int* __restrict__ aggmin, int* __restrict__ pmax,
                 int* __restrict__ smin) {
   constexpr int kPer = kF4Blk / kF4BlkThreads, kWarps = kF4BlkThreads / 32;
@@ -2341,8 +2392,10 @@ __global__ void __launch_bounds__(kF4BlkThreads)
   const int64_t n = nrec[layer + layer0], base = (int64_t)blockIdx.x * kF4Blk;
   if (base >= n) return;
   const F4Rec* R = rec + (int64_t)layer * rstride;
+  const F4RecD* D = recd + (int64_t)layer * rstride;
+  const double rdvr4 = plans[layer + layer0].rdvr4;
   const int nb = (int)((n + kF4Blk - 1) / kF4Blk);
-  int cm = -1, cn = 1 << 30;  // carries: blocks before, blocks after
+  int cm = -(1 << 30), cn = 1 << 30;  // carries: blocks before, blocks after
   for (int b = tid; b < nb; b += kF4BlkThreads) {
     if (b < (int)blockIdx.x) cm = max(cm, aggmax[(int64_t)layer * nblk + b]);
     if (b > (int)blockIdx.x) cn = min(cn, aggmin[(int64_t)layer * nblk + b]);
@@ -2351,8 +2404,9 @@ __global__ void __launch_bounds__(kF4BlkThreads)
   for (int q = 0; q < kPer; ++q) {
     const int k = tid + q * kF4BlkThreads;
     const int64_t i = base + k;
-    jmx[k] = i < n ? R[i].jmax : -1;
-    jmn[k] = i < n ? R[i].jmin : 1 << 30;
+    const int2 e = i < n ? f4_extent<Kind>(R, D, rdvr4, i) : make_int2(-(1 << 30), 1 << 30);
+    jmx[k] = e.x;
+    jmn[k] = e.y;
   }
   cm = block_max(cm, sh);
   cn = -block_max(-cn, sh);  // (its barriers also close the staging)
@@ -2360,7 +2414,7 @@ __global__ void __launch_bounds__(kF4BlkThreads)
   // then over the warp's and the block's threads
   int x[kPer], y[kPer];
 #pragma unroll
-  for (int q = 0; q < kPer; ++q) x[q] = max(jmx[tid * kPer + q], q ? x[q > 0 ? q - 1 : 0] : -1);
+  for (int q = 0; q < kPer; ++q) x[q] = max(jmx[tid * kPer + q], q ? x[q > 0 ? q - 1 : 0] : -(1 << 30));
 #pragma unroll
   for (int q = kPer - 1; q >= 0; --q) y[q] = min(jmn[tid * kPer + q], q < kPer - 1 ? y[q < kPer - 1 ? q + 1 : q] : 1 << 30);
   int tx = x[kPer - 1], ty = y[0];
@@ -2373,7 +2427,7 @@ __global__ void __launch_bounds__(kF4BlkThreads)
   if (lane == 0) wmin[warp] = ty;
   __syncthreads();
   int ex = __shfl_up_sync(0xffffffffu, tx, 1), ey = __shfl_down_sync(0xffffffffu, ty, 1);
-  if (lane == 0) ex = -1;
+  if (lane == 0) ex = -(1 << 30);
   if (lane == 31) ey = 1 << 30;
   ex = max(ex, cm);
   ey = min(ey, cn);
@@ -2389,6 +2443,11 @@ __global__ void __launch_bounds__(kF4BlkThreads)
       smin[o + q] = min(y[q], ey);
     }
 }
+template __global__ void k_f4_bounds<0>(CLBLM_F4_BOUNDS_ARGS);
+template __global__ void k_f4_bounds<1>(CLBLM_F4_BOUNDS_ARGS);
+template __global__ void k_f4_bounds<2>(CLBLM_F4_BOUNDS_ARGS);
+#undef CLBLM_F4_AGG_ARGS
+#undef CLBLM_F4_BOUNDS_ARGS
 
 // Per (layer, grid): running max of g_hi from the left and running min of
 // g_lo from the right over the convolution records, so that the records that

@@ -121,6 +121,7 @@ struct clblm_handle {
   DevBuf jprof, jod, jmap, jjobs, jblk;  // Jacobians: profiles, block ODs, maps, jobs, grid blocks
   DevBuf jvjp;                          // vector-Jacobian product: CTA partial sums and the totals
   DevBuf f4blk, f4ntot, f4cidx, f4vb, f4lb, f4src, f4flag, f4cut, f4grp, f4nxt, ragg;
+  DevBuf f4core;                   // points that no far-wing line's core reaches past, per layer
   DevBuf f4agg;                    // bounds of the far-wing records, per kF4Blk records
   DevBuf f4tab, f4calls, f4ncall;  // SHRINQ calls: counts of the possible ones, the list, its length
   DevBuf segpool;  // radiation-term segments of panels with more than kMaxSeg
@@ -143,7 +144,7 @@ struct clblm_handle {
                               &f4flag,    &f4cut,    &f4grp,     &f4nxt,   &ragg,    &segpool, &gpm,    &gsm,
                               &reclo,     &jprof,    &jod,       &jmap,    &jjobs,   &jblk,    &jvjp,   &isotab,
                               &linecpl,   &f4cpl,    &f4cpll,    &f4ncpl,   &pwork,
-                              &f4tab,     &f4calls,  &f4ncall,  &f4agg};
+                              &f4tab,     &f4calls,  &f4ncall,  &f4agg,     &f4core};
     for (auto& b : rt) v.push_back(&b);
     for (auto& b : imap) v.push_back(&b);
     v.push_back(&rtseg);
@@ -998,8 +999,9 @@ int64_t f4_records(int64_t f4stride) { return f4stride / 250 + 2; }
 
 // Runs the OD pipeline for `count` layers whose plans are already uploaded at
 // plans[first..]; OD of layer k lands at od + P.od_off (Real).
-int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int count, bool plain, int64_t lstride,
-                 int64_t f4stride, int64_t pstride) {
+// jac: the ODs of a Jacobian call (the mixed path keeps the order of their far-wing sums).
+int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int count, bool plain, bool jac,
+                 int64_t lstride, int64_t f4stride, int64_t pstride) {
   const LayerPlan* dplans = h->plans.as<const LayerPlan>();
   LineIn li = line_in(h);
   h->last_plain = plain;
@@ -1043,23 +1045,29 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     h->launches++;
     k_f4_next<<<dim3((unsigned)std::min<int64_t>((f4stride + 255) / 256, 4096), count), 256, 0, st>>>(
         h->f4vb.as<long long>(), h->f4lb.as<long long>(), h->f4ntot.as<int64_t>(), f4stride, h->f4nxt.as<int>());
-    h->launches++;
     const int64_t trec = f4_records(f4stride);
-    k_f4_calls<<<dim3((unsigned)((trec + kCallStarts - 1) / kCallStarts), count), 256, 0, st>>>(
-        dplans, first, f4stride, h->f4cidx.as<int64_t>(), h->f4vb.as<long long>(), h->f4lb.as<long long>(),
-        h->f4nxt.as<int>(), h->f4flag.as<unsigned char>(), h->f4ntot.as<int64_t>(), trec, h->f4tab.as<unsigned>());
-    h->launches++;
-    k_f4_walk<<<count, 256, 0, st>>>(dplans, first, count, h->nlines, f4stride, h->f4cidx.as<int64_t>(),
-                                     h->f4vb.as<long long>(), h->f4lb.as<long long>(), h->f4nxt.as<int>(),
-                                     h->f4flag.as<unsigned char>(), h->f4ntot.as<int64_t>(), h->f4cut.as<int64_t>(),
-                                     trec, h->f4tab.as<unsigned>(), h->f4calls.as<int4>(), h->f4ncall.as<int2>(),
-                                     h->f4nout.as<int64_t>());
-    h->launches++;
-    // (a call takes 250 lines or more but for the last: a CTA for each)
-    k_f4_groups<<<dim3((unsigned)std::min<int64_t>(trec + 1, 2048), count), 256, 0, st>>>(
-        first, f4stride, h->f4vb.as<long long>(), h->f4lb.as<long long>(), h->f4nxt.as<int>(),
-        h->f4flag.as<unsigned char>(), trec, h->f4calls.as<int4>(), h->f4ncall.as<int2>(), h->f4grp.as<int4>(),
-        h->f4nout.as<int64_t>());
+    auto walk = [&](auto* f) {
+      h->launches++;
+      f<<<count, kWalkThreads, 0, st>>>(dplans, first, count, h->nlines, f4stride, h->f4cidx.as<int64_t>(),
+                                        h->f4vb.as<long long>(), h->f4lb.as<long long>(), h->f4nxt.as<int>(),
+                                        h->f4flag.as<unsigned char>(), h->f4ntot.as<int64_t>(),
+                                        h->f4cut.as<int64_t>(), trec, h->f4tab.as<unsigned>(), h->f4calls.as<int4>(),
+                                        h->f4ncall.as<int2>(), h->f4grp.as<int4>(), h->f4nout.as<int64_t>());
+    };
+    if (count > h->nsm) {
+      walk(k_f4_walk<false>);
+    } else {
+      h->launches += 2;
+      k_f4_calls<<<dim3((unsigned)((trec + kCallStarts - 1) / kCallStarts), count), kWalkThreads, 0, st>>>(
+          dplans, first, f4stride, h->f4cidx.as<int64_t>(), h->f4vb.as<long long>(), h->f4lb.as<long long>(),
+          h->f4nxt.as<int>(), h->f4flag.as<unsigned char>(), h->f4ntot.as<int64_t>(), trec, h->f4tab.as<unsigned>());
+      walk(k_f4_walk<true>);
+      // (a call takes 250 lines or more but for the last: a CTA for each)
+      k_f4_groups<<<dim3((unsigned)std::min<int64_t>(trec + 1, 2048), count), kWalkThreads, 0, st>>>(
+          first, f4stride, h->f4vb.as<long long>(), h->f4lb.as<long long>(), h->f4nxt.as<int>(),
+          h->f4flag.as<unsigned char>(), trec, h->f4calls.as<int4>(), h->f4ncall.as<int2>(), h->f4grp.as<int4>(),
+          h->f4nout.as<int64_t>());
+    }
     h->launches++;
     // (about 16 CTAs per SM in all: a group is little work for a CTA's start)
     const int64_t gsum = std::max<int64_t>((int64_t)16 * h->nsm / count, 1);
@@ -1068,6 +1076,7 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
         h->f4nout.as<int64_t>(), h->f4sh.as<ShrunkLine>());
   }
   int64_t rstride = f4stride + 4096;
+  const bool far_nodes = plain || !jac;
   h->launches++;
   k_f4_lineinit<<<dim3((unsigned)std::min<int64_t>((f4stride + 255) / 256, 4096), count), blk, 0, st>>>(
       dplans, first, h->f4sh.as<ShrunkLine>(), f4stride, h->f4nout.as<int64_t>(), h->f4rec.as<F4Rec>(),
@@ -1092,11 +1101,21 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     int* amax = h->f4agg.as<int>();
     int* amin = amax + (int64_t)count * nblk;
     h->launches += 2;
-    k_f4_agg<<<dim3(nblk, count), kF4BlkThreads, 0, st>>>(h->f4rec.as<F4Rec>(), rstride, h->f4nrec.as<int64_t>(),
-                                                          first, nblk, amax, amin);
-    k_f4_bounds<<<dim3(nblk, count), kF4BlkThreads, 0, st>>>(h->f4rec.as<F4Rec>(), rstride, h->f4nrec.as<int64_t>(),
-                                                             first, nblk, amax, amin, h->f4pm.as<int>(),
-                                                             h->f4sm.as<int>());
+    const dim3 gb(nblk, count);
+    auto bounds = [&](auto* agg, auto* bnd) {
+      agg<<<gb, kF4BlkThreads, 0, st>>>(dplans, h->f4rec.as<F4Rec>(), h->f4recd.as<F4RecD>(), rstride,
+                                        h->f4nrec.as<int64_t>(), first, nblk, amax, amin, h->f4core.as<int>());
+      bnd<<<gb, kF4BlkThreads, 0, st>>>(dplans, h->f4rec.as<F4Rec>(), h->f4recd.as<F4RecD>(), rstride,
+                                        h->f4nrec.as<int64_t>(), first, nblk, amax, amin, h->f4pm.as<int>(),
+                                        h->f4sm.as<int>());
+    };
+    if (far_nodes) {
+      CUDA_TRY(h, cudaMemsetAsync(h->f4core.as<int>() + first, 0, sizeof(int) * count, st));
+      if (plain) bounds(k_f4_agg<2>, k_f4_bounds<2>);
+      else bounds(k_f4_agg<1>, k_f4_bounds<1>);
+    } else {
+      bounds(k_f4_agg<0>, k_f4_bounds<0>);
+    }
   }
   {
     int64_t maxr4 = 0;
@@ -1114,26 +1133,29 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     fa.r4_all = h->r4.p;
     fa.err = h->err.as<int>();
     fa.cpl = h->f4cpl.as<const double>();
-    dim3 grid((unsigned)((maxr4 + 2 + kF4Tile - 1) / kF4Tile), count);
-    auto f4 = [&](int v) {  // records per stage: 64, 128, 256
-      if (plain) {
-        if (v == 0) k_f4_conv<true, 64><<<grid, kF4Threads, 0, st>>>(fa);
-        else if (v == 1) k_f4_conv<true, 128><<<grid, kF4Threads, 0, st>>>(fa);
-        else k_f4_conv<true, 256><<<grid, kF4Threads, 0, st>>>(fa);
-      } else {
-        if (v == 0) k_f4_conv<false, 64><<<grid, kF4Threads, 0, st>>>(fa);
-        else if (v == 1) k_f4_conv<false, 128><<<grid, kF4Threads, 0, st>>>(fa);
-        else k_f4_conv<false, 256><<<grid, kF4Threads, 0, st>>>(fa);
+    fa.core = h->f4core.as<int>();
+    if (far_nodes) {
+      const dim3 grid((unsigned)((maxr4 + 2 + kFarTile - 1) / kFarTile), count);
+      h->launches++;
+      CUDA_TRY(h, cudaEventRecord(h->ev[0], st));
+      if (plain) k_f4_far<true><<<grid, kFarThreads, 0, st>>>(fa);
+      else k_f4_far<false><<<grid, kFarThreads, 0, st>>>(fa);
+    } else {
+      const dim3 grid((unsigned)((maxr4 + 2 + kF4Tile - 1) / kF4Tile), count);
+      auto f4 = [&](int v) {  // records per stage: 64, 128, 256
+        if (v == 0) k_f4_conv<64><<<grid, kF4Threads, 0, st>>>(fa);
+        else if (v == 1) k_f4_conv<128><<<grid, kF4Threads, 0, st>>>(fa);
+        else k_f4_conv<256><<<grid, kF4Threads, 0, st>>>(fa);
+      };
+      int tv = h->tune.f4[0];
+      if (tv < 0) {
+        int rc = tune_pick(h, st, 3, 2, f4, &h->tune.f4[0], &tv);
+        if (rc) return rc;
       }
-    };
-    int tv = h->tune.f4[plain ? 1 : 0];
-    if (tv < 0) {
-      int rc = tune_pick(h, st, 3, 2, f4, &h->tune.f4[plain ? 1 : 0], &tv);
-      if (rc) return rc;
+      h->launches++;
+      CUDA_TRY(h, cudaEventRecord(h->ev[0], st));
+      f4(tv);
     }
-    h->launches++;
-    CUDA_TRY(h, cudaEventRecord(h->ev[0], st));
-    f4(tv);
     if (h->has_cpl) {  // the coupled records' dispersion terms
       h->launches += 2;
       k_f4_cpl_list<<<count, 1024, 0, st>>>(fa, h->f4cpll.as<int64_t>(), h->f4ncpl.as<int64_t>());
@@ -1409,6 +1431,7 @@ cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int
   WS_ENSURE(h->f4calls.ensure(sizeof(int4) * (d.frecc + 2 * d.cnt)));
   WS_ENSURE(h->f4ncall.ensure(sizeof(int2) * d.cnt));
   WS_ENSURE(h->f4agg.ensure(sizeof(int) * 2 * d.f4aggc));
+  WS_ENSURE(h->f4core.ensure(sizeof(int) * nL));
   WS_ENSURE(h->f4rec.ensure(sizeof(F4Rec) * (d.fsc + 4096 * d.cnt)));
   WS_ENSURE(h->f4recd.ensure(plain ? sizeof(F4RecD) * (d.fsc + 4096 * d.cnt) : 256));
   WS_ENSURE(h->f4nrec.ensure(sizeof(int64_t) * nL));
@@ -1435,7 +1458,7 @@ std::vector<DevBuf*> ws_buffers(clblm_handle* h) {
           &h->f4vb,   &h->f4lb,   &h->f4src,  &h->f4flag,   &h->f4nxt,  &h->f4cut,  &h->f4grp,  &h->f4rec,
           &h->f4recd, &h->f4nrec, &h->f4nmir, &h->f4pm,     &h->f4sm,   &h->err,    &h->segpool, &h->pblk,
           &h->bv1,    &h->bn,     &h->bm0,    &h->bfac,   &h->isotab, &h->linecpl, &h->f4cpl, &h->f4cpll,
-          &h->f4ncpl, &h->pwork,  &h->f4tab,  &h->f4calls,  &h->f4ncall, &h->f4agg};
+          &h->f4ncpl, &h->pwork,  &h->f4tab,  &h->f4calls,  &h->f4ncall, &h->f4agg, &h->f4core};
 }
 
 // Frees every work buffer of the handle (all but the line list, the shape
@@ -1898,7 +1921,7 @@ int clblm_gpu_od(clblm_handle_t* h, const clblm_layer_t* layer, const clblm_grid
   int64_t ls, fs, ps, odt;
   rc = prepare_batch(h, hps, 0, 1, plain, &ls, &fs, &ps, &odt);
   if (rc) return rc;
-  rc = run_od_batch(h, hps, 0, 1, plain, ls, fs, ps);
+  rc = run_od_batch(h, hps, 0, 1, plain, false, ls, fs, ps);
   if (rc) return rc;
   const LayerPlan& P = hps[0].P;
   int64_t n = hps[0].n_out;
@@ -1993,7 +2016,8 @@ int clblm_gpu_od_stats(const clblm_handle_t* h, clblm_od_stats_t* stats) {
   if (!h || !stats) return CLBLM_ERR_ARG;
   *stats = h->last;
   const int p = h->last_plain ? 1 : 0;
-  stats->f4_stage_records = h->tune.f4[p] >= 0 ? kF4StageRecords[h->tune.f4[p]] : 0;
+  // (a call without k_f4_conv leaves the choice open: its default shape)
+  stats->f4_stage_records = h->tune.f4[p] >= 0 ? kF4StageRecords[h->tune.f4[p]] : (h->last.launches > 0 ? kF4StageRecords[2] : 0);
   stats->rt_threads = h->tune.rt[p] >= 0 ? kRtThreads[h->tune.rt[p]] : 0;
   stats->jac_threads = h->tune.jac[p] >= 0 ? kJacThreads[h->tune.jac[p]] : 0;
   return CLBLM_OK;
@@ -2156,7 +2180,7 @@ int clblm_gpu_rt_mode2(clblm_handle_t* h, const clblm_column_t* col, const clblm
     int64_t ls, fs, ps, odt;
     rc = prepare_batch(h, rp.hps, first, count, plain, &ls, &fs, &ps, &odt);
     if (rc) return rc;
-    rc = run_od_batch(h, rp.hps, first, count, plain, ls, fs, ps);
+    rc = run_od_batch(h, rp.hps, first, count, plain, false, ls, fs, ps);
     if (rc) return rc;
     CUDA_TRY(h, cudaEventRecord(h->ev[6], h->stream));
     // the layer tables of this batch: each layer's grid, its map onto the
@@ -2840,7 +2864,7 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
       int64_t ls, fs, ps, odt;
       rc = prepare_batch(h, hps, first, count, plain, &ls, &fs, &ps, &odt);
       if (rc) return rc;
-      rc = run_od_batch(h, hps, first, count, plain, ls, fs, ps);
+      rc = run_od_batch(h, hps, first, count, plain, true, ls, fs, ps);
       if (rc) return rc;
       rc = check_batch(h, hps, first, count, &h->last);
       if (rc) return rc;
@@ -3295,7 +3319,7 @@ int batch_enqueue(clblm_handle* h, BatchPlan& bp, const clblm_profile_t* prof, c
   double* stage = h->outbuf.as<double>();
   int unit_done = 0;
   for (const BChunk& c : bp.chunks) {
-    int rc = run_od_batch(h, bp.hps, c.first, c.count, plain, c.ls, c.fs, c.ps);
+    int rc = run_od_batch(h, bp.hps, c.first, c.count, plain, true, c.ls, c.fs, c.ps);
     if (rc) return rc;
     JacJob* jobs = h->jjobs.as<JacJob>() + c.first;
     const int64_t nmax = c.nmax;
