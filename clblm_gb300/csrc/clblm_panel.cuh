@@ -38,6 +38,10 @@ struct PanelArgs {
   const int* pmax_g;         // per grid: running max of g_hi over the records
   const int* smin_g;         // per grid: running min (from the right) of g_lo
   int* err;
+  // radiation-term segments of each panel (k_panel_segs)
+  const int* seg_n;
+  const int* seg_start;
+  const double2* seg_v;
   // radiation-term segments of panels with more than kMaxSeg of them (low
   // wavenumbers at coarse DV): slots of kSegSlot entries claimed by atomics
   int* seg_next;             // next free slot
@@ -100,8 +104,13 @@ template <bool Plain>
 __global__ void k_f4_cpl(const F4Args a, const int64_t* list, const int64_t* nlist);
 
 size_t panel_smem_bytes(bool plain, bool wings = false);  // wings: the mixed far-wing pass
-__global__ void k_r4_radfac(const LayerPlan* plans, int layer0, const double* blk_v1, const int* blk_n,
-                            double* blk_fac);
+constexpr int kRadfacWarps = 4;
+__global__ void __launch_bounds__(32 * kRadfacWarps)
+    k_r4_radfac(const LayerPlan* plans, int layer0, const double* blk_v1, const int* blk_n, double* blk_fac);
+constexpr int kSegTab = 24;  // radiation-term segments of a panel held by k_panel_segs
+__global__ void __launch_bounds__(64)
+    k_panel_segs(const LayerPlan* plans, int layer0, const double* vft_all, int64_t stride, int* seg_n, int* seg_start,
+                 double2* seg_v);
 
 // the passes of k_panel: the line sums (kPanelLines), then the far wings, the
 // continuum and the radiation term (kPanelWings)

@@ -251,11 +251,15 @@ __device__ __forceinline__ void xint_weights_f(float P, float w[4]) {
 
 // JRAD = 1: LBLF4Q multiplies each R4 block by the piecewise-linear
 // radiation term RADFNI started at the block origin
-// (clblm_ODLAY_LineF4.f90:142-177); one thread per block.
-__global__ void k_r4_radfac(const LayerPlan* __restrict__ plans, int layer0, const double* __restrict__ blk_v1,
-                            const int* __restrict__ blk_n, double* __restrict__ blk_fac) {
+// (clblm_ODLAY_LineF4.f90:142-177).  A warp per block: the lanes step through
+// the segments together and fill one's points side by side, RADVI + k RDEL
+// where the reference adds RDEL again and again (2500 dependent additions by
+// one thread took 310 us for a layer of 40,000 points).
+__global__ void __launch_bounds__(32 * kRadfacWarps)
+    k_r4_radfac(const LayerPlan* __restrict__ plans, int layer0, const double* __restrict__ blk_v1,
+                const int* __restrict__ blk_n, double* __restrict__ blk_fac) {
   const LayerPlan& P = plans[blockIdx.y + layer0];
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
+  const int b = blockIdx.x * kRadfacWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (b >= P.nblk4 || P.jrad != 1) return;
   const double V1R4 = blk_v1[P.blk_off + b];
   const int NPTR4 = blk_n[P.blk_off + b];
@@ -271,12 +275,47 @@ __global__ void k_r4_radfac(const LayerPlan* __restrict__ plans, int layer0, con
     double RADVI = radfni_d(VI, P.dvr4, XKT, &VITST, &RDEL, &RDLAST);
     N2 = (int)((VITST - V1R4) / P.dvr4 + 0.001);
     if (N2 > NPTR4) N2 = NPTR4;
-    double t = RADVI;
-    for (int I = N1; I <= N2; ++I) {
-      fac[I - 1] = t;
-      t = t + RDEL;
-    }
+    for (int I = N1 + lane; I <= N2; I += 32) fac[I - 1] = fma((double)(I - N1), RDEL, RADVI);
   } while (N2 < NPTR4);
+}
+
+// The radiation-term segments of every panel (panelOut, JRAD = 0: RADFNI from
+// the panel's first output point), a thread per panel: their number at
+// seg_n[layer * stride + panel] (-1: more than kSegTab, the far-wing pass
+// forms them itself), first points, values and slopes.  A segment is a chain of
+// exponentials and divisions in binary64 (about 3 us); formed by one lane of
+// the far-wing pass's CTA, those of a surface panel took two thirds of its 88 us.
+__global__ void __launch_bounds__(64)
+    k_panel_segs(const LayerPlan* __restrict__ plans, int layer0, const double* __restrict__ vft_all, int64_t stride,
+                 int* __restrict__ seg_n, int* __restrict__ seg_start, double2* __restrict__ seg_v) {
+  const LayerPlan& P = plans[blockIdx.y + layer0];
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= P.npanels || P.jrad != 0) return;
+  const int64_t k = (int64_t)blockIdx.y * stride + p;
+  const double dv = P.dv, VFT = vft_all[P.vft_off + p];
+  const int NHI = p == P.npanels - 1 ? P.nhi_last : (kNLIM1 + kNSHIFT - 1);
+  const int NLO = kNSHIFT + 1;
+  const double XKT = P.tave / kRADCN2;
+  const double V1P = VFT + (double)(NLO - 1) * dv;
+  double VITST = V1P - dv;
+  double RDLAST = -1.;
+  int N2 = NLO - 1, ns = 0;
+  do {
+    const int N1 = N2 + 1;
+    const double VI = VFT + (double)(N1 - 1) * dv;
+    double RDEL;
+    const double RADVI = radfni_d(VI, dv, XKT, &VITST, &RDEL, &RDLAST);
+    N2 = (int)((VITST - VFT) / dv + 0.001);
+    if (N2 > NHI) N2 = NHI;
+    if (ns == kSegTab) {
+      ns = -1;
+      break;
+    }
+    seg_start[k * kSegTab + ns] = N1;
+    seg_v[k * kSegTab + ns] = make_double2(RADVI, RDEL);
+    ns++;
+  } while (N2 < NHI);
+  seg_n[k] = ns;
 }
 
 // Record ranges of the T half tiles [G0 + 16t, G0 + 16t + 15] of one grid
@@ -716,9 +755,35 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
   // ---- R3: line sums on p-frame points 0..160 (new) and 0..7 (old) ----
   // units 0..kTiles3-1: 32 new points each; unit kTiles3: the 8 old points
   static_assert(kTiles3 + 1 < kPanelWarps, "the last warp has no R3 unit");
-  if (kWings && warp == kPanelWarps - 1 && lane == 0) {  // idle in the R3 phase: radiation-term segments (panelOut, JRAD = 0)
-    int ns = 0, slot = -1;
+  static_assert(kSegTab < kMaxSeg, "the tabulated segments fit in shared memory");
+  // radiation-term segments (panelOut, JRAD = 0): k_panel_segs' or, when they
+  // are more than it holds, formed by a lane idle in the R3 phase
+  int nseg = 0;
+  if constexpr (kWings) {
     if (P.jrad == 0) {
+      const int64_t k = (int64_t)layer * a.panel_stride + p;
+      nseg = a.seg_n[k];
+      for (int q = tid; q < nseg; q += kPanelThreads) {
+        S.seg_start[q] = a.seg_start[k * kSegTab + q];
+        const double2 v = a.seg_v[k * kSegTab + q];
+        if constexpr (Plain) {
+          S.seg_v[q] = v.x;
+          S.seg_d[q] = v.y;
+        } else {
+          S.segf_v[q] = (float)v.x;
+          S.segf_d[q] = (float)v.y;
+        }
+      }
+      if (tid == 0 && nseg >= 0) S.seg_start[nseg] = NHI + 1;
+    }
+    if (tid == 0 && nseg >= 0) {
+      S.nseg = nseg;
+      S.seg_slot = -1;
+    }
+  }
+  if (kWings && nseg < 0 && warp == kPanelWarps - 1 && lane == 0) {
+    int ns = 0, slot = -1;
+    {
       const int NLO = kNSHIFT + 1;
       double XKT = P.tave / kRADCN2;
       double V1P = VFT + (double)(NLO - 1) * dv;

@@ -563,45 +563,52 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
 }
 
 // ---- candidate line ranges of each panel on each grid ---------------------
+// first of a[lo, hi) not below x (line centres: positive, so that they order
+// like their bit patterns; a binary64 compare would wait for the FP64 unit)
 __device__ __forceinline__ int64_t lower_bound_d(const double* a, int64_t lo, int64_t hi, double x) {
+  const long long* b = reinterpret_cast<const long long*>(a);
+  const long long y = __double_as_longlong(x);
   while (lo < hi) {
     int64_t mid = (lo + hi) >> 1;
-    if (a[mid] < x) lo = mid + 1;
+    if (b[mid] < y) lo = mid + 1;
     else hi = mid;
   }
   return lo;
 }
 
+// eight threads a panel: a search each for its six bounds, the others its
+// entries in the line pass's list of CTAs
 __global__ void k_panel_ranges(const LayerPlan* __restrict__ plans, int layer0, const double* __restrict__ vnu_raw,
                                const double* __restrict__ alfvmax, double shiftmax, int64_t* __restrict__ ranges,
                                int64_t panel_stride, int2* __restrict__ work) {
   int layer = blockIdx.y;
   const LayerPlan& P = plans[layer + layer0];
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = threadIdx.x & 7;
+  int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   if (p >= P.npanels) return;
-  // the line pass's CTAs of this panel
-  for (int z = 0; z < P.nslice; ++z)
-    work[P.cta0 + (int64_t)p * P.nslice + z] = make_int2(layer * kMaxSlices + z, p);
+  if (k >= 6) {  // the line pass's CTAs of this panel
+    for (int z = k - 6; z < P.nslice; z += 2)
+      work[P.cta0 + (int64_t)p * P.nslice + z] = make_int2(layer * kMaxSlices + z, p);
+    return;
+  }
   double a = alfvmax[layer + layer0];
   double dv = P.dv;
   double s = shiftmax * P.rhorat + 1e-9;
-  // grid 1: output points J = 33..2432 of panel p
-  double r1lo = P.vft0 + (double)(kPanelPts * p + 32) * dv, r1hi = P.vft0 + (double)(kPanelPts * p + 2431) * dv;
-  double reach1 = 4. * a + 3. * dv + s;
-  // grid 2: points J = 5..612 (4 DV)
-  double r2lo = P.vft0 + (double)(kPanelR2 * p + 4) * 4. * dv, r2hi = P.vft0 + (double)(kPanelR2 * p + 611) * 4. * dv;
-  double reach2 = 16. * a + 12. * dv + s;
-  // grid 3: points J = 0..160 (16 DV)
-  double r3lo = P.vft0 + (double)(kPanelR3 * p - 1) * 16. * dv, r3hi = P.vft0 + (double)(kPanelR3 * p + 159) * 16. * dv;
-  double reach3 = 64. * a + 48. * dv + s;
-  int64_t lo = P.line_lo, hi = P.line_hi + 1;
-  int64_t* r = ranges + ((int64_t)layer * panel_stride + p) * 6;
-  r[0] = lower_bound_d(vnu_raw, lo, hi, r1lo - reach1) - P.line_lo;
-  r[1] = lower_bound_d(vnu_raw, lo, hi, r1hi + reach1) - P.line_lo;
-  r[2] = lower_bound_d(vnu_raw, lo, hi, r2lo - reach2) - P.line_lo;
-  r[3] = lower_bound_d(vnu_raw, lo, hi, r2hi + reach2) - P.line_lo;
-  r[4] = lower_bound_d(vnu_raw, lo, hi, r3lo - reach3) - P.line_lo;
-  r[5] = lower_bound_d(vnu_raw, lo, hi, r3hi + reach3) - P.line_lo;
+  double x;
+  if (k < 2) {  // grid 1: output points J = 33..2432 of panel p
+    const double reach = 4. * a + 3. * dv + s;
+    x = k == 0 ? P.vft0 + (double)(kPanelPts * p + 32) * dv - reach : P.vft0 + (double)(kPanelPts * p + 2431) * dv + reach;
+  } else if (k < 4) {  // grid 2: points J = 5..612 (4 DV)
+    const double reach = 16. * a + 12. * dv + s;
+    x = k == 2 ? P.vft0 + (double)(kPanelR2 * p + 4) * 4. * dv - reach
+               : P.vft0 + (double)(kPanelR2 * p + 611) * 4. * dv + reach;
+  } else {  // grid 3: points J = 0..160 (16 DV)
+    const double reach = 64. * a + 48. * dv + s;
+    x = k == 4 ? P.vft0 + (double)(kPanelR3 * p - 1) * 16. * dv - reach
+               : P.vft0 + (double)(kPanelR3 * p + 159) * 16. * dv + reach;
+  }
+  ranges[((int64_t)layer * panel_stride + p) * 6 + k] =
+      lower_bound_d(vnu_raw, P.line_lo, P.line_hi + 1, x) - P.line_lo;
 }
 
 // ---- H2O continuum on the ABSRB grid -----------------------------------------

@@ -117,6 +117,7 @@ struct clblm_handle {
   DevBuf pblk, bv1, bn, bm0, bfac;
   DevBuf gpm, gsm;  // per grid record bounds of the panel kernel
   DevBuf pwork;     // CTAs of the panel kernel's line pass
+  DevBuf psegn, psegs, psegv;  // radiation-term segments of the panels
   DevBuf reclo;     // low parts of the records' ZFL/ZSLOPE
   DevBuf jprof, jod, jmap, jjobs, jblk;  // Jacobians: profiles, block ODs, maps, jobs, grid blocks
   DevBuf jvjp;                          // vector-Jacobian product: CTA partial sums and the totals
@@ -144,7 +145,8 @@ struct clblm_handle {
                               &f4flag,    &f4cut,    &f4grp,     &f4nxt,   &ragg,    &segpool, &gpm,    &gsm,
                               &reclo,     &jprof,    &jod,       &jmap,    &jjobs,   &jblk,    &jvjp,   &isotab,
                               &linecpl,   &f4cpl,    &f4cpll,    &f4ncpl,   &pwork,
-                              &f4tab,     &f4calls,  &f4ncall,  &f4agg,     &f4core};
+                              &f4tab,     &f4calls,  &f4ncall,  &f4agg,     &f4core,  &psegn,
+                              &psegs,     &psegv};
     for (auto& b : rt) v.push_back(&b);
     for (auto& b : imap) v.push_back(&b);
     v.push_back(&rtseg);
@@ -170,8 +172,8 @@ struct clblm_handle {
   cudaEvent_t ev[10] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   // the far-wing chain runs on a second stream, forked from and joined back
   // into `stream` within each OD batch
-  cudaStream_t stream2 = nullptr;
-  cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
+  cudaStream_t stream2 = nullptr, stream3 = nullptr;  // (3: the continuum and the radiation terms)
+  cudaEvent_t fork_ev = nullptr, join_ev = nullptr, join3_ev = nullptr;
   int64_t acc_fnq = 0, acc_f4q = 0;
   double acc_ms_panel = 0., acc_ms_f4 = 0., acc_ms_line_chain = 0., acc_ms_f4_chain = 0., acc_ms_rt = 0.;
   int64_t acc_rt_bytes = 0;
@@ -929,7 +931,8 @@ size_t od_job_bytes(const LayerPlan& P, bool plain) {
                         (sizeof(unsigned) * kCallEnds + sizeof(int4) + 249) / 250;
   const size_t real = plain ? 8 : 4;
   return (size_t)(P.line_hi - P.line_lo + 1) * per_line + (size_t)(P.f4_hi - P.f4_lo) * per_f4 +
-         (size_t)(P.nsamp * P.nslice + P.nptr4) * real;
+         (size_t)(P.nsamp * P.nslice + P.nptr4) * real +
+         (size_t)P.npanels * (kSegTab * (sizeof(int) + sizeof(double2)) + sizeof(int));
 }
 
 // Bytes of OD-pipeline workspace one batch of layers may take: 60 % of the
@@ -1006,14 +1009,34 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
   LineIn li = line_in(h);
   h->last_plain = plain;
   dim3 blk(256);
-  // the continuum and the far-wing chain on the second stream, the line
-  // chain on the handle's stream; k_panel waits for both
+  // the far-wing chain on the second stream, the line chain on the handle's
+  // stream; k_panel's far-wing pass waits for both
   CUDA_TRY(h, cudaEventRecord(h->ev[4], h->stream));
   CUDA_TRY(h, cudaEventRecord(h->fork_ev, h->stream));
   CUDA_TRY(h, cudaStreamWaitEvent(h->stream2, h->fork_ev, 0));
   cudaStream_t st = h->stream2;
-  h->launches++;
-  k_continuum<<<dim3((kNABSRB + 255) / 256, count), blk, 0, st>>>(dplans, first, h->cont, h->absrb.as<double>());
+  {
+    // the continuum, the radiation term of the far-wing blocks and the panels'
+    // radiation segments need the plans alone: a stream of their own, joined
+    // before the far-wing pass of k_panel (50 us, 140 at a window of 1000
+    // cm-1, that the far-wing chain would wait for)
+    cudaStream_t s3 = h->stream3;
+    CUDA_TRY(h, cudaStreamWaitEvent(s3, h->fork_ev, 0));
+    int maxp = 1, maxb = 1;
+    for (int k = 0; k < count; ++k) {
+      maxp = std::max(maxp, hps[first + k].P.npanels);
+      maxb = std::max(maxb, hps[first + k].P.nblk4);
+    }
+    h->launches += 3;
+    k_continuum<<<dim3((kNABSRB + 255) / 256, count), blk, 0, s3>>>(dplans, first, h->cont, h->absrb.as<double>());
+    k_r4_radfac<<<dim3((maxb + kRadfacWarps - 1) / kRadfacWarps, count), 32 * kRadfacWarps, 0, s3>>>(
+        dplans, first, h->bv1.as<double>(), h->bn.as<int>(), h->bfac.as<double>());
+    k_panel_segs<<<dim3((maxp + 63) / 64, count), 64, 0, s3>>>(dplans, first, h->vft.as<double>(), pstride,
+                                                             h->psegn.as<int>(), h->psegs.as<int>(),
+                                                             h->psegv.as<double2>());
+    CUDA_TRY(h, cudaGetLastError());
+    CUDA_TRY(h, cudaEventRecord(h->join3_ev, s3));
+  }
   // far wings
   h->launches++;
   {
@@ -1210,7 +1233,7 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     ctas += (int64_t)hps[first + k].P.npanels * hps[first + k].P.nslice;
   }
   h->launches++;
-  k_panel_ranges<<<dim3((maxp + 127) / 128, count), 128, 0, st>>>(dplans, first, h->vkey.as<double>(),
+  k_panel_ranges<<<dim3((maxp + 15) / 16, count), 128, 0, st>>>(dplans, first, h->vkey.as<double>(),
                                                                    h->alfvmax.as<double>(), h->shiftmax,
                                                                    h->ranges.as<int64_t>(), pstride,
                                                                    h->pwork.as<int2>());
@@ -1251,13 +1274,9 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     pa.seg_pool_d = reinterpret_cast<double*>(b + 256 + start_b + val_b);
     CUDA_TRY(h, cudaMemsetAsync(pa.seg_next, 0, sizeof(int), st));
   }
-  {
-    int maxb = 1;
-    for (int k = 0; k < count; ++k) maxb = std::max(maxb, hps[first + k].P.nblk4);
-    h->launches++;
-    k_r4_radfac<<<dim3((maxb + 63) / 64, count), 64, 0, st>>>(dplans, first, h->bv1.as<double>(), h->bn.as<int>(),
-                                                            h->bfac.as<double>());
-  }
+  pa.seg_n = h->psegn.as<int>();
+  pa.seg_start = h->psegs.as<int>();
+  pa.seg_v = h->psegv.as<double2>();
   CUDA_TRY(h, cudaEventRecord(h->ev[5], st));
   // the line sums run beside the far-wing chain, then, once R4 and ABSRB are
   // ready, a second pass adds the far wings and the continuum through XINT and
@@ -1288,7 +1307,8 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     else k_panel<false, kPanelLines, false><<<(unsigned)ctas, kPanelThreads, smem, st>>>(pa);
   }
   CUDA_TRY(h, cudaEventRecord(h->ev[3], st));
-  CUDA_TRY(h, cudaStreamWaitEvent(st, h->join_ev, 0));  // R4 and ABSRB are ready
+  CUDA_TRY(h, cudaStreamWaitEvent(st, h->join_ev, 0));   // R4 is ready
+  CUDA_TRY(h, cudaStreamWaitEvent(st, h->join3_ev, 0));  // ABSRB and the radiation terms
   CUDA_TRY(h, cudaEventRecord(h->ev[8], st));
   // without the shape tables: six CTAs of the mixed far-wing pass share an SM
   if (plain) k_panel<true, kPanelWings, false><<<dim3(maxp, count), kPanelThreads, smem_w, st>>>(pa);
@@ -1408,6 +1428,9 @@ cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int
   WS_ENSURE(h->ranges.ensure(sizeof(int64_t) * 6 * d.psc));
   WS_ENSURE(h->od.ensure(real * d.odt));
   WS_ENSURE(h->pwork.ensure(sizeof(int2) * (size_t)d.ctas));
+  WS_ENSURE(h->psegn.ensure(sizeof(int) * d.psc));
+  WS_ENSURE(h->psegs.ensure(sizeof(int) * kSegTab * d.psc));
+  WS_ENSURE(h->psegv.ensure(sizeof(double2) * kSegTab * d.psc));
   WS_ENSURE(h->r4.ensure(real * d.r4t));
   WS_ENSURE(h->absrb.ensure(sizeof(double) * (kNABSRB + 8) * d.cnt));
   WS_ENSURE(h->stats.ensure(sizeof(unsigned long long) * kStatsPerLayer * nL));
@@ -1458,7 +1481,8 @@ std::vector<DevBuf*> ws_buffers(clblm_handle* h) {
           &h->f4vb,   &h->f4lb,   &h->f4src,  &h->f4flag,   &h->f4nxt,  &h->f4cut,  &h->f4grp,  &h->f4rec,
           &h->f4recd, &h->f4nrec, &h->f4nmir, &h->f4pm,     &h->f4sm,   &h->err,    &h->segpool, &h->pblk,
           &h->bv1,    &h->bn,     &h->bm0,    &h->bfac,   &h->isotab, &h->linecpl, &h->f4cpl, &h->f4cpll,
-          &h->f4ncpl, &h->pwork,  &h->f4tab,  &h->f4calls,  &h->f4ncall, &h->f4agg, &h->f4core};
+          &h->f4ncpl, &h->pwork,  &h->f4tab,  &h->f4calls,  &h->f4ncall, &h->f4agg, &h->f4core,
+          &h->psegn,  &h->psegs,  &h->psegv};
 }
 
 // Frees every work buffer of the handle (all but the line list, the shape
@@ -1671,7 +1695,9 @@ int clblm_gpu_create(const clblm_lines_t* lines, const clblm_cont_t* cont, int d
   }
   if (cudaStreamCreateWithFlags(&h->stream2, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&h->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&h->join_ev, cudaEventDisableTiming) != cudaSuccess) {
+      cudaEventCreateWithFlags(&h->join_ev, cudaEventDisableTiming) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&h->stream3, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->join3_ev, cudaEventDisableTiming) != cudaSuccess) {
     g_create_err = "cannot create the second stream";
     clblm_gpu_destroy(h);
     return CLBLM_ERR_CUDA;
@@ -1782,6 +1808,11 @@ int clblm_gpu_destroy(clblm_handle_t* h) {
   h->sf_io.release();
   if (h->fork_ev) cudaEventDestroy(h->fork_ev);
   if (h->join_ev) cudaEventDestroy(h->join_ev);
+  if (h->join3_ev) cudaEventDestroy(h->join3_ev);
+  if (h->stream3) {
+    cudaStreamSynchronize(h->stream3);
+    cudaStreamDestroy(h->stream3);
+  }
   if (h->stream2) {
     cudaStreamSynchronize(h->stream2);
     cudaStreamDestroy(h->stream2);
