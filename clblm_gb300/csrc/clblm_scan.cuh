@@ -30,6 +30,16 @@ __global__ void k_scan_load(const double* s, int64_t off, int64_t ltotal, int M,
 __global__ void k_scan_apod(ScanArgs a, double2* F);
 __global__ void k_scan_sfn(int jfn, double A, double dv, int64_t n, double p1, double p2, double p3, double* y);
 __global__ void k_scan_mulnum(const double2* H, int64_t nhalf, double2* F);
+// the scan through the low coefficients alone: terms of the expansion about a
+// block's centre, threads per CTA
+constexpr int kScanTerms = 12, kScanLowThreads = 256;
+constexpr int kScanLowRatio = 16;  // M >= kScanLowRatio K: theta < 0.2
+__global__ void __launch_bounds__(kScanLowThreads)
+    k_scan_moments(const double* s, int64_t off, int64_t ltotal, int M, int64_t ktotal, double fill, double* mom,
+                   int64_t nblk, int B, int64_t stride);
+__global__ void k_scan_low(ScanArgs a, double fill_n, int64_t K, int64_t M, double2* F);
+__global__ void __launch_bounds__(kScanLowThreads)
+    k_scan_expand(const double* y, int64_t stride, int B, int64_t first, int64_t count, double scale, double* out);
 __global__ void k_scan_out(const double* y, int64_t first, int64_t count, double scale, double* out);
 
 }  // namespace clblm

@@ -158,6 +158,7 @@ struct clblm_handle {
   // FFT scan: cuFFT plans of the last transform size, the transform buffer
   // and the per-record path differences
   int64_t scan_n = 0;
+  int scan_batch = 0;
   cufftHandle scan_fwd = 0, scan_inv = 0;
   bool scan_plans = false;
   DevBuf scan_buf, scan_buf2, scan_x0, scan_io;
@@ -3928,94 +3929,140 @@ int clblm_gpu_fftscn(clblm_handle_t* h, const clblm_scan_t* scan, const double* 
     din = sp;
   }
   h->launches += launches;
-  // transform buffer: N reals, in place as N/2+1 complex
-  CUDA_TRY(h, h->scan_buf.ensure(sizeof(double2) * (size_t)(N / 2 + 1)));
-  double* x = h->scan_buf.as<double>();
+  double* dscan = p.post ? reinterpret_cast<double*>(aux + a_pre + a_prews) : dfinal;
   const unsigned grid = (unsigned)std::min<int64_t>((N + 255) / 256, 152 * 32);
-  h->launches++;
-  k_scan_load<<<grid, 256, 0, st>>>(din, p.n1 - 1, p.ltotal, p.M, p.ktotal, scan->padding, x, N);
-  CUDA_TRY(h, cudaGetLastError());
-  if (p.fft) {
-    if (!h->scan_plans || h->scan_n != N) {
-      if (h->scan_plans) {
-        cufftDestroy(h->scan_fwd);
-        cufftDestroy(h->scan_inv);
-        h->scan_plans = false;
+  // path differences at the start of every record, accumulated as
+  // Scnfnt leaves X after each record (X0 + 32768*DX)
+  ScanArgs a;
+  std::memset(&a, 0, sizeof a);
+  a.jfn = p.ivx == 1 ? p.jfn : 0;  // the analytic apodization, or none (done above)
+  a.A = p.A;
+  a.DX = 1.0 / ((double)((int64_t)kScanRecord * p.nrec) * p.DV);
+  a.nhalf = N / 2;
+  std::vector<double> x0(p.nrec);
+  double X = 0.;
+  for (int j = 0; j < p.nrec; ++j) {
+    x0[j] = X;
+    if (a.jfn == 4 && a.nedge < kScanMaxEdges) {  // the rectangle's interpolated end point
+      const double alen = 1.0 / p.A;
+      int64_t nn = (int64_t)((alen - X) / a.DX) + 1;
+      double r = (alen - X) / a.DX + 1.0 - (double)nn;
+      if (r <= 0.5) {
+        r = r + 1.0;
+        nn = nn - 1;
       }
-      if (N > (int64_t)1 << 30 || cufftPlan1d(&h->scan_fwd, (int)N, CUFFT_D2Z, 1) != CUFFT_SUCCESS)
-        return set_err(h, CLBLM_ERR_OOM, "FFTSCN: no cuFFT plan for %lld points", (long long)N);
-      if (cufftPlan1d(&h->scan_inv, (int)N, CUFFT_Z2D, 1) != CUFFT_SUCCESS) {
-        cufftDestroy(h->scan_fwd);
-        return set_err(h, CLBLM_ERR_OOM, "FFTSCN: no cuFFT plan for %lld points", (long long)N);
+      if (nn >= 1 && nn <= kScanHalf - 1) {
+        a.edge_k[a.nedge] = (int64_t)j * kScanHalf + nn;
+        a.edge_v[a.nedge] = r - 0.5;
+        a.nedge++;
       }
-      h->scan_plans = true;
-      h->scan_n = N;
     }
+    X = X + (double)kScanRecord * a.DX / 2.0;
+  }
+  a.deconv = p.deconv ? 1 : 0;
+  a.deconv_a = p.deconv_a;
+  if (p.fft && (a.jfn > 0 || a.deconv)) {
+    CUDA_TRY(h, h->scan_x0.ensure(sizeof(double) * (size_t)p.nrec));
+    CUDA_TRY(h, cudaMemcpyAsync(h->scan_x0.p, x0.data(), sizeof(double) * p.nrec, cudaMemcpyHostToDevice, st));
+    a.X0 = h->scan_x0.as<double>();
+  }
+  // plans of `batch` real transforms of `len` points each way, kept for the next call
+  auto plans = [&](int64_t len, int batch) -> int {
+    if (h->scan_plans && h->scan_n == len && h->scan_batch == batch) return CLBLM_OK;
+    if (h->scan_plans) {
+      cufftDestroy(h->scan_fwd);
+      cufftDestroy(h->scan_inv);
+      h->scan_plans = false;
+    }
+    if (len > (int64_t)1 << 30 || cufftPlan1d(&h->scan_fwd, (int)len, CUFFT_D2Z, batch) != CUFFT_SUCCESS)
+      return set_err(h, CLBLM_ERR_OOM, "FFTSCN: no cuFFT plan for %lld points", (long long)len);
+    if (cufftPlan1d(&h->scan_inv, (int)len, CUFFT_Z2D, batch) != CUFFT_SUCCESS) {
+      cufftDestroy(h->scan_fwd);
+      return set_err(h, CLBLM_ERR_OOM, "FFTSCN: no cuFFT plan for %lld points", (long long)len);
+    }
+    h->scan_plans = true;
+    h->scan_n = len;
+    h->scan_batch = batch;
     if (cufftSetStream(h->scan_fwd, st) != CUFFT_SUCCESS || cufftSetStream(h->scan_inv, st) != CUFFT_SUCCESS)
       return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: cufftSetStream");
-    if (cufftExecD2Z(h->scan_fwd, x, reinterpret_cast<cufftDoubleComplex*>(x)) != CUFFT_SUCCESS)
-      return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: forward transform");
-    if (p.ivx == -1) {
-      // the scanning function sampled at DV, transformed; its first
-      // coefficient (the area) normalises it
-      CUDA_TRY(h, h->scan_buf2.ensure(sizeof(double2) * (size_t)(N / 2 + 1)));
-      double* y = h->scan_buf2.as<double>();
-      h->launches += 2;
-      k_scan_sfn<<<grid, 256, 0, st>>>(p.jfn, p.A, p.DV, N, p.parms[0], p.parms[1], p.parms[2], y);
-      CUDA_TRY(h, cudaGetLastError());
-      if (cufftExecD2Z(h->scan_fwd, y, reinterpret_cast<cufftDoubleComplex*>(y)) != CUFFT_SUCCESS)
-        return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: transform of the scanning function");
-      k_scan_mulnum<<<grid, 256, 0, st>>>(reinterpret_cast<const double2*>(y), N / 2,
-                                          reinterpret_cast<double2*>(x));
-      CUDA_TRY(h, cudaGetLastError());
-    }
-    // path differences at the start of every record, accumulated as
-    // Scnfnt leaves X after each record (X0 + 32768*DX)
-    ScanArgs a;
-    std::memset(&a, 0, sizeof a);
-    a.jfn = p.ivx == 1 ? p.jfn : 0;  // the analytic apodization, or none (done above)
-    a.A = p.A;
-    a.DX = 1.0 / ((double)((int64_t)kScanRecord * p.nrec) * p.DV);
-    a.nhalf = N / 2;
-    std::vector<double> x0(p.nrec);
-    double X = 0.;
-    for (int j = 0; j < p.nrec; ++j) {
-      x0[j] = X;
-      if (a.jfn == 4 && a.nedge < kScanMaxEdges) {  // the rectangle's interpolated end point
-        const double alen = 1.0 / p.A;
-        int64_t nn = (int64_t)((alen - X) / a.DX) + 1;
-        double r = (alen - X) / a.DX + 1.0 - (double)nn;
-        if (r <= 0.5) {
-          r = r + 1.0;
-          nn = nn - 1;
-        }
-        if (nn >= 1 && nn <= kScanHalf - 1) {
-          a.edge_k[a.nedge] = (int64_t)j * kScanHalf + nn;
-          a.edge_v[a.nedge] = r - 0.5;
-          a.nedge++;
-        }
-      }
-      X = X + (double)kScanRecord * a.DX / 2.0;
-    }
-    a.deconv = p.deconv ? 1 : 0;
-    a.deconv_a = p.deconv_a;
-    if (a.jfn > 0 || a.deconv) {
-      CUDA_TRY(h, h->scan_x0.ensure(sizeof(double) * (size_t)p.nrec));
-      CUDA_TRY(h, cudaMemcpyAsync(h->scan_x0.p, x0.data(), sizeof(double) * p.nrec, cudaMemcpyHostToDevice, st));
-      a.X0 = h->scan_x0.as<double>();
-      h->launches++;
-      k_scan_apod<<<grid, 256, 0, st>>>(a, reinterpret_cast<double2*>(x));
-      CUDA_TRY(h, cudaGetLastError());
-    }
-    if (cufftExecZ2D(h->scan_inv, reinterpret_cast<cufftDoubleComplex*>(x), x) != CUFFT_SUCCESS)
-      return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: inverse transform");
-    CUDA_TRY(h, cudaStreamSynchronize(st));  // x0 goes out of scope
+    return CLBLM_OK;
+  };
+  // An apodization that ends (functions 3 to 10 at 1/A; the Gaussian where its
+  // floor e^-34 = 2e-15 begins) at a small part of the transform's path
+  // differences: the first K coefficients alone, through M-point transforms
+  int64_t K = 0, M = 0;
+  if (p.ivx == 1 && p.jfn >= 2 && p.jfn <= 10) {
+    const double end = p.jfn == 2 ? std::sqrt(17.) / (3.141592653589793 * p.A) : 1. / p.A;
+    if (end / a.DX < 1.e9) K = (int64_t)(end / a.DX) + 3;
+    for (int e = 0; e < a.nedge; ++e) K = std::max<int64_t>(K, a.edge_k[e] + 1);
+    M = 1024;
+    while (M < kScanLowRatio * K) M *= 2;
   }
-  double* dscan = p.post ? reinterpret_cast<double*>(aux + a_pre + a_prews) : dfinal;
-  h->launches++;
-  k_scan_out<<<(unsigned)std::min<int64_t>((p.ntotal + 255) / 256, 152 * 32), 256, 0, st>>>(
-      x, p.N1 - 1, p.ntotal, p.fft ? 1.0 / (double)N : 1.0, dscan);
-  CUDA_TRY(h, cudaGetLastError());
+  if (K > 0 && K < N / 2 && M <= N / 32) {
+    const int B = (int)(N / M);
+    const int64_t pts = p.M > 1 ? p.ktotal : p.ltotal, nblk = (pts + B - 1) / B;
+    const int64_t ms = M + 2;  // a row: M reals, or M/2+1 complex in place
+    CUDA_TRY(h, h->scan_buf.ensure(sizeof(double) * (size_t)(2 * kScanTerms * ms)));
+    double* mom = h->scan_buf.as<double>();
+    double2* F = reinterpret_cast<double2*>(mom + (int64_t)kScanTerms * ms);
+    rc = plans(M, kScanTerms);
+    if (rc) return rc;
+    auto ctas = [&](int64_t warps) {
+      return (unsigned)std::max<int64_t>(std::min<int64_t>((warps + 7) / 8, (int64_t)h->nsm * 16), 1);
+    };
+    h->launches += 3;
+    CUDA_TRY(h, cudaMemsetAsync(mom, 0, sizeof(double) * (size_t)(kScanTerms * M), st));  // blocks past the data
+    k_scan_moments<<<ctas(nblk), kScanLowThreads, 0, st>>>(din, p.n1 - 1, p.ltotal, p.M, p.ktotal, scan->padding, mom,
+                                                           nblk, B, M);
+    CUDA_TRY(h, cudaGetLastError());
+    if (cufftExecD2Z(h->scan_fwd, mom, reinterpret_cast<cufftDoubleComplex*>(F)) != CUFFT_SUCCESS)
+      return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: forward transform");
+    k_scan_low<<<(unsigned)((M / 2 + 128) / 128), 128, 0, st>>>(a, scan->padding * (double)N, K, M, F);
+    CUDA_TRY(h, cudaGetLastError());
+    if (cufftExecZ2D(h->scan_inv, reinterpret_cast<cufftDoubleComplex*>(F), mom) != CUFFT_SUCCESS)
+      return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: inverse transform");
+    k_scan_expand<<<ctas(p.ntotal / B + 2), kScanLowThreads, 0, st>>>(mom, M, B, p.N1 - 1, p.ntotal, 1.0 / (double)N,
+                                                                      dscan);
+    CUDA_TRY(h, cudaGetLastError());
+  } else {
+    // transform buffer: N reals, in place as N/2+1 complex
+    CUDA_TRY(h, h->scan_buf.ensure(sizeof(double2) * (size_t)(N / 2 + 1)));
+    double* x = h->scan_buf.as<double>();
+    h->launches++;
+    k_scan_load<<<grid, 256, 0, st>>>(din, p.n1 - 1, p.ltotal, p.M, p.ktotal, scan->padding, x, N);
+    CUDA_TRY(h, cudaGetLastError());
+    if (p.fft) {
+      rc = plans(N, 1);
+      if (rc) return rc;
+      if (cufftExecD2Z(h->scan_fwd, x, reinterpret_cast<cufftDoubleComplex*>(x)) != CUFFT_SUCCESS)
+        return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: forward transform");
+      if (p.ivx == -1) {
+        // the scanning function sampled at DV, transformed; its first
+        // coefficient (the area) normalises it
+        CUDA_TRY(h, h->scan_buf2.ensure(sizeof(double2) * (size_t)(N / 2 + 1)));
+        double* y = h->scan_buf2.as<double>();
+        h->launches += 2;
+        k_scan_sfn<<<grid, 256, 0, st>>>(p.jfn, p.A, p.DV, N, p.parms[0], p.parms[1], p.parms[2], y);
+        CUDA_TRY(h, cudaGetLastError());
+        if (cufftExecD2Z(h->scan_fwd, y, reinterpret_cast<cufftDoubleComplex*>(y)) != CUFFT_SUCCESS)
+          return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: transform of the scanning function");
+        k_scan_mulnum<<<grid, 256, 0, st>>>(reinterpret_cast<const double2*>(y), N / 2,
+                                            reinterpret_cast<double2*>(x));
+        CUDA_TRY(h, cudaGetLastError());
+      }
+      if (a.jfn > 0 || a.deconv) {
+        h->launches++;
+        k_scan_apod<<<grid, 256, 0, st>>>(a, reinterpret_cast<double2*>(x));
+        CUDA_TRY(h, cudaGetLastError());
+      }
+      if (cufftExecZ2D(h->scan_inv, reinterpret_cast<cufftDoubleComplex*>(x), x) != CUFFT_SUCCESS)
+        return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: inverse transform");
+    }
+    h->launches++;
+    k_scan_out<<<(unsigned)std::min<int64_t>((p.ntotal + 255) / 256, 152 * 32), 256, 0, st>>>(
+        x, p.N1 - 1, p.ntotal, p.fft ? 1.0 / (double)N : 1.0, dscan);
+    CUDA_TRY(h, cudaGetLastError());
+  }
   if (p.post) {
     launches = 0;
     CUDA_TRY(h, sf_launch_interp(p.post_plan, dscan, dfinal, aux + a_pre + a_prews + a_scan, st, &launches));
