@@ -70,6 +70,35 @@ struct DevBuf {
   }
 };
 
+// a part of a device buffer
+struct DevView {
+  void* p = nullptr;
+  template <typename T>
+  T* as() const {
+    return reinterpret_cast<T*>(p);
+  }
+};
+
+// page-locked host memory that the handle keeps for its copies
+struct PinBuf {
+  unsigned char* p = nullptr;
+  size_t bytes = 0;
+  cudaError_t ensure(size_t n) {
+    if (n <= bytes) return cudaSuccess;
+    release();
+    const size_t want = n + n / 4 + 4096;
+    const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&p), want, cudaHostAllocDefault);
+    if (e == cudaSuccess) bytes = want;
+    else p = nullptr;
+    return e;
+  }
+  void release() {
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    bytes = 0;
+  }
+};
+
 }  // namespace
 
 namespace {
@@ -109,12 +138,20 @@ struct clblm_handle {
   bool first_pass_jrad = true;
   int jrad = 0;
   // workspace
-  DevBuf plans, vft, prep, qpanel, rec, recd, ranges, od, r4, absrb, stats, alfvmax, blockmax, nlines_d;
-  DevBuf isotab;  // isotopologue rows of the planned layers
+  DevBuf prep, qpanel, rec, recd, ranges, od, r4, absrb, blockmax;
+  // tables of the planned layers, counters and flags: parts of one buffer, so
+  // that a call uploads them with one copy, zeroes and reads back with one each
+  DevBuf tabbuf;
+  DevView plans, vft, nlines_d, pblk, bv1, bn, bm0;
+  DevView isotab;  // isotopologue rows of the planned layers
+  DevView err, stats, f4nout, alfvmax, f4core;
+  size_t tab_up = 0, tab_back = 0, tab_zero = 0;  // bytes uploaded, read back (from err on), zeroed (from err on)
+  PinBuf stage, back;                             // their host sides
+  cudaEvent_t stage_ev = nullptr;                 // the last upload has left `stage`
   DevBuf linecpl;  // SPPSP of the coupled lines, per line of each layer
   DevBuf f4cpl, f4cpll, f4ncpl;  // far wings: DPTRAT per record, the coupled records' list and counts
-  DevBuf f4prep, f4sh, f4nout, f4rec, f4recd, f4nrec, f4nmir, f4pm, f4sm, err;
-  DevBuf pblk, bv1, bn, bm0, bfac;
+  DevBuf f4prep, f4sh, f4rec, f4recd, f4nrec, f4nmir, f4pm, f4sm;
+  DevBuf bfac;
   DevBuf gpm, gsm;  // per grid record bounds of the panel kernel
   DevBuf pwork;     // CTAs of the panel kernel's line pass
   DevBuf psegn, psegs, psegv;  // radiation-term segments of the panels
@@ -122,7 +159,6 @@ struct clblm_handle {
   DevBuf jprof, jod, jmap, jjobs, jblk;  // Jacobians: profiles, block ODs, maps, jobs, grid blocks
   DevBuf jvjp;                          // vector-Jacobian product: CTA partial sums and the totals
   DevBuf f4blk, f4ntot, f4cidx, f4vb, f4lb, f4src, f4flag, f4cut, f4grp, f4nxt, ragg;
-  DevBuf f4core;                   // points that no far-wing line's core reaches past, per layer
   DevBuf f4agg;                    // bounds of the far-wing records, per kF4Blk records
   DevBuf f4tab, f4calls, f4ncall;  // SHRINQ calls: counts of the possible ones, the list, its length
   DevBuf segpool;  // radiation-term segments of panels with more than kMaxSeg
@@ -137,16 +173,13 @@ struct clblm_handle {
   int nsm = 1;  // SMs of the device
   // every device buffer of the handle but the line list
   std::vector<DevBuf*> buffers() {
-    std::vector<DevBuf*> v = {&cont_self, &cont_for, &cont_texp, &cont_co2, &tabs,    &plans,   &vft,    &prep,    &qpanel,
-                              &rec,       &recd,     &ranges,    &od,      &r4,      &absrb,  &stats,   &alfvmax,
-                              &blockmax,  &nlines_d, &f4prep,    &f4sh,    &f4nout,  &f4rec,  &f4recd,  &f4nrec,
-                              &f4nmir,    &f4pm,     &f4sm,      &err,     &outbuf,  &pblk,   &bv1,     &bn,
-                              &bm0,       &bfac,     &f4blk,     &f4ntot,  &f4cidx,  &f4vb,   &f4lb,    &f4src,
+    std::vector<DevBuf*> v = {&cont_self, &cont_for, &cont_texp, &cont_co2, &tabs,    &prep,    &qpanel,
+                              &rec,       &recd,     &ranges,    &od,      &r4,      &absrb,  &blockmax,  &f4prep,    &f4sh,    &f4rec,  &f4recd,  &f4nrec,
+                              &f4nmir,    &f4pm,     &f4sm,      &outbuf,  &bfac,     &f4blk,     &f4ntot,  &f4cidx,  &f4vb,   &f4lb,    &f4src,
                               &f4flag,    &f4cut,    &f4grp,     &f4nxt,   &ragg,    &segpool, &gpm,    &gsm,
-                              &reclo,     &jprof,    &jod,       &jmap,    &jjobs,   &jblk,    &jvjp,   &isotab,
-                              &linecpl,   &f4cpl,    &f4cpll,    &f4ncpl,   &pwork,
-                              &f4tab,     &f4calls,  &f4ncall,  &f4agg,     &f4core,  &psegn,
-                              &psegs,     &psegv};
+                              &reclo,     &jprof,    &jod,       &jmap,    &jjobs,   &jblk,    &jvjp,   &linecpl,   &f4cpl,    &f4cpll,    &f4ncpl,   &pwork,
+                              &f4tab,     &f4calls,  &f4ncall,  &f4agg,     &psegn,
+                              &psegs,     &psegv, &tabbuf};
     for (auto& b : rt) v.push_back(&b);
     for (auto& b : imap) v.push_back(&b);
     v.push_back(&rtseg);
@@ -941,11 +974,14 @@ size_t od_job_bytes(const LayerPlan& P, bool plain) {
 // already (the layers of a batch share launches, and every batch replays the
 // far-wing walk's serial record loop, so fewer, larger batches are faster),
 // between 8 and 192 GB.  CLBLM_OD_BUDGET_GB=<GB> sets it instead.
-size_t od_batch_budget(clblm_handle* h) {
+// `need`: what the call would take in one batch; at or below the least budget
+// the device is not asked.
+size_t od_batch_budget(clblm_handle* h, size_t need = ~(size_t)0) {
   if (const char* e = std::getenv("CLBLM_OD_BUDGET_GB")) {
     const double gb = std::atof(e);
     if (gb > 0.) return (size_t)(gb * (double)((size_t)1 << 30));
   }
+  if (need <= (size_t)8 << 30) return (size_t)8 << 30;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return (size_t)24 << 30;
   size_t held = 0;
@@ -1134,7 +1170,6 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
                                         h->f4sm.as<int>());
     };
     if (far_nodes) {
-      CUDA_TRY(h, cudaMemsetAsync(h->f4core.as<int>() + first, 0, sizeof(int) * count, st));
       if (plain) bounds(k_f4_agg<2>, k_f4_bounds<2>);
       else bounds(k_f4_agg<1>, k_f4_bounds<1>);
     } else {
@@ -1400,6 +1435,35 @@ WsDims batch_dims(std::vector<HostPlan>& hps, int first, int count, int64_t* lst
   return d;
 }
 
+// The parts of the tables' buffer for nL planned layers; returns its size.
+// (In order: what is uploaded; the error flags, counters and far-wing counts,
+// which are zeroed and read back; what is zeroed alone.)
+size_t tab_layout(clblm_handle* h, int nL, int64_t vftt, int64_t blkt, int64_t isot) {
+  size_t off = 0;
+  unsigned char* base = h->tabbuf.as<unsigned char>();
+  auto part = [&](DevView* v, size_t b) {
+    v->p = base ? base + off : nullptr;
+    off += (b + 255) & ~(size_t)255;
+  };
+  part(&h->plans, sizeof(LayerPlan) * (size_t)nL);
+  part(&h->isotab, sizeof(IsoRow) * (size_t)std::max<int64_t>(isot, 1));
+  part(&h->vft, sizeof(double) * (size_t)vftt);
+  part(&h->nlines_d, sizeof(int64_t) * (size_t)nL);
+  part(&h->pblk, sizeof(int) * (size_t)vftt);
+  part(&h->bv1, sizeof(double) * (size_t)(blkt + 1));
+  part(&h->bn, sizeof(int) * (size_t)(blkt + 1));
+  part(&h->bm0, sizeof(int64_t) * (size_t)(blkt + 1));
+  h->tab_up = off;
+  part(&h->err, sizeof(int) * 4);
+  part(&h->stats, sizeof(unsigned long long) * kStatsPerLayer * (size_t)nL);
+  part(&h->f4nout, sizeof(int64_t) * 2 * (size_t)nL);
+  h->tab_back = off - h->tab_up;
+  part(&h->alfvmax, sizeof(double) * (size_t)nL);
+  part(&h->f4core, sizeof(int) * (size_t)nL);
+  h->tab_zero = off - h->tab_up;
+  return off;
+}
+
 // Buffers of one OD batch (sized by d) and of all nL planned layers: the
 // first error, or success.
 cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int64_t blkt, int64_t isot,
@@ -1410,13 +1474,11 @@ cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int
   do {                                     \
     if ((e = (x)) != cudaSuccess) return e; \
   } while (0)
-  WS_ENSURE(h->plans.ensure(sizeof(LayerPlan) * nL));
-  WS_ENSURE(h->isotab.ensure(sizeof(IsoRow) * (size_t)std::max<int64_t>(isot, 1)));
+  WS_ENSURE(h->tabbuf.ensure(tab_layout(h, nL, vftt, blkt, isot)));
   WS_ENSURE(h->linecpl.ensure(h->has_cpl ? sizeof(double) * d.lsc : 256));
   WS_ENSURE(h->f4cpl.ensure(h->has_cpl ? sizeof(double) * (d.fsc + 4096 * d.cnt) : 256));
   WS_ENSURE(h->f4cpll.ensure(h->has_cpl ? sizeof(int64_t) * (d.fsc + 4096 * d.cnt) : 256));
   WS_ENSURE(h->f4ncpl.ensure(sizeof(int64_t) * std::max(nL, 1)));
-  WS_ENSURE(h->vft.ensure(sizeof(double) * vftt));
   WS_ENSURE(h->prep.ensure(sizeof(LinePrep) * d.lsc));
   WS_ENSURE(h->qpanel.ensure(sizeof(int) * d.lsc));
   WS_ENSURE(h->rec.ensure(sizeof(GridRec) * d.lsc * 3));
@@ -1434,13 +1496,9 @@ cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int
   WS_ENSURE(h->psegv.ensure(sizeof(double2) * kSegTab * d.psc));
   WS_ENSURE(h->r4.ensure(real * d.r4t));
   WS_ENSURE(h->absrb.ensure(sizeof(double) * (kNABSRB + 8) * d.cnt));
-  WS_ENSURE(h->stats.ensure(sizeof(unsigned long long) * kStatsPerLayer * nL));
-  WS_ENSURE(h->alfvmax.ensure(sizeof(double) * nL));
   WS_ENSURE(h->blockmax.ensure(sizeof(int) * d.smaxc));
-  WS_ENSURE(h->nlines_d.ensure(sizeof(int64_t) * nL));
   WS_ENSURE(h->f4prep.ensure(sizeof(F4Prep) * d.fsc));
   WS_ENSURE(h->f4sh.ensure(sizeof(ShrunkLine) * d.fsc));
-  WS_ENSURE(h->f4nout.ensure(sizeof(int64_t) * 2 * nL));
   WS_ENSURE(h->f4blk.ensure(sizeof(int64_t) * d.nblk4c));
   WS_ENSURE(h->f4ntot.ensure(sizeof(int64_t) * d.cnt));
   WS_ENSURE(h->f4cidx.ensure(sizeof(int64_t) * (d.fsc + d.cnt)));
@@ -1455,20 +1513,14 @@ cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int
   WS_ENSURE(h->f4calls.ensure(sizeof(int4) * (d.frecc + 2 * d.cnt)));
   WS_ENSURE(h->f4ncall.ensure(sizeof(int2) * d.cnt));
   WS_ENSURE(h->f4agg.ensure(sizeof(int) * 2 * d.f4aggc));
-  WS_ENSURE(h->f4core.ensure(sizeof(int) * nL));
   WS_ENSURE(h->f4rec.ensure(sizeof(F4Rec) * (d.fsc + 4096 * d.cnt)));
   WS_ENSURE(h->f4recd.ensure(plain ? sizeof(F4RecD) * (d.fsc + 4096 * d.cnt) : 256));
   WS_ENSURE(h->f4nrec.ensure(sizeof(int64_t) * nL));
   WS_ENSURE(h->f4nmir.ensure(sizeof(int64_t) * nL));
   WS_ENSURE(h->f4pm.ensure(sizeof(int) * (d.fsc + 4096 * d.cnt)));
   WS_ENSURE(h->f4sm.ensure(sizeof(int) * (d.fsc + 4096 * d.cnt)));
-  WS_ENSURE(h->err.ensure(sizeof(int) * 4));
   WS_ENSURE(h->segpool.ensure(256 + (sizeof(int) * (kSegSlot + 1) + 2 * sizeof(double) * kSegSlot) *
                                           (size_t)kSegPoolSlots));
-  WS_ENSURE(h->pblk.ensure(sizeof(int) * vftt));
-  WS_ENSURE(h->bv1.ensure(sizeof(double) * (blkt + 1)));
-  WS_ENSURE(h->bn.ensure(sizeof(int) * (blkt + 1)));
-  WS_ENSURE(h->bm0.ensure(sizeof(int64_t) * (blkt + 1)));
   WS_ENSURE(h->bfac.ensure(sizeof(double) * (kLIMOUT4 + 2) * (blkt + 1)));
 #undef WS_ENSURE
   return e;
@@ -1476,14 +1528,11 @@ cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int
 
 // The buffers ws_alloc sizes: scratch of one batch, nothing in them outlives it.
 std::vector<DevBuf*> ws_buffers(clblm_handle* h) {
-  return {&h->plans,  &h->vft,    &h->prep,   &h->qpanel,   &h->rec,    &h->recd,   &h->gpm,    &h->reclo,
-          &h->gsm,    &h->ragg,   &h->ranges, &h->od,       &h->r4,     &h->absrb,  &h->stats,  &h->alfvmax,
-          &h->blockmax, &h->nlines_d, &h->f4prep, &h->f4sh, &h->f4nout, &h->f4blk, &h->f4ntot, &h->f4cidx,
+  return {&h->prep,   &h->qpanel,   &h->rec,    &h->recd,   &h->gpm,    &h->reclo,
+          &h->gsm,    &h->ragg,   &h->ranges, &h->od,       &h->r4,     &h->absrb,  &h->blockmax, &h->f4prep, &h->f4sh, &h->f4blk, &h->f4ntot, &h->f4cidx,
           &h->f4vb,   &h->f4lb,   &h->f4src,  &h->f4flag,   &h->f4nxt,  &h->f4cut,  &h->f4grp,  &h->f4rec,
-          &h->f4recd, &h->f4nrec, &h->f4nmir, &h->f4pm,     &h->f4sm,   &h->err,    &h->segpool, &h->pblk,
-          &h->bv1,    &h->bn,     &h->bm0,    &h->bfac,   &h->isotab, &h->linecpl, &h->f4cpl, &h->f4cpll,
-          &h->f4ncpl, &h->pwork,  &h->f4tab,  &h->f4calls,  &h->f4ncall, &h->f4agg, &h->f4core,
-          &h->psegn,  &h->psegs,  &h->psegv};
+          &h->f4recd, &h->f4nrec, &h->f4nmir, &h->f4pm,     &h->f4sm,   &h->segpool, &h->bfac,   &h->linecpl, &h->f4cpl, &h->f4cpll,
+          &h->f4ncpl, &h->pwork,  &h->f4tab,  &h->f4calls,  &h->f4ncall, &h->f4agg, &h->psegn,  &h->psegs,  &h->psegv, &h->tabbuf};
 }
 
 // Frees every work buffer of the handle (all but the line list, the shape
@@ -1532,37 +1581,50 @@ void table_offsets(std::vector<HostPlan>& hps, int64_t* vftt, int64_t* blkt, int
 // zeroes the counters and error flags.
 int upload_plans(clblm_handle* h, std::vector<HostPlan>& hps, int64_t vftt, int64_t blkt, int64_t isot) {
   const int nL = (int)hps.size();
-  std::vector<int> pb(vftt, 0), bn(blkt + 1, 0);
-  std::vector<double> bv(blkt + 1, 0.);
-  std::vector<int64_t> bm(blkt + 1, 0);
-  std::vector<LayerPlan> plans(nL);
-  std::vector<double> vft(vftt, 0.);
-  std::vector<int64_t> nl(nL, 0);
-  std::vector<IsoRow> iso(std::max<int64_t>(isot, 1));
+  tab_layout(h, nL, vftt, blkt, isot);
+  if (!h->stage_ev) CUDA_TRY(h, cudaEventCreateWithFlags(&h->stage_ev, cudaEventDisableTiming));
+  CUDA_TRY(h, cudaEventSynchronize(h->stage_ev));  // the previous call's copy has been made
+  CUDA_TRY(h, h->stage.ensure(h->tab_up));
+  const unsigned char* base = h->tabbuf.as<unsigned char>();
+  auto host = [&](const DevView& v) { return h->stage.p + (v.as<const unsigned char>() - base); };
+  std::memset(h->stage.p, 0, h->tab_up);
+  LayerPlan* plans = reinterpret_cast<LayerPlan*>(host(h->plans));
+  IsoRow* iso = reinterpret_cast<IsoRow*>(host(h->isotab));
+  double* vft = reinterpret_cast<double*>(host(h->vft));
+  int64_t* nl = reinterpret_cast<int64_t*>(host(h->nlines_d));
+  int* pb = reinterpret_cast<int*>(host(h->pblk));
+  double* bv = reinterpret_cast<double*>(host(h->bv1));
+  int* bn = reinterpret_cast<int*>(host(h->bn));
+  int64_t* bm = reinterpret_cast<int64_t*>(host(h->bm0));
   for (int k = 0; k < nL; ++k) {
     const HostPlan& hp = hps[k];
-    std::copy(hp.iso.begin(), hp.iso.end(), iso.begin() + hp.P.iso_off);
-    std::copy(hp.panel_blk.begin(), hp.panel_blk.end(), pb.begin() + hp.P.vft_off);
-    std::copy(hp.blk_v1.begin(), hp.blk_v1.end(), bv.begin() + hp.P.blk_off);
-    std::copy(hp.blk_n.begin(), hp.blk_n.end(), bn.begin() + hp.P.blk_off);
-    std::copy(hp.blk_m0.begin(), hp.blk_m0.end(), bm.begin() + hp.P.blk_off);
+    std::copy(hp.iso.begin(), hp.iso.end(), iso + hp.P.iso_off);
+    std::copy(hp.panel_blk.begin(), hp.panel_blk.end(), pb + hp.P.vft_off);
+    std::copy(hp.blk_v1.begin(), hp.blk_v1.end(), bv + hp.P.blk_off);
+    std::copy(hp.blk_n.begin(), hp.blk_n.end(), bn + hp.P.blk_off);
+    std::copy(hp.blk_m0.begin(), hp.blk_m0.end(), bm + hp.P.blk_off);
     plans[k] = hp.P;
-    std::copy(hp.vft.begin(), hp.vft.end(), vft.begin() + hp.P.vft_off);
+    std::copy(hp.vft.begin(), hp.vft.end(), vft + hp.P.vft_off);
     nl[k] = hp.P.line_hi - hp.P.line_lo + 1;
   }
   cudaStream_t st = h->stream;
-  CUDA_TRY(h, cudaMemcpyAsync(h->pblk.p, pb.data(), sizeof(int) * vftt, cudaMemcpyHostToDevice, st));
-  CUDA_TRY(h, cudaMemcpyAsync(h->bv1.p, bv.data(), sizeof(double) * (blkt + 1), cudaMemcpyHostToDevice, st));
-  CUDA_TRY(h, cudaMemcpyAsync(h->bn.p, bn.data(), sizeof(int) * (blkt + 1), cudaMemcpyHostToDevice, st));
-  CUDA_TRY(h, cudaMemcpyAsync(h->bm0.p, bm.data(), sizeof(int64_t) * (blkt + 1), cudaMemcpyHostToDevice, st));
-  CUDA_TRY(h, cudaMemcpyAsync(h->plans.p, plans.data(), sizeof(LayerPlan) * nL, cudaMemcpyHostToDevice, st));
-  CUDA_TRY(h, cudaMemcpyAsync(h->isotab.p, iso.data(), sizeof(IsoRow) * iso.size(), cudaMemcpyHostToDevice, st));
-  CUDA_TRY(h, cudaMemcpyAsync(h->vft.p, vft.data(), sizeof(double) * vftt, cudaMemcpyHostToDevice, st));
-  CUDA_TRY(h, cudaMemcpyAsync(h->nlines_d.p, nl.data(), sizeof(int64_t) * nL, cudaMemcpyHostToDevice, st));
-  CUDA_TRY(h, cudaMemsetAsync(h->stats.p, 0, sizeof(unsigned long long) * kStatsPerLayer * nL, st));
-  CUDA_TRY(h, cudaMemsetAsync(h->alfvmax.p, 0, sizeof(double) * nL, st));
-  CUDA_TRY(h, cudaMemsetAsync(h->err.p, 0, sizeof(int) * 4, st));
-  CUDA_TRY(h, cudaStreamSynchronize(st));  // the host vectors go out of scope
+  CUDA_TRY(h, cudaMemcpyAsync(h->tabbuf.p, h->stage.p, h->tab_up, cudaMemcpyHostToDevice, st));
+  CUDA_TRY(h, cudaEventRecord(h->stage_ev, st));
+  CUDA_TRY(h, cudaMemsetAsync(h->err.p, 0, h->tab_zero, st));
+  return CLBLM_OK;
+}
+
+// Waits for the stream and reads back the error flags, the layers' counters and
+// their far-wing counts.
+int read_back(clblm_handle* h, const int** err, const unsigned long long** stats, const int64_t** nout) {
+  CUDA_TRY(h, h->back.ensure(h->tab_back));
+  CUDA_TRY(h, cudaMemcpyAsync(h->back.p, h->err.p, h->tab_back, cudaMemcpyDeviceToHost, h->stream));
+  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  CUDA_TRY(h, cudaGetLastError());
+  const unsigned char* base = h->err.as<const unsigned char>();
+  *err = reinterpret_cast<const int*>(h->back.p);
+  *stats = reinterpret_cast<const unsigned long long*>(h->back.p + (h->stats.as<const unsigned char>() - base));
+  *nout = reinterpret_cast<const int64_t*>(h->back.p + (h->f4nout.as<const unsigned char>() - base));
   return CLBLM_OK;
 }
 
@@ -1582,16 +1644,10 @@ int prepare_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int co
 
 // Reads back the error flags and the counters of layers [first, first+count).
 int check_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int count, clblm_od_stats_t* last_stats) {
-  int err[4];
-  int nL = (int)hps.size();
-  std::vector<unsigned long long> stats(kStatsPerLayer * nL);
-  std::vector<int64_t> nout(2 * nL);
-  CUDA_TRY(h, cudaMemcpyAsync(err, h->err.p, sizeof err, cudaMemcpyDeviceToHost, h->stream));
-  CUDA_TRY(h, cudaMemcpyAsync(stats.data(), h->stats.p, sizeof(unsigned long long) * stats.size(),
-                              cudaMemcpyDeviceToHost, h->stream));
-  CUDA_TRY(h, cudaMemcpyAsync(nout.data(), h->f4nout.p, sizeof(int64_t) * 2 * nL, cudaMemcpyDeviceToHost, h->stream));
-  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-  CUDA_TRY(h, cudaGetLastError());
+  const int* err;
+  const unsigned long long* stats;
+  const int64_t* nout;
+  if (int rc = read_back(h, &err, &stats, &nout)) return rc;
   if (err[0] & 1) return set_err(h, CLBLM_ERR_RANGE, "radiation-term segments: more than %d panels of a batch "
                                  "need more than %d", kSegPoolSlots, kMaxSeg);
   if (err[0] & 2) return set_err(h, CLBLM_ERR_RANGE, "shape-table index beyond NFMX");
@@ -1810,6 +1866,9 @@ int clblm_gpu_destroy(clblm_handle_t* h) {
   if (h->fork_ev) cudaEventDestroy(h->fork_ev);
   if (h->join_ev) cudaEventDestroy(h->join_ev);
   if (h->join3_ev) cudaEventDestroy(h->join3_ev);
+  if (h->stage_ev) cudaEventDestroy(h->stage_ev);
+  h->stage.release();
+  h->back.release();
   if (h->stream3) {
     cudaStreamSynchronize(h->stream3);
     cudaStreamDestroy(h->stream3);
@@ -2198,7 +2257,9 @@ int clblm_gpu_rt_mode2(clblm_handle_t* h, const clblm_column_t* col, const clblm
   CUDA_TRY(h, h->outbuf.ensure(sizeof(double) * nfinal));
   double* final_dst = flags == CLBLM_OUT_DEVICE ? rad : h->outbuf.as<double>();
   // layers in batches sized to the workspace budget
-  const size_t budget = od_batch_budget(h);
+  size_t all = 0;
+  for (const HostPlan& hp : rp.hps) all += od_job_bytes(hp.P, plain);
+  const size_t budget = od_batch_budget(h, all);
   int cur = 0;  // ping-pong index of the merged spectra
   for (int first = 0; first < n;) {
     int count = 0;
@@ -2625,6 +2686,9 @@ int jac_plan_block(clblm_handle* h, const clblm_rt_ctrl_t* ctrl, const clblm_jac
 // The blocks of noScattJacob (clblm_noScattJac.f90:206-232): V1B, V2B and
 // the block length, which is the first layer's OD length (:227-229); the next
 // block starts one DVout after the block's last point.
+// workspace, OD slabs and maps of the blocks whose ODs clblm_gpu_jac forms together
+constexpr size_t kJacGroupBytes = (size_t)24 << 30;
+
 struct JacBlock {
   double v1, v2;
   int64_t n;
@@ -2837,20 +2901,65 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
   int jr = h->jrad;
   bool fp = h->first_pass_jrad;
   int64_t total = 0;
+  // All blocks are planned first (host threads; in the reference's call order
+  // for the sticky JRAD).  The ODs of several blocks then share the pipeline's
+  // launches: a block's surface layers, few panels with long record lists,
+  // would leave the GPU idle at the end of each of its kernels (25 blocks of
+  // 240 ODs one after another: 110 ms, together 88 ms).
+  std::vector<std::vector<HostPlan>> plans;
+  std::vector<int64_t> nlims;
+  rc = jac_plan_blocks(h, ctrl, jac, js, dvn, dvf, blocks, &jr, &fp, &plans, &nlims);
+  if (rc) return rc;
+  for (size_t b = 0; b < blocks.size(); ++b)
+    if (nlims[b] != blocks[b].n) return set_err(h, CLBLM_ERR_GRID, "Jacobian block length changed");
   const size_t budget = od_batch_budget(h);
-  for (auto& blk : blocks) {
-    std::vector<HostPlan> hps;
-    int64_t nlim;
-    rc = jac_plan_block(h, ctrl, jac, js, dvn, dvf, blk.v1, blk.v2, &jr, &fp, &hps, &nlim);
-    if (rc) return rc;
-    if (nlim != blk.n) return set_err(h, CLBLM_ERR_GRID, "Jacobian block length changed");
-    const int njob = (int)hps.size();
-    // the block's ODs on the uniform grid, [variant][layer][point]
+  size_t limit = std::min(budget, kJacGroupBytes);  // of a group of blocks; 0: one block at a time
+  for (size_t ib = 0; ib < blocks.size();) {
+    // blocks [ib, ie): their ODs, OD slabs and maps within the limit
+    std::vector<int64_t> jod_off, map_off;
+    std::vector<int> job0, blk0, nblk;
+    std::vector<int64_t> j1;
+    std::vector<double> vo;
+    int64_t jods = 0, maps = 0, nlmax = 0;
+    int njob = 0, bmax = 0;
+    size_t ie = ib, bytes = 0;
+    for (; ie < blocks.size(); ++ie) {
+      const int64_t nlim = nlims[ie];
+      size_t w = real * (size_t)js.nvar * nl * nlim + 8 * plans[ie].size() * (size_t)nlim;
+      for (const HostPlan& hp : plans[ie]) w += od_job_bytes(hp.P, plain);
+      if (ie > ib && bytes + w > limit) break;
+      bytes += w;
+      jod_off.push_back(jods);
+      map_off.push_back(maps);
+      job0.push_back(njob);
+      jods += (int64_t)js.nvar * nl * nlim;
+      maps += (int64_t)plans[ie].size() * nlim;
+      njob += (int)plans[ie].size();
+      nlmax = std::max(nlmax, nlim);
+      // output-grid blocks of interpSpectrum's general branch (shared by the block's jobs)
+      blk0.push_back((int)j1.size());
+      const double TOL = 1.e-8;
+      const double V2out = blocks[ie].v1 + (double)(nlim - 1) * js.dvb;
+      double Vo = blocks[ie].v1;
+      while (Vo < V2out + TOL) {
+        int64_t J1 = (int64_t)((Vo - blocks[ie].v1) / js.dvb + 1.001);
+        int64_t J2 = std::min<int64_t>(nlim, J1 + 2400 - 1);
+        j1.push_back(J1);
+        vo.push_back(Vo);
+        Vo = blocks[ie].v1 + (double)J2 * js.dvb;
+        if (j1.size() - blk0.back() > (size_t)(nlim / 2400 + 8))
+          return set_err(h, CLBLM_ERR_GRID, "interpolation blocks");
+      }
+      nblk.push_back((int)j1.size() - blk0.back());
+      bmax = std::max(bmax, nblk.back());
+    }
+    // the blocks' ODs on the uniform grid, [variant][layer][point] each
     {  // (out of memory: the batch scratch and the block buffers, dead here, are freed, then once more)
       auto alloc = [&]() -> cudaError_t {
-        cudaError_t e = h->jod.ensure(real * (size_t)js.nvar * nl * nlim);
-        if (e == cudaSuccess) e = h->jmap.ensure(sizeof(int2) * (size_t)njob * nlim);
+        cudaError_t e = h->jod.ensure(real * (size_t)jods);
+        if (e == cudaSuccess) e = h->jmap.ensure(sizeof(int2) * (size_t)maps);
         if (e == cudaSuccess) e = h->jjobs.ensure(sizeof(JacJob) * (size_t)njob);
+        if (e == cudaSuccess) e = h->jblk.ensure(16 * (j1.size() + 1));
         return e;
       };
       cudaError_t e = alloc();
@@ -2859,138 +2968,149 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
         for (DevBuf* b : ws_buffers(h)) b->release();
         for (DevBuf* b : {&h->jod, &h->jmap, &h->jjobs}) b->release();
         e = alloc();
+        if (e == cudaErrorMemoryAllocation && ie - ib > 1) {  // one block at a time, as little as there is
+          cudaGetLastError();
+          limit = 0;
+          continue;
+        }
       }
       CUDA_TRY(h, e);
     }
-    // output-grid blocks of interpSpectrum's general branch (shared by all jobs)
-    std::vector<int64_t> j1;
-    std::vector<double> vo;
-    {
-      const double TOL = 1.e-8;
-      const double V2out = blk.v1 + (double)(nlim - 1) * js.dvb;
-      double Vo = blk.v1;
-      while (Vo < V2out + TOL) {
-        int64_t J1 = (int64_t)((Vo - blk.v1) / js.dvb + 1.001);
-        int64_t J2 = std::min<int64_t>(nlim, J1 + 2400 - 1);
-        j1.push_back(J1);
-        vo.push_back(Vo);
-        Vo = blk.v1 + (double)J2 * js.dvb;
-        if (j1.size() > (size_t)(nlim / 2400 + 8)) return set_err(h, CLBLM_ERR_GRID, "interpolation blocks");
-      }
-    }
-    const int nbt = (int)j1.size();
-    CUDA_TRY(h, h->jblk.ensure(16 * (size_t)(nbt + 1)));
+    std::vector<HostPlan> hps;
+    hps.reserve(njob);
+    for (size_t b = ib; b < ie; ++b)
+      for (HostPlan& hp : plans[b]) hps.push_back(std::move(hp));
     int64_t* dj1 = h->jblk.as<int64_t>();
-    double* dvo = reinterpret_cast<double*>(h->jblk.as<unsigned char>() + 8 * (size_t)(nbt + 1));
-    CUDA_TRY(h, cudaMemcpyAsync(dj1, j1.data(), 8 * (size_t)nbt, cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(h, cudaMemcpyAsync(dvo, vo.data(), 8 * (size_t)nbt, cudaMemcpyHostToDevice, h->stream));
+    double* dvo = reinterpret_cast<double*>(h->jblk.as<unsigned char>() + 8 * j1.size());
+    CUDA_TRY(h, cudaMemcpyAsync(dj1, j1.data(), 8 * j1.size(), cudaMemcpyHostToDevice, h->stream));
+    CUDA_TRY(h, cudaMemcpyAsync(dvo, vo.data(), 8 * j1.size(), cudaMemcpyHostToDevice, h->stream));
+    int last_first = 0, last_count = 0;  // the group's last batch
+    std::vector<JacJob> jobs(njob);
+    std::vector<std::vector<int>> of_layer;  // jobs of each layer of the block so far
+    bool shrink = false;
     for (int first = 0; first < njob;) {
       int count = 0;
-      size_t bytes = 0;
+      size_t wb = 0;
       while (first + count < njob) {
-        const size_t b = od_job_bytes(hps[first + count].P, plain);
-        if (count > 0 && bytes + b > budget) break;
-        bytes += b;
+        const size_t w = od_job_bytes(hps[first + count].P, plain);
+        if (count > 0 && wb + w > budget) break;
+        wb += w;
         count++;
       }
       int64_t ls, fs, ps, odt;
       rc = prepare_batch(h, hps, first, count, plain, &ls, &fs, &ps, &odt);
+      if (rc == CLBLM_ERR_OOM && ie - ib > 1 && first == 0) {  // one block at a time, as little as there is
+        cudaGetLastError();
+        shrink = true;
+        break;
+      }
       if (rc) return rc;
-      rc = run_od_batch(h, hps, first, count, plain, true, ls, fs, ps);
-      if (rc) return rc;
-      rc = check_batch(h, hps, first, count, &h->last);
-      if (rc) return rc;
-      std::vector<JacJob> jobs(count);
-      for (int k = 0; k < count; ++k) {
-        const int j = first + k;
+      size_t kb = 0;  // block of job j, counted from ib
+      for (int j = first; j < first + count; ++j) {
+        while (kb + 1 < job0.size() && job0[kb + 1] <= j) ++kb;
+        if (j == first || j == job0[kb]) of_layer.assign(nl, {});
+        const int q0 = job0[kb], q = j - q0;
+        const int64_t nlim = nlims[ib + kb];
         const LayerPlan& P = hps[j].P;
-        JacJob& jb = jobs[k];
-        jb.spec = interp_spec(P.v1, P.dv, P.nsamp, blk.v1, js.dvb, nlim);
+        JacJob& jb = jobs[j];
+        jb.spec = interp_spec(P.v1, P.dv, P.nsamp, blocks[ib + kb].v1, js.dvb, nlim);
         // the variants of a layer share its grid: one map per layer (built
-        // with the layer's first job), the others only read it
-        const int il = js.job_lay[j];
+        // with the batch's first job of the layer), the others only read it
+        const int il = js.job_lay[q];
         int owner = j;
-        for (int q = 0; q < j; ++q)
-          if (js.job_lay[q] == il && hps[q].P.dv == P.dv && hps[q].P.nsamp == P.nsamp) {
-            owner = q;
+        for (int k : of_layer[il])
+          if (hps[k].P.dv == P.dv && hps[k].P.nsamp == P.nsamp) {
+            owner = k;
             break;
           }
-        jb.map = h->jmap.as<int2>() + (size_t)owner * nlim;
+        of_layer[il].push_back(j);
+        jb.map = h->jmap.as<int2>() + map_off[kb] + (int64_t)(owner - q0) * nlim;
         jb.spec.map = jb.map;
         jb.build_map = (owner == j && jb.spec.kind != 0 && jb.spec.itype < 0) ? 1 : 0;
         jb.od_off = P.od_off;
         jb.n_in = P.nsamp;
         jb.nout = nlim;
-        jb.dst_off = (int64_t)(js.job_var[j] * nl + js.job_lay[j]) * nlim;
-        jb.blk_j1 = dj1;
-        jb.blk_vo = dvo;
-        jb.nblk = nbt;
+        jb.dst_off = jod_off[kb] + (int64_t)(js.job_var[q] * nl + js.job_lay[q]) * nlim;
+        jb.blk_j1 = dj1 + blk0[kb];
+        jb.blk_vo = dvo + blk0[kb];
+        jb.nblk = nblk[kb];
       }
-      CUDA_TRY(h, cudaMemcpyAsync(h->jjobs.p, jobs.data(), sizeof(JacJob) * count, cudaMemcpyHostToDevice,
+      // (before the pipeline's launches: a copy from pageable memory waits for
+      // what the stream holds)
+      JacJob* djobs = h->jjobs.as<JacJob>() + first;
+      CUDA_TRY(h, cudaMemcpyAsync(djobs, jobs.data() + first, sizeof(JacJob) * count, cudaMemcpyHostToDevice,
                                   h->stream));
+      rc = run_od_batch(h, hps, first, count, plain, true, ls, fs, ps);
+      if (rc) return rc;
       h->launches += 2;
-      k_interp_map_jobs<<<dim3((unsigned)nbt, count), kMapThreads, 0, h->stream>>>(h->jjobs.as<JacJob>(), count);
+      k_interp_map_jobs<<<dim3((unsigned)bmax, count), kMapThreads, 0, h->stream>>>(djobs, count);
+      const dim3 go((unsigned)((nlmax + kOdJobPoints - 1) / kOdJobPoints), count);
+      if (plain) k_od_jobs<true><<<go, kOdJobThreads, 0, h->stream>>>(djobs, count, h->od.p, h->jod.p);
+      else k_od_jobs<false><<<go, kOdJobThreads, 0, h->stream>>>(djobs, count, h->od.p, h->jod.p);
       {
         cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return set_err(h, CLBLM_ERR_CUDA, "k_interp_map_jobs: %s", cudaGetErrorString(e));
+        if (e != cudaSuccess) return set_err(h, CLBLM_ERR_CUDA, "Jacobian OD gather: %s", cudaGetErrorString(e));
       }
-      if (plain)
-        k_od_jobs<true><<<dim3((unsigned)((nlim + kOdJobPoints - 1) / kOdJobPoints), count), kOdJobThreads, 0,
-                          h->stream>>>(
-            h->jjobs.as<JacJob>(), count, h->od.p, h->jod.p);
-      else
-        k_od_jobs<false><<<dim3((unsigned)((nlim + kOdJobPoints - 1) / kOdJobPoints), count), kOdJobThreads, 0,
-                           h->stream>>>(
-            h->jjobs.as<JacJob>(), count, h->od.p, h->jod.p);
-      {
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return set_err(h, CLBLM_ERR_CUDA, "k_od_jobs: %s", cudaGetErrorString(e));
-      }
-      // the job table and the OD buffer are reused by the next batch
-      CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+      last_first = first;
+      last_count = count;
       first += count;
+      if (first < njob) {  // (the next batch's tables take this one's place)
+        rc = check_batch(h, hps, last_first, last_count, &h->last);
+        if (rc) return rc;
+      }
     }
-    JacArgs a;
-    std::memset(&a, 0, sizeof a);
-    a.jod = h->jod.p;
-    a.nlay = nl;
-    a.vT = js.vT;
-    a.vW = js.vW;
-    a.vM = js.vM;
-    a.nout = nlim;
-    a.v1 = blk.v1;
-    a.dv = js.dvb;
-    a.tlay = dprof;
-    a.tlev = dprof + nl;
-    a.amf_down = dprof + 2 * nl + 1;
-    a.wtot = dprof + 3 * nl + 1;
-    a.dT_dTup = dprof + 4 * nl + 1;
-    a.dT_dTlo = dprof + 5 * nl + 1;
-    a.dW_dQup = dprof + 6 * nl + 1;
-    a.dW_dQlo = dprof + 7 * nl + 1;
-    a.tsfc = col->tskin;
-    a.emis = col->emis;
-    a.lin_in_tau = ctrl->lin_in_tau;
-    a.do_temp = jac->do_temp;
-    a.rad = o_rad;
-    a.dtlev = o_dtl;
-    a.dqlev = o_dql;
-    a.dtsfc = o_dts;
-    a.demis = o_dem;
-    a.ld = ld;
-    a.off = total;
-    a.g = d_g;
-    a.part = d_part;
-    int grid = 0;
-    rc = launch_jac(h, a, plain, &grid);
+    if (shrink) {
+      for (size_t b = ib; b < ie; ++b)
+        for (size_t k = 0; k < plans[b].size(); ++k) plans[b][k] = std::move(hps[job0[b - ib] + k]);
+      limit = 0;
+      continue;
+    }
+    for (size_t b = ib; b < ie; ++b) {
+      const int64_t nlim = nlims[b];
+      JacArgs a;
+      std::memset(&a, 0, sizeof a);
+      a.jod = h->jod.as<unsigned char>() + real * jod_off[b - ib];
+      a.nlay = nl;
+      a.vT = js.vT;
+      a.vW = js.vW;
+      a.vM = js.vM;
+      a.nout = nlim;
+      a.v1 = blocks[b].v1;
+      a.dv = js.dvb;
+      a.tlay = dprof;
+      a.tlev = dprof + nl;
+      a.amf_down = dprof + 2 * nl + 1;
+      a.wtot = dprof + 3 * nl + 1;
+      a.dT_dTup = dprof + 4 * nl + 1;
+      a.dT_dTlo = dprof + 5 * nl + 1;
+      a.dW_dQup = dprof + 6 * nl + 1;
+      a.dW_dQlo = dprof + 7 * nl + 1;
+      a.tsfc = col->tskin;
+      a.emis = col->emis;
+      a.lin_in_tau = ctrl->lin_in_tau;
+      a.do_temp = jac->do_temp;
+      a.rad = o_rad;
+      a.dtlev = o_dtl;
+      a.dqlev = o_dql;
+      a.dtsfc = o_dts;
+      a.demis = o_dem;
+      a.ld = ld;
+      a.off = total;
+      a.g = d_g;
+      a.part = d_part;
+      int grid = 0;
+      rc = launch_jac(h, a, plain, &grid);
+      if (rc) return rc;
+      if (vjp) {
+        h->launches++;
+        k_vjp_accum<<<(unsigned)((nslot + 127) / 128), 128, 0, h->stream>>>(d_part, grid, nslot, d_acc);
+        CUDA_TRY(h, cudaGetLastError());
+      }
+      total += nlim;
+    }
+    rc = check_batch(h, hps, last_first, last_count, &h->last);  // (waits for the stream)
     if (rc) return rc;
-    if (vjp) {
-      h->launches++;
-      k_vjp_accum<<<(unsigned)((nslot + 127) / 128), 128, 0, h->stream>>>(d_part, grid, nslot, d_acc);
-      CUDA_TRY(h, cudaGetLastError());
-    }
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    total += nlim;
+    ib = ie;
   }
   h->first_pass_jrad = fp;
   h->jrad = jr;
@@ -3426,16 +3546,10 @@ int batch_enqueue(clblm_handle* h, BatchPlan& bp, const clblm_profile_t* prof, c
 // failing job fails its profile.  Returns the first failing profile's code.
 int batch_check(clblm_handle* h, const std::vector<int>& job_prof, std::vector<int>* status) {
   const int nL = (int)job_prof.size();
-  int err[4];
-  std::vector<unsigned long long> stats((size_t)kStatsPerLayer * nL);
-  std::vector<int64_t> nout(2 * (size_t)nL);
-  CUDA_TRY(h, cudaMemcpyAsync(err, h->err.p, sizeof err, cudaMemcpyDeviceToHost, h->stream));
-  CUDA_TRY(h, cudaMemcpyAsync(stats.data(), h->stats.p, sizeof(unsigned long long) * stats.size(),
-                              cudaMemcpyDeviceToHost, h->stream));
-  CUDA_TRY(h, cudaMemcpyAsync(nout.data(), h->f4nout.p, sizeof(int64_t) * nout.size(), cudaMemcpyDeviceToHost,
-                              h->stream));
-  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-  CUDA_TRY(h, cudaGetLastError());
+  const int* err;
+  const unsigned long long* stats;
+  const int64_t* nout;
+  if (int rc = read_back(h, &err, &stats, &nout)) return rc;
   if (err[0] & 1) return set_err(h, CLBLM_ERR_RANGE, "radiation-term segments: more than %d panels of a batch "
                                  "need more than %d", kSegPoolSlots, kMaxSeg);
   if (err[0] & 2) return set_err(h, CLBLM_ERR_RANGE, "shape-table index beyond NFMX");
