@@ -162,16 +162,32 @@ struct MapReplay {
       fixed = (double)q * (1. / 2305843009213693952.) == P ? 1 : 0;
     }
   }
-  // n steps.  At 0.5 <= RATIO < 0.999 a sum below 1 is exact on multiples of
+  // n steps.  Below 0.999 INT(iIn + P) is iIn + 1 and the chain has no binary64
+  // operation; at 0.5 <= RATIO < 0.999 a sum below 1 is exact on multiples of
   // 2^-53 and one above 1 rounds to a multiple of 2^-52: a chain of a few
   // integer operations.
   CLBLM_HD void steps(int n) {
     int k = 0;
-    while (k < n && !(fixed && ratio >= 0.5 && ratio < 0.999 && (q & 255) == 0)) {
+    const bool below = ratio < 0.999, half = ratio >= 0.5;
+    while (k < n && !(fixed && below && (!half || (q & 255) == 0))) {
       step();
       ++k;
     }
     if (k == n) return;
+    if (!half) {
+      int carries = 0;
+      for (; k < n; ++k) {
+        const uint64_t s = q + rq;
+        const int sh = 11 - clz32((uint32_t)(s >> 32));
+        const uint32_t one = 1u << sh, lo = (uint32_t)s;
+        const uint32_t up = (one >> 1) - 1u + ((lo >> sh) & 1u);
+        const uint64_t v = (s + (sh > 0 ? up : 0u)) & ~(uint64_t)(one - 1u);
+        carries += (int)(v >> 61);
+        q = v & (((uint64_t)1 << 61) - 1);
+      }
+      iIn += carries;
+      return;
+    }
     uint64_t p = q >> 8;
     const uint64_t r = rq >> 8;
     int carries = 0;
