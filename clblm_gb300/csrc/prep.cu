@@ -1992,39 +1992,81 @@ __device__ __forceinline__ ShrunkLine shrunk_line(int k, bool mixed, double SUMV
 // A surface layer's groups hold 64 lines and more (DVR4/2 = 0.32 cm-1 at 200
 // lines per cm-1): 170 us for one such layer with a thread per group, whose
 // loads followed one another.  Layers with fewer than kGroupWarpMin lines
-// per group keep a thread per group: their chains are short and there are
-// many of them (a warp each would leave most lanes idle).
+// per group keep a thread per group: there are many of them, and the FP64
+// unit, which takes 16 cycles for an instruction of any number of lanes, adds
+// 32 groups' members at once.
 constexpr int kGroupWarps = kGroupSumThreads / 32;
-constexpr int kGroupWarpMin = 6;  // mean lines per group from which a warp takes a group
+constexpr int kGroupWarpMin = 20;  // mean lines per group from which a warp takes a group
 
-// one group by one thread
+// Fields of a corrected line, as 16-byte loads (48 bytes a line)
+struct F4Member {
+  double vnu, sp, spp;
+  float4 w;  // the widths: w.f of the mixed path, the bits of w.d on the FP64 path
+  int mol;
+};
+__device__ __forceinline__ F4Member load_member(const F4Prep* __restrict__ r) {
+  static_assert(sizeof(F4Prep) == 48, "three 16-byte loads");
+  const double2 a = __ldg(reinterpret_cast<const double2*>(r));
+  const int4 b = __ldg(reinterpret_cast<const int4*>(r) + 1);  // spp, first half of w
+  const int4 c = __ldg(reinterpret_cast<const int4*>(r) + 2);  // second half of w, mol, pass
+  F4Member m;
+  m.vnu = a.x;
+  m.sp = a.y;
+  m.spp = __hiloint2double(b.y, b.x);
+  m.w = make_float4(__int_as_float(b.z), __int_as_float(b.w), __int_as_float(c.x), __int_as_float(c.y));
+  m.mol = c.z;
+  return m;
+}
+// SP < 1e-35 (not of a NaN of either sign) and SPP != 0 on the bits: a binary64
+// compare takes the FP64 unit, which bounds the sums
+__device__ __forceinline__ bool weak_sp(double sp) {
+  const long long b = __double_as_longlong(sp);
+  return b < __double_as_longlong(1.0e-35) && (unsigned long long)b << 1 <= 0xFFE0000000000000ull;
+}
+__device__ __forceinline__ bool nonzero_d(double x) { return (__double_as_longlong(x) << 1) != 0; }
+
+// one group by one thread, the next member loaded while one is added
 __device__ __forceinline__ void group_sum_thread(const F4Prep* __restrict__ pr, const int64_t* __restrict__ S,
                                                  const int4 gr, bool mixed, ShrunkLine* __restrict__ O) {
   int slot = gr.z;
   double SUMS[2] = {0., 0.}, SUMV[2] = {0., 0.}, AL[2] = {0., 0.}, AD[2] = {0., 0.};
   float ALf[2] = {0.f, 0.f}, ADf[2] = {0.f, 0.f};
+  F4Member nxt = load_member(pr + S[gr.x]);
   for (int u = gr.x; u <= gr.y; ++u) {
-    const F4Prep& r = pr[S[u]];
-    const bool weak = r.sp < 1.0e-35;
-    if (!weak && r.spp != 0.) {  // a coupled line is not shrunk (SHRINQ :1566-1578)
-      O[slot++] = shrunk_coupled(r, mixed);
+    const F4Member r = nxt;
+    if (u < gr.y) nxt = load_member(pr + S[u + 1]);
+    const bool weak = weak_sp(r.sp);
+    if (!weak && nonzero_d(r.spp)) {  // a coupled line is not shrunk (SHRINQ :1566-1578)
+      O[slot++] = shrunk_coupled(pr[S[u]], mixed);
       continue;
     }
     const double sp = weak ? 0.0 : r.sp;
+    const double vs = r.vnu * sp;
     auto add = [&](int k) {
-      SUMV[k] = SUMV[k] + r.vnu * sp;
+      SUMV[k] = SUMV[k] + vs;
       SUMS[k] = SUMS[k] + sp;
-      if (mixed) {  // widths set no index: FP32
-        const float spf = weak ? 0.f : r.w.f[2];
-        ALf[k] = ALf[k] + spf * r.w.f[0];
-        ADf[k] = ADf[k] + spf * r.w.f[1];
-      } else {
-        AL[k] = AL[k] + sp * r.w.d[0];
-        AD[k] = AD[k] + sp * r.w.d[1];
-      }
     };
     if (r.mol != 2) add(0);
     else add(1);
+    if (mixed) {  // widths set no index: FP32
+      const float spf = weak ? 0.f : r.w.z;
+      const float al = spf * r.w.x, ad = spf * r.w.y;
+      ALf[0] = ALf[0] + (r.mol != 2 ? al : 0.f);
+      ADf[0] = ADf[0] + (r.mol != 2 ? ad : 0.f);
+      ALf[1] = ALf[1] + (r.mol != 2 ? 0.f : al);
+      ADf[1] = ADf[1] + (r.mol != 2 ? 0.f : ad);
+    } else {
+      const double al = sp * __hiloint2double(__float_as_int(r.w.y), __float_as_int(r.w.x));
+      const double ad = sp * __hiloint2double(__float_as_int(r.w.w), __float_as_int(r.w.z));
+      const int k = r.mol != 2 ? 0 : 1;
+      if (k == 0) {
+        AL[0] = AL[0] + al;
+        AD[0] = AD[0] + ad;
+      } else {
+        AL[1] = AL[1] + al;
+        AD[1] = AD[1] + ad;
+      }
+    }
   }
 #pragma unroll
   for (int k = 0; k < 2; ++k)
@@ -2064,8 +2106,8 @@ __global__ void __launch_bounds__(kGroupSumThreads)
       F4Prep r;
       if (lane < cnt) {
         r = pr[S[u0 + lane]];
-        const bool weak = r.sp < 1.0e-35;
-        coupled = !weak && r.spp != 0.;  // a coupled line is not shrunk (SHRINQ :1566-1578)
+        const bool weak = weak_sp(r.sp);
+        coupled = !weak && nonzero_d(r.spp);  // a coupled line is not shrunk (SHRINQ :1566-1578)
         const double sp = weak || coupled ? 0.0 : r.sp;
         const int k = r.mol != 2 ? 0 : 1;
         D[4 * k][lane] = coupled ? 0. : r.vnu * sp;

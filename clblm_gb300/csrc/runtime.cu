@@ -1065,7 +1065,8 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
       maxb = std::max(maxb, hps[first + k].P.nblk4);
     }
     h->launches += 3;
-    k_continuum<<<dim3((kNABSRB + 255) / 256, count), blk, 0, s3>>>(dplans, first, h->cont, h->absrb.as<double>());
+    // (small CTAs: the FP64 unit bounds it, one point a lane over all SMs)
+    k_continuum<<<dim3((kNABSRB + 8 + 63) / 64, count), 64, 0, s3>>>(dplans, first, h->cont, h->absrb.as<double>());
     k_r4_radfac<<<dim3((maxb + kRadfacWarps - 1) / kRadfacWarps, count), 32 * kRadfacWarps, 0, s3>>>(
         dplans, first, h->bv1.as<double>(), h->bn.as<int>(), h->bfac.as<double>());
     k_panel_segs<<<dim3((maxp + 63) / 64, count), 64, 0, s3>>>(dplans, first, h->vft.as<double>(), pstride,
@@ -1129,9 +1130,7 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
           h->f4nout.as<int64_t>());
     }
     h->launches++;
-    // (about 16 CTAs per SM in all: a group is little work for a CTA's start)
-    const int64_t gsum = std::max<int64_t>((int64_t)16 * h->nsm / count, 1);
-    k_f4_groupsum<<<dim3((unsigned)std::min<int64_t>((f4stride + 255) / 256, gsum), count), kGroupSumThreads, 0, st>>>(
+    k_f4_groupsum<<<dim3((unsigned)std::min<int64_t>((f4stride + 255) / 256, 4096), count), kGroupSumThreads, 0, st>>>(
         dplans, first, h->f4prep.as<F4Prep>(), f4stride, h->f4src.as<int64_t>(), h->f4grp.as<int4>(),
         h->f4nout.as<int64_t>(), h->f4sh.as<ShrunkLine>());
   }
