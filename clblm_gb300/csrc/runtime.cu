@@ -4079,7 +4079,8 @@ int clblm_gpu_fftscn(clblm_handle_t* h, const clblm_scan_t* scan, const double* 
     CUDA_TRY(h, cudaMemcpyAsync(h->scan_x0.p, x0.data(), sizeof(double) * p.nrec, cudaMemcpyHostToDevice, st));
     a.X0 = h->scan_x0.as<double>();
   }
-  // plans of `batch` real transforms of `len` points each way, kept for the next call
+  // plans of one real transform of `len` points, or of a batch of complex ones,
+  // each way, kept for the next call
   auto plans = [&](int64_t len, int batch) -> int {
     if (h->scan_plans && h->scan_n == len && h->scan_batch == batch) return CLBLM_OK;
     if (h->scan_plans) {
@@ -4087,9 +4088,9 @@ int clblm_gpu_fftscn(clblm_handle_t* h, const clblm_scan_t* scan, const double* 
       cufftDestroy(h->scan_inv);
       h->scan_plans = false;
     }
-    if (len > (int64_t)1 << 30 || cufftPlan1d(&h->scan_fwd, (int)len, CUFFT_D2Z, batch) != CUFFT_SUCCESS)
+    if (len > (int64_t)1 << 30 || cufftPlan1d(&h->scan_fwd, (int)len, batch == 1 ? CUFFT_D2Z : CUFFT_Z2Z, batch) != CUFFT_SUCCESS)
       return set_err(h, CLBLM_ERR_OOM, "FFTSCN: no cuFFT plan for %lld points", (long long)len);
-    if (cufftPlan1d(&h->scan_inv, (int)len, CUFFT_Z2D, batch) != CUFFT_SUCCESS) {
+    if (cufftPlan1d(&h->scan_inv, (int)len, batch == 1 ? CUFFT_Z2D : CUFFT_Z2Z, batch) != CUFFT_SUCCESS) {
       cufftDestroy(h->scan_fwd);
       return set_err(h, CLBLM_ERR_OOM, "FFTSCN: no cuFFT plan for %lld points", (long long)len);
     }
@@ -4114,28 +4115,47 @@ int clblm_gpu_fftscn(clblm_handle_t* h, const clblm_scan_t* scan, const double* 
   if (K > 0 && K < N / 2 && M <= N / 32) {
     const int B = (int)(N / M);
     const int64_t pts = p.M > 1 ? p.ktotal : p.ltotal, nblk = (pts + B - 1) / B;
-    const int64_t ms = M + 2;  // a row: M reals, or M/2+1 complex in place
-    CUDA_TRY(h, h->scan_buf.ensure(sizeof(double) * (size_t)(2 * kScanTerms * ms)));
-    double* mom = h->scan_buf.as<double>();
-    double2* F = reinterpret_cast<double2*>(mom + (int64_t)kScanTerms * ms);
-    rc = plans(M, kScanTerms);
-    if (rc) return rc;
+    // Z: the moments, then the way back's spectra; X: the transforms of the
+    // one, then of the other; W: exp(-2 pi i j / M)
+    constexpr int kPairs = kScanTerms / 2;
+    CUDA_TRY(h, h->scan_buf.ensure(sizeof(double2) * (size_t)((2 * kPairs + 1) * M)));
+    double2* Z = h->scan_buf.as<double2>();
+    double2 *X = Z + kPairs * M, *W = X + kPairs * M;
+    const bool own = M / kScanFftR <= kScanFftMaxC;
+    const int C = (int)(M / kScanFftR), logC = 63 - __builtin_clzll((unsigned long long)C);
+    const size_t smem = sizeof(double2) * 3 * (size_t)C;
+    const dim3 parts(kScanFftR, kPairs);
     auto ctas = [&](int64_t warps) {
       return (unsigned)std::max<int64_t>(std::min<int64_t>((warps + 7) / 8, (int64_t)h->nsm * 16), 1);
     };
-    h->launches += 3;
-    CUDA_TRY(h, cudaMemsetAsync(mom, 0, sizeof(double) * (size_t)(kScanTerms * M), st));  // blocks past the data
-    k_scan_moments<<<ctas(nblk), kScanLowThreads, 0, st>>>(din, p.n1 - 1, p.ltotal, p.M, p.ktotal, scan->padding, mom,
-                                                           nblk, B, M);
+    h->launches += own ? 5 : 3;
+    k_scan_moments<<<ctas(M / 4), kScanLowThreads, 0, st>>>(din, p.n1 - 1, p.ltotal, p.M, p.ktotal, scan->padding, Z,
+                                                            nblk, B, M, own ? W : nullptr);
     CUDA_TRY(h, cudaGetLastError());
-    if (cufftExecD2Z(h->scan_fwd, mom, reinterpret_cast<cufftDoubleComplex*>(F)) != CUFFT_SUCCESS)
-      return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: forward transform");
-    k_scan_low<<<(unsigned)((M / 2 + 128) / 128), 128, 0, st>>>(a, scan->padding * (double)N, K, M, F);
+    if (own) {
+      CUDA_TRY(h, cudaFuncSetAttribute(k_scan_fft<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      CUDA_TRY(h, cudaFuncSetAttribute(k_scan_fft<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      k_scan_fft<false><<<parts, kScanFftThreads, smem, st>>>(Z, X, W, M, K, logC);
+      CUDA_TRY(h, cudaGetLastError());
+    } else {
+      rc = plans(M, kPairs);
+      if (rc) return rc;
+      if (cufftExecZ2Z(h->scan_fwd, reinterpret_cast<cufftDoubleComplex*>(Z), reinterpret_cast<cufftDoubleComplex*>(X),
+                       CUFFT_FORWARD) != CUFFT_SUCCESS)
+        return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: forward transform");
+      CUDA_TRY(h, cudaMemsetAsync(Z, 0, sizeof(double2) * (size_t)(kPairs * M), st));
+    }
+    k_scan_low<<<(unsigned)((K + kScanLowK - 1) / kScanLowK), 32 * kPairs, 0, st>>>(
+        a, scan->padding * (double)N, 1.0 / (double)N, K, M, own ? kScanFftR : 1, X, W, Z);
     CUDA_TRY(h, cudaGetLastError());
-    if (cufftExecZ2D(h->scan_inv, reinterpret_cast<cufftDoubleComplex*>(F), mom) != CUFFT_SUCCESS)
+    if (own) {
+      k_scan_fft<true><<<parts, kScanFftThreads, smem, st>>>(Z, X, W, M, K, logC);
+      CUDA_TRY(h, cudaGetLastError());
+    } else if (cufftExecZ2Z(h->scan_inv, reinterpret_cast<cufftDoubleComplex*>(Z),
+                            reinterpret_cast<cufftDoubleComplex*>(X), CUFFT_INVERSE) != CUFFT_SUCCESS) {
       return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: inverse transform");
-    k_scan_expand<<<ctas(p.ntotal / B + 2), kScanLowThreads, 0, st>>>(mom, M, B, p.N1 - 1, p.ntotal, 1.0 / (double)N,
-                                                                      dscan);
+    }
+    k_scan_expand<<<ctas(p.ntotal / B + 2), kScanLowThreads, 0, st>>>(X, M, B, p.N1 - 1, p.ntotal, dscan);
     CUDA_TRY(h, cudaGetLastError());
   } else {
     // transform buffer: N reals, in place as N/2+1 complex

@@ -28,13 +28,13 @@
 //   exp(-2 pi i k n / N) = phase(k, b) exp(-i theta t),  theta = pi k / M,
 // and exp(-i theta t) = sum_p (-i theta)^p / p! t^p: 12 terms below 1e-16 for
 // theta < 0.2, so
-//   k_scan_moments   sum_j x_j t_j^p of each block, p = 0 .. 11
-//   (cuFFT)          12 transforms of M points
-//   k_scan_low       the coefficients k < K from them, times the apodization,
-//                    and the 12 spectra of the way back, (i theta)^p / p! of
-//                    each (the block centres' phases cancel)
-//   (cuFFT)          12 transforms of M points
-//   k_scan_expand    sum_p t^p Y_p(b) at the scanned points
+//   k_scan_moments     sum_j x_j t_j^p of each block, p = 0 .. 11
+//   k_scan_fft<false>  their transforms of M points, two moments as one complex
+//   k_scan_low         the coefficients k < K from them, times the apodization,
+//                      and the 12 spectra of the way back, (i theta)^p / p! of
+//                      each (the block centres' phases cancel)
+//   k_scan_fft<true>   their transforms
+//   k_scan_expand      sum_p t^p Y_p(b) at the scanned points
 // The spectrum is read once and the scanned points written once; a 2^23-point
 // scan took 2.0 ms, nearly all of it in the transforms' passes over memory.
 #include <cuda_runtime.h>
@@ -214,134 +214,306 @@ __global__ void k_scan_mulnum(const double2* __restrict__ H, int64_t nhalf, doub
   }
 }
 
-// moments of a block of B points (even): thread t of the warp takes the pairs
-// (j, B-1-j) with j = t, t + 32, ... of the lower half, whose t are opposite
+// t_j^(2q) of a block's lower half (q = 0: t itself) in shared memory
+__device__ __forceinline__ void scan_powers(int B, double (*T)[kScanPowers], int n) {
+  const double rh = 2. / (double)B, c = 0.5 * (double)(B - 1);
+  for (int j = threadIdx.x; j < B / 2; j += blockDim.x) {
+    const double t = ((double)j - c) * rh, t2 = t * t;
+    T[0][j] = t;
+    double e = t2;
+    for (int q = 1; q < n; ++q) {
+      T[q][j] = e;
+      e *= t2;
+    }
+  }
+  __syncthreads();
+}
+
+// moments of a block of B points (even): the pairs (j, B-1-j), whose t are
+// opposite, over the kMomLanes lanes of a block; the FP64 unit bounds it (16
+// cycles an instruction: 17 a pair), so the powers of t come from a table and
+// a lane group is as small as the reduction's 16 values allow (lane q ends
+// with moments 2q and 2q+1): 77 -> 33 us on 2,000,000 points against a warp
+// per block and powers by multiplication.  The blocks past the data are
+// zeroed, and W gets exp(-2 pi i j / M) for the transforms.
 __global__ void __launch_bounds__(kScanLowThreads)
-    k_scan_moments(const double* __restrict__ s, int64_t off, int64_t ltotal, int M, int64_t ktotal, double fill,
-                   double* __restrict__ mom, int64_t nblk, int B, int64_t stride) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  const int64_t n = M <= 1 ? ltotal : ktotal;
+    k_scan_moments(const double* __restrict__ s, int64_t off, int64_t ltotal, int boxed, int64_t ktotal, double fill,
+                   double2* __restrict__ mom, int64_t nblk, int B, int64_t M, double2* __restrict__ W) {
+  constexpr int kMomLanes = 8;
+  __shared__ double T[kScanTerms / 2][kScanPowers];
+  const bool table = B / 2 <= kScanPowers;
+  if (table) scan_powers(B, T, kScanTerms / 2);
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthr = (int64_t)gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & (kMomLanes - 1);
+  const int64_t n = boxed <= 1 ? ltotal : ktotal;
   auto value = [&](int64_t i) -> double {  // less FILL, which reaches k = 0 alone
     if (i >= n) return 0.;
-    if (M <= 1) return __dadd_rn(s[off + i], -fill);
+    if (boxed <= 1) return fill != 0. ? __dadd_rn(s[off + i], -fill) : s[off + i];
     double sum = 0.0;
-    for (int m = 0; m < M; ++m) sum = __dadd_rn(sum, s[off + i * M + m]);
-    return __dadd_rn(__ddiv_rn(sum, (double)M), -fill);
+    for (int m = 0; m < boxed; ++m) sum = __dadd_rn(sum, s[off + i * boxed + m]);
+    return __dadd_rn(__ddiv_rn(sum, (double)boxed), -fill);
   };
   const double rh = 2. / (double)B, c = 0.5 * (double)(B - 1);
-  for (int64_t b = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b < nblk; b += warps) {
+  // (whole warps: the last one's spare groups take block M - 1 again)
+  const int64_t groups = (M * kMomLanes + 31) / 32 * (32 / kMomLanes);
+  for (int64_t g = tid / kMomLanes; g < groups; g += nthr / kMomLanes) {
+    const int64_t b = g < M ? g : M - 1;
     double v[16];
 #pragma unroll
     for (int p = 0; p < 16; ++p) v[p] = 0.;
-    for (int j = lane; j < B / 2; j += 32) {
-      const double x0 = value(b * B + j), x1 = value(b * B + B - 1 - j);
-      const double t = ((double)j - c) * rh, t2 = t * t;
-      double e = x0 + x1, o = (x0 - x1) * t;  // (t of the other point is -t)
+    if (b < nblk) {
+      const int64_t i0 = b * B;
+      if (table) {
+#pragma unroll 4
+        for (int j = lane; j < B / 2; j += kMomLanes) {
+          const double x0 = value(i0 + j), x1 = value(i0 + B - 1 - j);
+          const double e = x0 + x1, o = (x0 - x1) * T[0][j];  // (t of the other point is -t)
+          v[0] += e;
+          v[1] += o;
 #pragma unroll
-      for (int p = 0; p < kScanTerms; p += 2) {
-        v[p] += e;
-        v[p + 1] += o;
-        e *= t2;
-        o *= t2;
+          for (int q = 1; q < kScanTerms / 2; ++q) {
+            v[2 * q] = fma(e, T[q][j], v[2 * q]);
+            v[2 * q + 1] = fma(o, T[q][j], v[2 * q + 1]);
+          }
+        }
+      } else {
+        for (int j = lane; j < B / 2; j += kMomLanes) {
+          const double x0 = value(i0 + j), x1 = value(i0 + B - 1 - j);
+          const double t = ((double)j - c) * rh, t2 = t * t;
+          double e = x0 + x1, o = (x0 - x1) * t;
+#pragma unroll
+          for (int p = 0; p < kScanTerms; p += 2) {
+            v[p] += e;
+            v[p + 1] += o;
+            e *= t2;
+            o *= t2;
+          }
+        }
       }
     }
-    // totals over the lanes: lane l ends with that of v[l >> 1]
+    // totals over the lanes: lane l ends with those of v[2l], v[2l+1]
 #pragma unroll
-    for (int h = 8; h >= 1; h >>= 1) {
-      const int bit = 2 * h;
-      const bool up = (lane & bit) != 0;
+    for (int h = 8; h >= 2; h >>= 1) {
+      const bool up = (lane & (h >> 1)) != 0;
 #pragma unroll
       for (int i = 0; i < h; ++i) {
         const double send = up ? v[i] : v[i + h];
         const double keep = up ? v[i + h] : v[i];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h >> 1);
       }
     }
-    const double tot = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-    if (!(lane & 1) && (lane >> 1) < kScanTerms) mom[(int64_t)(lane >> 1) * stride + b] = tot;
+    if (lane < kScanTerms / 2) mom[(int64_t)lane * M + b] = make_double2(v[0], v[1]);
+  }
+  if (W)
+    for (int64_t j = tid; j < M; j += nthr) {
+      double sn, cs;
+      sincospi(2. * (double)j / (double)M, &sn, &cs);
+      W[j] = make_double2(cs, -sn);
+    }
+}
+
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, -(a.y * b.y)), fma(a.x, b.y, a.y * b.x));
+}
+__device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
+
+// One transform of C = M / kScanFftR points per CTA: the part r (mod kScanFftR)
+// of an M-point transform of which only the coefficients |k| < K are wanted.
+// Forward:
+//   X_r[j] = sum_c z[r + R c] w_C^(j c), so that X[k] = sum_r w_M^(r k) X_r[k mod C]
+// (the sum over r in k_scan_low); way back, from the Z[k] of |k| < K alone:
+//   y[r + R c] = sum_j conj(w_C)^(j c) sum_{k = j mod C} conj(w_M)^(r k) Z[k].
+// Radix-4 Stockham passes (Stockham's autosort transform) in shared memory.
+// The 6 transforms of M = 32768 points were 255 us each way as 12 real ones of
+// a library with a CTA per transform (12 of 152 SMs); 192 CTAs take 13 us.
+// The parts' number is fixed, so that the sum over r stays 32 terms; above
+// kScanFftMaxC points a part, M is enough work for the library's transforms.
+template <bool Back>
+__global__ void __launch_bounds__(kScanFftThreads)
+    k_scan_fft(const double2* __restrict__ in, double2* __restrict__ out, const double2* __restrict__ W, int64_t M,
+               int64_t K, int logC) {
+  extern __shared__ double2 sm[];
+  const int C = 1 << logC, r = blockIdx.x;
+  double2 *x = sm, *y = sm + C, *w = sm + 2 * C;
+  const int64_t row = (int64_t)blockIdx.y * M;
+  for (int j = threadIdx.x; j < C; j += blockDim.x) {
+    const double2 wc = W[(int64_t)j * kScanFftR];
+    w[j] = Back ? cconj(wc) : wc;
+    if (!Back) {
+      x[j] = in[row + r + (int64_t)kScanFftR * j];
+    } else {
+      double2 u = make_double2(0., 0.);
+      for (int64_t k = j; k < K; k += C) {
+        const double2 t = cmul(in[row + k], cconj(W[(r * k) & (M - 1)]));
+        u.x += t.x;
+        u.y += t.y;
+      }
+      for (int64_t k = C - j; k < K; k += C) {  // -k = j mod C
+        const double2 t = cmul(in[row + M - k], W[(r * k) & (M - 1)]);
+        u.x += t.x;
+        u.y += t.y;
+      }
+      x[j] = u;
+    }
+  }
+  __syncthreads();
+  int ls = 0;  // log2 of the stride
+  for (; logC - ls >= 2; ls += 2) {
+    const int s = 1 << ls, quarter = C >> 2;
+    for (int t = threadIdx.x; t < quarter; t += blockDim.x) {
+      const int q = t & (s - 1), ps = t - q;  // ps = p * s
+      const double2 a = x[t], b = x[t + quarter], c = x[t + 2 * quarter], d = x[t + 3 * quarter];
+      const double2 apc = make_double2(a.x + c.x, a.y + c.y), amc = make_double2(a.x - c.x, a.y - c.y);
+      const double2 bpd = make_double2(b.x + d.x, b.y + d.y), bmd = make_double2(b.x - d.x, b.y - d.y);
+      // -i (b - d) forward, i (b - d) back
+      const double2 jd = Back ? make_double2(-bmd.y, bmd.x) : make_double2(bmd.y, -bmd.x);
+      double2* o = y + q + 4 * ps;
+      o[0] = make_double2(apc.x + bpd.x, apc.y + bpd.y);
+      o[s] = cmul(w[ps], make_double2(amc.x + jd.x, amc.y + jd.y));
+      o[2 * s] = cmul(w[2 * ps], make_double2(apc.x - bpd.x, apc.y - bpd.y));
+      o[3 * s] = cmul(w[3 * ps], make_double2(amc.x - jd.x, amc.y - jd.y));
+    }
+    __syncthreads();
+    double2* z = x;
+    x = y;
+    y = z;
+  }
+  if (logC - ls == 1) {
+    const int s = 1 << ls;
+    for (int t = threadIdx.x; t < s; t += blockDim.x) {
+      const double2 a = x[t], b = x[t + s];
+      y[t] = make_double2(a.x + b.x, a.y + b.y);
+      y[t + s] = make_double2(a.x - b.x, a.y - b.y);
+    }
+    __syncthreads();
+    x = y;
+  }
+  for (int j = threadIdx.x; j < C; j += blockDim.x) {
+    if (Back) out[row + r + (int64_t)kScanFftR * j] = x[j];
+    else out[row + (int64_t)r * C + j] = x[j];
   }
 }
 
 // Coefficients k < K of the spectrum from the transforms of its moments, times
-// the apodization (k_scan_apod's), and the spectra of the way back.  F holds
-// kScanTerms transforms of nhalf + 1 coefficients, the rest of which is zeroed.
-__global__ void k_scan_low(ScanArgs a, double fill_n, int64_t K, int64_t M, double2* __restrict__ F) {
+// the apodization (k_scan_apod's) and `scale`, and the spectra of the way
+// back: pair q = (moments 2q, 2q+1) by warp q, 16 k's by halves of the parts.
+// With z = m_2q + i m_(2q+1), A = Z[k] and D = conj(Z[M-k]), a and b the
+// theta^p / p! of the two moments and s = (-1)^q, the pair adds
+//   s/2 ((a - b) A + (a + b) D)
+// to the coefficient w, and y_2q + i y_(2q+1) has the spectrum s (a - b) w at
+// k, s (a + b) conj(w) at -k.  R = kScanFftR parts (k_scan_fft), or 1 part (W
+// not read).
+__global__ void __launch_bounds__(32 * kScanTerms / 2)
+    k_scan_low(ScanArgs a, double fill_n, double scale, int64_t K, int64_t M, int R, const double2* __restrict__ X,
+               const double2* __restrict__ W, double2* __restrict__ Z) {
   const double PI = 3.141592653589793;
-  const int64_t mh = M / 2;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k <= mh; k += (int64_t)gridDim.x * blockDim.x) {
-    if (k >= K) {
-#pragma unroll
-      for (int p = 0; p < kScanTerms; ++p) F[p * (mh + 1) + k] = make_double2(0., 0.);
-      continue;
+  __shared__ double2 part[kScanTerms / 2][kScanLowK], tot[kScanLowK];
+  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31, kl = lane & (kScanLowK - 1);
+  const int64_t k = (int64_t)blockIdx.x * kScanLowK + kl;
+  const bool in = k < K;
+  const int64_t C = M / R, kc = k & (C - 1), kn = (C - kc) & (C - 1);
+  double2 A = make_double2(0., 0.), D = make_double2(0., 0.);
+  const double2* x = X + (int64_t)q * M;
+  if (in) {
+    if (R == 1) {
+      if (lane < kScanLowK) {
+        A = x[kc];
+        D = cconj(x[kn]);
+      }
+    } else {
+#pragma unroll 8
+      for (int i = 0; i < kScanFftR / 2; ++i) {
+        const int r = i + (lane / kScanLowK) * (kScanFftR / 2);
+        const double2 w = W[(r * k) & (M - 1)], f = x[r * C + kc], g = x[r * C + kn];
+        A.x = fma(w.x, f.x, fma(-w.y, f.y, A.x));
+        A.y = fma(w.x, f.y, fma(w.y, f.x, A.y));
+        D.x = fma(w.x, g.x, fma(w.y, g.y, D.x));
+        D.y = fma(-w.x, g.y, fma(w.y, g.x, D.y));
+      }
     }
-    const double th = PI * (double)k / (double)M;
-    // sum of (-i theta)^p / p! F_p
-    double cr = 1., wr = 0., wi = 0.;  // theta^p / p!
+  }
+  A.x += __shfl_xor_sync(0xffffffffu, A.x, kScanLowK);
+  A.y += __shfl_xor_sync(0xffffffffu, A.y, kScanLowK);
+  D.x += __shfl_xor_sync(0xffffffffu, D.x, kScanLowK);
+  D.y += __shfl_xor_sync(0xffffffffu, D.y, kScanLowK);
+  const double th = PI * (double)k / (double)M;
+  double ca = 1., cb = th;  // theta^p / p! of p = 2q and 2q + 1
+  for (int p = 1; p <= q; ++p) {
+    ca = ca * (th * th) * (1. / (double)((2 * p - 1) * (2 * p)));
+    cb = cb * (th * th) * (1. / (double)((2 * p) * (2 * p + 1)));
+  }
+  const double sg = q & 1 ? -1. : 1., cm = sg * (ca - cb), cp = sg * (ca + cb);
+  if (lane < kScanLowK)
+    part[q][kl] = make_double2(0.5 * (cm * A.x + cp * D.x), 0.5 * (cm * A.y + cp * D.y));
+  __syncthreads();
+  if (q == 0 && lane < kScanLowK && in) {
+    double wr = 0., wi = 0.;
 #pragma unroll
-    for (int p = 0; p < kScanTerms; ++p) {
-      if (p) cr = cr * th * (1. / (double)p);
-      const double2 f = F[p * (mh + 1) + k];
-      const int q = p & 3;  // (-i)^p = 1, -i, -1, i
-      const double sr = q == 0 ? f.x : q == 1 ? f.y : q == 2 ? -f.x : -f.y;
-      const double si = q == 0 ? f.y : q == 1 ? -f.x : q == 2 ? -f.y : f.x;
-      wr += cr * sr;
-      wi += cr * si;
+    for (int p = 0; p < kScanTerms / 2; ++p) {
+      wr += part[p][kl].x;
+      wi += part[p][kl].y;
     }
     if (k == 0) wr += fill_n;
     const int64_t j = k / kScanHalf, kk = k - j * kScanHalf;
-    const double x = __dadd_rn(a.X0[j], __dmul_rn((double)kk, a.DX));
-    double h = apod(a.jfn, x, a.A);
+    const double xd = __dadd_rn(a.X0[j], __dmul_rn((double)kk, a.DX));
+    double h = apod(a.jfn, xd, a.A);
     for (int e = 0; e < a.nedge; ++e)
       if (k == a.edge_k[e]) h = a.edge_v[e];
     wr *= h;
     wi *= h;
     if (a.deconv) {
-      const double z = __dmul_rn(__dmul_rn(__dmul_rn(2.0, PI), x), a.deconv_a);
+      const double z = __dmul_rn(__dmul_rn(__dmul_rn(2.0, PI), xd), a.deconv_a);
       const double d = z != 0.0 ? __ddiv_rn(z, sin(z)) : 1.0;
       wr *= d;
       wi *= d;
     }
-    cr = 1.;
-#pragma unroll
-    for (int p = 0; p < kScanTerms; ++p) {
-      if (p) cr = cr * th * (1. / (double)p);
-      const int q = p & 3;  // i^p = 1, i, -1, -i
-      const double gr = q == 0 ? wr : q == 1 ? -wi : q == 2 ? -wr : wi;
-      const double gi = q == 0 ? wi : q == 1 ? wr : q == 2 ? -wi : -wr;
-      F[p * (mh + 1) + k] = make_double2(cr * gr, cr * gi);
-    }
+    tot[kl] = make_double2(wr * scale, wi * scale);
+  }
+  __syncthreads();
+  if (lane < kScanLowK && in) {
+    const double2 w = tot[kl];
+    Z[(int64_t)q * M + k] = make_double2(cm * w.x, cm * w.y);
+    if (k > 0) Z[(int64_t)q * M + M - k] = make_double2(cp * w.x, -cp * w.y);
   }
 }
 
 // The scanned points [first, first + count): a warp per block, a lane per
-// pair of opposite points
+// pair of opposite points (13 FP64 instructions a pair bound it; 42 -> 27 us
+// with t from a table and the scale in the coefficients)
 __global__ void __launch_bounds__(kScanLowThreads)
-    k_scan_expand(const double* __restrict__ y, int64_t stride, int B, int64_t first, int64_t count, double scale,
+    k_scan_expand(const double2* __restrict__ y, int64_t M, int B, int64_t first, int64_t count,
                   double* __restrict__ out) {
+  __shared__ double T[2][kScanPowers];
+  const bool table = B / 2 <= kScanPowers;
+  if (table) scan_powers(B, T, 2);
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   const int64_t b0 = first / B, b1 = (first + count - 1) / B;
   const double rh = 2. / (double)B, c = 0.5 * (double)(B - 1);
   for (int64_t b = b0 + (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b <= b1; b += warps) {
-    double Y[kScanTerms];
+    double2 Y[kScanTerms / 2];
 #pragma unroll
-    for (int p = 0; p < kScanTerms; ++p) Y[p] = y[(int64_t)p * stride + b];
+    for (int q = 0; q < kScanTerms / 2; ++q) Y[q] = y[(int64_t)q * M + b];
     for (int j = lane; j < B / 2; j += 32) {
-      const double t = ((double)j - c) * rh, t2 = t * t;
-      double e = Y[kScanTerms - 2], o = Y[kScanTerms - 1];
+      const double t = table ? T[0][j] : ((double)j - c) * rh, t2 = table ? T[1][j] : t * t;
+      double e = Y[kScanTerms / 2 - 1].x, o = Y[kScanTerms / 2 - 1].y;
 #pragma unroll
-      for (int p = kScanTerms - 4; p >= 0; p -= 2) {
-        e = fma(e, t2, Y[p]);
-        o = fma(o, t2, Y[p + 1]);
+      for (int q = kScanTerms / 2 - 2; q >= 0; --q) {
+        e = fma(e, t2, Y[q].x);
+        o = fma(o, t2, Y[q].y);
       }
       o *= t;
       const int64_t i0 = b * B + j - first, i1 = b * B + B - 1 - j - first;
-      if (i0 >= 0 && i0 < count) out[i0] = (e + o) * scale;
-      if (i1 >= 0 && i1 < count) out[i1] = (e - o) * scale;
+      if (i0 >= 0 && i0 < count) out[i0] = e + o;
+      if (i1 >= 0 && i1 < count) out[i1] = e - o;
     }
   }
 }
+
+template __global__ void k_scan_fft<false>(const double2* __restrict__, double2* __restrict__, const double2* __restrict__,
+                                          int64_t, int64_t, int);
+template __global__ void k_scan_fft<true>(const double2* __restrict__, double2* __restrict__, const double2* __restrict__,
+                                          int64_t, int64_t, int);
 
 __global__ void k_scan_out(const double* __restrict__ y, int64_t first, int64_t count, double scale,
                            double* __restrict__ out) {

@@ -55,3 +55,12 @@ def test_data_ending_at_records_and_blocks(gpu_lib, n):
     dv = 0.0005 if n > 100000 else 0.001
     v2 = 1000.0 + dv * (n - 1)
     _check(gpu_lib, n, dv, 3, 0.8, 1000.0 + 0.3 * (v2 - 1000.0), v2)
+
+
+# transforms of 4096 to 131072 points in parts (odd and even powers of two a
+# part), and of 262144 points whole
+@pytest.mark.parametrize("n,dv,hw", [(1000000, 5e-4, 2.6), (600000, 5e-4, 1.3), (600000, 5e-4, 0.65),
+                                     (1100000, 5e-4, 0.65), (4300000, 2e-4, 0.5), (4300000, 2e-4, 0.26),
+                                     (4300000, 2e-4, 0.2)])
+def test_transform_sizes(gpu_lib, n, dv, hw):
+    _check(gpu_lib, n, dv, 5, hw, 1000.0 + 0.4 * dv * n, 1000.0 + 0.9 * dv * n, fill=0.5)
