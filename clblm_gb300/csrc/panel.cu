@@ -109,7 +109,7 @@ constexpr int kBatch = 16;  // records per staging batch of a warp
 // (ranges are kept per 16-point half tile: half tile 2t + h is lanes 16h..16h+15 of tile t)
 struct PanelTiles {
   int lo1[2 * kTiles1], hi1[2 * kTiles1], lo2[2 * kTiles2], hi2[2 * kTiles2], lo3[2 * kTiles3], hi3[2 * kTiles3];
-  GridRec wrec[kPanelWarps][kBatch];
+  GridRec wrec[kPanelWarps][kBatch];  // (mixed path: as StagedRec)
   XintPanel X;
   int layer;
 };
@@ -392,34 +392,98 @@ __device__ __forceinline__ int fast_index(int k, const GridRec& r, float* d) {
   return __float_as_int(t) - 0x4B400000;
 }
 
-// Contribution of one record at global point g of the lane (mixed path),
-// without branches: zero unless the record's range holds g and its panel is
-// at most qmax.  A hit whose FP32 index is within 1e-3 of a rounding
-// boundary, or beyond the tables, sets `bit` in *fix; the caller redoes those
+// A record as the mixed path's gather stages it, for the points at a distance
+// `pos` from the tile's first: kk = pos - f0 and the hit test 1 <= kk <= span
+// are exact FP32 (an integer kk and its conversion took a quarter of the
+// inner loop), a record that adds nothing (its panel past qmax, coupled, or
+// beyond the batch) has span 0, and thr is the largest | |ZF| - index | that
+// settles the table index.  FP32's ZF is off by at most 2^-24 (|kk ZS| +
+// |ZFL| + |ZF|) <= 2^-23 (|ZFL| + max |ZF|), 2e-4 to 7e-4 where a fixed 1e-3
+// sent twice as many terms to fix_terms; a record that may pass the tables'
+// end sends all of its own there.
+struct __align__(16) StagedRec {
+  float f0, span, zfl, zs;
+  float a0, thr, a1, a2;
+};
+static_assert(sizeof(StagedRec) == sizeof(GridRec), "staged in the records' place");
+__device__ __forceinline__ StagedRec stage_rec(const GridRec& r, int g0, int qmax, bool valid) {
+  StagedRec t;
+  const int n = r.g_hi - r.g_lo + 1;
+  t.f0 = (float)(r.g_lo - 1 - g0);
+  t.span = valid && r.q <= qmax ? (float)n : 0.f;
+  t.zfl = r.zfl;
+  t.zs = r.zs;
+  const float z1 = fabsf(r.zfl + r.zs), zn = fabsf(fmaf((float)n, r.zs, r.zfl)), top = (float)kNFMX - 0.75f;
+  const float near = 0.4999999f - 1.21e-7f * (fabsf(r.zfl) + fmaxf(z1, zn));
+  t.thr = z1 <= top && zn <= top ? fmaxf(near, 0.499f) : -1.f;
+  t.a0 = r.a0;
+  t.a1 = r.a1;
+  t.a2 = r.a2;
+  return t;
+}
+
+// The tables of a grid in shared memory, addressed by the bits of 1.5 2^23 +
+// index: 32-bit addresses less those of the bits of index 1
+constexpr uint32_t kIndexBits = 0x4B400001u;
+__device__ __forceinline__ float lds_f(uint32_t p) {
+  float v;
+  asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(p));
+  return v;
+}
+__device__ __forceinline__ float2 lds_f2(uint32_t p) {
+  float2 v;
+  asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(p));
+  return v;
+}
+struct TabAddr {
+  uint32_t a, c;
+};
+template <int GRID>
+__device__ __forceinline__ TabAddr tab_addr(const PanelSmem<false>& S) {
+  TabAddr t;
+  if constexpr (GRID == 1) {
+    t.a = smem_u32(S.tab.t1ab) - 8u * kIndexBits;
+    t.c = smem_u32(S.tab.t1c) - 4u * kIndexBits;
+  } else {
+    t.a = smem_u32(GRID == 2 ? S.tab.t2 : S.tab.t3) - 4u * kIndexBits;
+    t.c = 0;
+  }
+  return t;
+}
+
+// Adds one staged record at position pos to *s, without branches.  A hit
+// whose FP32 index is not certain sets `bit` in *fix; the caller redoes those
 // terms with the reference's FP64 index.
 template <int GRID>
-__device__ __forceinline__ float term_fast(const PanelSmem<false>& S, const GridRec& r, int g, int qmax,
-                                           unsigned* fix, unsigned bit, bool valid = true) {
-  const int kk = g - r.g_lo + 1;
-  const bool hit = valid && kk >= 1 && g <= r.g_hi && r.q <= qmax;
-  float d;
-  int iz = fast_index(kk, r, &d);
-  *fix |= (hit && (fabsf(d) > 0.499f || iz > kNFMX)) ? bit : 0u;
-  iz = min(iz, kNFMX);
-  const float v = table_term<GRID>(S, r, iz);
-  return hit ? v : 0.f;
+__device__ __forceinline__ void term_fast(const TabAddr& T, const StagedRec& r, float pos, unsigned* fix, unsigned bit,
+                                          float* s) {
+  const float kk = pos - r.f0;
+  const bool hit = kk >= 1.f && kk <= r.span;
+  const float az = fabsf(fmaf(kk, r.zs, r.zfl));
+  const float t = az + 12582913.0f;  // fast_index
+  const float d = az - (t - 12582913.0f);
+  const uint32_t ti = min(__float_as_uint(t), kIndexBits + (uint32_t)(kNFMX - 1));
+  float v;
+  if constexpr (GRID == 1) {
+    const float2 ab = lds_f2(T.a + 8u * ti);
+    v = fmaf(r.a0, ab.x, fmaf(r.a1, ab.y, __fmul_rn(r.a2, lds_f(T.c + 4u * ti))));
+  } else {
+    v = __fmul_rn(r.a0, lds_f(T.a + 4u * ti));
+  }
+  if (hit) *s = __fadd_rn(*s, v);
+  if (hit && !(fabsf(d) <= r.thr)) *fix |= bit;
 }
 
 // Correction of a batch sum for the terms flagged by term_fast: the term with
 // the FP64-exact index replaces the FP32-index one (both hits by construction)
 template <int GRID>
-__device__ __forceinline__ float fix_terms(const PanelSmem<false>& S, const GridRec* buf, int64_t base,
+__device__ __forceinline__ float fix_terms(const PanelSmem<false>& S, const GridRec* __restrict__ rec, int64_t base,
                                         const GridRecLo* __restrict__ reclo, const PanelArgs& a, int g, unsigned fix) {
   float c = 0.f;
   while (fix) {
     const int k = __ffs(fix) - 1;
     fix &= fix - 1;
-    const GridRec r = buf[k];
+    const GridRec r = rec[base + k];
     const int kk = g - r.g_lo + 1;
     float d;
     const int izf = fast_index(kk, r, &d);
@@ -441,7 +505,7 @@ __device__ __forceinline__ float fix_terms(const PanelSmem<false>& S, const Grid
 // shape with the exact index, plus its dispersion term, the shape times
 // CLCk * DPTRAT * ZF (CNVFNQ's line-coupling loop, clblm_ODLAY.f90:2195-2239)
 template <int GRID>
-__device__ __forceinline__ float cpl_terms(const PanelSmem<false>& S, const GridRec* buf, int64_t base,
+__device__ __forceinline__ float cpl_terms(const PanelSmem<false>& S, const GridRec* __restrict__ rec, int64_t base,
                                         const GridRecLo* __restrict__ reclo, const PanelArgs& a, int g, int qmax,
                                         unsigned m) {
   const float clc = GRID == 1 ? (float)kCLC1 : (GRID == 2 ? (float)kCLC2 : (float)kCLC3);
@@ -449,7 +513,7 @@ __device__ __forceinline__ float cpl_terms(const PanelSmem<false>& S, const Grid
   while (m) {
     const int k = __ffs(m) - 1;
     m &= m - 1;
-    const GridRec r = buf[k];
+    const GridRec r = rec[base + k];
     const int q = r.q & ~kCplBit;
     const int kk = g - r.g_lo + 1;
     if (kk < 1 || g > r.g_hi || q > qmax) continue;
@@ -536,7 +600,10 @@ __device__ __forceinline__ void gather_grid(PanelSmem<Plain>& S, const PanelArgs
     }
   } else {
     const int half = lane >> 4, hl = lane & 15;
-    GridRec* hb = S.wrec[warp] + half * kHalfBatch;
+    StagedRec* hb = reinterpret_cast<StagedRec*>(S.wrec[warp]) + half * kHalfBatch;
+    const TabAddr T = tab_addr<GRID>(S);
+    const int g0 = g - lane;  // the tile's first point
+    const float pos = (float)lane;
     // a half warp without an active lane sums nothing
     const unsigned act = __ballot_sync(0xffffffffu, active);
     const int n = ((act >> (16 * half)) & 0xFFFFu) ? (int)(hi - lo) : 0;
@@ -545,38 +612,35 @@ __device__ __forceinline__ void gather_grid(PanelSmem<Plain>& S, const PanelArgs
     if (hl < kHalfBatch && hl < n) nxt = rec[lo + hl];
     for (int b = 0; b < nmax; b += kHalfBatch) {
       __syncwarp();
-      if (hl < kHalfBatch) hb[hl] = nxt;
-      // the batch's coupled records: term_fast skips them (q carries kCplBit)
+      // (a coupled record's panel carries kCplBit: past qmax)
+      if (hl < kHalfBatch) hb[hl] = stage_rec(nxt, g0, qmax, b + hl < n);
       unsigned cpl_bits = 0;
       if constexpr (Cpl) cpl_bits = __ballot_sync(0xffffffffu, hl < kHalfBatch && (nxt.q & kCplBit) != 0);
       __syncwarp();
       const int cnt = min(n - b, kHalfBatch);
       if (hl < kHalfBatch && b + kHalfBatch + hl < n) nxt = rec[lo + b + kHalfBatch + hl];
-      if (!active || cnt <= 0) continue;
       unsigned fix = 0;
       float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-      if (cnt == kHalfBatch) {
+      if (nmax - b > kHalfBatch / 2) {  // (both halves alike: records past cnt add nothing)
 #pragma unroll
         for (int k = 0; k < kHalfBatch; k += 4) {
-          s0 += term_fast<GRID>(S, hb[k], g, qmax, &fix, 1u << k);
-          s1 += term_fast<GRID>(S, hb[k + 1], g, qmax, &fix, 2u << k);
-          s2 += term_fast<GRID>(S, hb[k + 2], g, qmax, &fix, 4u << k);
-          s3 += term_fast<GRID>(S, hb[k + 3], g, qmax, &fix, 8u << k);
+          term_fast<GRID>(T, hb[k], pos, &fix, 1u << k, &s0);
+          term_fast<GRID>(T, hb[k + 1], pos, &fix, 2u << k, &s1);
+          term_fast<GRID>(T, hb[k + 2], pos, &fix, 4u << k, &s2);
+          term_fast<GRID>(T, hb[k + 3], pos, &fix, 8u << k, &s3);
         }
       } else {
-        // a partial batch in groups of four; entries past cnt are masked
-        for (int k = 0; k < cnt; k += 4) {
-          s0 += term_fast<GRID>(S, hb[k], g, qmax, &fix, 1u << k);
-          s1 += term_fast<GRID>(S, hb[k + 1], g, qmax, &fix, 2u << k, k + 1 < cnt);
-          s2 += term_fast<GRID>(S, hb[k + 2], g, qmax, &fix, 4u << k, k + 2 < cnt);
-          s3 += term_fast<GRID>(S, hb[k + 3], g, qmax, &fix, 8u << k, k + 3 < cnt);
-        }
+        term_fast<GRID>(T, hb[0], pos, &fix, 1u, &s0);
+        term_fast<GRID>(T, hb[1], pos, &fix, 2u, &s1);
+        term_fast<GRID>(T, hb[2], pos, &fix, 4u, &s2);
+        term_fast<GRID>(T, hb[3], pos, &fix, 8u, &s3);
       }
+      if (!active || cnt <= 0) continue;
       float bsum = (s0 + s1) + (s2 + s3);
-      if (fix) bsum += fix_terms<GRID>(S, hb, lo + b, reclo, a, g, fix);
+      if (fix) bsum += fix_terms<GRID>(S, rec, lo + b, reclo, a, g, fix);
       if constexpr (Cpl) {
         const unsigned cm = (cpl_bits >> (16 * half)) & ((1u << cnt) - 1u);
-        if (cm) bsum += cpl_terms<GRID>(S, hb, lo + b, reclo, a, g, qmax, cm);
+        if (cm) bsum += cpl_terms<GRID>(S, rec, lo + b, reclo, a, g, qmax, cm);
       }
       acc.add(bsum);
     }
