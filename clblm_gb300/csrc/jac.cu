@@ -373,18 +373,21 @@ __global__ void __launch_bounds__(128) k_jac(JacArgs a) {
 __global__ void k_vjp_accum(const double* __restrict__ part, int nctas, int nslot, double* __restrict__ acc) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nslot) return;
-  // in the CTAs' order, their sums loaded ahead (800 dependent loads and
-  // additions took 160 us a block)
-  double sum = acc[k];
-  int c = 0;
-  for (; c + 16 <= nctas; c += 16) {
-    double v[16];
+  // sixteen chains: a binary64 addition takes 140 ns to the next, and one chain
+  // of 800 CTAs took 114 us a block
+  double v[16];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) v[q] = part[(int64_t)(c + q) * nslot + k];
+  for (int q = 0; q < 16; ++q) v[q] = 0.;
+  for (int c = 0; c < nctas; c += 16) {
 #pragma unroll
-    for (int q = 0; q < 16; ++q) sum += v[q];
+    for (int q = 0; q < 16; ++q)
+      if (c + q < nctas) v[q] += part[(int64_t)(c + q) * nslot + k];
   }
-  for (; c < nctas; ++c) sum += part[(int64_t)c * nslot + k];
+#pragma unroll
+  for (int h = 8; h > 0; h >>= 1)
+#pragma unroll
+    for (int q = 0; q < h; ++q) v[q] += v[q + h];
+  const double sum = acc[k] + v[0];
   acc[k] = sum;
 }
 

@@ -56,10 +56,10 @@ struct SumD {
 // FP32 argument lies within 1e-3 of a rounding boundary it is redone in
 // float-float (ZFL and ZSLOPE as hi + lo pairs, products and sums with their
 // exact errors, about 1e-8 absolute), and within 1e-7 of the boundary after
-// that, in FP64 with ZFL and ZSLOPE formed again from the line record `rec`
-// of this CTA's layer, as CNVFNQ's set-up forms them.
+// that, in FP64 with ZFL and ZSLOPE formed again from the line of the
+// record `off` of this CTA's layer, as CNVFNQ's set-up forms them.
 __device__ __noinline__ int table_index_near_boundary(int k, float zfl, float zs, GridRecLo lo, const PanelArgs* pa,
-                                                      int64_t rec, int q, int grid, int layer) {
+                                                      unsigned off, int grid, int layer) {
   const float kf = (float)k;
   const float p = kf * zs;
   const float pe = fmaf(kf, zs, -p);                // kf*zs = p + pe exactly
@@ -73,7 +73,8 @@ __device__ __noinline__ int table_index_near_boundary(int k, float zfl, float zs
   if (fabsf(fabsf(dd) - 0.5f) < 1e-7f) {
     // ZFkL and ZSLOPE in FP64 from the line, as the record set-up forms them
     const LayerPlan& P = pa->plans[layer + pa->layer0];
-    const LinePrep L = pa->prep[(int64_t)layer * pa->stride + rec];
+    const LinePrep L = pa->prep[(int64_t)(layer - grid + 1) * pa->stride + off];
+    const int q = pa->rec[(int64_t)layer * 3 * pa->stride + off].q & ~kCplBit;
     const CnvfnqSetup cs = cnvfnq_setup(P, pa->vft_all[P.vft_off + q], L.vnu, L.recalf, L.bhwdxf);
     const double zf64 = fma((double)k, cs.zslope, cs.zf[grid - 1]);
     return (int)(fabs(zf64) + 1.5);
@@ -105,11 +106,11 @@ constexpr int kPanelWarps = kPanelThreads / 32;
 
 // record index range [lo, hi) of every tile, one 32-record staging buffer
 // per warp, and the panel's XINT set-up
-constexpr int kBatch = 16;  // records per staging batch of a warp
+constexpr int kBatch = 16;  // records per staging batch of a warp (FP64 path), of a half warp (mixed)
 // (ranges are kept per 16-point half tile: half tile 2t + h is lanes 16h..16h+15 of tile t)
 struct PanelTiles {
   int lo1[2 * kTiles1], hi1[2 * kTiles1], lo2[2 * kTiles2], hi2[2 * kTiles2], lo3[2 * kTiles3], hi3[2 * kTiles3];
-  GridRec wrec[kPanelWarps][kBatch];  // (mixed path: as StagedRec)
+  GridRec wrec[kPanelWarps][2 * kBatch];  // (mixed path: as StagedRec)
   XintPanel X;
   int layer;
 };
@@ -124,8 +125,16 @@ struct PanelSmem<false> : PanelTiles {
   float r3n[kR3Pts];     // R3 p-frame 0..160, lines of panels <= p
   float r3o[8];          // R3 p-frame 0..7, lines of panels <= p-1
   float r2[kR2Pts];      // R2 p-frame 0..615
-  int seg_start[kMaxSeg + 1];
-  float segf_v[kMaxSeg], segf_d[kMaxSeg];
+  union {
+    struct {  // far-wing pass
+      int seg_start[kMaxSeg + 1];
+      float segf_v[kMaxSeg], segf_d[kMaxSeg];
+    };
+    struct {  // line pass
+      float r2c[kR2Pts];  // compensation of R2's line sums
+      int unit;           // next unit of the R3 and R2 line sums
+    };
+  };
   int nseg, seg_slot;  // seg_slot >= 0: the segments are in that pool slot
   uint64_t tab_bar;      // completes the table copy
   MixedTables tab;       // shape tables (one bulk copy)
@@ -369,24 +378,20 @@ __device__ __forceinline__ void tile_ranges(const int* __restrict__ pm, const in
   }
 }
 
-// Table value of record r at table index iz (mixed path)
-template <int GRID>
-__device__ __forceinline__ float table_term(const PanelSmem<false>& S, const GridRec& r, int iz) {
-  if constexpr (GRID == 1) {
+// Table value of a record at table index iz (mixed path)
+__device__ __forceinline__ float table_term(const PanelSmem<false>& S, float a0, float a1, float a2, int iz, int grid) {
+  if (grid == 1) {
     const float2 ab = S.tab.t1ab[iz - 1];
-    return fmaf(r.a0, ab.x, fmaf(r.a1, ab.y, r.a2 * S.tab.t1c[iz - 1]));
-  } else if constexpr (GRID == 2) {
-    return r.a0 * S.tab.t2[iz - 1];
-  } else {
-    return r.a0 * S.tab.t3[iz - 1];
+    return fmaf(a0, ab.x, fmaf(a1, ab.y, a2 * S.tab.t1c[iz - 1]));
   }
+  return a0 * (grid == 2 ? S.tab.t2 : S.tab.t3)[iz - 1];
 }
 
 // FP32 table index rint(|ZF|) + 1 = INT(|ZF| + 1.5) away from ties, and the
 // distance d = |ZF| - rint(|ZF|) (exact) that tells how near the rounding
 // boundary |d| = 0.5 the FP32 argument lies.  Always >= 1.
-__device__ __forceinline__ int fast_index(int k, const GridRec& r, float* d) {
-  const float az = fabsf(fmaf((float)k, r.zs, r.zfl));
+__device__ __forceinline__ int fast_index(float k, float zfl, float zs, float* d) {
+  const float az = fabsf(fmaf(k, zs, zfl));
   const float t = az + 12582913.0f;            // 1.5*2^23 + 1: rounds |ZF| + 1
   *d = az - (t - 12582913.0f);
   return __float_as_int(t) - 0x4B400000;
@@ -413,9 +418,10 @@ __device__ __forceinline__ StagedRec stage_rec(const GridRec& r, int g0, int qma
   t.span = valid && r.q <= qmax ? (float)n : 0.f;
   t.zfl = r.zfl;
   t.zs = r.zs;
-  const float z1 = fabsf(r.zfl + r.zs), zn = fabsf(fmaf((float)n, r.zs, r.zfl)), top = (float)kNFMX - 0.75f;
-  const float near = 0.4999999f - 1.21e-7f * (fabsf(r.zfl) + fmaxf(z1, zn));
-  t.thr = z1 <= top && zn <= top ? fmaxf(near, 0.499f) : -1.f;
+  // |ZF| over kk = 0 .. n is largest at an end
+  const float z0 = fabsf(r.zfl), zn = fabsf(fmaf((float)n, r.zs, r.zfl)), top = (float)kNFMX - 0.75f;
+  const float near = 0.4999999f - 1.21e-7f * (z0 + fmaxf(z0, zn));
+  t.thr = z0 <= top && zn <= top ? fmaxf(near, 0.499f) : -1.f;
   t.a0 = r.a0;
   t.a1 = r.a1;
   t.a2 = r.a2;
@@ -438,14 +444,13 @@ __device__ __forceinline__ float2 lds_f2(uint32_t p) {
 struct TabAddr {
   uint32_t a, c;
 };
-template <int GRID>
-__device__ __forceinline__ TabAddr tab_addr(const PanelSmem<false>& S) {
+__device__ __forceinline__ TabAddr tab_addr(const PanelSmem<false>& S, int grid) {
   TabAddr t;
-  if constexpr (GRID == 1) {
+  if (grid == 1) {
     t.a = smem_u32(S.tab.t1ab) - 8u * kIndexBits;
     t.c = smem_u32(S.tab.t1c) - 4u * kIndexBits;
   } else {
-    t.a = smem_u32(GRID == 2 ? S.tab.t2 : S.tab.t3) - 4u * kIndexBits;
+    t.a = smem_u32(grid == 2 ? S.tab.t2 : S.tab.t3) - 4u * kIndexBits;
     t.c = 0;
   }
   return t;
@@ -454,7 +459,7 @@ __device__ __forceinline__ TabAddr tab_addr(const PanelSmem<false>& S) {
 // Adds one staged record at position pos to *s, without branches.  A hit
 // whose FP32 index is not certain sets `bit` in *fix; the caller redoes those
 // terms with the reference's FP64 index.
-template <int GRID>
+template <bool R1>
 __device__ __forceinline__ void term_fast(const TabAddr& T, const StagedRec& r, float pos, unsigned* fix, unsigned bit,
                                           float* s) {
   const float kk = pos - r.f0;
@@ -464,7 +469,7 @@ __device__ __forceinline__ void term_fast(const TabAddr& T, const StagedRec& r, 
   const float d = az - (t - 12582913.0f);
   const uint32_t ti = min(__float_as_uint(t), kIndexBits + (uint32_t)(kNFMX - 1));
   float v;
-  if constexpr (GRID == 1) {
+  if constexpr (R1) {
     const float2 ab = lds_f2(T.a + 8u * ti);
     v = fmaf(r.a0, ab.x, fmaf(r.a1, ab.y, __fmul_rn(r.a2, lds_f(T.c + 4u * ti))));
   } else {
@@ -475,27 +480,28 @@ __device__ __forceinline__ void term_fast(const TabAddr& T, const StagedRec& r, 
 }
 
 // Correction of a batch sum for the terms flagged by term_fast: the term with
-// the FP64-exact index replaces the FP32-index one (both hits by construction)
-template <int GRID>
-__device__ __forceinline__ float fix_terms(const PanelSmem<false>& S, const GridRec* __restrict__ rec, int64_t base,
-                                        const GridRecLo* __restrict__ reclo, const PanelArgs& a, int g, unsigned fix) {
+// the FP64-exact index replaces the FP32-index one (both hits by construction).
+// buf: the staged batch, off: its first record among the layer's of all grids
+__device__ __forceinline__ float fix_terms(const PanelSmem<false>& S, const StagedRec* buf,
+                                           const GridRecLo* __restrict__ reclo, const PanelArgs& a, unsigned off,
+                                           float pos, unsigned fix, int grid) {
   float c = 0.f;
   while (fix) {
     const int k = __ffs(fix) - 1;
     fix &= fix - 1;
-    const GridRec r = rec[base + k];
-    const int kk = g - r.g_lo + 1;
+    const GridRecLo l = reclo[off + k];
+    const StagedRec r = buf[k];
+    const float kk = pos - r.f0;
     float d;
-    const int izf = fast_index(kk, r, &d);
-    const float vf = table_term<GRID>(S, r, min(izf, kNFMX));
-    const int iz = fabsf(d) > 0.499f
-                       ? table_index_near_boundary(kk, r.zfl, r.zs, reclo[base + k], &a, base + k, r.q, GRID, S.layer)
-                       : izf;
+    const int izf = fast_index(kk, r.zfl, r.zs, &d);
+    const float vf = table_term(S, r.a0, r.a1, r.a2, min(izf, kNFMX), grid);
+    const int iz =
+        fabsf(d) > 0.499f ? table_index_near_boundary((int)kk, r.zfl, r.zs, l, &a, off + k, grid, S.layer) : izf;
     if (iz > kNFMX) {
       atomicOr(a.err, 2);
       c -= vf;
     } else if (iz != izf) {
-      c += table_term<GRID>(S, r, iz) - vf;
+      c += table_term(S, r.a0, r.a1, r.a2, iz, grid) - vf;
     }
   }
   return c;
@@ -504,143 +510,159 @@ __device__ __forceinline__ float fix_terms(const PanelSmem<false>& S, const Grid
 // The terms of the coupled records (bits of m) at point g (mixed path): the
 // shape with the exact index, plus its dispersion term, the shape times
 // CLCk * DPTRAT * ZF (CNVFNQ's line-coupling loop, clblm_ODLAY.f90:2195-2239)
-template <int GRID>
-__device__ __forceinline__ float cpl_terms(const PanelSmem<false>& S, const GridRec* __restrict__ rec, int64_t base,
+__device__ __forceinline__ float cpl_terms(const PanelSmem<false>& S, const GridRec* __restrict__ rec, unsigned off,
                                         const GridRecLo* __restrict__ reclo, const PanelArgs& a, int g, int qmax,
-                                        unsigned m) {
-  const float clc = GRID == 1 ? (float)kCLC1 : (GRID == 2 ? (float)kCLC2 : (float)kCLC3);
+                                        unsigned m, int grid) {
+  const float clc = grid == 1 ? (float)kCLC1 : (grid == 2 ? (float)kCLC2 : (float)kCLC3);
   float c = 0.f;
   while (m) {
     const int k = __ffs(m) - 1;
     m &= m - 1;
-    const GridRec r = rec[base + k];
+    const GridRec r = rec[off + k];
     const int q = r.q & ~kCplBit;
     const int kk = g - r.g_lo + 1;
     if (kk < 1 || g > r.g_hi || q > qmax) continue;
     float d;
-    int iz = fast_index(kk, r, &d);
-    if (fabsf(d) > 0.499f) iz = table_index_near_boundary(kk, r.zfl, r.zs, reclo[base + k], &a, base + k, q, GRID, S.layer);
+    int iz = fast_index((float)kk, r.zfl, r.zs, &d);
+    if (fabsf(d) > 0.499f)
+      iz = table_index_near_boundary(kk, r.zfl, r.zs, reclo[off + k], &a, off + k, grid, S.layer);
     if (iz > kNFMX) {
       atomicOr(a.err, 2);
       continue;
     }
-    const float v = table_term<GRID>(S, r, iz);
+    const float v = table_term(S, r.a0, r.a1, r.a2, iz, grid);
     const float zf = fmaf((float)kk, r.zs, r.zfl);
-    const float dpt = (float)a.cpl[(int64_t)S.layer * a.stride + base + k];
+    const float dpt = (float)a.cpl[(int64_t)(S.layer - grid + 1) * a.stride + off + k];
     c += v + (v * (clc * dpt)) * zf;
   }
   return c;
 }
 
-// Sum over the records [lo, hi) of one grid at global point g of the lane.
-// FP64 path: [lo, hi) is the warp's 32-point tile's; the records pass through
-// the warp's shared-memory buffer kBatch at a time (the next batch already in
-// registers) and are added one by one in record order.  Mixed path: [lo, hi)
-// is the lane's 16-point half tile's, so each half warp sums only the records
-// that reach its half (narrow lines reach a few points: a 32-point range
-// would pair most records with lanes they miss); the halves stage
-// kHalfBatch records each, every batch is summed in FP32 (four partial sums)
-// and added to the Kahan sum.
-constexpr int kHalfBatch = kBatch / 2;
-template <bool Plain, int GRID, bool Cpl>
-__device__ __forceinline__ void gather_grid(PanelSmem<Plain>& S, const PanelArgs& a, const GridRec* __restrict__ rec,
-                                            const GridRecD* __restrict__ recd, const GridRecLo* __restrict__ reclo,
-                                            int64_t lo, int64_t hi, int g, bool active, int qmax,
-                                            typename std::conditional<Plain, SumD, KahanF>::type& acc) {
+// Sum over the records [lo, hi) of a 32-point tile of one grid at global point
+// g of the lane, FP64 path: the records pass through the warp's shared-memory
+// buffer kBatch at a time (the next batch already in registers) and are added
+// one by one in record order.
+template <int GRID, bool Cpl>
+__device__ __forceinline__ void gather_plain(PanelSmem<true>& S, const PanelArgs& a, const GridRec* __restrict__ rec,
+                                             const GridRecD* __restrict__ recd, int64_t lo, int64_t hi, int g,
+                                             bool active, int qmax, SumD& acc) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if constexpr (Plain) {
-    const int sl = lane & (kBatch - 1);
-    GridRec* buf = S.wrec[warp];
-    GridRec nxt;
-    GridRecD nxtd;
-    if (lo + sl < hi) {
-      nxt = rec[lo + sl];
-      nxtd = recd[lo + sl];
+  const int sl = lane & (kBatch - 1);
+  GridRec* buf = S.wrec[warp];
+  GridRec nxt;
+  GridRecD nxtd;
+  if (lo + sl < hi) {
+    nxt = rec[lo + sl];
+    nxtd = recd[lo + sl];
+  }
+  for (int64_t base = lo; base < hi; base += kBatch) {
+    __syncwarp();
+    if (lane < kBatch) {
+      buf[lane] = nxt;
+      S.wrecd[warp][lane] = nxtd;
     }
-    for (int64_t base = lo; base < hi; base += kBatch) {
-      __syncwarp();
-      if (lane < kBatch) {
-        buf[lane] = nxt;
-        S.wrecd[warp][lane] = nxtd;
+    __syncwarp();
+    const int cnt = (int)(hi - base < kBatch ? hi - base : kBatch);
+    if (base + kBatch + sl < hi) {
+      nxt = rec[base + kBatch + sl];
+      nxtd = recd[base + kBatch + sl];
+    }
+    if (!active) continue;
+    for (int k = 0; k < cnt; ++k) {
+      const GridRec r = buf[k];
+      if (g < r.g_lo || g > r.g_hi || (Cpl ? (r.q & ~kCplBit) : r.q) > qmax) continue;
+      const GridRecD& d = S.wrecd[warp][k];
+      const double zf = fma((double)(g - r.g_lo + 1), d.zs, d.zfl);
+      const int iz = (int)(fabs(zf) + 1.5);
+      if (iz > kNFMX) {
+        atomicOr(a.err, 2);
+        continue;
       }
-      __syncwarp();
-      const int cnt = (int)(hi - base < kBatch ? hi - base : kBatch);
-      if (base + kBatch + sl < hi) {
-        nxt = rec[base + kBatch + sl];
-        nxtd = recd[base + kBatch + sl];
-      }
-      if (!active) continue;
-      for (int k = 0; k < cnt; ++k) {
-        const GridRec r = buf[k];
-        if (g < r.g_lo || g > r.g_hi || (Cpl ? (r.q & ~kCplBit) : r.q) > qmax) continue;
-        const GridRecD& d = S.wrecd[warp][k];
-        const double zf = fma((double)(g - r.g_lo + 1), d.zs, d.zfl);
-        const int iz = (int)(fabs(zf) + 1.5);
-        if (iz > kNFMX) {
-          atomicOr(a.err, 2);
-          continue;
-        }
-        // a coupled line adds its dispersion term: the strengths times CLCk
-        // times DPTRAT, the shape times ZF (clblm_ODLAY.f90:2195-2239)
-        const double dpt = (Cpl && (r.q & kCplBit)) ? a.cpl[(int64_t)S.layer * a.stride + base + k] : 0.;
-        if constexpr (GRID == 1) {
-          const double* T = S.t1 + 3 * (iz - 1);
-          acc.add(d.a0 * T[0] + d.a1 * T[1] + d.a2 * T[2]);
-          if (dpt != 0.)
-            acc.add((((d.a0 * kCLC1) * dpt) * T[0] + ((d.a1 * kCLC1) * dpt) * T[1] + ((d.a2 * kCLC1) * dpt) * T[2]) *
-                    zf);
-        } else if constexpr (GRID == 2) {
-          acc.add(d.a0 * S.t2[iz - 1]);
-          if (dpt != 0.) acc.add((((d.a0 * kCLC2) * dpt) * S.t2[iz - 1]) * zf);
-        } else {
-          acc.add(d.a0 * S.t3[iz - 1]);
-          if (dpt != 0.) acc.add((((d.a0 * kCLC3) * dpt) * S.t3[iz - 1]) * zf);
-        }
+      // a coupled line adds its dispersion term: the strengths times CLCk
+      // times DPTRAT, the shape times ZF (clblm_ODLAY.f90:2195-2239)
+      const double dpt = (Cpl && (r.q & kCplBit)) ? a.cpl[(int64_t)S.layer * a.stride + base + k] : 0.;
+      if constexpr (GRID == 1) {
+        const double* T = S.t1 + 3 * (iz - 1);
+        acc.add(d.a0 * T[0] + d.a1 * T[1] + d.a2 * T[2]);
+        if (dpt != 0.)
+          acc.add((((d.a0 * kCLC1) * dpt) * T[0] + ((d.a1 * kCLC1) * dpt) * T[1] + ((d.a2 * kCLC1) * dpt) * T[2]) *
+                  zf);
+      } else if constexpr (GRID == 2) {
+        acc.add(d.a0 * S.t2[iz - 1]);
+        if (dpt != 0.) acc.add((((d.a0 * kCLC2) * dpt) * S.t2[iz - 1]) * zf);
+      } else {
+        acc.add(d.a0 * S.t3[iz - 1]);
+        if (dpt != 0.) acc.add((((d.a0 * kCLC3) * dpt) * S.t3[iz - 1]) * zf);
       }
     }
-  } else {
-    const int half = lane >> 4, hl = lane & 15;
-    StagedRec* hb = reinterpret_cast<StagedRec*>(S.wrec[warp]) + half * kHalfBatch;
-    const TabAddr T = tab_addr<GRID>(S);
-    const int g0 = g - lane;  // the tile's first point
-    const float pos = (float)lane;
-    // a half warp without an active lane sums nothing
-    const unsigned act = __ballot_sync(0xffffffffu, active);
-    const int n = ((act >> (16 * half)) & 0xFFFFu) ? (int)(hi - lo) : 0;
-    const int nmax = max(n, __shfl_xor_sync(0xffffffffu, n, 16));  // the warp's batch loop
-    GridRec nxt = {};
-    if (hl < kHalfBatch && hl < n) nxt = rec[lo + hl];
-    for (int b = 0; b < nmax; b += kHalfBatch) {
-      __syncwarp();
-      // (a coupled record's panel carries kCplBit: past qmax)
-      if (hl < kHalfBatch) hb[hl] = stage_rec(nxt, g0, qmax, b + hl < n);
-      unsigned cpl_bits = 0;
-      if constexpr (Cpl) cpl_bits = __ballot_sync(0xffffffffu, hl < kHalfBatch && (nxt.q & kCplBit) != 0);
-      __syncwarp();
-      const int cnt = min(n - b, kHalfBatch);
-      if (hl < kHalfBatch && b + kHalfBatch + hl < n) nxt = rec[lo + b + kHalfBatch + hl];
+  }
+  __syncwarp();
+}
+
+// Mixed path: a unit of the line pass is a 32-point tile of one grid; its two
+// halves sum the records of their own 16-point half tile (narrow lines reach a
+// few points: a 32-point range would pair most records with lanes they miss),
+// kHalfBatch at a time in FP32 (four partial sums) and then into the Kahan
+// sum.  A lane of the half stages one record, so two such groups are staged at
+// once (staging is as many instructions as three terms).  `nxt` holds the
+// lane's record of the unit's first batch on entry, of the next unit's on
+// return: a thin layer's tiles have a record or two, and each unit waited for a
+// load.
+constexpr int kHalfBatch = kBatch / 2;
+struct MixedUnit {  // of a lane's half
+  unsigned off;  // first record among the layer's of all grids
+  int n;
+};
+__device__ __forceinline__ GridRec unit_first(const GridRec* __restrict__ rec, const MixedUnit& u) {
+  const unsigned hl = threadIdx.x & 15;
+  GridRec r = {};
+  if ((int)hl < u.n) r = rec[u.off + hl];
+  return r;
+}
+template <bool R1, bool Cpl>
+__device__ __forceinline__ void gather_mixed(PanelSmem<false>& S, const PanelArgs& a, const MixedUnit& u,
+                                             const MixedUnit& next, const GridRec* __restrict__ rec,
+                                             const GridRecLo* __restrict__ reclo, int grid, int g, bool active,
+                                             int qmax, GridRec& nxt, KahanF& acc) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int half = lane >> 4, hl = lane & 15, n = u.n;
+  StagedRec* buf = reinterpret_cast<StagedRec*>(S.wrec[warp]) + half * kBatch;
+  const TabAddr T = tab_addr(S, R1 ? 1 : grid);
+  const int g0 = g - lane;  // the tile's first point
+  const float pos = (float)lane;
+  const int nmax = max(n, __shfl_xor_sync(0xffffffffu, n, 16));  // the warp's batch loop
+  if (nmax <= 0) nxt = unit_first(rec, next);
+  for (int b = 0; b < nmax; b += kBatch) {
+    __syncwarp();
+    // (a coupled record's panel carries kCplBit: past qmax)
+    buf[hl] = stage_rec(nxt, g0, qmax, b + hl < n);
+    unsigned cpl_bits = 0;
+    if constexpr (Cpl) cpl_bits = __ballot_sync(0xffffffffu, (nxt.q & kCplBit) != 0);
+    __syncwarp();
+    if (b + kBatch >= nmax) nxt = unit_first(rec, next);
+    else if (b + kBatch + hl < n) nxt = rec[u.off + (unsigned)(b + kBatch + hl)];
+    const int bend = min(b + kBatch, nmax);
+#pragma unroll 1
+    for (int c = b; c < bend; c += kHalfBatch) {
+      const StagedRec* hb = buf + (c - b);
       unsigned fix = 0;
       float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-      if (nmax - b > kHalfBatch / 2) {  // (both halves alike: records past cnt add nothing)
-#pragma unroll
-        for (int k = 0; k < kHalfBatch; k += 4) {
-          term_fast<GRID>(T, hb[k], pos, &fix, 1u << k, &s0);
-          term_fast<GRID>(T, hb[k + 1], pos, &fix, 2u << k, &s1);
-          term_fast<GRID>(T, hb[k + 2], pos, &fix, 4u << k, &s2);
-          term_fast<GRID>(T, hb[k + 3], pos, &fix, 8u << k, &s3);
-        }
-      } else {
-        term_fast<GRID>(T, hb[0], pos, &fix, 1u, &s0);
-        term_fast<GRID>(T, hb[1], pos, &fix, 2u, &s1);
-        term_fast<GRID>(T, hb[2], pos, &fix, 4u, &s2);
-        term_fast<GRID>(T, hb[3], pos, &fix, 8u, &s3);
+      term_fast<R1>(T, hb[0], pos, &fix, 1u, &s0);
+      term_fast<R1>(T, hb[1], pos, &fix, 2u, &s1);
+      term_fast<R1>(T, hb[2], pos, &fix, 4u, &s2);
+      term_fast<R1>(T, hb[3], pos, &fix, 8u, &s3);
+      if (bend - c > kHalfBatch / 2) {  // (both halves alike: records past n add nothing)
+        term_fast<R1>(T, hb[4], pos, &fix, 16u, &s0);
+        term_fast<R1>(T, hb[5], pos, &fix, 32u, &s1);
+        term_fast<R1>(T, hb[6], pos, &fix, 64u, &s2);
+        term_fast<R1>(T, hb[7], pos, &fix, 128u, &s3);
       }
-      if (!active || cnt <= 0) continue;
+      if (!active || c >= n) continue;
       float bsum = (s0 + s1) + (s2 + s3);
-      if (fix) bsum += fix_terms<GRID>(S, rec, lo + b, reclo, a, g, fix);
+      if (fix) bsum += fix_terms(S, hb, reclo, a, u.off + c, pos, fix, R1 ? 1 : grid);
       if constexpr (Cpl) {
-        const unsigned cm = (cpl_bits >> (16 * half)) & ((1u << cnt) - 1u);
-        if (cm) bsum += cpl_terms<GRID>(S, rec, lo + b, reclo, a, g, qmax, cm);
+        const unsigned cm = (cpl_bits >> (16 * half + c - b)) & ((1u << min(n - c, kHalfBatch)) - 1u);
+        if (cm) bsum += cpl_terms(S, rec, u.off + c, reclo, a, g, qmax, cm, R1 ? 1 : grid);
       }
       acc.add(bsum);
     }
@@ -682,7 +704,10 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
   const int nslice = P.nslice;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) S.layer = layer;
+  if (tid == 0) {
+    S.layer = layer;
+    if constexpr (kLines && !Plain) S.unit = kPanelWarps;
+  }
   const double dv = P.dv;
   const double* vft = a.vft_all + P.vft_off;
   const double VFT = vft[p];
@@ -724,8 +749,6 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
   const GridRecD* rd2 = rd1 + a.stride;
   const GridRecD* rd3 = rd2 + a.stride;
   const GridRecLo* rl1 = a.reclo + (int64_t)layer * a.stride * 3;
-  const GridRecLo* rl2 = rl1 + a.stride;
-  const GridRecLo* rl3 = rl2 + a.stride;
   const int64_t* rg = a.ranges + ((int64_t)layer * a.panel_stride + p) * 6;
   const int* pm1 = a.pmax_g + (int64_t)layer * a.stride * 3;
   const int* sm1 = a.smin_g + (int64_t)layer * a.stride * 3;
@@ -745,9 +768,9 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
     }
   }
   // a slice's share of the records [lo, hi) of a tile
-  auto share = [&](int64_t* lo, int64_t* hi) {
+  auto share = [&](int* lo, int* hi) {
     if (nslice > 1) {
-      const int n = (int)(*hi - *lo), q = n / nslice, r = n - q * nslice;
+      const int n = *hi - *lo, q = n / nslice, r = n - q * nslice;
       *lo += q * slice + min(slice, r);
       *hi = *lo + q + (slice < r ? 1 : 0);
     }
@@ -915,20 +938,93 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
     S.nseg = ns;
     S.seg_slot = slot;
   }
-  for (int u = warp; u <= kTiles3; u += kPanelWarps) {
+  // Mixed line pass: the units of R3 and R2, which are independent of each
+  // other, go to whichever warp is free (the R3 units of 160 points hold as
+  // much work as the four times as many of R2: as phases of their own the CTA
+  // waited a fifth of its time for the last warp); R1's follow by tile, the
+  // first of each warp loaded before the barrier.
+  MixedUnit nu = {};
+  GridRec nxt = {};
+  auto unit_of = [&](int grid, const int* L, const int* H, int h, bool active) {
+    const unsigned act = __ballot_sync(0xffffffffu, active);
+    int lo = L[h], hi = max(L[h], H[h]);
+    share(&lo, &hi);
+    MixedUnit m;
+    m.off = (unsigned)((grid - 1) * a.stride + lo);
+    m.n = ((act >> (lane & 16)) & 0xFFFFu) ? hi - lo : 0;  // a half without an active lane sums nothing
+    return m;
+  };
+  auto unit1 = [&](int tile) {
+    const bool in = tile < nT1;
+    return unit_of(1, S.lo1, S.hi1, in ? 2 * tile + (lane >> 4) : 0,
+                   in && kNSHIFT + 1 + tile * 32 + lane <= NHI);
+  };
+  if constexpr (kLines && !Plain) {
+    // p-frame index of unit u, and whether it is a point of the unit
+    auto point = [&](int u, bool* active) {
+      int J;
+      if (u < kTiles3) {
+        J = u * 32 + lane;
+        *active = J < kR3Pts;
+      } else if (u == kTiles3) {  // the 8 old points
+        J = lane;
+        *active = J < 8 && p > 0;
+      } else {
+        J = (u - kTiles3 - 1) * 32 + lane;
+        *active = J >= 5 && J < kR2Pts;
+      }
+      return J;
+    };
+    constexpr int kUnits = kTiles3 + 1 + kTiles2;
+    auto unit32 = [&](int u) {
+      bool active;
+      point(u, &active);
+      if (u >= kUnits) return unit_of(3, S.lo3, S.hi3, 0, false);
+      const int h = lane >> 4;
+      if (u <= kTiles3) return unit_of(3, S.lo3, S.hi3, (u < kTiles3 ? 2 * u : 0) + h, active);
+      return unit_of(2, S.lo2, S.hi2, 2 * (u - kTiles3 - 1) + h, active);
+    };
+    auto take = [&] {
+      int u = 0;
+      if (lane == 0) u = atomicAdd(&S.unit, 1);
+      return __shfl_sync(0xffffffffu, u, 0);
+    };
+    int u = warp;
+    nu = unit32(u);
+    nxt = unit_first(rec1, nu);
+    while (u < kUnits) {
+      const int un = take();
+      const MixedUnit cur = nu;
+      nu = un < kUnits ? unit32(un) : unit1(warp);
+      bool active;
+      const int J = point(u, &active);
+      KahanF acc;
+      const bool r3 = u <= kTiles3, old = u == kTiles3;
+      gather_mixed<false, Cpl>(S, a, cur, nu, rec1, rl1, r3 ? 3 : 2, (r3 ? kPanelR3 : kPanelR2) * p + J - 1, active,
+                               old ? p - 1 : p, nxt, acc);
+      if (active) {
+        if (old) S.r3o[J] = acc.value();
+        else if (r3) S.r3n[J] = acc.value();
+        else {
+          S.r2[J] = acc.s;
+          S.r2c[J] = acc.c;
+        }
+      }
+      u = un;
+    }
+  }
+  for (int u = warp; u <= kTiles3 && (Plain || kWings); u += kPanelWarps) {
     const bool old = (u == kTiles3);
     const int J3 = old ? lane : u * 32 + lane;  // p-frame index
     const bool active = old ? (J3 < 8 && p > 0) : (J3 < kR3Pts);
     const int qmax = old ? p - 1 : p;
     const int g = kPanelR3 * p + J3 - 1;
     const int t = old ? 0 : u;
-    // the FP64 path: the 32-point tile's range; mixed: the lane's half tile's
-    const int h0 = 2 * t + (Plain ? 0 : (lane >> 4)), h1 = Plain ? 2 * t + 1 : h0;
     Acc acc;
-    if constexpr (kLines) {
-      int64_t lo = S.lo3[h0], hi = max(S.lo3[h0], S.hi3[h1]);
+    if constexpr (kLines && Plain) {
+      int lo = S.lo3[2 * t], hi = max(S.lo3[2 * t], S.hi3[2 * t + 1]);
       share(&lo, &hi);
-      gather_grid<Plain, 3, Cpl>(S, a, rec3, rd3, rl3, lo, hi, g, active, qmax, acc);
+      gather_plain<3, Cpl>(S, a, rec3, rd3, lo, hi, g, active, qmax, acc);
     }
     if (active && kWings) {
       // far wings (R4) and continuum (ABSRB) interpolated into R3 (XINT).
@@ -1012,11 +1108,14 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
       bool active = J >= 5 && J < kR2Pts;
       int g = kPanelR2 * p + J - 1;
       Acc acc;
-      const int h0 = 2 * tile + (Plain ? 0 : (lane >> 4)), h1 = Plain ? 2 * tile + 1 : h0;
-      if constexpr (kLines) {
-        int64_t lo = S.lo2[h0], hi = max(S.lo2[h0], S.hi2[h1]);
+      if constexpr (kLines && Plain) {
+        int lo = S.lo2[2 * tile], hi = max(S.lo2[2 * tile], S.hi2[2 * tile + 1]);
         share(&lo, &hi);
-        gather_grid<Plain, 2, Cpl>(S, a, rec2, rd2, rl2, lo, hi, g, active, p, acc);
+        gather_plain<2, Cpl>(S, a, rec2, rd2, lo, hi, g, active, p, acc);
+      }
+      if constexpr (kLines && !Plain) {
+        acc.s = active ? S.r2[J] : 0.f;
+        acc.c = active ? S.r2c[J] : 0.f;
       }
       if (active) {
         int off = (J - 1) & 3;
@@ -1056,11 +1155,15 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
       bool active = J <= NHI;
       int g = kPanelPts * p + J - 1;
       Acc acc;
-      const int h0 = 2 * tile + (Plain ? 0 : (lane >> 4)), h1 = Plain ? 2 * tile + 1 : h0;
-      if constexpr (kLines) {
-        int64_t lo = S.lo1[h0], hi = max(S.lo1[h0], S.hi1[h1]);
+      if constexpr (kLines && Plain) {
+        int lo = S.lo1[2 * tile], hi = max(S.lo1[2 * tile], S.hi1[2 * tile + 1]);
         share(&lo, &hi);
-        gather_grid<Plain, 1, Cpl>(S, a, rec1, rd1, rl1, lo, hi, g, active, p, acc);
+        gather_plain<1, Cpl>(S, a, rec1, rd1, lo, hi, g, active, p, acc);
+      }
+      if constexpr (kLines && !Plain) {
+        const MixedUnit cur = nu;
+        nu = unit1(tile + kPanelWarps);
+        gather_mixed<true, Cpl>(S, a, cur, nu, rec1, rl1, 1, g, active, p, nxt, acc);
       }
       if (active) {
         int off = (J - 33) & 3;
