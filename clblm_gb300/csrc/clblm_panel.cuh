@@ -13,6 +13,19 @@ constexpr int kR3Pts = 161;  // R3 p-frame 0..160
 constexpr int kR2Pts = 616;  // R2 p-frame 0..615
 constexpr int kMaxSeg = 256; // radiation-term segments per panel
 
+// XINT set-up of one panel (clblm_Spectrum.f90:874-915 as called by HIRACQ,
+// clblm_ODLAY.f90:1451-1459): the R4 blocks in use (index 0: the previous
+// panel's, for the carried points 1..5; 1: this panel's), the R3 index
+// limits of both interpolations and the reciprocal spacings
+struct XintPanel {
+  double v1r4[2], recdva4, recdvab;
+  long long m0[2];
+  int nptr4[2], ilo4[2], ihi4[2], blk[2];
+  int iloab, ihiab;
+  int ab0, nab;  // mixed path: ABSRB(ab0 .. ab0+nab-1) staged as FP32 (nab = 0: read from global)
+};
+constexpr int kAbsStage = 64;
+
 struct PanelArgs {
   const LayerPlan* plans;
   int layer0;
@@ -38,7 +51,8 @@ struct PanelArgs {
   const int* pmax_g;         // per grid: running max of g_hi over the records
   const int* smin_g;         // per grid: running min (from the right) of g_lo
   int* err;
-  // radiation-term segments of each panel (k_panel_segs)
+  // radiation-term segments and XINT set-up of each panel (k_panel_setup)
+  const XintPanel* xint;
   const int* seg_n;
   const int* seg_start;
   const double2* seg_v;
@@ -107,10 +121,11 @@ size_t panel_smem_bytes(bool plain, bool wings = false);  // wings: the mixed fa
 constexpr int kRadfacWarps = 4;
 __global__ void __launch_bounds__(32 * kRadfacWarps)
     k_r4_radfac(const LayerPlan* plans, int layer0, const double* blk_v1, const int* blk_n, double* blk_fac);
-constexpr int kSegTab = 24;  // radiation-term segments of a panel held by k_panel_segs
+constexpr int kSegTab = 24;  // radiation-term segments of a panel held by k_panel_setup
 __global__ void __launch_bounds__(64)
-    k_panel_segs(const LayerPlan* plans, int layer0, const double* vft_all, int64_t stride, int* seg_n, int* seg_start,
-                 double2* seg_v);
+    k_panel_setup(const LayerPlan* plans, int layer0, const double* vft_all, int64_t stride, const int* panel_blk,
+                  const double* blk_v1, const int* blk_n, const int64_t* blk_m0, int* seg_n, int* seg_start,
+                  double2* seg_v, XintPanel* xint);
 
 // the passes of k_panel: the line sums (kPanelLines), then the far wings, the
 // continuum and the radiation term (kPanelWings)

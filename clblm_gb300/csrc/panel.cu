@@ -82,19 +82,6 @@ __device__ __noinline__ int table_index_near_boundary(int k, float zfl, float zs
   return (int)n + 1 + (dd >= 0.5f ? 1 : (dd < -0.5f ? -1 : 0));
 }
 
-// XINT set-up of one panel (clblm_Spectrum.f90:874-915 as called by HIRACQ,
-// clblm_ODLAY.f90:1451-1459): the R4 blocks in use (index 0: the previous
-// panel's, for the carried points 1..5; 1: this panel's), the R3 index
-// limits of both interpolations and the reciprocal spacings
-struct XintPanel {
-  double v1r4[2], recdva4, recdvab;
-  long long m0[2];
-  int nptr4[2], ilo4[2], ihi4[2], blk[2];
-  int iloab, ihiab;
-  int ab0, nab;  // mixed path: ABSRB(ab0 .. ab0+nab-1) staged as FP32 (nab = 0: read from global)
-};
-constexpr int kAbsStage = 64;
-
 // ---------------------------------------------------------------------------
 // shared-memory layout of k_panel
 template <bool Plain>
@@ -288,20 +275,63 @@ __global__ void __launch_bounds__(32 * kRadfacWarps)
   } while (N2 < NPTR4);
 }
 
-// The radiation-term segments of every panel (panelOut, JRAD = 0: RADFNI from
-// the panel's first output point), a thread per panel: their number at
-// seg_n[layer * stride + panel] (-1: more than kSegTab, the far-wing pass
-// forms them itself), first points, values and slopes.  A segment is a chain of
-// exponentials and divisions in binary64 (about 3 us); formed by one lane of
-// the far-wing pass's CTA, those of a surface panel took two thirds of its 88 us.
+// What the far-wing pass needs of every panel and one thread can form, ahead of
+// it: by the CTA's first warp, a lane per panel, the radiation-term segments
+// (panelOut, JRAD = 0: RADFNI from the panel's first output point), their
+// number at seg_n[layer * stride + panel] (-1: more than kSegTab, the far-wing
+// pass forms them itself), first points, values and slopes; by its second, the
+// XINT set-up.  Both are chains of binary64 divisions and exponentials (a
+// segment takes about 3 us, the set-up 15): formed by one lane of the far-wing
+// pass's CTA, the segments of a surface panel were two thirds of its 88 us,
+// and the set-up a third of the others' 43 us.
 __global__ void __launch_bounds__(64)
-    k_panel_segs(const LayerPlan* __restrict__ plans, int layer0, const double* __restrict__ vft_all, int64_t stride,
-                 int* __restrict__ seg_n, int* __restrict__ seg_start, double2* __restrict__ seg_v) {
+    k_panel_setup(const LayerPlan* __restrict__ plans, int layer0, const double* __restrict__ vft_all, int64_t stride,
+                  const int* __restrict__ panel_blk, const double* __restrict__ blk_v1,
+                  const int* __restrict__ blk_n, const int64_t* __restrict__ blk_m0, int* __restrict__ seg_n,
+                  int* __restrict__ seg_start, double2* __restrict__ seg_v, XintPanel* __restrict__ xint) {
   const LayerPlan& P = plans[blockIdx.y + layer0];
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P.npanels || P.jrad != 0) return;
+  const int p = blockIdx.x * 32 + (threadIdx.x & 31);
+  if (p >= P.npanels) return;
   const int64_t k = (int64_t)blockIdx.y * stride + p;
   const double dv = P.dv, VFT = vft_all[P.vft_off + p];
+  if (threadIdx.x >= 32) {
+    XintPanel X = {};
+    const double DVR3 = 16. * dv;
+    if (P.nptr4 > 0) {
+      X.recdva4 = 1. / P.dvr4;
+      for (int c = 0; c < 2; ++c) {
+        const int b = panel_blk[P.vft_off + ((c == 0 && p > 0) ? p - 1 : p)];
+        const double V1R4 = blk_v1[P.blk_off + b];
+        const int NPTR4 = blk_n[P.blk_off + b];
+        const double V2R4 = V1R4 + P.dvr4 * (double)(NPTR4 - 1);
+        X.blk[c] = b;
+        X.v1r4[c] = V1R4;
+        X.nptr4[c] = NPTR4;
+        X.m0[c] = blk_m0[P.blk_off + b];
+        X.ilo4[c] = (int)((V1R4 + P.dvr4 - VFT) / DVR3 + 1. + kONEMI);
+        X.ihi4[c] = (int)((V2R4 - P.dvr4 - VFT) / DVR3 + kONEMI);
+      }
+    }
+    if (P.contnm) {
+      X.recdvab = 1. / P.dvabs;
+      X.iloab = (int)((P.v1abs + P.dvabs - VFT) / DVR3 + 1. + kONEMI);
+      X.ihiab = (int)((P.v2abs - P.dvabs - VFT) / DVR3 + kONEMI);
+      if (P.mixed) {
+        const int j3a = max(X.iloab, 0), j3b = min(X.ihiab, kR3Pts - 1);
+        if (j3a <= j3b) {
+          const int Ja = (int)((VFT + DVR3 * (double)(j3a - 1) - P.v1abs) * X.recdvab + kONEPL);
+          const int Jb = (int)((VFT + DVR3 * (double)(j3b - 1) - P.v1abs) * X.recdvab + kONEPL);
+          if (Jb + 2 - (Ja - 1) + 1 <= kAbsStage) {
+            X.ab0 = Ja - 1;
+            X.nab = Jb + 2 - (Ja - 1) + 1;
+          }
+        }
+      }
+    }
+    xint[k] = X;
+    return;
+  }
+  if (P.jrad != 0) return;
   const int NHI = p == P.npanels - 1 ? P.nhi_last : (kNLIM1 + kNSHIFT - 1);
   const int NLO = kNSHIFT + 1;
   const double XKT = P.tave / kRADCN2;
@@ -781,41 +811,9 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
     for (int t = tid; t < 2 * kTiles2; t += blockDim.x) S.lo2[t] = S.hi2[t] = (int)rg[3];
     for (int t = tid; t < 2 * kTiles3; t += blockDim.x) S.lo3[t] = S.hi3[t] = (int)rg[5];
   }
-  if (kWings && tid == 0) {  // XINT set-up of the panel (once, in FP64)
-    XintPanel& X = S.X;
-    const double DVR3 = 16. * dv;
-    if (P.nptr4 > 0) {
-      X.recdva4 = 1. / P.dvr4;
-      for (int c = 0; c < 2; ++c) {
-        const int b = a.panel_blk[P.vft_off + ((c == 0 && p > 0) ? p - 1 : p)];
-        const double V1R4 = a.blk_v1[P.blk_off + b];
-        const int NPTR4 = a.blk_n[P.blk_off + b];
-        const double V2R4 = V1R4 + P.dvr4 * (double)(NPTR4 - 1);
-        X.blk[c] = b;
-        X.v1r4[c] = V1R4;
-        X.nptr4[c] = NPTR4;
-        X.m0[c] = a.blk_m0[P.blk_off + b];
-        X.ilo4[c] = (int)((V1R4 + P.dvr4 - VFT) / DVR3 + 1. + kONEMI);
-        X.ihi4[c] = (int)((V2R4 - P.dvr4 - VFT) / DVR3 + kONEMI);
-      }
-    }
-    X.nab = 0;
-    if (P.contnm) {
-      X.recdvab = 1. / P.dvabs;
-      X.iloab = (int)((P.v1abs + P.dvabs - VFT) / DVR3 + 1. + kONEMI);
-      X.ihiab = (int)((P.v2abs - P.dvabs - VFT) / DVR3 + kONEMI);
-      if constexpr (!Plain) {
-        const int j3a = max(X.iloab, 0), j3b = min(X.ihiab, kR3Pts - 1);
-        if (j3a <= j3b) {
-          const int Ja = (int)((VFT + DVR3 * (double)(j3a - 1) - P.v1abs) * X.recdvab + kONEPL);
-          const int Jb = (int)((VFT + DVR3 * (double)(j3b - 1) - P.v1abs) * X.recdvab + kONEPL);
-          if (Jb + 2 - (Ja - 1) + 1 <= kAbsStage) {
-            X.ab0 = Ja - 1;
-            X.nab = Jb + 2 - (Ja - 1) + 1;
-          }
-        }
-      }
-    }
+  if constexpr (kWings) {  // XINT set-up of the panel (k_panel_setup)
+    const int* x = reinterpret_cast<const int*>(&a.xint[(int64_t)layer * a.panel_stride + p]);
+    for (int i = tid; i < (int)(sizeof(XintPanel) / sizeof(int)); i += kPanelThreads) reinterpret_cast<int*>(&S.X)[i] = x[i];
   }
   __syncthreads();
   if constexpr (!Plain && kWings) {  // ABSRB of the panel as FP32
@@ -843,7 +841,7 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
   // units 0..kTiles3-1: 32 new points each; unit kTiles3: the 8 old points
   static_assert(kTiles3 + 1 < kPanelWarps, "the last warp has no R3 unit");
   static_assert(kSegTab < kMaxSeg, "the tabulated segments fit in shared memory");
-  // radiation-term segments (panelOut, JRAD = 0): k_panel_segs' or, when they
+  // radiation-term segments (panelOut, JRAD = 0): k_panel_setup's or, when they
   // are more than it holds, formed by a lane idle in the R3 phase
   int nseg = 0;
   if constexpr (kWings) {

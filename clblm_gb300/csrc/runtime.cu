@@ -154,7 +154,7 @@ struct clblm_handle {
   DevBuf bfac;
   DevBuf gpm, gsm;  // per grid record bounds of the panel kernel
   DevBuf pwork;     // CTAs of the panel kernel's line pass
-  DevBuf psegn, psegs, psegv;  // radiation-term segments of the panels
+  DevBuf psegn, psegs, psegv, pxint;  // radiation-term segments and XINT set-up of the panels
   DevBuf reclo;     // low parts of the records' ZFL/ZSLOPE
   DevBuf jprof, jod, jmap, jjobs, jblk;  // Jacobians: profiles, block ODs, maps, jobs, grid blocks
   DevBuf jvjp;                          // vector-Jacobian product: CTA partial sums and the totals
@@ -179,7 +179,7 @@ struct clblm_handle {
                               &f4flag,    &f4cut,    &f4grp,     &f4nxt,   &ragg,    &segpool, &gpm,    &gsm,
                               &reclo,     &jprof,    &jod,       &jmap,    &jjobs,   &jblk,    &jvjp,   &linecpl,   &f4cpl,    &f4cpll,    &f4ncpl,   &pwork,
                               &f4tab,     &f4calls,  &f4ncall,  &f4agg,     &psegn,
-                              &psegs,     &psegv, &tabbuf};
+                              &psegs,     &psegv, &pxint, &tabbuf};
     for (auto& b : rt) v.push_back(&b);
     for (auto& b : imap) v.push_back(&b);
     v.push_back(&rtseg);
@@ -966,7 +966,7 @@ size_t od_job_bytes(const LayerPlan& P, bool plain) {
   const size_t real = plain ? 8 : 4;
   return (size_t)(P.line_hi - P.line_lo + 1) * per_line + (size_t)(P.f4_hi - P.f4_lo) * per_f4 +
          (size_t)(P.nsamp * P.nslice + P.nptr4) * real +
-         (size_t)P.npanels * (kSegTab * (sizeof(int) + sizeof(double2)) + sizeof(int));
+         (size_t)P.npanels * (kSegTab * (sizeof(int) + sizeof(double2)) + sizeof(int) + sizeof(XintPanel));
 }
 
 // Bytes of OD-pipeline workspace one batch of layers may take: 60 % of the
@@ -1054,7 +1054,7 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
   cudaStream_t st = h->stream2;
   {
     // the continuum, the radiation term of the far-wing blocks and the panels'
-    // radiation segments need the plans alone: a stream of their own, joined
+    // set-up need the plans alone: a stream of their own, joined
     // before the far-wing pass of k_panel (50 us, 140 at a window of 1000
     // cm-1, that the far-wing chain would wait for)
     cudaStream_t s3 = h->stream3;
@@ -1069,9 +1069,10 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     k_continuum<<<dim3((kNABSRB + 8 + 63) / 64, count), 64, 0, s3>>>(dplans, first, h->cont, h->absrb.as<double>());
     k_r4_radfac<<<dim3((maxb + kRadfacWarps - 1) / kRadfacWarps, count), 32 * kRadfacWarps, 0, s3>>>(
         dplans, first, h->bv1.as<double>(), h->bn.as<int>(), h->bfac.as<double>());
-    k_panel_segs<<<dim3((maxp + 63) / 64, count), 64, 0, s3>>>(dplans, first, h->vft.as<double>(), pstride,
-                                                             h->psegn.as<int>(), h->psegs.as<int>(),
-                                                             h->psegv.as<double2>());
+    k_panel_setup<<<dim3((maxp + 31) / 32, count), 64, 0, s3>>>(
+        dplans, first, h->vft.as<double>(), pstride, h->pblk.as<int>(), h->bv1.as<double>(), h->bn.as<int>(),
+        h->bm0.as<int64_t>(), h->psegn.as<int>(), h->psegs.as<int>(), h->psegv.as<double2>(),
+        h->pxint.as<XintPanel>());
     CUDA_TRY(h, cudaGetLastError());
     CUDA_TRY(h, cudaEventRecord(h->join3_ev, s3));
   }
@@ -1309,6 +1310,7 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     pa.seg_pool_d = reinterpret_cast<double*>(b + 256 + start_b + val_b);
     CUDA_TRY(h, cudaMemsetAsync(pa.seg_next, 0, sizeof(int), st));
   }
+  pa.xint = h->pxint.as<XintPanel>();
   pa.seg_n = h->psegn.as<int>();
   pa.seg_start = h->psegs.as<int>();
   pa.seg_v = h->psegv.as<double2>();
@@ -1493,6 +1495,7 @@ cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int
   WS_ENSURE(h->psegn.ensure(sizeof(int) * d.psc));
   WS_ENSURE(h->psegs.ensure(sizeof(int) * kSegTab * d.psc));
   WS_ENSURE(h->psegv.ensure(sizeof(double2) * kSegTab * d.psc));
+  WS_ENSURE(h->pxint.ensure(sizeof(XintPanel) * d.psc));
   WS_ENSURE(h->r4.ensure(real * d.r4t));
   WS_ENSURE(h->absrb.ensure(sizeof(double) * (kNABSRB + 8) * d.cnt));
   WS_ENSURE(h->blockmax.ensure(sizeof(int) * d.smaxc));
@@ -1531,7 +1534,7 @@ std::vector<DevBuf*> ws_buffers(clblm_handle* h) {
           &h->gsm,    &h->ragg,   &h->ranges, &h->od,       &h->r4,     &h->absrb,  &h->blockmax, &h->f4prep, &h->f4sh, &h->f4blk, &h->f4ntot, &h->f4cidx,
           &h->f4vb,   &h->f4lb,   &h->f4src,  &h->f4flag,   &h->f4nxt,  &h->f4cut,  &h->f4grp,  &h->f4rec,
           &h->f4recd, &h->f4nrec, &h->f4nmir, &h->f4pm,     &h->f4sm,   &h->segpool, &h->bfac,   &h->linecpl, &h->f4cpl, &h->f4cpll,
-          &h->f4ncpl, &h->pwork,  &h->f4tab,  &h->f4calls,  &h->f4ncall, &h->f4agg, &h->psegn,  &h->psegs,  &h->psegv, &h->tabbuf};
+          &h->f4ncpl, &h->pwork,  &h->f4tab,  &h->f4calls,  &h->f4ncall, &h->f4agg, &h->psegn,  &h->psegs,  &h->psegv, &h->pxint, &h->tabbuf};
 }
 
 // Frees every work buffer of the handle (all but the line list, the shape
