@@ -54,12 +54,14 @@ __host__ __device__ constexpr int jac_vjp_slots(int nlay) { return 2 * (nlay + 1
 __global__ void __launch_bounds__(kMapThreads) k_interp_map_jobs(const JacJob* jobs, int njob);
 // k_od_jobs: threads per CTA and output points per CTA
 constexpr int kOdJobThreads = 256;
-constexpr int kOdJobPoints = 2048;
+constexpr int kOdJobPoints = 8192;
 template <bool Plain>
 __global__ void k_od_jobs(const JacJob* jobs, int njob, const void* od_all, void* out);
 template <bool Plain>
 __global__ void k_jac(JacArgs a);
-// acc[k] += the CTAs' partial sums part[c][k], c = 0 .. nctas-1 in order
-__global__ void k_vjp_accum(const double* part, int nctas, int nslot, double* acc);
+// acc[k] += the CTAs' partial sums part[c][k], c = 0 .. nctas-1, in a fixed order
+constexpr int kVjpRows = 32;
+__global__ void __launch_bounds__(32 * kVjpRows)
+    k_vjp_accum(const double* part, int nctas, int nslot, double* acc);
 
 }  // namespace clblm

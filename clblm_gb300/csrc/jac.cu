@@ -11,7 +11,7 @@
 //                      (:899-1065) and the molecule derivatives of
 //                      drv_LevelConc (:1069-1203)
 //
-// The per-point recurrence keeps its per-layer arrays in local memory
+// The per-point recurrence keeps two per-layer arrays in local memory
 // (at most kMaxJacLayers layers).  The mixed path runs it in FP32, the FP64
 // path in binary64 with the reference's operation order.
 #include <cuda_runtime.h>
@@ -34,6 +34,10 @@ __global__ void __launch_bounds__(kMapThreads) k_interp_map_jobs(const JacJob* _
   if (J1 < 1 || J1 > jb.nout) return;  // a block start off the output grid writes nothing
   interp_map_block(jb.spec.v1, jb.spec.dvin, jb.spec.ratio, J1, jb.blk_vo[b], jb.nout, jb.map);
 }
+
+// a product rounded on its own
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
 // interpSpectrum's linear extension by two points past either end
 template <typename Real>
@@ -79,10 +83,16 @@ __global__ void __launch_bounds__(kOdJobThreads) k_od_jobs(const JacJob* jobs, i
       const int2 mp = map[I - 1];
       const int64_t i = mp.x;
       const Real4 c = ia[mp.y];
-      Real v = c.x * od_ext_t(x, n_in, i - 1);
-      v += c.y * od_ext_t(x, n_in, i);
-      v += c.z * od_ext_t(x, n_in, i + 1);
-      v += c.w * od_ext_t(x, n_in, i + 2);
+      Real v;
+      if (i >= 2 && i + 2 <= n_in) {  // (the extension's tests took most of the kernel)
+        const Real* q = x + (i - 2);
+        v = fma(c.w, q[3], fma(c.z, q[2], fma(c.y, q[1], mul_rn(c.x, q[0]))));
+      } else {
+        v = c.x * od_ext_t(x, n_in, i - 1);
+        v += c.y * od_ext_t(x, n_in, i);
+        v += c.z * od_ext_t(x, n_in, i + 1);
+        v += c.w * od_ext_t(x, n_in, i + 2);
+      }
       o[I - 1] = v;
     }
     return;
@@ -205,129 +215,174 @@ __global__ void __launch_bounds__(128) k_jac(JacArgs a) {
       dst[idx] = (double)val;
     }
   };
-  Real viewOD[M], downOD[M], Bbar[M], dBbar[M], Blev[M], dBlev[M], cumTxA[M], cumTxB2[M];
-  Real dRad_dT_up[M], dRad_dT_dn[M], dRad_dTbar[M], dRad_dTau[M], dRad_dTlev[M];
+  // Of the recurrence's arrays two stay, in local memory: cumTxA, summed from
+  // the top and used from the surface, and the down path's dRad_dTau, which
+  // first holds cumTxB2 (summed from the surface, used from the top).  The
+  // rest is formed again where it is used, an exponential or two each: 13
+  // arrays of 62 layers, 3 KB a point, went through L2 and DRAM (8.8 ms of a
+  // 60-layer 500 cm-1 call's 85).
+  Real cumTxA[M], dTauDn[M];
   const Real* jod = reinterpret_cast<const Real*>(a.jod);
   const double vn = a.v1 + (double)iv * a.dv;
   const Real vr = (Real)vn;  // the point's wavenumber in the working precision, converted once
-  for (int l = 1; l <= N2; ++l) {
-    viewOD[l] = jod[(int64_t)(l - 1) * a.nout + iv];
-    downOD[l] = viewOD[l] * lc(kAmf, a.amf_down, l - 1);
-  }
-  if (a.lin_in_tau != 0)
-    for (int lv = 1; lv <= N2 + 1; ++lv) planck_drv_t<Real>(vr, lc(kTlev, a.tlev, lv - 1), &Blev[lv], &dBlev[lv]);
-  for (int l = 1; l <= N2; ++l) planck_drv_t<Real>(vr, lc(kTlay, a.tlay, l - 1), &Bbar[l], &dBbar[l]);
+  // (read-only loads, issued layers ahead: the recurrence is a chain, and a
+  // launch of 100,000 points leaves 20 warps an SM to hide 600 cycles a load)
+  auto view = [&](int l) -> Real { return __ldg(jod + ((int64_t)(l - 1) * a.nout + iv)); };
+  auto variant = [&](int v, int il) -> Real { return __ldg(jod + (((int64_t)v * N2 + il) * a.nout + iv)); };
+  auto amf = [&](int l) -> Real { return lc(kAmf, a.amf_down, l - 1); };
+  auto down_od = [&](int l, Real od) -> Real { return mul_rn(od, amf(l)); };
+  const int lit = a.lin_in_tau;
+  const bool dT = a.do_temp != 0;
+  auto planck_lev = [&](int lv, Real* B, Real* dB) {  // (levels enter where the source is linear in tau)
+    *B = *dB = 0;
+    if (lit != 0) planck_drv_t<Real>(vr, lc(kTlev, a.tlev, lv - 1), B, dB);
+  };
+  auto planck_lay = [&](int l, Real* B, Real* dB) { planck_drv_t<Real>(vr, lc(kTlay, a.tlay, l - 1), B, dB); };
   Real Bsfc, dBsfc;
   planck_drv_t<Real>(vr, (Real)a.tsfc, &Bsfc, &dBsfc);
   Real rad = 0;
-  for (int l = 1; l <= N2; ++l) dRad_dTau[l] = dRad_dTbar[l] = 0;
-  for (int l = 1; l <= N2 + 1; ++l) dRad_dT_up[l] = dRad_dT_dn[l] = dRad_dTlev[l] = 0;
-  const int obsLay = N2 + 1;
   // 0- transmittance along the upwelling path from TOA down
   Real cumODA = 0;
   cumTxA[N2 + 1] = 1;
-  for (int l = obsLay - 1; l >= 1; --l) {
-    cumODA = cumODA + viewOD[l];
+#pragma unroll 8
+  for (int l = N2; l >= 1; --l) {
+    cumODA = cumODA + view(l);
     cumTxA[l] = dev_exp(-cumODA);
   }
   const Real totODUp = cumODA, totTxUp = cumTxA[1];
+  const bool down = totTxUp > (Real)1.e-06;
   Real dbavgdb, dbavgdbdod, Blt, dTran;
-  const int lit = a.lin_in_tau;
-  const bool dT = a.do_temp != 0;
   // 1- downwelling thermal radiance
-  if (totTxUp > (Real)1.e-06) {
-    cumTxB2[1] = totTxUp;
+  if (down) {
+    dTauDn[1] = totTxUp;  // cumTxB2
     Real cumODB = 0;
+#pragma unroll 8
     for (int l = 1; l <= N2; ++l) {
-      cumODB = cumODB + downOD[l];
-      cumTxB2[l + 1] = dev_exp(-(totODUp + cumODB));
+      cumODB = cumODB + down_od(l, view(l));
+      dTauDn[l + 1] = dev_exp(-(totODUp + cumODB));
     }
+    Real tx1 = dTauDn[N2 + 1], Bup, dBup;  // of the layer's upper level
+    planck_lev(N2 + 1, &Bup, &dBup);
+    Real od_next = view(N2);
     for (int l = N2; l >= 1; --l) {
-      dTran = cumTxB2[l] - cumTxB2[l + 1];
-      const Real amf = lc(kAmf, a.amf_down, l - 1);
+      const Real tx = dTauDn[l], od = down_od(l, od_next);
+      od_next = l > 1 ? view(l - 1) : (Real)0;
+      dTran = tx - tx1;
+      const Real am = amf(l);
+      Real B = 0, dB, Blo, dBlo, dtau;
+      planck_lev(l, &Blo, &dBlo);
+      if (lit != 2) planck_lay(l, &B, &dB);
       if (lit != 0) {
-        rlin_t(downOD[l], &dbavgdb, &dbavgdbdod);
+        rlin_t(od, &dbavgdb, &dbavgdbdod);
         if (lit == 2) {
-          Blt = Blev[l] + (Blev[l + 1] - Blev[l]) * dbavgdb;
-          dRad_dTau[l] = (cumTxB2[l + 1] * Blt - rad + dTran * dbavgdbdod * (Blev[l + 1] - Blev[l])) * amf;
-          if (dT) {
-            dRad_dT_dn[l + 1] = dRad_dT_dn[l + 1] + dTran * dBlev[l + 1] * dbavgdb;
-            dRad_dT_dn[l] = dTran * dBlev[l] * (1 - dbavgdb);
-            dRad_dTbar[l] = 0;
-          }
+          Blt = Blo + (Bup - Blo) * dbavgdb;
+          dtau = (tx1 * Blt - rad + dTran * dbavgdbdod * (Bup - Blo)) * am;
         } else {
-          Blt = 2 * Bbar[l] * dbavgdb + Blev[l] * (1 - 2 * dbavgdb);
-          dRad_dTau[l] = (cumTxB2[l + 1] * Blt - rad + 2 * dTran * dbavgdbdod * (Bbar[l] - Blev[l])) * amf;
-          if (dT) {
-            dRad_dT_dn[l] = dTran * dBlev[l] * (1 - 2 * dbavgdb);
-            dRad_dTbar[l] = dTran * 2 * dBbar[l] * dbavgdb;
-          }
+          Blt = 2 * B * dbavgdb + Blo * (1 - 2 * dbavgdb);
+          dtau = (tx1 * Blt - rad + 2 * dTran * dbavgdbdod * (B - Blo)) * am;
         }
         rad = rad + dTran * Blt;
       } else {
-        dRad_dTau[l] = (cumTxB2[l + 1] * Bbar[l] - rad) * amf;
-        rad = rad + dTran * Bbar[l];
-        if (dT) dRad_dTbar[l] = dTran * dBbar[l];
+        dtau = (tx1 * B - rad) * am;
+        rad = rad + dTran * B;
       }
+      dTauDn[l] = dtau;
+      tx1 = tx;
+      Bup = Blo;
     }
+  } else {
+    for (int l = 1; l <= N2; ++l) dTauDn[l] = 0;
   }
   // 2- surface reflectance; 3- surface terms
   const Real emis = (Real)a.emis, rsfc = 1 - emis;
-  for (int l = 1; l <= N2; ++l) {
-    dRad_dTau[l] = dRad_dTau[l] * rsfc;
-    if (dT) dRad_dTbar[l] = dRad_dTbar[l] * rsfc;
-  }
   const Real dRad_dEmis = totTxUp * Bsfc - rad;
   const Real dRad_dTsfc = emis * totTxUp * dBsfc;
   rad = rad * rsfc + emis * totTxUp * Bsfc;
-  // 5- upwelling thermal radiance
-  for (int l = 1; l <= obsLay - 1; ++l) {
-    dTran = cumTxA[l + 1] - cumTxA[l];
-    if (lit != 0) {
-      rlin_t(viewOD[l], &dbavgdb, &dbavgdbdod);
-      if (lit == 2) {
-        Blt = Blev[l + 1] * (1 - dbavgdb) + Blev[l] * dbavgdb;
-        dRad_dTau[l] = dRad_dTau[l] + (cumTxA[l] * Blt - rad + dTran * dbavgdbdod * (Blev[l] - Blev[l + 1]));
-        if (dT) {
-          dRad_dT_up[l + 1] = dTran * dBlev[l + 1] * (1 - dbavgdb);
-          dRad_dT_up[l] = dRad_dT_up[l] + dTran * dBlev[l] * dbavgdb;
+  // 5- upwelling thermal radiance, and each layer's derivatives as its level
+  // below is complete.
+  // drv_LevelTemp: dTau/dT = [tau(T+1) - tau(T)] - (Wtot/T) dTau/dWtot
+  // drv_LevelConc: dTau/dln W = the OD of the molecule alone
+  // (amfView = 1: the viewing path is the reference path)
+  const int64_t o = a.off + iv;
+  const bool wantT = dT && (a.dtlev || vjp) && a.vT >= 0, wantM = (a.dqlev || vjp) && a.vM >= 0;
+  Real Blo, dBlo, txB = totTxUp, cumODB = 0;  // down path: level l
+  planck_lev(1, &Blo, &dBlo);
+  Real tx = cumTxA[1];
+  Real dTup = 0, dTdn = 0;      // dRad_dT_up(l) and dRad_dT_dn(l) from the layer below
+  Real barB = 0;                // dRad_dTbar of the layer below
+  Real loT = 0, loM = 0;        // of the layer below at its upper level
+  Real m_next = view(1), t_next = wantT ? variant(a.vT, 0) : (Real)0, w_next = wantT ? variant(a.vW, 0) : (Real)0,
+       q_next = wantM ? variant(a.vM, 0) : (Real)0;
+  for (int l = 1; l <= N2; ++l) {
+    const int il = l - 1;
+    const Real m = m_next, tp = t_next, wp = w_next, mol = q_next, tx1 = cumTxA[l + 1];
+    if (l < N2) {
+      m_next = view(l + 1);
+      if (wantT) {
+        t_next = variant(a.vT, l);
+        w_next = variant(a.vW, l);
+      }
+      if (wantM) q_next = variant(a.vM, l);
+    }
+    Real Bup, dBup, B = 0, dB = 0;
+    planck_lev(l + 1, &Bup, &dBup);
+    if (lit != 2) planck_lay(l, &B, &dB);
+    // the down path's level and layer temperature terms
+    Real dnUp = 0, bar = 0;  // dRad_dT_dn(l + 1) of lit = 2; dRad_dTbar(l)
+    if (down && dT) {
+      const Real od = down_od(l, m);
+      cumODB = cumODB + od;
+      const Real txB1 = dev_exp(-(totODUp + cumODB));
+      dTran = txB - txB1;
+      if (lit != 0) {
+        rlin_t(od, &dbavgdb, &dbavgdbdod);
+        if (lit == 2) {
+          dTdn = dTran * dBlo * (1 - dbavgdb) + dTdn;
+          dnUp = dTran * dBup * dbavgdb;
+        } else {
+          dTdn = dTran * dBlo * (1 - 2 * dbavgdb);
+          bar = dTran * 2 * dB * dbavgdb;
         }
       } else {
-        Blt = 2 * Bbar[l] * dbavgdb + Blev[l + 1] * (1 - 2 * dbavgdb);
-        dRad_dTau[l] = dRad_dTau[l] + (cumTxA[l] * Blt - rad + dTran * dbavgdbdod * 2 * (Bbar[l] - Blev[l + 1]));
+        bar = dTran * dB;
+      }
+      txB = txB1;
+    }
+    Real dtau = dTauDn[l] * rsfc;
+    if (dT) bar = bar * rsfc;
+    dTran = tx1 - tx;
+    Real upUp = 0;  // dRad_dT_up(l + 1)
+    if (lit != 0) {
+      rlin_t(m, &dbavgdb, &dbavgdbdod);
+      if (lit == 2) {
+        Blt = Bup * (1 - dbavgdb) + Blo * dbavgdb;
+        dtau = dtau + (tx * Blt - rad + dTran * dbavgdbdod * (Blo - Bup));
         if (dT) {
-          dRad_dT_up[l + 1] = dTran * dBlev[l + 1] * (1 - 2 * dbavgdb);
-          dRad_dTbar[l] = dRad_dTbar[l] + dTran * 2 * dBbar[l] * dbavgdb;
+          upUp = dTran * dBup * (1 - dbavgdb);
+          dTup = dTup + dTran * dBlo * dbavgdb;
+        }
+      } else {
+        Blt = 2 * B * dbavgdb + Bup * (1 - 2 * dbavgdb);
+        dtau = dtau + (tx * Blt - rad + dTran * dbavgdbdod * 2 * (B - Bup));
+        if (dT) {
+          upUp = dTran * dBup * (1 - 2 * dbavgdb);
+          bar = bar + dTran * 2 * dB * dbavgdb;
         }
       }
       rad = rad + dTran * Blt;
     } else {
-      dRad_dTau[l] = dRad_dTau[l] + (cumTxA[l] * Bbar[l] - rad);
-      rad = rad + dTran * Bbar[l];
-      if (dT) dRad_dTbar[l] = dRad_dTbar[l] + dTran * dBbar[l];
+      dtau = dtau + (tx * B - rad);
+      rad = rad + dTran * B;
+      if (dT) bar = bar + dTran * dB;
     }
-  }
-  // (amfView = 1: the viewing path is the reference path)
-  if (dT) {
-    if (lit != 0)
-      for (int lv = 1; lv <= N2 + 1; ++lv) dRad_dTlev[lv] = dRad_dT_up[lv] + dRad_dT_dn[lv] * rsfc;
-    if (lit == 0 || lit == 1)
-      for (int l = N2; l >= 1; --l) {
-        dRad_dTlev[l + 1] = dRad_dTlev[l + 1] + dRad_dTbar[l] * lc(kTup, a.dT_dTup, l - 1);
-        dRad_dTlev[l] = dRad_dTlev[l] + dRad_dTbar[l] * lc(kTlo, a.dT_dTlo, l - 1);
+    if (wantT) {
+      Real lev = 0;  // dRad_dTlev(l)
+      if (lit != 0) lev = dTup + dTdn * rsfc;
+      if (lit != 2) {
+        lev = lev + bar * lc(kTlo, a.dT_dTlo, il);
+        if (l > 1) lev = lev + barB * lc(kTup, a.dT_dTup, il - 1);
+        barB = bar;
       }
-  }
-  const int64_t o = a.off + iv;
-  if (a.rad && !vjp) a.rad[o] = (double)rad;
-  put(a.dtsfc, o, 2 * N2 + 2, dRad_dTsfc);
-  put(a.demis, o, 2 * N2 + 3, dRad_dEmis);
-  // drv_LevelTemp: dTau/dT = [tau(T+1) - tau(T)] - (Wtot/T) dTau/dWtot
-  if (dT && (a.dtlev || vjp) && a.vT >= 0) {
-    Real lo = 0;
-    for (int il = 0; il < N2; ++il) {
-      const Real m = jod[(int64_t)il * a.nout + iv];
-      const Real tp = jod[((int64_t)a.vT * N2 + il) * a.nout + iv];
-      const Real wp = jod[((int64_t)a.vW * N2 + il) * a.nout + iv];
       Real dTau_dT;
       if constexpr (Plain) {
         dTau_dT = tp - m;
@@ -339,26 +394,35 @@ __global__ void __launch_bounds__(128) k_jac(JacArgs a) {
         // (wp - m) / (0.01 Wtot) * (Wtot / T) = (wp - m) * 100 / T
         dTau_dT = (tp - m) - (wp - m) * s_c[kRt100][il];
       }
-      const Real dRaddT = dRad_dTau[il + 1] * dTau_dT;
+      const Real dRaddT = dtau * dTau_dT;
       const Real up = dRaddT * lc(kTup, a.dT_dTup, il);
-      lo = lo + dRaddT * lc(kTlo, a.dT_dTlo, il) + dRad_dTlev[il + 1];
-      put(a.dtlev, (int64_t)il * a.ld + o, il, lo);
-      if (il == N2 - 1) put(a.dtlev, (int64_t)N2 * a.ld + o, N2, up + dRad_dTlev[il + 2]);
-      lo = up;
+      loT = loT + dRaddT * lc(kTlo, a.dT_dTlo, il) + lev;
+      put(a.dtlev, (int64_t)il * a.ld + o, il, loT);
+      loT = up;
     }
-  }
-  // drv_LevelConc: dTau/dln W = the OD of the molecule alone
-  if ((a.dqlev || vjp) && a.vM >= 0) {
-    Real lo = 0;
-    for (int il = 0; il < N2; ++il) {
-      const Real dRad_dW = dRad_dTau[il + 1] * jod[((int64_t)a.vM * N2 + il) * a.nout + iv];
+    if (wantM) {
+      const Real dRad_dW = dtau * mol;
       const Real up = dRad_dW * lc(kQup, a.dW_dQup, il);
-      lo = lo + dRad_dW * lc(kQlo, a.dW_dQlo, il);
-      put(a.dqlev, (int64_t)il * a.ld + o, N2 + 1 + il, lo);
-      if (il == N2 - 1) put(a.dqlev, (int64_t)N2 * a.ld + o, 2 * N2 + 1, up);
-      lo = up;
+      loM = loM + dRad_dW * lc(kQlo, a.dW_dQlo, il);
+      put(a.dqlev, (int64_t)il * a.ld + o, N2 + 1 + il, loM);
+      loM = up;
     }
+    dTup = upUp;
+    dTdn = dnUp;
+    tx = tx1;
+    Blo = Bup;
+    dBlo = dBup;
   }
+  if (wantT) {  // the top level
+    Real lev = 0;
+    if (lit != 0) lev = dTup + dTdn * rsfc;
+    if (lit != 2) lev = lev + barB * lc(kTup, a.dT_dTup, N2 - 1);
+    put(a.dtlev, (int64_t)N2 * a.ld + o, N2, loT + lev);
+  }
+  if (wantM) put(a.dqlev, (int64_t)N2 * a.ld + o, 2 * N2 + 1, loM);
+  if (a.rad && !vjp) a.rad[o] = (double)rad;
+  put(a.dtsfc, o, 2 * N2 + 2, dRad_dTsfc);
+  put(a.demis, o, 2 * N2 + 3, dRad_dEmis);
   if (vjp) {  // the CTA's sums, warp by warp in order
     __syncthreads();
     const int nw = (int)(blockDim.x >> 5);
@@ -370,24 +434,23 @@ __global__ void __launch_bounds__(128) k_jac(JacArgs a) {
   }
 }
 
-__global__ void k_vjp_accum(const double* __restrict__ part, int nctas, int nslot, double* __restrict__ acc) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nslot) return;
-  // sixteen chains: a binary64 addition takes 140 ns to the next, and one chain
-  // of 800 CTAs took 114 us a block
-  double v[16];
-#pragma unroll
-  for (int q = 0; q < 16; ++q) v[q] = 0.;
-  for (int c = 0; c < nctas; c += 16) {
-#pragma unroll
-    for (int q = 0; q < 16; ++q)
-      if (c + q < nctas) v[q] += part[(int64_t)(c + q) * nslot + k];
+// Sums over the CTAs: a lane per slot, the CTAs dealt to kVjpRows warps, whose
+// sums are added in order (one thread per slot waited for 800 loads in turn:
+// 114 to 190 us a block)
+__global__ void __launch_bounds__(32 * kVjpRows)
+    k_vjp_accum(const double* __restrict__ part, int nctas, int nslot, double* __restrict__ acc) {
+  __shared__ double rows[kVjpRows][33];
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
+  double sum = 0.;
+  if (k < nslot) {
+#pragma unroll 8
+    for (int c = row; c < nctas; c += kVjpRows) sum += part[(int64_t)c * nslot + k];
   }
-#pragma unroll
-  for (int h = 8; h > 0; h >>= 1)
-#pragma unroll
-    for (int q = 0; q < h; ++q) v[q] += v[q + h];
-  const double sum = acc[k] + v[0];
+  rows[row][lane] = sum;
+  __syncthreads();
+  if (row != 0 || k >= nslot) return;
+  sum = acc[k];
+  for (int w = 0; w < kVjpRows; ++w) sum += rows[w][lane];
   acc[k] = sum;
 }
 

@@ -3105,7 +3105,7 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
       if (rc) return rc;
       if (vjp) {
         h->launches++;
-        k_vjp_accum<<<(unsigned)((nslot + 127) / 128), 128, 0, h->stream>>>(d_part, grid, nslot, d_acc);
+        k_vjp_accum<<<(unsigned)((nslot + 31) / 32), 32 * kVjpRows, 0, h->stream>>>(d_part, grid, nslot, d_acc);
         CUDA_TRY(h, cudaGetLastError());
       }
       total += nlim;
