@@ -162,6 +162,16 @@ struct MapReplay {
       fixed = (double)q * (1. / 2305843009213693952.) == P ? 1 : 0;
     }
   }
+  // IP of the point: INT(P*201. + 1.00001) in integers (the binary64 argument is
+  // within 2^-44 of the exact one), in binary64 nearer an integer than that
+  CLBLM_HD int ip() const {
+    if (fixed) {
+      const uint64_t one = (uint64_t)1 << 53, t = (q >> 8) * 201 + one + 90071992547ull;  // 1.00001 * 2^53
+      const uint64_t f = t & (one - 1);
+      if (f >= 8192 && f <= one - 8192) return (int)(t >> 53);
+    }
+    return map_ip(phase());
+  }
   // n steps.  Below 0.999 INT(iIn + P) is iIn + 1 and the chain has no binary64
   // operation; at 0.5 <= RATIO < 0.999 a sum below 1 is exact on multiples of
   // 2^-53 and one above 1 rounds to a multiple of 2^-52: a chain of a few
@@ -169,11 +179,28 @@ struct MapReplay {
   CLBLM_HD void steps(int n) {
     int k = 0;
     const bool below = ratio < 0.999, half = ratio >= 0.5;
-    while (k < n && !(fixed && below && (!half || (q & 255) == 0))) {
+    while (k < n && !(fixed && (!below || !half || (q & 255) == 0))) {
       step();
       ++k;
     }
     if (k == n) return;
+    if (!below) {
+      for (; k < n; ++k) {
+        const uint64_t s = q + rq;
+        const int sh = 11 - clz32((uint32_t)(s >> 32));
+        const uint32_t one = 1u << sh, lo = (uint32_t)s;
+        const uint32_t up = (one >> 1) - 1u + ((lo >> sh) & 1u);
+        const uint64_t v = (s + (sh > 0 ? up : 0u)) & ~(uint64_t)(one - 1u);
+        const uint64_t p = v & (((uint64_t)1 << 61) - 1);
+        if ((p >> 40) == 0x1FFFFF) {  // INT(iIn + P) may round up
+          step();
+          continue;
+        }
+        iIn += (int64_t)(v >> 61);
+        q = p;
+      }
+      return;
+    }
     if (!half) {
       int carries = 0;
       for (; k < n; ++k) {
@@ -202,6 +229,41 @@ struct MapReplay {
     iIn += carries;
   }
 };
+
+// The flagged (undecided) points of a block, first .. last, from the reference's
+// steps: emit(k, iIn, IP).  Where INT(iIn + P) may round up at one of them
+// (sticky) iIn stays ahead for the rest of the block: seen at the point after
+// it, and only then the rest is replayed as well (point by point, 1.7 us each:
+// a gradient's two such blocks of 4700 took 600 us when the rest always was).
+template <class Emit>
+CLBLM_HD void map_replay(const MapLin& m, double P0, double ratio, const unsigned* flags, int first, int last, int n,
+                         const Emit& emit) {
+  MapReplay r;
+  r.start(m.i0, P0, ratio);
+  int k = 0;
+  for (int w = first >> 5; w <= last >> 5; ++w) {
+    unsigned f = flags[w];
+    for (int i = 0; f; ++i, f >>= 1) {
+      if (!(f & 1u)) continue;
+      const int t = 32 * w + i;
+      r.steps(t - k);
+      k = t;
+      emit(k, (int)r.iIn, r.ip());
+      if (!m.sticky || t + 1 >= n || (flags[(t + 1) >> 5] >> ((t + 1) & 31) & 1u)) continue;
+      r.steps(1);
+      k = t + 1;
+      int64_t iIn;
+      int IP;
+      map_point(m, (uint32_t)k, &iIn, &IP);
+      if (iIn == r.iIn) continue;
+      for (; k < n; ++k) {
+        emit(k, (int)r.iIn, r.ip());
+        r.step();
+      }
+      return;
+    }
+  }
+}
 
 #ifdef __CUDACC__
 // The map of one block (first output point J1, wavenumber Vo) by one CTA of
@@ -242,22 +304,8 @@ __device__ __forceinline__ void interp_map_block(double v1, double dvin, double 
   }
   __syncthreads();
   if (threadIdx.x != 0 || last < 0) return;
-  // from one undecided point to the next
-  MapReplay r;
-  r.start(lin.i0, p0, ratio);
-  int k = 0;
-  for (int w = first >> 5; w < (n + 31) / 32 && (lin.sticky || w <= last >> 5); ++w) {
-    unsigned f = flags[w];
-    if (lin.sticky) f = 32 * w >= first ? 0xffffffffu : f | (0xffffffffu << (first & 31));
-    while (f) {
-      const int t = 32 * w + __ffs(f) - 1;
-      f &= f - 1;
-      if (t >= n) break;
-      r.steps(t - k);
-      k = t;
-      out[k] = make_int2((int)r.iIn, map_ip(r.phase()));
-    }
-  }
+  map_replay(lin, p0, ratio, flags, first, last, n,
+             [&](int k, int iIn, int IP) { out[k] = make_int2(iIn, IP); });
 }
 #endif
 

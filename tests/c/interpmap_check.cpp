@@ -20,6 +20,23 @@ static void block(int64_t i0, double P0, double r) {
   int64_t iIn = i0;
   double P = P0;
   bool from = false;
+  // the block's map as the device forms it: decided points, then the others
+  static unsigned flags[(kMapBlock + 31) / 32];
+  static int64_t wi[kMapBlock];
+  static int wp[kMapBlock];
+  int first = kMapBlock, last = -1;
+  for (unsigned& f : flags) f = 0;
+  for (int k = 0; k < kMapBlock; ++k) {
+    if (map_point(m, (uint32_t)k, &wi[k], &wp[k])) continue;
+    flags[k >> 5] |= 1u << (k & 31);
+    first = k < first ? k : first;
+    last = k;
+  }
+  if (last >= 0)
+    map_replay(m, P0, r, flags, first, last, kMapBlock, [](int k, int i, int ip) {
+      wi[k] = i;
+      wp[k] = ip;
+    });
   for (int k = 0; k < kMapBlock; ++k) {
     // the reference's step
     const int IPr = (int)(P * 201. + 1.00001);
@@ -42,6 +59,9 @@ static void block(int64_t i0, double P0, double r) {
       }
     }
     points++;
+    if ((int)wi[k] != (int)iIn || wp[k] != IP) {
+      if (bad++ < 5) printf("block: i0 %lld P0 %.17g r %.17g k %d\n", (long long)i0, P0, r, k);
+    }
     if (gi != iIn || gp != IP) {
       if (bad++ < 5) printf("i0 %lld P0 %.17g r %.17g k %d: %lld %d, want %lld %d\n", (long long)i0, P0, r, k, (long long)gi, gp, (long long)iIn, IP);
     }
