@@ -2154,6 +2154,19 @@ __global__ void __launch_bounds__(kGroupSumThreads)
   }
 }
 
+// INT(x / d + c) with r = 1 / d to rounding: the product is within 4e-16 of the
+// quotient, so it decides unless it lies within 1e-6 of an integer (|x / d| <
+// 2^30), where the reference's division does.  The conversions and the test are
+// integer operations; a division is ten of the FP64 unit's, which bounds the
+// set-up.
+__device__ __forceinline__ int quotient_int(double x, double d, double r, double c) {
+  const double a = x * r + c;
+  const int J = f64_to_i32_trunc(a);
+  const long long f = __double_as_longlong(a - i32_to_f64(J)) & 0x7FFFFFFFFFFFFFFFll;
+  if (f > __double_as_longlong(1e-6) && f < __double_as_longlong(1. - 1e-6)) return J;
+  return (int)(x / d + c);
+}
+
 // CNVF4Q per-line set-up of each shrunk line (clblm_ODLAY_LineF4.f90:320-385):
 // Voigt width, the Lorentz/Voigt strengths and the point range JMIN..JMAX on
 // the global far-wing grid V1R4 + (J-1)*DVR4.  Lines at 0 < vnu <= 25 cm-1
@@ -2172,9 +2185,9 @@ __device__ void f4_record(const LayerPlan& P, const ShrunkLine& L, double VNUI, 
   const double B3 = -1. / ((1. + ZSQBND) * (1. + ZSQBND));
   const double RECPI = P.recpi;
   const double XNUI = VNUI - P.v1r4;
-  int JMIN = (int)((XNUI - P.bound4) / P.dvr4 + 2.);
+  int JMIN = quotient_int(XNUI - P.bound4, P.dvr4, P.rdvr4, 2.);
   if (JMIN < 1) JMIN = 1;
-  int JMAX = (int)((XNUI + P.bound4) / P.dvr4 + 1.);
+  int JMAX = quotient_int(XNUI + P.bound4, P.dvr4, P.rdvr4, 1.);
   if (JMAX > (int)P.nptr4) JMAX = (int)P.nptr4;
   const bool co2 = (L.mol == 2);
   r->jmin = JMIN;
