@@ -101,9 +101,10 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
                 unsigned long long* __restrict__ stats);
 __global__ void k_scan_blockmax(const LinePrep* prep, int64_t stride, const int64_t* nlines, int* blockmax,
                                 int nblk_stride);
-__global__ void k_scan_blocks(int* blockmax, int nblk_stride, const int64_t* nlines, int nlayers);
-__global__ void k_scan_apply(const LinePrep* prep, int64_t stride, const int64_t* nlines, const int* blockmax,
-                             int nblk_stride, int* qpanel);
+constexpr int kScanBlock = 1024, kScanThreads = 256;  // lines and threads of a CTA of the scans over a layer's lines
+__global__ void __launch_bounds__(kScanThreads)
+    k_scan_apply(const LinePrep* prep, int64_t stride, const int64_t* nlines, const int* blockmax, int nblk_stride,
+                 int* qpanel);
 __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
     k_line_records(const LayerPlan* plans, int layer0, const double* vft_all, const LinePrep* prep,
                                const int* qpanel, int64_t stride, GridRec* rec, GridRecD* recd,
@@ -118,12 +119,11 @@ __global__ void __launch_bounds__(kSetupThreads, 4)
                           const IsoRow* __restrict__ iso_tab, F4Prep* __restrict__ out, int64_t stride,
                           unsigned long long* __restrict__ stats);
 __global__ void k_f4_count(const F4Prep* prep, int64_t stride, const LayerPlan* plans, int layer0, int64_t* blocksum,
-                           int nblk);
-__global__ void k_f4_blockscan(int64_t* blocksum, int nblk, const LayerPlan* plans, int layer0, int nlayers,
-                               int64_t* ntot);
-__global__ void k_f4_compact(const F4Prep* prep, int64_t stride, const LayerPlan* plans, int layer0,
-                             const int64_t* blocksum, int nblk, int64_t* cidx, long long* vbits, long long* lbits,
-                             int64_t* src, unsigned char* flags, int64_t* cut);
+                           int nblk, int64_t* cut);
+__global__ void __launch_bounds__(kScanThreads)
+    k_f4_compact(const F4Prep* prep, int64_t stride, const LayerPlan* plans, int layer0, const int64_t* blocksum,
+                 int nblk, int64_t* cidx, long long* vbits, long long* lbits, int64_t* src, unsigned char* flags,
+                 int64_t* cut, int64_t* ntot);
 __global__ void k_f4_next(const long long* vbits, const long long* lbits, const int64_t* ntot, int64_t stride,
                           int* gnxt);
 constexpr int kCallEnds = 32;    // records a tabulated SHRINQ call may span

@@ -311,7 +311,6 @@ template __global__ void k_line_prep<true>(const LayerPlan* __restrict__, int, L
                                           unsigned long long* __restrict__);
 
 // ---- prefix maximum of fpanel over a layer's line range -------------------
-constexpr int kScanBlock = 1024;
 
 __global__ void k_scan_blockmax(const LinePrep* __restrict__ prep, int64_t stride, const int64_t* __restrict__ nlines,
                                 int* __restrict__ blockmax, int nblk_stride) {
@@ -334,60 +333,51 @@ __global__ void k_scan_blockmax(const LinePrep* __restrict__ prep, int64_t strid
   }
 }
 
-// exclusive prefix max of the block maxima (one thread per layer; a few
-// thousand blocks at most)
-__global__ void k_scan_blocks(int* __restrict__ blockmax, int nblk_stride, const int64_t* __restrict__ nlines,
-                              int nlayers) {
-  int layer = blockIdx.x * blockDim.x + threadIdx.x;
-  if (layer >= nlayers) return;
-  int64_t n = nlines[layer];
-  int nb = (int)((n + kScanBlock - 1) / kScanBlock);
-  int run = -1;
-  for (int b = 0; b < nb; ++b) {
-    int v = blockmax[layer * nblk_stride + b];
-    blockmax[layer * nblk_stride + b] = run;
-    run = max(run, v);
+// panel of each line = max(largest of the blocks before, inclusive in-block
+// prefix).  A CTA takes the maximum of the blocks before its own itself (a few
+// hundred words from L2; a kernel of its own for their prefix was 12 us of a
+// layer's chain), and scans by warps of 4 times 32 lines (32 lanes with 32
+// consecutive lines each met in one bank of shared memory: 0.33 -> 0.28 ms for 30
+// million lines, 1.87 -> 0.97 ms for 120 million).
+__global__ void __launch_bounds__(kScanThreads)
+    k_scan_apply(const LinePrep* __restrict__ prep, int64_t stride, const int64_t* __restrict__ nlines,
+                 const int* __restrict__ blockmax, int nblk_stride, int* __restrict__ qpanel) {
+  constexpr int kWarps = kScanThreads / 32, kRows = kScanBlock / kScanThreads;
+  __shared__ int before[kWarps], total[kWarps];
+  const int layer = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t n = nlines[layer];
+  const int64_t base = (int64_t)blockIdx.x * kScanBlock + warp * (32 * kRows);
+  if ((int64_t)blockIdx.x * kScanBlock >= n) return;
+  int pre = -1;
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += kScanThreads) pre = max(pre, blockmax[layer * nblk_stride + b]);
+  int v[kRows], run = -1;
+#pragma unroll
+  for (int j = 0; j < kRows; ++j) {
+    const int64_t i = base + 32 * j + lane;
+    v[j] = i < n ? prep[layer * stride + i].fpanel : -1;
   }
-}
-
-// panel of each line = max(exclusive block prefix, inclusive in-block prefix)
-__global__ void k_scan_apply(const LinePrep* __restrict__ prep, int64_t stride, const int64_t* __restrict__ nlines,
-                             const int* __restrict__ blockmax, int nblk_stride, int* __restrict__ qpanel) {
-  int layer = blockIdx.y;
-  int64_t n = nlines[layer];
-  int64_t base = (int64_t)blockIdx.x * kScanBlock;
-  __shared__ int sh[kScanBlock];
-  for (int k = threadIdx.x; k < kScanBlock; k += blockDim.x) {
-    int64_t i = base + k;
-    sh[k] = i < n ? prep[layer * stride + i].fpanel : -1;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    // each lane scans 32 entries, then a warp scan of the lane totals
-    int lane = threadIdx.x;
-    int run = -1;
-    for (int k = 0; k < kScanBlock / 32; ++k) {
-      int idx = lane * (kScanBlock / 32) + k;
-      run = max(run, sh[idx]);
-      sh[idx] = run;
-    }
-    int tot = run;
+  pre = __reduce_max_sync(0xffffffffu, pre);
+#pragma unroll
+  for (int j = 0; j < kRows; ++j) {
+#pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-      int o = __shfl_up_sync(0xffffffffu, tot, off);
-      if (lane >= off) tot = max(tot, o);
+      const int o = __shfl_up_sync(0xffffffffu, v[j], off);
+      if (lane >= off) v[j] = max(v[j], o);
     }
-    int excl = __shfl_up_sync(0xffffffffu, tot, 1);
-    if (lane == 0) excl = -1;
-    excl = max(excl, blockmax[layer * nblk_stride + blockIdx.x]);
-    for (int k = 0; k < kScanBlock / 32; ++k) {
-      int idx = lane * (kScanBlock / 32) + k;
-      sh[idx] = max(sh[idx], excl);
-    }
+    v[j] = max(v[j], run);
+    run = __shfl_sync(0xffffffffu, v[j], 31);
+  }
+  if (lane == 0) {
+    before[warp] = pre;
+    total[warp] = run;
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < kScanBlock; k += blockDim.x) {
-    int64_t i = base + k;
-    if (i < n) qpanel[layer * stride + i] = sh[k];
+  pre = -1;
+  for (int w = 0; w < kWarps; ++w) pre = max(pre, w < warp ? max(before[w], total[w]) : before[w]);
+#pragma unroll
+  for (int j = 0; j < kRows; ++j) {
+    const int64_t i = base + 32 * j + lane;
+    if (i < n) qpanel[layer * stride + i] = max(v[j], pre);
   }
 }
 
@@ -1327,9 +1317,37 @@ template __global__ void k_f4_prep<true>(const LayerPlan* __restrict__, int, Lin
 // loop over them and the groups of its calls, (5) the groups' sums in the
 // reference's order.
 
+// Fields of a corrected line, as 16-byte loads (48 bytes a line)
+struct F4Member {
+  double vnu, sp, spp;
+  float4 w;  // the widths: w.f of the mixed path, the bits of w.d on the FP64 path
+  int mol;
+};
+__device__ __forceinline__ F4Member load_member(const F4Prep* __restrict__ r) {
+  static_assert(sizeof(F4Prep) == 48, "three 16-byte loads");
+  const double2 a = __ldg(reinterpret_cast<const double2*>(r));
+  const int4 b = __ldg(reinterpret_cast<const int4*>(r) + 1);  // spp, first half of w
+  const int4 c = __ldg(reinterpret_cast<const int4*>(r) + 2);  // second half of w, mol, pass
+  F4Member m;
+  m.vnu = a.x;
+  m.sp = a.y;
+  m.spp = __hiloint2double(b.y, b.x);
+  m.w = make_float4(__int_as_float(b.z), __int_as_float(b.w), __int_as_float(c.x), __int_as_float(c.y));
+  m.mol = c.z;
+  return m;
+}
+// SP < 1e-35 (not of a NaN of either sign) and SPP != 0 on the bits: a binary64
+// compare takes the FP64 unit, which bounds the sums
+__device__ __forceinline__ bool weak_sp(double sp) {
+  const long long b = __double_as_longlong(sp);
+  return b < __double_as_longlong(1.0e-35) && (unsigned long long)b << 1 <= 0xFFE0000000000000ull;
+}
+__device__ __forceinline__ bool nonzero_d(double x) { return (__double_as_longlong(x) << 1) != 0; }
+
 __global__ void k_f4_count(const F4Prep* __restrict__ prep, int64_t stride, const LayerPlan* __restrict__ plans,
-                           int layer0, int64_t* __restrict__ blocksum, int nblk) {
+                           int layer0, int64_t* __restrict__ blocksum, int nblk, int64_t* __restrict__ cut) {
   const int layer = blockIdx.y;
+  if (blockIdx.x == 0 && threadIdx.x == 0) cut[layer] = -1;  // k_f4_compact's minimum
   const LayerPlan& P = plans[layer + layer0];
   const int64_t n = P.f4_hi - P.f4_lo;
   const int64_t base = (int64_t)blockIdx.x * 1024;
@@ -1349,76 +1367,69 @@ __global__ void k_f4_count(const F4Prep* __restrict__ prep, int64_t stride, cons
   }
 }
 
-__global__ void k_f4_blockscan(int64_t* __restrict__ blocksum, int nblk, const LayerPlan* __restrict__ plans,
-                               int layer0, int nlayers, int64_t* __restrict__ ntot) {
-  int layer = blockIdx.x * blockDim.x + threadIdx.x;
-  if (layer >= nlayers) return;
-  const LayerPlan& P = plans[layer + layer0];
-  const int64_t n = P.f4_hi - P.f4_lo;
-  const int nb = (int)((n + 1 + 1023) / 1024);  // blocks covering t = 0..n
-  int64_t run = 0;
-  for (int b = 0; b < nb; ++b) {
-    int64_t v = blocksum[(int64_t)layer * nblk + b];
-    blocksum[(int64_t)layer * nblk + b] = run;
-    run += v;
-  }
-  ntot[layer] = run;
-}
-
 // cidx[t] = passing lines before t (t = 0..n, cidx[n] = total); the passing
 // lines are compacted into vbits / lbits (centre, centre + DVR4/2) and src.
-__global__ void k_f4_compact(const F4Prep* __restrict__ prep, int64_t stride, const LayerPlan* __restrict__ plans,
-                             int layer0, const int64_t* __restrict__ blocksum, int nblk, int64_t* __restrict__ cidx,
-                             long long* __restrict__ vbits, long long* __restrict__ lbits, int64_t* __restrict__ src,
-                             unsigned char* __restrict__ flags, int64_t* __restrict__ cut) {
-  const int layer = blockIdx.y;
+// A CTA adds up the blocks before its own (a kernel of its own for their prefix
+// was 19 us of a layer's chain); the warps count with ballots.
+__global__ void __launch_bounds__(kScanThreads)
+    k_f4_compact(const F4Prep* __restrict__ prep, int64_t stride, const LayerPlan* __restrict__ plans, int layer0,
+                 const int64_t* __restrict__ blocksum, int nblk, int64_t* __restrict__ cidx,
+                 long long* __restrict__ vbits, long long* __restrict__ lbits, int64_t* __restrict__ src,
+                 unsigned char* __restrict__ flags, int64_t* __restrict__ cut, int64_t* __restrict__ ntot) {
+  constexpr int kWarps = kScanThreads / 32, kRows = kScanBlock / kScanThreads;
+  __shared__ long long before[kWarps];
+  __shared__ int total[kWarps];
+  const int layer = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const LayerPlan& P = plans[layer + layer0];
   const int64_t n = P.f4_hi - P.f4_lo;
-  const int64_t base = (int64_t)blockIdx.x * 1024;
-  __shared__ int sh[1024];
-  for (int k = threadIdx.x; k < 1024; k += blockDim.x) {
-    int64_t t = base + k;
-    sh[k] = t < n ? prep[(int64_t)layer * stride + t].pass : 0;
+  if ((int64_t)blockIdx.x * kScanBlock > n) return;
+  const int64_t base = (int64_t)blockIdx.x * kScanBlock + warp * (32 * kRows);
+  long long pre = 0;
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += kScanThreads) pre += blocksum[(int64_t)layer * nblk + b];
+  unsigned in[kRows];
+  int count = 0;
+#pragma unroll
+  for (int j = 0; j < kRows; ++j) {
+    const int64_t t = base + 32 * j + lane;
+    in[j] = __ballot_sync(0xffffffffu, t < n && prep[(int64_t)layer * stride + t].pass != 0);
+    count += __popc(in[j]);
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) pre += __shfl_xor_sync(0xffffffffu, pre, off);
+  if (lane == 0) {
+    before[warp] = pre;
+    total[warp] = count;
   }
   __syncthreads();
-  if (threadIdx.x < 32) {
-    int lane = threadIdx.x, run = 0;
-    for (int k = 0; k < 32; ++k) {
-      int idx = lane * 32 + k;
-      int v = sh[idx];
-      sh[idx] = run;  // exclusive within the lane's 32
-      run += v;
-    }
-    int tot = run;
-    for (int off = 1; off < 32; off <<= 1) {
-      int o = __shfl_up_sync(0xffffffffu, tot, off);
-      if (lane >= off) tot += o;
-    }
-    int excl = tot - run;
-    for (int k = 0; k < 32; ++k) sh[lane * 32 + k] += excl;
-  }
-  __syncthreads();
-  const int64_t off0 = blocksum[(int64_t)layer * nblk + blockIdx.x];
+  long long c0 = 0;
+  for (int w = 0; w < kWarps; ++w) c0 += before[w] + (w < warp ? total[w] : 0);
   const double half = P.dvr4 / 2.;
-  for (int k = threadIdx.x; k < 1024; k += blockDim.x) {
-    int64_t t = base + k;
+  const bool v2pos = P.v2l4 >= 0.;  // then doubles order like their bits against it
+#pragma unroll
+  for (int j = 0; j < kRows; ++j) {
+    const int64_t t = base + 32 * j + lane;
+    const int64_t c = c0 + __popc(in[j] & ((1u << lane) - 1u));
+    c0 += __popc(in[j]);
     if (t > n) continue;
-    int64_t c = off0 + sh[k];
     cidx[(int64_t)layer * (stride + 1) + t] = c;
-    if (t == n) continue;
-    const F4Prep& r = prep[(int64_t)layer * stride + t];
-    if (r.pass) {
+    if (t == n) {
+      ntot[layer] = c;
+      continue;
+    }
+    if (in[j] >> lane & 1u) {
+      const F4Member r = load_member(prep + ((int64_t)layer * stride + t));
       vbits[(int64_t)layer * stride + c] = __double_as_longlong(r.vnu);
       lbits[(int64_t)layer * stride + c] = __double_as_longlong(r.vnu + half);
       src[(int64_t)layer * stride + c] = t;
       // SHRINQ zeroes SP < 1e-35 (and SPP with it); a coupled line (SPP
       // still nonzero) is a record of its own (4), else a group emits a
       // non-CO2 / CO2 line when its strength sum of that kind is positive
-      bool strong = !(r.sp < 1.0e-35);
-      const bool coupled = strong && r.spp != 0.;
+      const bool strong = !weak_sp(r.sp);
+      const bool coupled = strong && nonzero_d(r.spp);
       flags[(int64_t)layer * stride + c] =
           (unsigned char)(coupled ? 4 : ((strong && r.mol != 2 ? 1 : 0) | (strong && r.mol == 2 ? 2 : 0)));
-      if (r.vnu > P.v2l4) atomicMin((unsigned long long*)&cut[layer], (unsigned long long)c);
+      if (v2pos ? __double_as_longlong(r.vnu) > __double_as_longlong(P.v2l4) : r.vnu > P.v2l4)
+        atomicMin((unsigned long long*)&cut[layer], (unsigned long long)c);
     }
   }
 }
@@ -1439,7 +1450,17 @@ __global__ void k_f4_next(const long long* __restrict__ vbits, const long long* 
   for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < total; b += (int64_t)gridDim.x * blockDim.x) {
     const long long lim = lbits[(int64_t)layer * stride + b];
     int64_t j = b + 2;
+    // four loads at a time: the walk from line to line waited for each
+    for (; j + 4 <= total; j += 4) {
+      const long long v0 = V[j], v1 = V[j + 1], v2 = V[j + 2], v3 = V[j + 3];
+      const int k = v0 > lim ? 0 : v1 > lim ? 1 : v2 > lim ? 2 : v3 > lim ? 3 : 4;
+      if (k < 4) {
+        j += k;
+        goto found;
+      }
+    }
     while (j < total && V[j] <= lim) ++j;
+  found:
     gnxt[(int64_t)layer * stride + b] = (int)(j - 1);
   }
 }
@@ -1997,33 +2018,6 @@ __device__ __forceinline__ ShrunkLine shrunk_line(int k, bool mixed, double SUMV
 // 32 groups' members at once.
 constexpr int kGroupWarps = kGroupSumThreads / 32;
 constexpr int kGroupWarpMin = 20;  // mean lines per group from which a warp takes a group
-
-// Fields of a corrected line, as 16-byte loads (48 bytes a line)
-struct F4Member {
-  double vnu, sp, spp;
-  float4 w;  // the widths: w.f of the mixed path, the bits of w.d on the FP64 path
-  int mol;
-};
-__device__ __forceinline__ F4Member load_member(const F4Prep* __restrict__ r) {
-  static_assert(sizeof(F4Prep) == 48, "three 16-byte loads");
-  const double2 a = __ldg(reinterpret_cast<const double2*>(r));
-  const int4 b = __ldg(reinterpret_cast<const int4*>(r) + 1);  // spp, first half of w
-  const int4 c = __ldg(reinterpret_cast<const int4*>(r) + 2);  // second half of w, mol, pass
-  F4Member m;
-  m.vnu = a.x;
-  m.sp = a.y;
-  m.spp = __hiloint2double(b.y, b.x);
-  m.w = make_float4(__int_as_float(b.z), __int_as_float(b.w), __int_as_float(c.x), __int_as_float(c.y));
-  m.mol = c.z;
-  return m;
-}
-// SP < 1e-35 (not of a NaN of either sign) and SPP != 0 on the bits: a binary64
-// compare takes the FP64 unit, which bounds the sums
-__device__ __forceinline__ bool weak_sp(double sp) {
-  const long long b = __double_as_longlong(sp);
-  return b < __double_as_longlong(1.0e-35) && (unsigned long long)b << 1 <= 0xFFE0000000000000ull;
-}
-__device__ __forceinline__ bool nonzero_d(double x) { return (__double_as_longlong(x) << 1) != 0; }
 
 // one group by one thread, the next member loaded while one is added
 __device__ __forceinline__ void group_sum_thread(const F4Prep* __restrict__ pr, const int64_t* __restrict__ S,

@@ -1093,17 +1093,13 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     int nblk4 = (int)((f4stride + 1 + 1023) / 1024);
     h->launches++;
     k_f4_count<<<dim3(nblk4, count), 256, 0, st>>>(h->f4prep.as<F4Prep>(), f4stride, dplans, first,
-                                                   h->f4blk.as<int64_t>(), nblk4);
+                                                   h->f4blk.as<int64_t>(), nblk4, h->f4cut.as<int64_t>());
     h->launches++;
-    k_f4_blockscan<<<(count + 63) / 64, 64, 0, st>>>(h->f4blk.as<int64_t>(), nblk4, dplans, first, count,
-                                                     h->f4ntot.as<int64_t>());
-    CUDA_TRY(h, cudaMemsetAsync(h->f4cut.p, 0xff, sizeof(int64_t) * count, st));
-    h->launches++;
-    k_f4_compact<<<dim3(nblk4, count), 256, 0, st>>>(h->f4prep.as<F4Prep>(), f4stride, dplans, first,
+    k_f4_compact<<<dim3(nblk4, count), kScanThreads, 0, st>>>(h->f4prep.as<F4Prep>(), f4stride, dplans, first,
                                                      h->f4blk.as<int64_t>(), nblk4, h->f4cidx.as<int64_t>(),
                                                      h->f4vb.as<long long>(), h->f4lb.as<long long>(),
                                                      h->f4src.as<int64_t>(), h->f4flag.as<unsigned char>(),
-                                                     h->f4cut.as<int64_t>());
+                                                     h->f4cut.as<int64_t>(), h->f4ntot.as<int64_t>());
     h->launches++;
     k_f4_next<<<dim3((unsigned)std::min<int64_t>((f4stride + 255) / 256, 4096), count), 256, 0, st>>>(
         h->f4vb.as<long long>(), h->f4lb.as<long long>(), h->f4ntot.as<int64_t>(), f4stride, h->f4nxt.as<int>());
@@ -1244,9 +1240,7 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
   k_scan_blockmax<<<dim3(nblk, count), 256, 0, st>>>(h->prep.as<LinePrep>(), lstride, h->nlines_d.as<int64_t>() + first,
                                                       h->blockmax.as<int>(), nblk);
   h->launches++;
-  k_scan_blocks<<<(count + 63) / 64, 64, 0, st>>>(h->blockmax.as<int>(), nblk, h->nlines_d.as<int64_t>() + first, count);
-  h->launches++;
-  k_scan_apply<<<dim3(nblk, count), 256, 0, st>>>(h->prep.as<LinePrep>(), lstride, h->nlines_d.as<int64_t>() + first,
+  k_scan_apply<<<dim3(nblk, count), kScanThreads, 0, st>>>(h->prep.as<LinePrep>(), lstride, h->nlines_d.as<int64_t>() + first,
                                                    h->blockmax.as<int>(), nblk, h->qpanel.as<int>());
   const int nagg = (int)((lstride + kRecBlock - 1) / kRecBlock);
   h->launches++;
