@@ -82,10 +82,12 @@ struct alignas(16) MixedTables {
 static_assert(sizeof(MixedTables) % 16 == 0, "a bulk copy moves multiples of 16 bytes");
 
 // kernels of prep.cu (FP64, no FMA contraction)
-extern __constant__ double c_AVRAT[102], c_CGAUSS[102], c_CF1[102], c_CF2[102], c_CF3[102], c_CER[102];
-// FP32 copies of CF1, CF2, CF3, CGAUSS, CER (mixed-path shape coefficients)
-extern __constant__ float c_SHAPEf[5][102];
-extern __constant__ float c_AVRATf[102];
+// Tables that every lane reads at its line's own place, in global memory: from
+// the constant cache a warp's 32 places come one after another
+extern __device__ double c_AVRAT[102], c_CGAUSS[102], c_CF1[102], c_CF2[102], c_CF3[102], c_CER[102];
+// FP32 copies of CF1, CF2, CF3, CGAUSS, CER (mixed-path shape coefficients), a row per place
+extern __device__ float4 c_SHAPEf[102][2];
+extern __device__ float c_AVRATf[102];
 // Cpl: the line list holds coupled lines (IFLG 1 or 3) with their coefficient
 // records.  (A template kernel's declaration repeats its definition's
 // parameter qualifiers exactly: nvcc takes a difference in __restrict__ for

@@ -71,9 +71,10 @@ struct RtSegArgs {
 };
 
 // 201-point interpolation coefficients of interpSpectrum (clblm_Spectrum.f90:350-365),
-// in FP64 and as FP32 copies for the mixed path (defined in rt.cu)
-extern __constant__ double c_IA1[203], c_IA2[203], c_IA3[203], c_IA4[203];
-extern __constant__ float c_IAf[4][203];
+// in FP64 and as FP32 copies for the mixed path (defined in rt.cu), in global
+// memory: lanes read them at different IP
+extern __device__ double2 c_IA[203][2];
+extern __device__ float4 c_IAf[203];
 
 // Stencil of output point I (1-based) of grid (V1, dvout, nout) on the input
 // grid (V1, dvin, nin): up to four input indices and weights of type W.
@@ -85,9 +86,20 @@ struct Stencil {
 };
 
 template <typename W>
-__device__ __forceinline__ W ia_coef(int k, int IP) {
-  if constexpr (sizeof(W) == 8) return k == 0 ? c_IA1[IP] : k == 1 ? c_IA2[IP] : k == 2 ? c_IA3[IP] : c_IA4[IP];
-  else return c_IAf[k][IP];
+__device__ __forceinline__ void ia_coefs(int IP, W* w) {
+  if constexpr (sizeof(W) == 8) {
+    const double2 a = __ldg(&c_IA[IP][0]), b = __ldg(&c_IA[IP][1]);
+    w[0] = a.x;
+    w[1] = a.y;
+    w[2] = b.x;
+    w[3] = b.y;
+  } else {
+    const float4 a = __ldg(&c_IAf[IP]);
+    w[0] = a.x;
+    w[1] = a.y;
+    w[2] = a.z;
+    w[3] = a.w;
+  }
 }
 template <typename W>
 __device__ __forceinline__ W b_coef(const InterpSpec& s, int k, int NL) {
@@ -140,7 +152,7 @@ __device__ __forceinline__ Stencil<W> interp_stencil(const InterpSpec& s, int64_
   st.i[1] = iIn;
   st.i[2] = iIn + 1;
   st.i[3] = iIn + 2;
-  for (int k = 0; k < 4; ++k) st.w[k] = ia_coef<W>(k, IP);
+  ia_coefs<W>(IP, st.w);
   st.n = 4;
   return st;
 }

@@ -70,12 +70,9 @@ __global__ void __launch_bounds__(kOdJobThreads) k_od_jobs(const JacJob* jobs, i
   const bool general = jb.spec.kind != 0 && jb.spec.itype < 0;
   if (general) {  // CTA-uniform
     for (int k = threadIdx.x; k < 203; k += blockDim.x) {
-      Real4 c;
-      c.x = ia_coef<Real>(0, k);
-      c.y = ia_coef<Real>(1, k);
-      c.z = ia_coef<Real>(2, k);
-      c.w = ia_coef<Real>(3, k);
-      ia[k] = c;
+      Real c[4];
+      ia_coefs<Real>(k, c);
+      ia[k] = {c[0], c[1], c[2], c[3]};
     }
     __syncthreads();
     const int2* map = jb.spec.map;

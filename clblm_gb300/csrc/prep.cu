@@ -23,11 +23,11 @@
 
 namespace clblm {
 
-__constant__ double c_AVRAT[102], c_CGAUSS[102], c_CF1[102], c_CF2[102], c_CF3[102], c_CER[102];
-__constant__ float c_SHAPEf[5][102];
-__constant__ float c_AVRATf[102];
+__device__ double c_AVRAT[102], c_CGAUSS[102], c_CF1[102], c_CF2[102], c_CF3[102], c_CER[102];
+__device__ float4 c_SHAPEf[102][2];
+__device__ float c_AVRATf[102];
 // MaxISOTPL_smass, clblm_ConstParam.f90:246-251 (index: HITRAN molecule 0..47)
-__constant__ int c_MAXISO[kMaxMol + 1] = {0, 6, 10, 9, 5, 6, 4, 3, 3, 2, 1, 2, 2, 3, 2, 4, 4, 2,
+__device__ const int c_MAXISO[kMaxMol + 1] = {0, 6, 10, 9, 5, 6, 4, 3, 3, 2, 1, 2, 2, 3, 2, 4, 4, 2,
                                           2,  5, 3, 2, 2, 3, 2, 1, 3, 2, 1, 2, 1, 3, 1, 1,
                                           1,  2, 1, 2, 2, 1, 2, 1, 1, 1, 1, 2, 4, 1};
 
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
     int iso = (molf % 1000) / 100;
     if (iso == 0) iso = 10;
     bool ok = iflg >= 0 && m >= 1 && m <= kMaxMol && P.mrow[m] >= 0;
-    if (ok && iso > c_MAXISO[m]) ok = false;
+    if (ok && iso > __ldg(c_MAXISO + m)) ok = false;
     double SUI = 0.;
     if (ok) {
       SUI = f32_to_f64(lines.sp[i]) * P.wk[m];
@@ -210,7 +210,8 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
         ok = false;
       } else {
         double ZETDIF = FZETA - i32_to_f64(IZ - 1);
-        double ALFV = (c_AVRAT[IZ - 1] + ZETDIF * (c_AVRAT[IZ] - c_AVRAT[IZ - 1])) * (ALFL + ALFAD);
+        const double av0 = __ldg(c_AVRAT + IZ - 1), av1 = __ldg(c_AVRAT + IZ);
+        double ALFV = (av0 + ZETDIF * (av1 - av0)) * (ALFL + ALFAD);
         int nmin = 0, npl = 0;
         if (ALFV < P.dv) {
           ALFV = P.dv;
@@ -383,7 +384,8 @@ __global__ void __launch_bounds__(kScanThreads)
 
 // ---- CNVFNQ per-line set-up ----------------------------------------------
 __device__ __forceinline__ void interp_coef(const double* tab, int IZM, double ZETDIF, double DEPTHA, double* out) {
-  *out = DEPTHA * (tab[IZM - 1] + ZETDIF * (tab[IZM] - tab[IZM - 1]));
+  const double t0 = __ldg(tab + IZM - 1), t1 = __ldg(tab + IZM);
+  *out = DEPTHA * (t0 + ZETDIF * (t1 - t0));
 }
 
 __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
@@ -436,10 +438,14 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
       float c[5];  // the same, FP32 (mixed path)
       if (P.mixed) {  // shape coefficients set no index: FP32
         const float zd = f64_to_f32(ZETDIF), de = f64_to_f32(DEPTHA);
-        for (int q5 = 0; q5 < 5; ++q5) {
-          const float* T = c_SHAPEf[q5];
-          c[q5] = de * (T[IZM - 1] + zd * (T[IZM] - T[IZM - 1]));
-        }
+        const float4 a0 = __ldg(&c_SHAPEf[IZM - 1][0]), a1 = __ldg(&c_SHAPEf[IZM][0]);
+        const float b0 = __ldg(&c_SHAPEf[IZM - 1][1].x), b1 = __ldg(&c_SHAPEf[IZM][1].x);
+        auto at = [&](float t0, float t1) { return de * (t0 + zd * (t1 - t0)); };
+        c[0] = at(a0.x, a1.x);
+        c[1] = at(a0.y, a1.y);
+        c[2] = at(a0.z, a1.z);
+        c[3] = at(a0.w, a1.w);
+        c[4] = at(b0, b1);
       } else {
         interp_coef(c_CF1, IZM, ZETDIF, DEPTHA, &STRFA1);
         interp_coef(c_CF2, IZM, ZETDIF, DEPTHA, &STRFA2);
@@ -1219,7 +1225,7 @@ __global__ void __launch_bounds__(kSetupThreads, 4)
     int iso = (molf % 1000) / 100;
     if (iso == 0) iso = 10;
     bool ok = iflg >= 0 && m >= 1 && m <= kMaxMol && P.mrow[m] >= 0;
-    if (ok && iso > c_MAXISO[m]) ok = false;
+    if (ok && iso > __ldg(c_MAXISO + m)) ok = false;
     if (ok) {
       double SUI = (double)lines.sp[i] * P.wk[m];
       if (SUI != 0. && !(lines.vnu[i] < P.v1l4)) {
@@ -2200,7 +2206,7 @@ __device__ void f4_record(const LayerPlan& P, const ShrunkLine& L, double VNUI, 
     int IZ = (int)(100.f * ZETAI + (float)kONEPL);
     IZ = IZ < 1 ? 1 : (IZ > 101 ? 101 : IZ);
     const float ZETDIF = 100.f * ZETAI - (float)(IZ - 1);
-    const float a0 = c_AVRATf[IZ - 1], a1 = c_AVRATf[IZ];
+    const float a0 = __ldg(c_AVRATf + IZ - 1), a1 = __ldg(c_AVRATf + IZ);
     const float ALFAVI = (a0 + ZETDIF * (a1 - a0)) * (ALFALI + ALFADI);
     const float RALFVI = 1.f / ALFAVI;
     const float SP = L.w.f[2], rpi = (float)(1. / 3.14159265358979323846);
@@ -2224,7 +2230,8 @@ __device__ void f4_record(const LayerPlan& P, const ShrunkLine& L, double VNUI, 
     const double ZETAI = ALFALI / (ALFALI + ALFADI);
     const int IZ = (int)(100. * ZETAI + kONEPL);
     const double ZETDIF = 100. * ZETAI - (double)(IZ - 1);
-    const double ALFAVI = (c_AVRAT[IZ - 1] + ZETDIF * (c_AVRAT[IZ] - c_AVRAT[IZ - 1])) * (ALFALI + ALFADI);
+    const double av0 = __ldg(c_AVRAT + IZ - 1), av1 = __ldg(c_AVRAT + IZ);
+    const double ALFAVI = (av0 + ZETDIF * (av1 - av0)) * (ALFALI + ALFADI);
     const double RALFVI = 1. / ALFAVI;
     const double SIL = L.sp * RECPI * ALFALI;
     const double SIV = (ALFALI * RALFVI) * L.sp * RECPI * RALFVI;

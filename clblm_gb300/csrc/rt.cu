@@ -26,8 +26,8 @@ namespace clblm {
 
 // 201-point interpolation coefficients of interpSpectrum (clblm_Spectrum.f90:350-365),
 // in FP64 and as FP32 copies for the mixed path
-__constant__ double c_IA1[203], c_IA2[203], c_IA3[203], c_IA4[203];
-__constant__ float c_IAf[4][203];
+__device__ double2 c_IA[203][2];
+__device__ float4 c_IAf[203];
 
 // The general-ratio branch of interpSpectrum (clblm_Spectrum.f90:528-565)
 // steps the phase P by DVout/DVin with a carry into iIn and restarts it from
@@ -476,28 +476,22 @@ template __global__ void k_od_out<false>(const void*, int64_t, InterpSpec, int64
 template __global__ void k_od_out<true>(const void*, int64_t, InterpSpec, int64_t, double*);
 
 cudaError_t rt_upload_interp_coef(cudaStream_t st) {
-  double a1[203], a2[203], a3[203], a4[203];
+  double2 a[203][2];  // (staged by the copies before they return: pageable sources)
+  float4 af[203];
   const double XNUMCF = 201.;
   for (int IP = 0; IP <= 202; ++IP) {
     double P = ((double)IP - 1.0) / (XNUMCF - 1.0);
     double PP = P * P;
-    a1[IP] = -P / 2.0 * ((1 - P) * (1 - P));
-    a2[IP] = 1.0 - PP * (3.0 - 2.0 * P) + PP / 2.0 * (1.0 - P);
-    a3[IP] = PP * (3.0 - 2.0 * P) + P / 2.0 * ((1.0 - P) * (1.0 - P));
-    a4[IP] = -PP / 2 * (1.0 - P);
+    const double a1 = -P / 2.0 * ((1 - P) * (1 - P));
+    const double a2 = 1.0 - PP * (3.0 - 2.0 * P) + PP / 2.0 * (1.0 - P);
+    const double a3 = PP * (3.0 - 2.0 * P) + P / 2.0 * ((1.0 - P) * (1.0 - P));
+    const double a4 = -PP / 2 * (1.0 - P);
+    a[IP][0] = make_double2(a1, a2);
+    a[IP][1] = make_double2(a3, a4);
+    af[IP] = make_float4((float)a1, (float)a2, (float)a3, (float)a4);
   }
-  cudaError_t e = cudaMemcpyToSymbolAsync(c_IA1, a1, sizeof a1, 0, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(c_IA2, a2, sizeof a2, 0, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(c_IA3, a3, sizeof a3, 0, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(c_IA4, a4, sizeof a4, 0, cudaMemcpyHostToDevice, st);
+  const cudaError_t e = cudaMemcpyToSymbolAsync(c_IA, a, sizeof a, 0, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return e;
-  static float af[4][203];  // staged by the copy before it returns (pageable source)
-  for (int IP = 0; IP <= 202; ++IP) {
-    af[0][IP] = (float)a1[IP];
-    af[1][IP] = (float)a2[IP];
-    af[2][IP] = (float)a3[IP];
-    af[3][IP] = (float)a4[IP];
-  }
   return cudaMemcpyToSymbolAsync(c_IAf, af, sizeof af, 0, cudaMemcpyHostToDevice, st);
 }
 

@@ -408,10 +408,10 @@ int upload_tables(clblm_handle* h) {
   CUDA_TRY(h, cudaMemcpyToSymbol(c_CF3, CLBLM_CF3, sizeof CLBLM_CF3));
   CUDA_TRY(h, cudaMemcpyToSymbol(c_CER, CLBLM_CER, sizeof CLBLM_CER));
   {
-    float sf[5][102];
+    float sf[102][8] = {};
     const double* src[5] = {CLBLM_CF1, CLBLM_CF2, CLBLM_CF3, CLBLM_CGAUSS, CLBLM_CER};
     for (int q = 0; q < 5; ++q)
-      for (int i = 0; i < 102; ++i) sf[q][i] = (float)src[q][i];
+      for (int i = 0; i < 102; ++i) sf[i][q] = (float)src[q][i];
     CUDA_TRY(h, cudaMemcpyToSymbol(c_SHAPEf, sf, sizeof sf));
     float af[102];
     for (int i = 0; i < 102; ++i) af[i] = (float)CLBLM_AVRAT[i];
