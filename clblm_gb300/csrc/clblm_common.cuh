@@ -51,7 +51,7 @@ constexpr int kMaxSlices = 32;
 struct LayerPlan {
   // grid
   double v1, v2, dv, dvr2, dvr3, alfav, alfmax, bound, vbot, vtop, vft0;
-  double wavdxf, rdv;             // DV/DXF1 (CNVFNQ's WAVDXF) and 1/DV (estimates only)
+  double wavdxf, rdv;             // DV/DXF1 (CNVFNQ's WAVDXF) and 1/DV (estimates, div_by)
   double conf2, conf3;            // CNVFNQ's CONF2 = DV/DVR2, CONF3 = DV/DVR3
   double omconf2, omconf3;        // 1 - CONF2, 1 - CONF3
   double pave, tave, wtot, xkt, xkt0, betacr, tratio, rhorat, pavp0, pavp2;
@@ -149,13 +149,13 @@ __device__ __forceinline__ CnvfnqSetup cnvfnq_setup(const LayerPlan& P, double v
   // layer's, formed once on the host with the same operations
   const double CONF2 = P.conf2, CONF3 = P.conf3;
   s.zslope = __dmul_rn(recalf, P.wavdxf);
-  const double ZINT = __ddiv_rn(__dsub_rn(vnu, vft_q), P.dv);
+  const double ZINT = div_by(__dsub_rn(vnu, vft_q), P.dv, P.rdv);
   s.zint = ZINT;
   // INT truncations and the integer-to-binary64 conversions are exact
   // integer arithmetic (clblm_fpconv.cuh): the binary64 pipe keeps the sums
   s.jmax1 = f64_to_i32_trunc(__dadd_rn(__dadd_rn(ZINT, bhwdxf), 1.5));
   s.jmin1 = f64_to_i32_trunc(__dadd_rn(__dsub_rn(ZINT, bhwdxf), 1.5));
-  const double RSHFT = ZINT < 0.0 ? -0.5 : 0.5;
+  const double RSHFT = (int64_t)fpc_bits(ZINT) < 0 && !zero_bits(ZINT) ? -0.5 : 0.5;
   s.j2shft = f64_to_i32_trunc(__dadd_rn(__dmul_rn(ZINT, P.omconf2), RSHFT));
   s.j3shft = f64_to_i32_trunc(__dadd_rn(__dmul_rn(ZINT, P.omconf3), RSHFT));
   const int JMIN2 = s.jmin1 - s.j2shft, JMIN3 = s.jmin1 - s.j3shft;

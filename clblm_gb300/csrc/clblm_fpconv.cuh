@@ -11,6 +11,7 @@
 // conversion.  The functions are host and device code, so that a host test
 // checks them against the compiler's own conversions.
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 
@@ -145,5 +146,29 @@ CLBLM_HD int32_t f64_to_i32_trunc(double x) {
   const int32_t t = (int32_t)(M >> (52 - E));
   return (b >> 63) ? -t : t;
 }
+
+// x / d correctly rounded, with r = 1 / d correctly rounded: two steps of
+// Markstein's division (IBM J. Res. Dev. 34, 1990; the second remainder is
+// exact and its correction rounds once). For a divisor known ahead this is five
+// operations of the binary64 unit, where a division is about ten. No quotient
+// or remainder may leave the normal range (x = 0 does not).
+CLBLM_HD double div_by(double x, double d, double r) {
+#ifdef __CUDA_ARCH__
+  const double q0 = __dmul_rn(x, r);
+  const double q1 = __fma_rn(__fma_rn(-q0, d, x), r, q0);
+  return __fma_rn(__fma_rn(-q1, d, x), r, q1);
+#else
+  const double q0 = x * r;
+  const double q1 = std::fma(std::fma(-q0, d, x), r, q0);
+  return std::fma(std::fma(-q1, d, x), r, q1);
+#endif
+}
+// a < b and x == 0 on the bits, for values that are not NaN: nonnegative doubles
+// order like their bits, and below a nonnegative b every negative a lies (-0
+// apart, which no caller has)
+CLBLM_HD bool less_bits(double a, double b) {
+  return (int64_t)fpc_bits(b) >= 0 ? (int64_t)fpc_bits(a) < (int64_t)fpc_bits(b) : a < b;
+}
+CLBLM_HD bool zero_bits(double x) { return (fpc_bits(x) << 1) == 0; }
 
 }  // namespace clblm

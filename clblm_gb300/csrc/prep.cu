@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
     double SUI = 0.;
     if (ok) {
       SUI = f32_to_f64(lines.sp[i]) * P.wk[m];
-      if (SUI == 0.) ok = false;
+      if (zero_bits(SUI)) ok = false;
     }
     if (ok) {
       nlin++;
@@ -213,11 +213,11 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
         const double av0 = __ldg(c_AVRAT + IZ - 1), av1 = __ldg(c_AVRAT + IZ);
         double ALFV = (av0 + ZETDIF * (av1 - av0)) * (ALFL + ALFAD);
         int nmin = 0, npl = 0;
-        if (ALFV < P.dv) {
+        if (less_bits(ALFV, P.dv)) {
           ALFV = P.dv;
           nmin = 1;
         }
-        if (ALFV > P.alfmax) {
+        if (less_bits(P.alfmax, ALFV)) {
           ALFV = P.alfmax;
           npl = 1;
         }
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
         // in.  Lines of the first record are read with panel 0; k_line_records
         // checks that no later line would be dropped at its own read panel.
         // (ALFV > 0: the sum is at least VNU, so only VNU < VFT can drop.)
-        if (VNU < vft[0] && kHWF3 * ALFV + VNU < vft[0]) ok = false;
+        if (less_bits(VNU, vft[0]) && kHWF3 * ALFV + VNU < vft[0]) ok = false;
         if (ok) {
           double RECALF = 1. / ALFV;
           const float EPP0 = lines.epp[i];
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
   const LayerPlan& P = plans[layer + layer0];
   int64_t n = P.line_hi - P.line_lo + 1;
   const double* vft = vft_all + P.vft_off;
-  double amax = 0.;
+  long long amax = 0;  // the bits of ALFV > 0 order like their values
   unsigned long long bad = 0;
   unsigned long long steps = 0;  // CNVFNQ inner steps JMAX1-JMIN1+1 of the accepted lines
   __shared__ int red[3][2][kRecBlock / 32];
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
         int qr = 0;
         if (rs - 1 >= P.line_lo) qr = max(0, qpanel[layer * stride + (rs - 1 - P.line_lo)]);
         // (ALFV > 0: only VNU < VFT can drop the line)
-        if (qr > 0 && qr < P.npanels && lp.vnu < vft[qr] && kHWF3 * lp.alfv + lp.vnu < vft[qr]) bad++;
+        if (qr > 0 && qr < P.npanels && less_bits(lp.vnu, vft[qr]) && kHWF3 * lp.alfv + lp.vnu < vft[qr]) bad++;
       }
       double DEPTHA = lp.sp * lp.recalf;
       int IZM = lp.iz;
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
       l1 = {lo1, zs_lo};
       l2 = {lo2, zs_lo};
       l3 = {lo3, zs_lo};
-      amax = fmax(amax, lp.alfv);
+      amax = max(amax, __double_as_longlong(lp.alfv));
       // a coupled line (SPPSP != 0, tested on the bits: no FP64 compare) has
       // its records go the exact way
       if ((__double_as_longlong(lp.sppsp) << 1) != 0) {
@@ -547,12 +547,12 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
       __syncthreads();
     }
   }
-  for (int off = 16; off > 0; off >>= 1) amax = fmax(amax, __shfl_down_sync(0xffffffffu, amax, off));
+  for (int off = 16; off > 0; off >>= 1) amax = max(amax, __shfl_down_sync(0xffffffffu, amax, off));
   unsigned long long b = bad;
   for (int off = 16; off > 0; off >>= 1) b += __shfl_down_sync(0xffffffffu, b, off);
   for (int off = 16; off > 0; off >>= 1) steps += __shfl_down_sync(0xffffffffu, steps, off);
   if ((threadIdx.x & 31) == 0) {
-    if (amax > 0.) atomicMax((unsigned long long*)&alfvmax[layer + layer0], (unsigned long long)__double_as_longlong(amax));
+    if (amax > 0) atomicMax((unsigned long long*)&alfvmax[layer + layer0], (unsigned long long)amax);
     if (b) atomicAdd(&stats[(layer + layer0) * kStatsPerLayer + 4], b);
     if (steps) atomicAdd(&stats[(layer + layer0) * kStatsPerLayer + 5], steps);
   }
