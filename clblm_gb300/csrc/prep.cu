@@ -2019,66 +2019,152 @@ __device__ __forceinline__ ShrunkLine shrunk_line(int k, bool mixed, double SUMV
 // A surface layer's groups hold 64 lines and more (DVR4/2 = 0.32 cm-1 at 200
 // lines per cm-1): 170 us for one such layer with a thread per group, whose
 // loads followed one another.  Layers with fewer than kGroupWarpMin lines
-// per group keep a thread per group: there are many of them, and the FP64
-// unit, which takes 16 cycles for an instruction of any number of lanes, adds
-// 32 groups' members at once.
+// per group take a thread per group, sorted by length: there are many of them,
+// and the FP64 unit, which takes as long for one lane as for 32, adds 32
+// groups' members at once.
 constexpr int kGroupWarps = kGroupSumThreads / 32;
-constexpr int kGroupWarpMin = 20;  // mean lines per group from which a warp takes a group
+// Launches of many lines do so at any length: a warp's group costs an addition
+// of the FP64 unit per line where 32 threads' groups cost three per 32 lines
+// (10 million lines near the surface of a 60-layer column: 0.75 ms), and a
+// chain of 100 lines by a thread, 50 us, hides behind the others.
+constexpr int kGroupWarpMin = 20;            // mean lines per group from which a warp takes a group
+constexpr int64_t kGroupWarpMax = 1 << 20;   // lines of the launch up to which it does
 
-// one group by one thread, the next member loaded while one is added
+// sums of one group: SUMV, SUMS and the widths' of either kind
+struct GroupSums {
+  double v[2], s[2], al[2], ad[2];
+  float alf[2], adf[2];
+};
+// one group by one thread, the next member loaded while one is added; coupled
+// lines are written on the way.  (A kind's sums are picked and put back by
+// selects: a branch would issue either kind's additions for the warp.)
+template <bool Mixed>
 __device__ __forceinline__ void group_sum_thread(const F4Prep* __restrict__ pr, const int64_t* __restrict__ S,
-                                                 const int4 gr, bool mixed, ShrunkLine* __restrict__ O) {
-  int slot = gr.z;
-  double SUMS[2] = {0., 0.}, SUMV[2] = {0., 0.}, AL[2] = {0., 0.}, AD[2] = {0., 0.};
-  float ALf[2] = {0.f, 0.f}, ADf[2] = {0.f, 0.f};
+                                                 const int4 gr, ShrunkLine* __restrict__ O, int* slot, GroupSums* g) {
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    g->v[k] = g->s[k] = g->al[k] = g->ad[k] = 0.;
+    g->alf[k] = g->adf[k] = 0.f;
+  }
   F4Member nxt = load_member(pr + S[gr.x]);
   for (int u = gr.x; u <= gr.y; ++u) {
     const F4Member r = nxt;
     if (u < gr.y) nxt = load_member(pr + S[u + 1]);
     const bool weak = weak_sp(r.sp);
     if (!weak && nonzero_d(r.spp)) {  // a coupled line is not shrunk (SHRINQ :1566-1578)
-      O[slot++] = shrunk_coupled(pr[S[u]], mixed);
+      O[(*slot)++] = shrunk_coupled(pr[S[u]], Mixed);
       continue;
     }
     const double sp = weak ? 0.0 : r.sp;
-    const double vs = r.vnu * sp;
-    auto add = [&](int k) {
-      SUMV[k] = SUMV[k] + vs;
-      SUMS[k] = SUMS[k] + sp;
-    };
-    if (r.mol != 2) add(0);
-    else add(1);
-    if (mixed) {  // widths set no index: FP32
+    const bool co2 = r.mol == 2;
+    const double v = (co2 ? g->v[1] : g->v[0]) + r.vnu * sp, t = (co2 ? g->s[1] : g->s[0]) + sp;
+    g->v[0] = co2 ? g->v[0] : v;
+    g->v[1] = co2 ? v : g->v[1];
+    g->s[0] = co2 ? g->s[0] : t;
+    g->s[1] = co2 ? t : g->s[1];
+    if constexpr (Mixed) {  // widths set no index: FP32
       const float spf = weak ? 0.f : r.w.z;
       const float al = spf * r.w.x, ad = spf * r.w.y;
-      ALf[0] = ALf[0] + (r.mol != 2 ? al : 0.f);
-      ADf[0] = ADf[0] + (r.mol != 2 ? ad : 0.f);
-      ALf[1] = ALf[1] + (r.mol != 2 ? 0.f : al);
-      ADf[1] = ADf[1] + (r.mol != 2 ? 0.f : ad);
+      g->alf[0] = g->alf[0] + (co2 ? 0.f : al);
+      g->adf[0] = g->adf[0] + (co2 ? 0.f : ad);
+      g->alf[1] = g->alf[1] + (co2 ? al : 0.f);
+      g->adf[1] = g->adf[1] + (co2 ? ad : 0.f);
     } else {
-      const double al = sp * __hiloint2double(__float_as_int(r.w.y), __float_as_int(r.w.x));
-      const double ad = sp * __hiloint2double(__float_as_int(r.w.w), __float_as_int(r.w.z));
-      const int k = r.mol != 2 ? 0 : 1;
-      if (k == 0) {
-        AL[0] = AL[0] + al;
-        AD[0] = AD[0] + ad;
-      } else {
-        AL[1] = AL[1] + al;
-        AD[1] = AD[1] + ad;
-      }
+      const double al = (co2 ? g->al[1] : g->al[0]) +
+                        sp * __hiloint2double(__float_as_int(r.w.y), __float_as_int(r.w.x));
+      const double ad = (co2 ? g->ad[1] : g->ad[0]) +
+                        sp * __hiloint2double(__float_as_int(r.w.w), __float_as_int(r.w.z));
+      g->al[0] = co2 ? g->al[0] : al;
+      g->al[1] = co2 ? al : g->al[1];
+      g->ad[0] = co2 ? g->ad[0] : ad;
+      g->ad[1] = co2 ? ad : g->ad[1];
     }
   }
-#pragma unroll
-  for (int k = 0; k < 2; ++k)
-    if (SUMS[k] > 0.) O[slot++] = shrunk_line(k, mixed, SUMV[k], SUMS[k], AL[k], AD[k], ALf[k], ADf[k]);
+}
+// > 0 on the bits (not of a NaN)
+__device__ __forceinline__ bool positive_d(double x) {
+  const long long b = __double_as_longlong(x);
+  return b > 0 && b <= 0x7FF0000000000000ll;
+}
+
+// The groups [g0, g0 + kGroupSumThreads) of a layer, a thread each, the longest
+// first: with 1.9 lines a group on average and eight in the longest of any 32,
+// the FP64 unit issued three times the additions it had to, and as many
+// quotients again for the few groups with a line of either kind (those wait
+// in a queue until all are done).
+struct GroupShared {
+  int4 gr[kGroupSumThreads];
+  unsigned short order[kGroupSumThreads];
+  int bin[33], start[33], queued;
+  int slot[kGroupSumThreads];
+  double v[kGroupSumThreads], s[kGroupSumThreads], al[kGroupSumThreads], ad[kGroupSumThreads];
+};
+template <bool Mixed>
+__device__ __forceinline__ void group_sums_sorted(GroupShared& W, const F4Prep* __restrict__ pr,
+                                                  const int64_t* __restrict__ S, const int4* __restrict__ G, int64_t g0,
+                                                  int64_t ng, ShrunkLine* __restrict__ O) {
+  const int t = threadIdx.x;
+  if (t < 33) W.bin[t] = 0;
+  if (t == 0) W.queued = 0;
+  __syncthreads();
+  int4 gr = make_int4(0, -1, 0, 0);
+  if (g0 + t < ng) gr = G[g0 + t];
+  const int b = 32 - min(gr.y - gr.x + 1, 32);
+  const int pos = atomicAdd(&W.bin[b], 1);
+  W.gr[t] = gr;
+  __syncthreads();
+  if (t < 32) {
+    const int n = W.bin[t];
+    int x = n;
+    for (int off = 1; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, x, off);
+      if (t >= off) x += o;
+    }
+    W.start[t] = x - n;
+    if (t == 31) W.start[32] = x;
+  }
+  __syncthreads();
+  W.order[W.start[b] + pos] = (unsigned short)t;
+  __syncthreads();
+  gr = W.gr[W.order[t]];
+  if (gr.y >= gr.x) {
+    GroupSums g;
+    int slot = gr.z;
+    group_sum_thread<Mixed>(pr, S, gr, O, &slot, &g);
+    const bool e0 = positive_d(g.s[0]), e1 = positive_d(g.s[1]);
+    if (e0 || e1)
+      O[slot++] = shrunk_line(e0 ? 0 : 1, Mixed, e0 ? g.v[0] : g.v[1], e0 ? g.s[0] : g.s[1], e0 ? g.al[0] : g.al[1],
+                              e0 ? g.ad[0] : g.ad[1], e0 ? g.alf[0] : g.alf[1], e0 ? g.adf[0] : g.adf[1]);
+    if (e0 && e1) {
+      const int q = atomicAdd(&W.queued, 1);
+      W.slot[q] = slot;
+      W.v[q] = g.v[1];
+      W.s[q] = g.s[1];
+      W.al[q] = Mixed ? __hiloint2double(__float_as_int(g.adf[1]), __float_as_int(g.alf[1])) : g.al[1];
+      W.ad[q] = g.ad[1];
+    }
+  }
+  __syncthreads();
+  if (t < W.queued)
+    O[W.slot[t]] = shrunk_line(1, Mixed, W.v[t], W.s[t], W.al[t], W.ad[t], __int_as_float(__double2loint(W.al[t])),
+                               __int_as_float(__double2hiint(W.al[t])));
+  __syncthreads();
 }
 
 __global__ void __launch_bounds__(kGroupSumThreads)
     k_f4_groupsum(const LayerPlan* __restrict__ plans, int layer0, const F4Prep* __restrict__ prep, int64_t stride,
                   const int64_t* __restrict__ src, const int4* __restrict__ groups,
                   const int64_t* __restrict__ ngroups, ShrunkLine* __restrict__ out) {
-  __shared__ double sd[kGroupWarps][8][33];
-  __shared__ float sf[kGroupWarps][4][33];
+  struct Rows {
+    double d[kGroupWarps][8][33];
+    float f[kGroupWarps][4][33];
+  };
+  union Shared {
+    __device__ Shared() {}
+    Rows rows;
+    GroupShared sorted;
+  };
+  __shared__ Shared sh;
   const int layer = blockIdx.y;
   const int64_t ng = ngroups[2 * (layer + layer0)];
   if (ng <= 0) return;
@@ -2087,14 +2173,17 @@ __global__ void __launch_bounds__(kGroupSumThreads)
   const F4Prep* pr = prep + (int64_t)layer * stride;
   ShrunkLine* O = out + (int64_t)layer * stride;
   const bool mixed = plans[layer + layer0].mixed != 0;
-  if ((int64_t)G[ng - 1].y + 1 < kGroupWarpMin * ng) {  // (groups cover the stream from its start)
-    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < ng; g += (int64_t)gridDim.x * blockDim.x)
-      group_sum_thread(pr, S, G[g], mixed, O);
+  const int64_t members = (int64_t)G[ng - 1].y + 1;  // (groups cover the stream from its start)
+  if (members < kGroupWarpMin * ng || members * gridDim.y >= kGroupWarpMax) {
+    for (int64_t g = blockIdx.x * (int64_t)kGroupSumThreads; g < ng; g += (int64_t)gridDim.x * kGroupSumThreads) {
+      if (mixed) group_sums_sorted<true>(sh.sorted, pr, S, G, g, ng, O);
+      else group_sums_sorted<false>(sh.sorted, pr, S, G, g, ng, O);
+    }
     return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double(*D)[33] = sd[warp];
-  float(*F)[33] = sf[warp];
+  double(*D)[33] = sh.rows.d[warp];
+  float(*F)[33] = sh.rows.f[warp];
   for (int64_t g = (int64_t)blockIdx.x * kGroupWarps + warp; g < ng; g += (int64_t)gridDim.x * kGroupWarps) {
     const int4 gr = G[g];
     int slot = gr.z;
