@@ -26,6 +26,24 @@ struct XintPanel {
 };
 constexpr int kAbsStage = 64;
 
+// Radiation-term segments of panels with more than kSegTab of them (low
+// wavenumbers at coarse DV), in slots claimed by atomics: of kMaxSeg entries,
+// or, past that, of kSegSlot
+constexpr int kSegSlot = kNLIM1 + 1;  // at most one segment per point of a panel
+constexpr int kSegPoolSlots = 4096, kMedPoolSlots = 4096;
+struct SegPool {
+  int* next;      // next free slot, of kSegSlot entries and of kMaxSeg
+  int slots;      // slots of kSegSlot entries
+  int* start;     // [slot][kSegSlot + 1]
+  double* v;      // [slot][kSegSlot]
+  double* d;
+  int* med_start;  // [kMedPoolSlots][kMaxSeg]
+  double2* med_v;  // [kMedPoolSlots][kMaxSeg]
+};
+// bytes of the pool, next included
+constexpr size_t kSegPoolBytes = 256 + (sizeof(int) * (kSegSlot + 1) + 2 * sizeof(double) * kSegSlot) * (size_t)kSegPoolSlots +
+                                 (sizeof(int) + sizeof(double2)) * (size_t)kMaxSeg * kMedPoolSlots;
+
 struct PanelArgs {
   const LayerPlan* plans;
   int layer0;
@@ -56,16 +74,8 @@ struct PanelArgs {
   const int* seg_n;
   const int* seg_start;
   const double2* seg_v;
-  // radiation-term segments of panels with more than kMaxSeg of them (low
-  // wavenumbers at coarse DV): slots of kSegSlot entries claimed by atomics
-  int* seg_next;             // next free slot
-  int seg_slots;             // slots in the pool
-  int* seg_pool_start;       // [slot][kSegSlot + 1]
-  double* seg_pool_v;        // [slot][kSegSlot]
-  double* seg_pool_d;
+  SegPool seg;
 };
-constexpr int kSegSlot = kNLIM1 + 1;  // at most one segment per point of a panel
-constexpr int kSegPoolSlots = 4096;
 
 // far-wing pseudo-line prepared for the convolution (CNVF4Q per-line set-up),
 // FP32 form of the mixed path: 80 bytes, staged in shared memory in chunks.
@@ -125,7 +135,7 @@ constexpr int kSegTab = 24;  // radiation-term segments of a panel held by k_pan
 __global__ void __launch_bounds__(64)
     k_panel_setup(const LayerPlan* plans, int layer0, const double* vft_all, int64_t stride, const int* panel_blk,
                   const double* blk_v1, const int* blk_n, const int64_t* blk_m0, int* seg_n, int* seg_start,
-                  double2* seg_v, XintPanel* xint);
+                  double2* seg_v, XintPanel* xint, SegPool pool);
 
 // the passes of k_panel: the line sums (kPanelLines), then the far wings, the
 // continuum and the radiation term (kPanelWings)

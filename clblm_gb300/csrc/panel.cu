@@ -275,12 +275,17 @@ __global__ void __launch_bounds__(32 * kRadfacWarps)
   } while (N2 < NPTR4);
 }
 
+// seg_n of a panel whose segments are in a slot: -2 and below
+__device__ __forceinline__ int seg_code(bool big, int slot) { return -2 - (2 * slot + (big ? 1 : 0)); }
+
 // What the far-wing pass needs of every panel and one thread can form, ahead of
 // it: by the CTA's first warp, a lane per panel, the radiation-term segments
 // (panelOut, JRAD = 0: RADFNI from the panel's first output point), their
-// number at seg_n[layer * stride + panel] (-1: more than kSegTab, the far-wing
-// pass forms them itself), first points, values and slopes; by its second, the
-// XINT set-up.  Both are chains of binary64 divisions and exponentials (a
+// number at seg_n[layer * stride + panel], first points, values and slopes; by
+// its second, the XINT set-up.  Past kSegTab segments they go to a slot of the
+// pool, and seg_n is the slot (seg_code) and seg_start[.. kSegTab] their
+// number; with no slot left seg_n is -1 and the far-wing pass forms them itself
+// (far infrared, 24 cm-1 panels: up to 800, 2 ms of that pass's CTA).  Both are chains of binary64 divisions and exponentials (a
 // segment takes about 3 us, the set-up 15): formed by one lane of the far-wing
 // pass's CTA, the segments of a surface panel were two thirds of its 88 us,
 // and the set-up a third of the others' 43 us.
@@ -288,7 +293,8 @@ __global__ void __launch_bounds__(64)
     k_panel_setup(const LayerPlan* __restrict__ plans, int layer0, const double* __restrict__ vft_all, int64_t stride,
                   const int* __restrict__ panel_blk, const double* __restrict__ blk_v1,
                   const int* __restrict__ blk_n, const int64_t* __restrict__ blk_m0, int* __restrict__ seg_n,
-                  int* __restrict__ seg_start, double2* __restrict__ seg_v, XintPanel* __restrict__ xint) {
+                  int* __restrict__ seg_start, double2* __restrict__ seg_v, XintPanel* __restrict__ xint,
+                  SegPool pool) {
   const LayerPlan& P = plans[blockIdx.y + layer0];
   const int p = blockIdx.x * 32 + (threadIdx.x & 31);
   if (p >= P.npanels) return;
@@ -338,7 +344,7 @@ __global__ void __launch_bounds__(64)
   const double V1P = VFT + (double)(NLO - 1) * dv;
   double VITST = V1P - dv;
   double RDLAST = -1.;
-  int N2 = NLO - 1, ns = 0;
+  int N2 = NLO - 1, ns = 0, med = -1, big = -1;
   do {
     const int N1 = N2 + 1;
     const double VI = VFT + (double)(N1 - 1) * dv;
@@ -347,14 +353,49 @@ __global__ void __launch_bounds__(64)
     N2 = (int)((VITST - VFT) / dv + 0.001);
     if (N2 > NHI) N2 = NHI;
     if (ns == kSegTab) {
-      ns = -1;
-      break;
+      med = atomicAdd(&pool.next[1], 1);
+      if (med >= kMedPoolSlots) {
+        seg_n[k] = -1;
+        return;
+      }
+      for (int q = 0; q < ns; ++q) {
+        pool.med_start[(int64_t)med * kMaxSeg + q] = seg_start[k * kSegTab + q];
+        pool.med_v[(int64_t)med * kMaxSeg + q] = seg_v[k * kSegTab + q];
+      }
     }
-    seg_start[k * kSegTab + ns] = N1;
-    seg_v[k * kSegTab + ns] = make_double2(RADVI, RDEL);
+    if (ns == kMaxSeg) {
+      big = atomicAdd(&pool.next[0], 1);
+      if (big >= pool.slots) {  // the far-wing pass reports it
+        seg_n[k] = -1;
+        return;
+      }
+      for (int q = 0; q < ns; ++q) {
+        const double2 v = pool.med_v[(int64_t)med * kMaxSeg + q];
+        pool.start[(int64_t)big * (kSegSlot + 1) + q] = pool.med_start[(int64_t)med * kMaxSeg + q];
+        pool.v[(int64_t)big * kSegSlot + q] = v.x;
+        pool.d[(int64_t)big * kSegSlot + q] = v.y;
+      }
+    }
+    if (ns >= kSegSlot) {  // cannot happen: a segment spans at least one point
+      seg_n[k] = -1;
+      return;
+    }
+    if (big >= 0) {
+      pool.start[(int64_t)big * (kSegSlot + 1) + ns] = N1;
+      pool.v[(int64_t)big * kSegSlot + ns] = RADVI;
+      pool.d[(int64_t)big * kSegSlot + ns] = RDEL;
+    } else if (med >= 0) {
+      pool.med_start[(int64_t)med * kMaxSeg + ns] = N1;
+      pool.med_v[(int64_t)med * kMaxSeg + ns] = make_double2(RADVI, RDEL);
+    } else {
+      seg_start[k * kSegTab + ns] = N1;
+      seg_v[k * kSegTab + ns] = make_double2(RADVI, RDEL);
+    }
     ns++;
   } while (N2 < NHI);
-  seg_n[k] = ns;
+  if (big >= 0) pool.start[(int64_t)big * (kSegSlot + 1) + ns] = NHI + 1;
+  if (med >= 0) seg_start[k * kSegTab] = ns;
+  seg_n[k] = big >= 0 ? seg_code(true, big) : med >= 0 ? seg_code(false, med) : ns;
 }
 
 // Record ranges of the T half tiles [G0 + 16t, G0 + 16t + 15] of one grid
@@ -848,9 +889,22 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
     if (P.jrad == 0) {
       const int64_t k = (int64_t)layer * a.panel_stride + p;
       nseg = a.seg_n[k];
-      for (int q = tid; q < nseg; q += kPanelThreads) {
-        S.seg_start[q] = a.seg_start[k * kSegTab + q];
-        const double2 v = a.seg_v[k * kSegTab + q];
+      const int* first = a.seg_start + k * kSegTab;
+      const double2* val = a.seg_v + k * kSegTab;
+      int slot = -1;
+      if (nseg <= -2) {  // in a slot of the pool (seg_code)
+        const int code = -2 - nseg, id = code >> 1;
+        nseg = first[0];
+        if (code & 1) {
+          slot = id;
+        } else {
+          first = a.seg.med_start + (int64_t)id * kMaxSeg;
+          val = a.seg.med_v + (int64_t)id * kMaxSeg;
+        }
+      }
+      for (int q = tid; q < nseg && slot < 0; q += kPanelThreads) {
+        S.seg_start[q] = first[q];
+        const double2 v = val[q];
         if constexpr (Plain) {
           S.seg_v[q] = v.x;
           S.seg_d[q] = v.y;
@@ -859,10 +913,13 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
           S.segf_d[q] = (float)v.y;
         }
       }
-      if (tid == 0 && nseg >= 0) S.seg_start[nseg] = NHI + 1;
-    }
-    if (tid == 0 && nseg >= 0) {
-      S.nseg = nseg;
+      if (tid == 0 && nseg >= 0) {
+        if (slot < 0) S.seg_start[nseg] = NHI + 1;
+        S.nseg = nseg;
+        S.seg_slot = slot;
+      }
+    } else if (tid == 0) {
+      S.nseg = 0;
       S.seg_slot = -1;
     }
   }
@@ -893,16 +950,16 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
           }
         } else {
           if (slot < 0) {  // more segments than shared memory holds: move to a pool slot
-            slot = atomicAdd(a.seg_next, 1);
-            if (slot >= a.seg_slots) {
+            slot = atomicAdd(&a.seg.next[0], 1);
+            if (slot >= a.seg.slots) {
               atomicOr(a.err, 1);
               slot = -1;
               ns = 0;
               break;
             }
-            int* gs = a.seg_pool_start + (int64_t)slot * (kSegSlot + 1);
-            double* gv = a.seg_pool_v + (int64_t)slot * kSegSlot;
-            double* gd = a.seg_pool_d + (int64_t)slot * kSegSlot;
+            int* gs = a.seg.start + (int64_t)slot * (kSegSlot + 1);
+            double* gv = a.seg.v + (int64_t)slot * kSegSlot;
+            double* gd = a.seg.d + (int64_t)slot * kSegSlot;
             for (int q = 0; q < kMaxSeg; ++q) {
               gs[q] = S.seg_start[q];
               if constexpr (Plain) {
@@ -919,18 +976,18 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
             ns = 0;
             break;
           }
-          a.seg_pool_start[(int64_t)slot * (kSegSlot + 1) + ns] = N1;
+          a.seg.start[(int64_t)slot * (kSegSlot + 1) + ns] = N1;
           if constexpr (Plain) {
-            a.seg_pool_v[(int64_t)slot * kSegSlot + ns] = RADVI;
-            a.seg_pool_d[(int64_t)slot * kSegSlot + ns] = RDEL;
+            a.seg.v[(int64_t)slot * kSegSlot + ns] = RADVI;
+            a.seg.d[(int64_t)slot * kSegSlot + ns] = RDEL;
           } else {  // the values the mixed path uses are FP32
-            a.seg_pool_v[(int64_t)slot * kSegSlot + ns] = (float)RADVI;
-            a.seg_pool_d[(int64_t)slot * kSegSlot + ns] = (float)RDEL;
+            a.seg.v[(int64_t)slot * kSegSlot + ns] = (float)RADVI;
+            a.seg.d[(int64_t)slot * kSegSlot + ns] = (float)RDEL;
           }
         }
         ns++;
       } while (N2 < NHI);
-      if (slot >= 0) a.seg_pool_start[(int64_t)slot * (kSegSlot + 1) + ns] = NHI + 1;
+      if (slot >= 0) a.seg.start[(int64_t)slot * (kSegSlot + 1) + ns] = NHI + 1;
       else S.seg_start[ns] = NHI + 1;
     }
     S.nseg = ns;
@@ -1189,7 +1246,7 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
           if (P.jrad == 0 && S.nseg > 0) {
             // segment of J: largest s with seg_start[s] <= J
             const int slot = S.seg_slot;
-            const int* ss = slot < 0 ? S.seg_start : a.seg_pool_start + (int64_t)slot * (kSegSlot + 1);
+            const int* ss = slot < 0 ? S.seg_start : a.seg.start + (int64_t)slot * (kSegSlot + 1);
             int s0 = 0, s1 = S.nseg;
             while (s1 - s0 > 1) {
               int m = (s0 + s1) >> 1;
@@ -1201,8 +1258,8 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
               if constexpr (Plain) f = S.seg_v[s0] + (double)(J - S.seg_start[s0]) * S.seg_d[s0];
               else f = fmaf((float)(J - S.seg_start[s0]), S.segf_d[s0], S.segf_v[s0]);
             } else {
-              const double gv = a.seg_pool_v[(int64_t)slot * kSegSlot + s0];
-              const double gd = a.seg_pool_d[(int64_t)slot * kSegSlot + s0];
+              const double gv = a.seg.v[(int64_t)slot * kSegSlot + s0];
+              const double gd = a.seg.d[(int64_t)slot * kSegSlot + s0];
               if constexpr (Plain) f = gv + (double)(J - ss[s0]) * gd;
               else f = fmaf((float)(J - ss[s0]), (float)gd, (float)gv);
             }

@@ -1037,6 +1037,23 @@ int tune_pick(clblm_handle* h, cudaStream_t st, int n, int def, F launch, int* s
 // 250-line records that a layer's far-wing range of at most f4stride lines meets
 int64_t f4_records(int64_t f4stride) { return f4stride / 250 + 2; }
 
+// the segment pool's arrays (allocated with the workspace, before any capture)
+SegPool seg_pool(const clblm_handle* h) {
+  const size_t start_b = sizeof(int) * (size_t)kSegPoolSlots * (kSegSlot + 1);
+  const size_t val_b = sizeof(double) * (size_t)kSegPoolSlots * kSegSlot;
+  unsigned char* b = h->segpool.as<unsigned char>();
+  SegPool s;
+  s.next = reinterpret_cast<int*>(b);
+  s.slots = kSegPoolSlots;
+  b += 256;
+  s.start = reinterpret_cast<int*>(b);
+  s.v = reinterpret_cast<double*>(b += start_b);
+  s.d = reinterpret_cast<double*>(b += val_b);
+  s.med_v = reinterpret_cast<double2*>(b += val_b);
+  s.med_start = reinterpret_cast<int*>(b + sizeof(double2) * (size_t)kMaxSeg * kMedPoolSlots);
+  return s;
+}
+
 // Runs the OD pipeline for `count` layers whose plans are already uploaded at
 // plans[first..]; OD of layer k lands at od + P.od_off (Real).
 // jac: the ODs of a Jacobian call (the mixed path keeps the order of their far-wing sums).
@@ -1069,10 +1086,12 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     k_continuum<<<dim3((kNABSRB + 8 + 63) / 64, count), 64, 0, s3>>>(dplans, first, h->cont, h->absrb.as<double>());
     k_r4_radfac<<<dim3((maxb + kRadfacWarps - 1) / kRadfacWarps, count), 32 * kRadfacWarps, 0, s3>>>(
         dplans, first, h->bv1.as<double>(), h->bn.as<int>(), h->bfac.as<double>());
+    const SegPool pool = seg_pool(h);
+    CUDA_TRY(h, cudaMemsetAsync(pool.next, 0, 2 * sizeof(int), s3));
     k_panel_setup<<<dim3((maxp + 31) / 32, count), 64, 0, s3>>>(
         dplans, first, h->vft.as<double>(), pstride, h->pblk.as<int>(), h->bv1.as<double>(), h->bn.as<int>(),
         h->bm0.as<int64_t>(), h->psegn.as<int>(), h->psegs.as<int>(), h->psegv.as<double2>(),
-        h->pxint.as<XintPanel>());
+        h->pxint.as<XintPanel>(), pool);
     CUDA_TRY(h, cudaGetLastError());
     CUDA_TRY(h, cudaEventRecord(h->join3_ev, s3));
   }
@@ -1292,18 +1311,7 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
   pa.pmax_g = h->gpm.as<int>();
   pa.smin_g = h->gsm.as<int>();
   pa.err = h->err.as<int>();
-  {
-    // (allocated with the workspace, before any capture)
-    const size_t start_b = sizeof(int) * (size_t)kSegPoolSlots * (kSegSlot + 1);
-    const size_t val_b = sizeof(double) * (size_t)kSegPoolSlots * kSegSlot;
-    unsigned char* b = h->segpool.as<unsigned char>();
-    pa.seg_next = reinterpret_cast<int*>(b);
-    pa.seg_slots = kSegPoolSlots;
-    pa.seg_pool_start = reinterpret_cast<int*>(b + 256);
-    pa.seg_pool_v = reinterpret_cast<double*>(b + 256 + start_b);
-    pa.seg_pool_d = reinterpret_cast<double*>(b + 256 + start_b + val_b);
-    CUDA_TRY(h, cudaMemsetAsync(pa.seg_next, 0, sizeof(int), st));
-  }
+  pa.seg = seg_pool(h);
   pa.xint = h->pxint.as<XintPanel>();
   pa.seg_n = h->psegn.as<int>();
   pa.seg_start = h->psegs.as<int>();
@@ -1515,8 +1523,7 @@ cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int
   WS_ENSURE(h->f4nmir.ensure(sizeof(int64_t) * nL));
   WS_ENSURE(h->f4pm.ensure(sizeof(int) * (d.fsc + 4096 * d.cnt)));
   WS_ENSURE(h->f4sm.ensure(sizeof(int) * (d.fsc + 4096 * d.cnt)));
-  WS_ENSURE(h->segpool.ensure(256 + (sizeof(int) * (kSegSlot + 1) + 2 * sizeof(double) * kSegSlot) *
-                                          (size_t)kSegPoolSlots));
+  WS_ENSURE(h->segpool.ensure(kSegPoolBytes));
   WS_ENSURE(h->bfac.ensure(sizeof(double) * (kLIMOUT4 + 2) * (blkt + 1)));
 #undef WS_ENSURE
   return e;
