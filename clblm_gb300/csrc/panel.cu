@@ -410,29 +410,6 @@ __device__ __forceinline__ long long floordiv16(long long x) { return x >> 4; } 
 __device__ __forceinline__ void tile_ranges(const int* __restrict__ pm, const int* __restrict__ sm, int64_t w0,
                                             int64_t w1, int G0, int T, int* lo, int* hi) {
   const long long g0 = G0;
-  if (w1 - w0 > 2048) {
-    // a long window (wide lines): two searches per half tile instead of a pass
-    // over it, which every slice of the panel would repeat
-    for (int t = threadIdx.x; t < T; t += blockDim.x) {
-      const long long b = g0 + 16 * t;
-      int64_t l = w0, h = w1;
-      while (l < h) {
-        const int64_t m = (l + h) >> 1;
-        if (pm[m] < b) l = m + 1;
-        else h = m;
-      }
-      lo[t] = (int)l;
-      h = w1;
-      l = w0;
-      while (l < h) {
-        const int64_t m = (l + h) >> 1;
-        if (sm[m] <= b + 15) l = m + 1;
-        else h = m;
-      }
-      hi[t] = (int)l;
-    }
-    return;
-  }
   for (int64_t i = w0 + threadIdx.x; i < w1; i += blockDim.x) {
     // lo: tiles t with prev < G0 + 16 t <= cur
     const long long cur = pm[i];
@@ -446,6 +423,34 @@ __device__ __forceinline__ void tile_ranges(const int* __restrict__ pm, const in
     ta = (prevs - g0 - 15 <= 0) ? 0 : floordiv16(prevs - g0);
     tb = (curs - g0 - 16 < 0) ? -1 : min(floordiv16(curs - g0 - 16), (long long)T - 1);
     for (long long t = ta; t <= tb; ++t) hi[t] = (int)i;
+  }
+}
+
+// The same for a panel whose windows are long (wide lines), which a pass over
+// them by every slice of the panel would go through again: two searches per
+// half tile, all grids' side by side (one grid after the other, they were 24 us
+// of a single panel's 84).  rg: the windows of R1, R2, R3.
+constexpr int64_t kLongWindow = 2048;
+__device__ __noinline__ void tile_ranges_long(const int* __restrict__ pm, const int* __restrict__ sm, int64_t stride,
+                                              const int64_t* __restrict__ rg, int G01, int G02, int G03, int nT1,
+                                              PanelTiles& S) {
+  const int T1 = 2 * nT1, T2 = 2 * kTiles2, total = T1 + T2 + 2 * kTiles3;
+  for (int q = threadIdx.x; q < 2 * total; q += blockDim.x) {
+    const bool upper = q >= total;
+    int t = upper ? q - total : q;
+    const int k = t < T1 ? 0 : (t < T1 + T2 ? 1 : 2);
+    t -= k == 0 ? 0 : (k == 1 ? T1 : T1 + T2);
+    const int* arr = (upper ? sm : pm) + k * stride;
+    // lo: the first record with pm >= G0 + 16 t; hi: the first with sm > G0 + 16 t + 15
+    const long long lim = (long long)(k == 0 ? G01 : (k == 1 ? G02 : G03)) + 16 * t + (upper ? 16 : 0);
+    int64_t l = rg[2 * k], h = rg[2 * k + 1];
+    while (l < h) {
+      const int64_t m = (l + h) >> 1;
+      if (arr[m] < lim) l = m + 1;
+      else h = m;
+    }
+    int* out = k == 0 ? (upper ? S.hi1 : S.lo1) : (k == 1 ? (upper ? S.hi2 : S.lo2) : (upper ? S.hi3 : S.lo3));
+    out[t] = (int)l;
   }
 }
 
@@ -862,9 +867,14 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
     for (int i = tid; i < S.X.nab; i += blockDim.x) S.absf[i] = (float)AB[S.X.ab0 + i];
   }
   if (kLines) {
-    if (nT1 > 0) tile_ranges(pm1, sm1, rg[0], rg[1], G01, 2 * nT1, S.lo1, S.hi1);
-    tile_ranges(pm1 + a.stride, sm1 + a.stride, rg[2], rg[3], G02, 2 * kTiles2, S.lo2, S.hi2);
-    tile_ranges(pm1 + 2 * a.stride, sm1 + 2 * a.stride, rg[4], rg[5], G03, 2 * kTiles3, S.lo3, S.hi3);
+    // (the windows of the three grids hold nearly the same records)
+    if (max(rg[1] - rg[0], max(rg[3] - rg[2], rg[5] - rg[4])) > kLongWindow) {
+      tile_ranges_long(pm1, sm1, a.stride, rg, G01, G02, G03, max(nT1, 0), S);
+    } else {
+      if (nT1 > 0) tile_ranges(pm1, sm1, rg[0], rg[1], G01, 2 * nT1, S.lo1, S.hi1);
+      tile_ranges(pm1 + a.stride, sm1 + a.stride, rg[2], rg[3], G02, 2 * kTiles2, S.lo2, S.hi2);
+      tile_ranges(pm1 + 2 * a.stride, sm1 + 2 * a.stride, rg[4], rg[5], G03, 2 * kTiles3, S.lo3, S.hi3);
+    }
   }
   __syncthreads();
   if constexpr (!Plain && kLines) {  // the tables have landed (bounded wait; the error flag otherwise)
