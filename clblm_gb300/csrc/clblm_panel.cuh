@@ -140,6 +140,7 @@ __global__ void __launch_bounds__(64)
 // the passes of k_panel: the line sums (kPanelLines), then the far wings, the
 // continuum and the radiation term (kPanelWings)
 constexpr int kPanelLines = 1, kPanelWings = 2;
+constexpr int kWingParts = 5;  // CTAs per panel of a far-wing pass over few panels
 // Cpl: the line list holds coupled lines, whose grid records carry kCplBit
 // (the branch-free sums of the mixed path skip them; they are added with
 // their dispersion term); without it the line sums stay as lean as before

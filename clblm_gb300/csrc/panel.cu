@@ -834,13 +834,16 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
   // the far-wing pass adds to the OD the line pass wrote: its loads are
   // issued here, ahead of the R3 and R2 phases
   constexpr int kT1PerWarp = (kTiles1 + kPanelWarps - 1) / kPanelWarps;
+  // (few panels: kWingParts CTAs each, which share out the R1 tiles)
+  static_assert(kT1PerWarp % kWingParts == 0, "as many tiles a warp in every part");
+  auto mine = [&](int i) { return gridDim.z == 1 || i % kWingParts == (int)blockIdx.z; };
   Real od_pre[Part == kPanelWings ? kT1PerWarp : 1];
   if constexpr (Part == kPanelWings) {
     const Real* od = reinterpret_cast<const Real*>(a.od_all) + P.od_off + (int64_t)kPanelPts * p;
 #pragma unroll
     for (int i = 0; i < kT1PerWarp; ++i) {
       const int J = kNSHIFT + 1 + (warp + i * kPanelWarps) * 32 + lane;
-      od_pre[i] = (warp + i * kPanelWarps < nT1 && J <= NHI) ? od[J - kNSHIFT - 1] : (Real)0;
+      od_pre[i] = (mine(i) && warp + i * kPanelWarps < nT1 && J <= NHI) ? od[J - kNSHIFT - 1] : (Real)0;
     }
   }
   // a slice's share of the records [lo, hi) of a tile
@@ -1290,7 +1293,7 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
     if constexpr (Part == kPanelWings) {
 #pragma unroll
       for (int i = 0; i < kT1PerWarp; ++i)
-        if (warp + i * kPanelWarps < nT1) r1_tile(warp + i * kPanelWarps, od_pre[i]);
+        if (mine(i) && warp + i * kPanelWarps < nT1) r1_tile(warp + i * kPanelWarps, od_pre[i]);
     } else {
       for (int tile = warp; tile < nT1; tile += kPanelWarps) r1_tile(tile, (Real)0);
     }

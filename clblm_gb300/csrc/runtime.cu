@@ -1350,8 +1350,12 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
   CUDA_TRY(h, cudaStreamWaitEvent(st, h->join3_ev, 0));  // ABSRB and the radiation terms
   CUDA_TRY(h, cudaEventRecord(h->ev[8], st));
   // without the shape tables: six CTAs of the mixed far-wing pass share an SM
-  if (plain) k_panel<true, kPanelWings, false><<<dim3(maxp, count), kPanelThreads, smem_w, st>>>(pa);
-  else k_panel<false, kPanelWings, false><<<dim3(maxp, count), kPanelThreads, smem_w, st>>>(pa);
+  // a panel's CTA goes through ten R1 tiles a warp (28 us for the panel of a
+  // channel-wide layer): while all fit at once, parts of it side by side, which
+  // form R3 and R2 each
+  const unsigned parts = (int64_t)maxp * count * kWingParts <= 2 * (int64_t)h->nsm ? kWingParts : 1;
+  if (plain) k_panel<true, kPanelWings, false><<<dim3(maxp, count, parts), kPanelThreads, smem_w, st>>>(pa);
+  else k_panel<false, kPanelWings, false><<<dim3(maxp, count, parts), kPanelThreads, smem_w, st>>>(pa);
   CUDA_TRY(h, cudaEventRecord(h->ev[9], st));
   // RSYM: the first panel of a layer whose panel origin is at or below 0 cm-1
   bool fold = false;
