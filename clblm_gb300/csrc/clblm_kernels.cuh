@@ -100,18 +100,17 @@ template <bool Cpl>
 __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
     k_line_prep(const LayerPlan* __restrict__ plans, int layer0, LineIn lines, const IsoRow* __restrict__ iso_tab,
                 const double* __restrict__ vft_all, LinePrep* __restrict__ out, int64_t out_stride,
-                unsigned long long* __restrict__ stats);
-__global__ void k_scan_blockmax(const LinePrep* prep, int64_t stride, const int64_t* nlines, int* blockmax,
+                int* __restrict__ fpanel, unsigned long long* __restrict__ stats);
+__global__ void k_scan_blockmax(const int* fpanel, int64_t stride, const int64_t* nlines, int* blockmax,
                                 int nblk_stride);
 constexpr int kScanBlock = 1024, kScanThreads = 256;  // lines and threads of a CTA of the scans over a layer's lines
 __global__ void __launch_bounds__(kScanThreads)
-    k_scan_apply(const LinePrep* prep, int64_t stride, const int64_t* nlines, const int* blockmax, int nblk_stride,
-                 int* qpanel);
+    k_scan_apply(int* qpanel, int64_t stride, const int64_t* nlines, const int* blockmax, int nblk_stride);
 __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
     k_line_records(const LayerPlan* plans, int layer0, const double* vft_all, const LinePrep* prep,
                                const int* qpanel, int64_t stride, GridRec* rec, GridRecD* recd,
                                GridRecLo* reclo, double* cpl, unsigned long long* stats,
-                               double* alfvmax, int* aggmax, int* aggmin, int nagg);
+                               double* alfvmax, int* aggmax, int* aggmin, int nagg, int* pmax, int* smin);
 __global__ void k_panel_ranges(const LayerPlan* plans, int layer0, const double* vnu_raw, const double* alfvmax,
                                double shiftmax, int64_t* ranges, int64_t panel_stride, int2* work);
 __global__ void k_continuum(const LayerPlan* plans, int layer0, ContIn cont, double* absrb_all);
@@ -119,12 +118,13 @@ template <bool Cpl>
 __global__ void __launch_bounds__(kSetupThreads, 4)
     k_f4_prep(const LayerPlan* __restrict__ plans, int layer0, LineIn lines,
                           const IsoRow* __restrict__ iso_tab, F4Prep* __restrict__ out, int64_t stride,
-                          unsigned long long* __restrict__ stats);
-__global__ void k_f4_count(const F4Prep* prep, int64_t stride, const LayerPlan* plans, int layer0, int64_t* blocksum,
-                           int nblk, int64_t* cut);
+                          unsigned* __restrict__ mask, int64_t mstride, unsigned long long* __restrict__ stats);
 __global__ void __launch_bounds__(kScanThreads)
-    k_f4_compact(const F4Prep* prep, int64_t stride, const LayerPlan* plans, int layer0, const int64_t* blocksum,
-                 int nblk, int64_t* cidx, long long* vbits, long long* lbits, int64_t* src, unsigned char* flags,
+    k_f4_count(const unsigned* mask, int64_t mstride, const LayerPlan* plans, int layer0, int64_t* blocksum, int nblk,
+               int64_t* cut);
+__global__ void __launch_bounds__(kScanThreads)
+    k_f4_compact(const F4Prep* prep, const unsigned* mask, int64_t mstride, int64_t stride, const LayerPlan* plans,
+                 int layer0, const int64_t* blocksum, int nblk, int64_t* cidx, long long* vbits, long long* lbits, int64_t* src, unsigned char* flags,
                  int64_t* cut, int64_t* ntot);
 __global__ void k_f4_next(const long long* vbits, const long long* lbits, const int64_t* ntot, int64_t stride,
                           int* gnxt);
@@ -170,8 +170,9 @@ __global__ void k_layer_amounts(int nlev, int nmol, const double* z, const doubl
 constexpr int kRecBlock = 256;
 constexpr int kRecNone = 0x7fffffff;
 __global__ void k_rec_carry(const LayerPlan* plans, int layer0, int* aggmax, int* aggmin, int nagg);
-__global__ void k_rec_bounds(const LayerPlan* plans, int layer0, const GridRec* rec, int64_t stride,
-                             const int* aggmax, const int* aggmin, int nagg, int* pmax, int* smin);
+__global__ void __launch_bounds__(kRecBlock)
+    k_rec_bounds(const LayerPlan* plans, int layer0, int64_t stride, const int* aggmax, const int* aggmin, int nagg,
+                 int* pmax, int* smin);
 // running bounds of the far-wing records, in blocks of kF4Blk records
 constexpr int kF4Blk = 1024, kF4BlkThreads = 256;
 template <int Kind>

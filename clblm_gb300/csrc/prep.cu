@@ -140,7 +140,8 @@ template <bool Cpl>
 __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
     k_line_prep(const LayerPlan* __restrict__ plans, int layer0, LineIn lines,
                             const IsoRow* __restrict__ iso_tab, const double* __restrict__ vft_all,
-                            LinePrep* __restrict__ out, int64_t out_stride, unsigned long long* __restrict__ stats) {
+                            LinePrep* __restrict__ out, int64_t out_stride, int* __restrict__ fpanel,
+                            unsigned long long* __restrict__ stats) {
   const LayerPlan& P = plans[blockIdx.y + layer0];
   int64_t n = P.line_hi - P.line_lo + 1;
   LinePrep* o = out + (int64_t)blockIdx.y * out_stride;
@@ -286,6 +287,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
       }
     }
     o[t] = r;
+    fpanel[(int64_t)blockIdx.y * out_stride + t] = r.fpanel;  // for the scan over lines, by itself
   }
   // block reduction of the counters
   __shared__ unsigned long long sh[5][32];
@@ -306,14 +308,14 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
 }
 template __global__ void k_line_prep<false>(const LayerPlan* __restrict__, int, LineIn, const IsoRow* __restrict__,
                                            const double* __restrict__, LinePrep* __restrict__, int64_t,
-                                           unsigned long long* __restrict__);
+                                           int* __restrict__, unsigned long long* __restrict__);
 template __global__ void k_line_prep<true>(const LayerPlan* __restrict__, int, LineIn, const IsoRow* __restrict__,
                                           const double* __restrict__, LinePrep* __restrict__, int64_t,
-                                          unsigned long long* __restrict__);
+                                          int* __restrict__, unsigned long long* __restrict__);
 
 // ---- prefix maximum of fpanel over a layer's line range -------------------
 
-__global__ void k_scan_blockmax(const LinePrep* __restrict__ prep, int64_t stride, const int64_t* __restrict__ nlines,
+__global__ void k_scan_blockmax(const int* __restrict__ fpanel, int64_t stride, const int64_t* __restrict__ nlines,
                                 int* __restrict__ blockmax, int nblk_stride) {
   int layer = blockIdx.y;
   int64_t n = nlines[layer];
@@ -321,7 +323,7 @@ __global__ void k_scan_blockmax(const LinePrep* __restrict__ prep, int64_t strid
   int mx = -1;
   for (int k = threadIdx.x; k < kScanBlock; k += blockDim.x) {
     int64_t i = base + k;
-    if (i < n) mx = max(mx, prep[layer * stride + i].fpanel);
+    if (i < n) mx = max(mx, fpanel[layer * stride + i]);
   }
   for (int off = 16; off > 0; off >>= 1) mx = max(mx, __shfl_down_sync(0xffffffffu, mx, off));
   __shared__ int sh[32];
@@ -335,14 +337,14 @@ __global__ void k_scan_blockmax(const LinePrep* __restrict__ prep, int64_t strid
 }
 
 // panel of each line = max(largest of the blocks before, inclusive in-block
-// prefix).  A CTA takes the maximum of the blocks before its own itself (a few
+// prefix), in place of its own first panel.  A CTA takes the maximum of the blocks before its own itself (a few
 // hundred words from L2; a kernel of its own for their prefix was 12 us of a
 // layer's chain), and scans by warps of 4 times 32 lines (32 lanes with 32
 // consecutive lines each met in one bank of shared memory: 0.33 -> 0.28 ms for 30
 // million lines, 1.87 -> 0.97 ms for 120 million).
 __global__ void __launch_bounds__(kScanThreads)
-    k_scan_apply(const LinePrep* __restrict__ prep, int64_t stride, const int64_t* __restrict__ nlines,
-                 const int* __restrict__ blockmax, int nblk_stride, int* __restrict__ qpanel) {
+    k_scan_apply(int* qpanel, int64_t stride, const int64_t* __restrict__ nlines, const int* __restrict__ blockmax,
+                 int nblk_stride) {
   constexpr int kWarps = kScanThreads / 32, kRows = kScanBlock / kScanThreads;
   __shared__ int before[kWarps], total[kWarps];
   const int layer = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(kScanThreads)
 #pragma unroll
   for (int j = 0; j < kRows; ++j) {
     const int64_t i = base + 32 * j + lane;
-    v[j] = i < n ? prep[layer * stride + i].fpanel : -1;
+    v[j] = i < n ? qpanel[layer * stride + i] : -1;
   }
   pre = __reduce_max_sync(0xffffffffu, pre);
 #pragma unroll
@@ -395,7 +397,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
                                GridRecLo* __restrict__ reclo, double* __restrict__ cpl,
                                unsigned long long* __restrict__ stats,
                                double* __restrict__ alfvmax, int* __restrict__ aggmax, int* __restrict__ aggmin,
-                               int nagg) {
+                               int nagg, int* __restrict__ pmax, int* __restrict__ smin) {
   int layer = blockIdx.y;
   const LayerPlan& P = plans[layer + layer0];
   int64_t n = P.line_hi - P.line_lo + 1;
@@ -517,32 +519,47 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks)
       reclo[o + stride + t] = l2;
       reclo[o + 2 * stride + t] = l3;
     }
+    // running bounds within the block, and its own: the largest g_hi up to each
+    // record, the least g_lo from it on (empty records do not bound)
     {
-      const GridRec* gg[3] = {&g1, &g2, &g3};
       const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-      for (int k = 0; k < 3; ++k) {
-        const bool ne = gg[k]->g_hi >= gg[k]->g_lo;  // empty records do not bound
-        int mx = ne ? gg[k]->g_hi : -1, mn = ne ? gg[k]->g_lo : kRecNone;
-        for (int off = 16; off > 0; off >>= 1) {
-          mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-          mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, off));
+      constexpr int kWarps = kRecBlock / 32;
+      int x[3], y[3];
+      auto scan = [&](int k, const GridRec& g) {
+        const bool ne = g.g_hi >= g.g_lo;
+        x[k] = ne ? g.g_hi : -1;
+        y[k] = ne ? g.g_lo : kRecNone;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, x[k], d);
+          const int v = __shfl_down_sync(0xffffffffu, y[k], d);
+          if (lane >= d) x[k] = max(x[k], u);
+          if (lane + d < 32) y[k] = min(y[k], v);
         }
-        if (lane == 0) {
-          red[k][0][warp] = mx;
-          red[k][1][warp] = mn;
-        }
-      }
+        if (lane == 31) red[k][0][warp] = x[k];
+        if (lane == 0) red[k][1][warp] = y[k];
+      };
+      scan(0, g1);
+      scan(1, g2);
+      scan(2, g3);
       __syncthreads();
-      if (threadIdx.x < 3) {
-        const int k = threadIdx.x;
-        int mx = -1, mn = kRecNone;
-        for (int w = 0; w < kRecBlock / 32; ++w) {
-          mx = max(mx, red[k][0][w]);
-          mn = min(mn, red[k][1][w]);
+      const int64_t o = (int64_t)layer * stride * 3 + t;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        int cm = -1, cn = kRecNone;
+        for (int w = 0; w < kWarps; ++w) {
+          if (w < warp) cm = max(cm, red[k][0][w]);
+          if (w > warp) cn = min(cn, red[k][1][w]);
+        }
+        cm = max(cm, x[k]);
+        cn = min(cn, y[k]);
+        if (live) {
+          pmax[o + k * stride] = cm;
+          smin[o + k * stride] = cn;
         }
         const int64_t a = ((int64_t)layer * 3 + k) * nagg + base / kRecBlock;
-        aggmax[a] = mx;
-        aggmin[a] = mn;
+        if (threadIdx.x == kRecBlock - 1) aggmax[a] = cm;
+        if (threadIdx.x == 0) aggmin[a] = cn;
       }
       __syncthreads();
     }
@@ -1207,7 +1224,7 @@ template <bool Cpl>
 __global__ void __launch_bounds__(kSetupThreads, 4)
     k_f4_prep(const LayerPlan* __restrict__ plans, int layer0, LineIn lines,
                           const IsoRow* __restrict__ iso_tab, F4Prep* __restrict__ out, int64_t stride,
-                          unsigned long long* __restrict__ stats) {
+                          unsigned* __restrict__ mask, int64_t mstride, unsigned long long* __restrict__ stats) {
   const LayerPlan& P = plans[blockIdx.y + layer0];
   int64_t n = P.f4_hi - P.f4_lo;
   F4Prep* o = out + (int64_t)blockIdx.y * stride;
@@ -1298,14 +1315,22 @@ __global__ void __launch_bounds__(kSetupThreads, 4)
       }
     }
     o[t] = r;
+    // a bit per line that passes, for the compaction (the flag itself is four
+    // bytes of every 48)
+    const int lane = threadIdx.x & 31;
+    const int64_t left = n - (t - lane);
+    const unsigned pass = __ballot_sync(left >= 32 ? 0xffffffffu : (1u << left) - 1u, r.pass != 0);
+    if (lane == 0) mask[(int64_t)blockIdx.y * mstride + (t >> 5)] = pass;
   }
   for (int off = 16; off > 0; off >>= 1) bad += __shfl_down_sync(0xffffffffu, bad, off);
   if ((threadIdx.x & 31) == 0 && bad) atomicAdd(&stats[(blockIdx.y + layer0) * kStatsPerLayer + 4], bad);
 }
 template __global__ void k_f4_prep<false>(const LayerPlan* __restrict__, int, LineIn, const IsoRow* __restrict__,
-                                         F4Prep* __restrict__, int64_t, unsigned long long* __restrict__);
+                                         F4Prep* __restrict__, int64_t, unsigned* __restrict__, int64_t,
+                                          unsigned long long* __restrict__);
 template __global__ void k_f4_prep<true>(const LayerPlan* __restrict__, int, LineIn, const IsoRow* __restrict__,
-                                        F4Prep* __restrict__, int64_t, unsigned long long* __restrict__);
+                                        F4Prep* __restrict__, int64_t, unsigned* __restrict__, int64_t,
+                                          unsigned long long* __restrict__);
 
 // ---- LINF4Q record loop with SHRINQ, in parallel pieces -------------------
 // The reference appends the corrected lines of each 250-line record to a
@@ -1350,27 +1375,20 @@ __device__ __forceinline__ bool weak_sp(double sp) {
 }
 __device__ __forceinline__ bool nonzero_d(double x) { return (__double_as_longlong(x) << 1) != 0; }
 
-__global__ void k_f4_count(const F4Prep* __restrict__ prep, int64_t stride, const LayerPlan* __restrict__ plans,
-                           int layer0, int64_t* __restrict__ blocksum, int nblk, int64_t* __restrict__ cut) {
-  const int layer = blockIdx.y;
+// passing lines of every block of 1024: a warp per block, a word of 32 per lane
+__global__ void __launch_bounds__(kScanThreads)
+    k_f4_count(const unsigned* __restrict__ mask, int64_t mstride, const LayerPlan* __restrict__ plans, int layer0,
+               int64_t* __restrict__ blocksum, int nblk, int64_t* __restrict__ cut) {
+  static_assert(kScanBlock == 1024, "a word of 32 lines per lane");
+  const int layer = blockIdx.y, lane = threadIdx.x & 31;
   if (blockIdx.x == 0 && threadIdx.x == 0) cut[layer] = -1;  // k_f4_compact's minimum
   const LayerPlan& P = plans[layer + layer0];
-  const int64_t n = P.f4_hi - P.f4_lo;
-  const int64_t base = (int64_t)blockIdx.x * 1024;
-  int c = 0;
-  for (int k = threadIdx.x; k < 1024; k += blockDim.x) {
-    int64_t t = base + k;
-    if (t < n) c += prep[(int64_t)layer * stride + t].pass;
-  }
-  for (int off = 16; off > 0; off >>= 1) c += __shfl_down_sync(0xffffffffu, c, off);
-  __shared__ int sh[32];
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int64_t tot = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += sh[w];
-    blocksum[(int64_t)layer * nblk + blockIdx.x] = tot;
-  }
+  const int64_t words = (P.f4_hi - P.f4_lo + 31) / 32;
+  const int blk = blockIdx.x * (kScanThreads / 32) + (threadIdx.x >> 5);
+  if (blk >= nblk) return;
+  const int64_t w = (int64_t)blk * 32 + lane;
+  const int c = __reduce_add_sync(0xffffffffu, w < words ? __popc(mask[(int64_t)layer * mstride + w]) : 0);
+  if (lane == 0) blocksum[(int64_t)layer * nblk + blk] = c;
 }
 
 // cidx[t] = passing lines before t (t = 0..n, cidx[n] = total); the passing
@@ -1378,8 +1396,8 @@ __global__ void k_f4_count(const F4Prep* __restrict__ prep, int64_t stride, cons
 // A CTA adds up the blocks before its own (a kernel of its own for their prefix
 // was 19 us of a layer's chain); the warps count with ballots.
 __global__ void __launch_bounds__(kScanThreads)
-    k_f4_compact(const F4Prep* __restrict__ prep, int64_t stride, const LayerPlan* __restrict__ plans, int layer0,
-                 const int64_t* __restrict__ blocksum, int nblk, int64_t* __restrict__ cidx,
+    k_f4_compact(const F4Prep* __restrict__ prep, const unsigned* __restrict__ mask, int64_t mstride, int64_t stride,
+                 const LayerPlan* __restrict__ plans, int layer0, const int64_t* __restrict__ blocksum, int nblk, int64_t* __restrict__ cidx,
                  long long* __restrict__ vbits, long long* __restrict__ lbits, int64_t* __restrict__ src,
                  unsigned char* __restrict__ flags, int64_t* __restrict__ cut, int64_t* __restrict__ ntot) {
   constexpr int kWarps = kScanThreads / 32, kRows = kScanBlock / kScanThreads;
@@ -1396,8 +1414,8 @@ __global__ void __launch_bounds__(kScanThreads)
   int count = 0;
 #pragma unroll
   for (int j = 0; j < kRows; ++j) {
-    const int64_t t = base + 32 * j + lane;
-    in[j] = __ballot_sync(0xffffffffu, t < n && prep[(int64_t)layer * stride + t].pass != 0);
+    const int64_t t = base + 32 * j;
+    in[j] = t < n ? mask[(int64_t)layer * mstride + (t >> 5)] : 0u;
     count += __popc(in[j]);
   }
 #pragma unroll
@@ -2666,47 +2684,55 @@ __global__ void k_rec_carry(const LayerPlan* __restrict__ plans, int layer0, int
   }
 }
 
+// A warp per block and grid: the bounds of the blocks before (after) raise
+// (lower) the first (last) few of a block's own, which are monotone. (Formed
+// from the records again, 32 bytes each for two of their words, they were 0.70
+// ms for 30 million lines.)
 __global__ void __launch_bounds__(kRecBlock)
-    k_rec_bounds(const LayerPlan* __restrict__ plans, int layer0, const GridRec* __restrict__ rec, int64_t stride,
-                 const int* __restrict__ aggmax, const int* __restrict__ aggmin, int nagg, int* __restrict__ pmax,
-                 int* __restrict__ smin) {
-  const int layer = blockIdx.y / 3;
+    k_rec_bounds(const LayerPlan* __restrict__ plans, int layer0, int64_t stride, const int* __restrict__ aggmax,
+                 const int* __restrict__ aggmin, int nagg, int* __restrict__ pmax, int* __restrict__ smin) {
+  const int layer = blockIdx.y / 3, lane = threadIdx.x & 31;
   const LayerPlan& P = plans[layer + layer0];
   const int64_t n = P.line_hi - P.line_lo + 1;
-  const int64_t base = (int64_t)blockIdx.x * kRecBlock;
+  const int64_t blk = (int64_t)blockIdx.x * (kRecBlock / 32) + (threadIdx.x >> 5), base = blk * kRecBlock;
   if (base >= n) return;
-  const int64_t o = (int64_t)blockIdx.y * stride;
-  const int64_t i = base + threadIdx.x;
-  const bool live = i < n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __shared__ int wmax[kRecBlock / 32], wmin[kRecBlock / 32];
-  int hi = -1, lo = kRecNone;
-  if (live) {
-    const GridRec r = rec[o + i];
-    if (r.g_hi >= r.g_lo) {
-      hi = r.g_hi;
-      lo = r.g_lo;
+  const int64_t end = base + kRecBlock < n ? base + kRecBlock : n;
+  int* pm = pmax + (int64_t)blockIdx.y * stride;
+  int* sm = smin + (int64_t)blockIdx.y * stride;
+  const int cm = aggmax[(int64_t)blockIdx.y * nagg + blk], cn = aggmin[(int64_t)blockIdx.y * nagg + blk];
+  // (64 records at first, nearly always enough; the others' loads all at once)
+  constexpr int kRows = kRecBlock / 32;
+  int v[kRows];
+  auto raise = [&](int j0, int j1) {
+    bool all = true;
+#pragma unroll
+    for (int j = j0; j < j1; ++j) {
+      const int64_t i = base + 32 * j + lane;
+      v[j] = i < end ? pm[i] : cm;
     }
-  }
-  // inclusive prefix max within the warp, inclusive suffix min within the warp
-  int x = hi, y = lo;
-  for (int d = 1; d < 32; d <<= 1) {
-    const int a = __shfl_up_sync(0xffffffffu, x, d);
-    const int b = __shfl_down_sync(0xffffffffu, y, d);
-    if (lane >= d) x = max(x, a);
-    if (lane + d < 32) y = min(y, b);
-  }
-  if (lane == 31) wmax[warp] = x;
-  if (lane == 0) wmin[warp] = y;
-  __syncthreads();
-  int cm = aggmax[(int64_t)blockIdx.y * nagg + blockIdx.x];
-  for (int w = 0; w < warp; ++w) cm = max(cm, wmax[w]);
-  int cn = aggmin[(int64_t)blockIdx.y * nagg + blockIdx.x];
-  for (int w = warp + 1; w < kRecBlock / 32; ++w) cn = min(cn, wmin[w]);
-  if (live) {
-    pmax[o + i] = max(cm, x);
-    smin[o + i] = min(cn, y);
-  }
+#pragma unroll
+    for (int j = j0; j < j1; ++j) {
+      if (v[j] < cm) pm[base + 32 * j + lane] = cm;
+      else all = false;
+    }
+    return __all_sync(0xffffffffu, all) != 0;
+  };
+  auto lower = [&](int j0, int j1) {
+    bool all = true;
+#pragma unroll
+    for (int j = j0; j < j1; ++j) {
+      const int64_t i = end - 1 - lane - 32 * j;
+      v[j] = i >= base ? sm[i] : cn;
+    }
+#pragma unroll
+    for (int j = j0; j < j1; ++j) {
+      if (v[j] > cn) sm[end - 1 - lane - 32 * j] = cn;
+      else all = false;
+    }
+    return __all_sync(0xffffffffu, all) != 0;
+  };
+  if (raise(0, 2)) raise(2, kRows);
+  if (lower(0, 2)) lower(2, kRows);
 }
 
 }  // namespace clblm

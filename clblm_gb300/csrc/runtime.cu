@@ -158,7 +158,7 @@ struct clblm_handle {
   DevBuf reclo;     // low parts of the records' ZFL/ZSLOPE
   DevBuf jprof, jod, jmap, jjobs, jblk;  // Jacobians: profiles, block ODs, maps, jobs, grid blocks
   DevBuf jvjp;                          // vector-Jacobian product: CTA partial sums and the totals
-  DevBuf f4blk, f4ntot, f4cidx, f4vb, f4lb, f4src, f4flag, f4cut, f4grp, f4nxt, ragg;
+  DevBuf f4mask, f4blk, f4ntot, f4cidx, f4vb, f4lb, f4src, f4flag, f4cut, f4grp, f4nxt, ragg;
   DevBuf f4agg;                    // bounds of the far-wing records, per kF4Blk records
   DevBuf f4tab, f4calls, f4ncall;  // SHRINQ calls: counts of the possible ones, the list, its length
   DevBuf segpool;  // radiation-term segments of panels with more than kMaxSeg
@@ -175,7 +175,7 @@ struct clblm_handle {
   std::vector<DevBuf*> buffers() {
     std::vector<DevBuf*> v = {&cont_self, &cont_for, &cont_texp, &cont_co2, &tabs,    &prep,    &qpanel,
                               &rec,       &recd,     &ranges,    &od,      &r4,      &absrb,  &blockmax,  &f4prep,    &f4sh,    &f4rec,  &f4recd,  &f4nrec,
-                              &f4nmir,    &f4pm,     &f4sm,      &outbuf,  &bfac,     &f4blk,     &f4ntot,  &f4cidx,  &f4vb,   &f4lb,    &f4src,
+                              &f4nmir,    &f4pm,     &f4sm,      &outbuf,  &bfac,     &f4mask,    &f4blk,     &f4ntot,  &f4cidx,  &f4vb,   &f4lb,    &f4src,
                               &f4flag,    &f4cut,    &f4grp,     &f4nxt,   &ragg,    &segpool, &gpm,    &gsm,
                               &reclo,     &jprof,    &jod,       &jmap,    &jjobs,   &jblk,    &jvjp,   &linecpl,   &f4cpl,    &f4cpll,    &f4ncpl,   &pwork,
                               &f4tab,     &f4calls,  &f4ncall,  &f4agg,     &psegn,
@@ -1037,6 +1037,9 @@ int tune_pick(clblm_handle* h, cudaStream_t st, int n, int def, F launch, int* s
 // 250-line records that a layer's far-wing range of at most f4stride lines meets
 int64_t f4_records(int64_t f4stride) { return f4stride / 250 + 2; }
 
+// words of a layer's mask of passing far-wing lines
+int64_t f4_mask_words(int64_t f4stride) { return f4stride / 32 + 1; }
+
 // the segment pool's arrays (allocated with the workspace, before any capture)
 SegPool seg_pool(const clblm_handle* h) {
   const size_t start_b = sizeof(int) * (size_t)kSegPoolSlots * (kSegSlot + 1);
@@ -1096,26 +1099,28 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     CUDA_TRY(h, cudaEventRecord(h->join3_ev, s3));
   }
   // far wings
+  unsigned* mask = h->f4mask.as<unsigned>();
+  const int64_t mstride = f4_mask_words(f4stride);
   h->launches++;
   {
     const dim3 g4((unsigned)std::min<int64_t>((f4stride + 255) / 256, 4096), count);
     if (h->has_cpl)
       k_f4_prep<true><<<g4, blk, 0, st>>>(dplans, first, li, h->isotab.as<const IsoRow>(), h->f4prep.as<F4Prep>(),
-                                          f4stride, h->stats.as<unsigned long long>());
+                                          f4stride, mask, mstride, h->stats.as<unsigned long long>());
     else
       k_f4_prep<false><<<g4, blk, 0, st>>>(dplans, first, li, h->isotab.as<const IsoRow>(), h->f4prep.as<F4Prep>(),
-                                           f4stride, h->stats.as<unsigned long long>());
+                                           f4stride, mask, mstride, h->stats.as<unsigned long long>());
     CUDA_TRY(h, cudaGetLastError());  // the chain after it reads what it writes
   }
   {
     // LINF4Q record loop + SHRINQ: count, compact, walk, group sums
     int nblk4 = (int)((f4stride + 1 + 1023) / 1024);
     h->launches++;
-    k_f4_count<<<dim3(nblk4, count), 256, 0, st>>>(h->f4prep.as<F4Prep>(), f4stride, dplans, first,
-                                                   h->f4blk.as<int64_t>(), nblk4, h->f4cut.as<int64_t>());
+    k_f4_count<<<dim3((nblk4 + kScanThreads / 32 - 1) / (kScanThreads / 32), count), kScanThreads, 0, st>>>(
+        mask, mstride, dplans, first, h->f4blk.as<int64_t>(), nblk4, h->f4cut.as<int64_t>());
     h->launches++;
-    k_f4_compact<<<dim3(nblk4, count), kScanThreads, 0, st>>>(h->f4prep.as<F4Prep>(), f4stride, dplans, first,
-                                                     h->f4blk.as<int64_t>(), nblk4, h->f4cidx.as<int64_t>(),
+    k_f4_compact<<<dim3(nblk4, count), kScanThreads, 0, st>>>(h->f4prep.as<F4Prep>(), mask, mstride, f4stride, dplans,
+                                                     first, h->f4blk.as<int64_t>(), nblk4, h->f4cidx.as<int64_t>(),
                                                      h->f4vb.as<long long>(), h->f4lb.as<long long>(),
                                                      h->f4src.as<int64_t>(), h->f4flag.as<unsigned char>(),
                                                      h->f4cut.as<int64_t>(), h->f4ntot.as<int64_t>());
@@ -1248,33 +1253,35 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
     const dim3 gl((unsigned)std::min<int64_t>((lstride + 255) / 256, 8192), count);
     if (h->has_cpl)
       k_line_prep<true><<<gl, blk, 0, st>>>(dplans, first, li, h->isotab.as<const IsoRow>(), h->vft.as<double>(),
-                                            h->prep.as<LinePrep>(), lstride, h->stats.as<unsigned long long>());
+                                            h->prep.as<LinePrep>(), lstride, h->qpanel.as<int>(),
+                                            h->stats.as<unsigned long long>());
     else
       k_line_prep<false><<<gl, blk, 0, st>>>(dplans, first, li, h->isotab.as<const IsoRow>(), h->vft.as<double>(),
-                                             h->prep.as<LinePrep>(), lstride, h->stats.as<unsigned long long>());
+                                             h->prep.as<LinePrep>(), lstride, h->qpanel.as<int>(),
+                                             h->stats.as<unsigned long long>());
     CUDA_TRY(h, cudaGetLastError());  // the chain after it reads what it writes
   }
   int nblk = (int)((lstride + 1023) / 1024);
   h->launches++;
-  k_scan_blockmax<<<dim3(nblk, count), 256, 0, st>>>(h->prep.as<LinePrep>(), lstride, h->nlines_d.as<int64_t>() + first,
+  k_scan_blockmax<<<dim3(nblk, count), 256, 0, st>>>(h->qpanel.as<int>(), lstride, h->nlines_d.as<int64_t>() + first,
                                                       h->blockmax.as<int>(), nblk);
   h->launches++;
-  k_scan_apply<<<dim3(nblk, count), kScanThreads, 0, st>>>(h->prep.as<LinePrep>(), lstride, h->nlines_d.as<int64_t>() + first,
-                                                   h->blockmax.as<int>(), nblk, h->qpanel.as<int>());
+  k_scan_apply<<<dim3(nblk, count), kScanThreads, 0, st>>>(h->qpanel.as<int>(), lstride,
+                                                           h->nlines_d.as<int64_t>() + first, h->blockmax.as<int>(), nblk);
   const int nagg = (int)((lstride + kRecBlock - 1) / kRecBlock);
   h->launches++;
   k_line_records<<<dim3((unsigned)std::min<int64_t>(nagg, 8192), count), kRecBlock, 0, st>>>(
       dplans, first, h->vft.as<double>(), h->prep.as<LinePrep>(), h->qpanel.as<int>(), lstride, h->rec.as<GridRec>(),
       h->recd.as<GridRecD>(), h->reclo.as<GridRecLo>(), h->linecpl.as<double>(), h->stats.as<unsigned long long>(),
-      h->alfvmax.as<double>(), h->ragg.as<int>(), h->ragg.as<int>() + (int64_t)3 * count * nagg, nagg);
+      h->alfvmax.as<double>(), h->ragg.as<int>(), h->ragg.as<int>() + (int64_t)3 * count * nagg, nagg,
+      h->gpm.as<int>(), h->gsm.as<int>());
   h->launches++;
   k_rec_carry<<<3 * count, 1024, 0, st>>>(dplans, first, h->ragg.as<int>(),
                                           h->ragg.as<int>() + (int64_t)3 * count * nagg, nagg);
   h->launches++;
-  k_rec_bounds<<<dim3(nagg, 3 * count), kRecBlock, 0, st>>>(dplans, first, h->rec.as<GridRec>(), lstride,
-                                                            h->ragg.as<int>(),
-                                                            h->ragg.as<int>() + (int64_t)3 * count * nagg, nagg,
-                                                            h->gpm.as<int>(), h->gsm.as<int>());
+  k_rec_bounds<<<dim3((nagg + kRecBlock / 32 - 1) / (kRecBlock / 32), 3 * count), kRecBlock, 0, st>>>(
+      dplans, first, lstride, h->ragg.as<int>(), h->ragg.as<int>() + (int64_t)3 * count * nagg, nagg,
+      h->gpm.as<int>(), h->gsm.as<int>());
   int maxp = 0;
   int64_t ctas = 0;  // of the line pass
   for (int k = 0; k < count; ++k) {
@@ -1509,6 +1516,7 @@ cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int
   WS_ENSURE(h->f4sh.ensure(sizeof(ShrunkLine) * d.fsc));
   WS_ENSURE(h->f4blk.ensure(sizeof(int64_t) * d.nblk4c));
   WS_ENSURE(h->f4ntot.ensure(sizeof(int64_t) * d.cnt));
+  WS_ENSURE(h->f4mask.ensure(sizeof(unsigned) * (d.fsc / 32 + d.cnt)));
   WS_ENSURE(h->f4cidx.ensure(sizeof(int64_t) * (d.fsc + d.cnt)));
   WS_ENSURE(h->f4vb.ensure(sizeof(long long) * d.fsc));
   WS_ENSURE(h->f4lb.ensure(sizeof(long long) * d.fsc));
@@ -1536,7 +1544,7 @@ cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int
 // The buffers ws_alloc sizes: scratch of one batch, nothing in them outlives it.
 std::vector<DevBuf*> ws_buffers(clblm_handle* h) {
   return {&h->prep,   &h->qpanel,   &h->rec,    &h->recd,   &h->gpm,    &h->reclo,
-          &h->gsm,    &h->ragg,   &h->ranges, &h->od,       &h->r4,     &h->absrb,  &h->blockmax, &h->f4prep, &h->f4sh, &h->f4blk, &h->f4ntot, &h->f4cidx,
+          &h->gsm,    &h->ragg,   &h->ranges, &h->od,       &h->r4,     &h->absrb,  &h->blockmax, &h->f4prep, &h->f4sh, &h->f4mask, &h->f4blk, &h->f4ntot, &h->f4cidx,
           &h->f4vb,   &h->f4lb,   &h->f4src,  &h->f4flag,   &h->f4nxt,  &h->f4cut,  &h->f4grp,  &h->f4rec,
           &h->f4recd, &h->f4nrec, &h->f4nmir, &h->f4pm,     &h->f4sm,   &h->segpool, &h->bfac,   &h->linecpl, &h->f4cpl, &h->f4cpll,
           &h->f4ncpl, &h->pwork,  &h->f4tab,  &h->f4calls,  &h->f4ncall, &h->f4agg, &h->psegn,  &h->psegs,  &h->psegv, &h->pxint, &h->tabbuf};
