@@ -17,6 +17,7 @@
 #include <climits>
 
 #include "clblm_common.cuh"
+#include "clblm_fpconv.cuh"
 #include "clblm_interpmap.cuh"
 #include "clblm_kernels.cuh"
 #include "clblm_panel.cuh"
@@ -83,41 +84,55 @@ __device__ __forceinline__ double hlf_d(double od) {
   return 1. / (od)-1. / (tex - 1.);
 }
 
+// FP64 path: XKT = T / RADCN2 of a layer's top, bottom and mean temperatures
+// and their reciprocals (div_by), formed once per CTA: three divisions a point
+// otherwise, of a path that the FP64 unit bounds
+struct LayerXkt {
+  double top, bot, ave, rtop, rbot, rave;
+};
+__device__ __forceinline__ LayerXkt layer_xkt(const RtSegLayer& L) {
+  LayerXkt x;
+  x.top = L.ttop / kRADCN2;
+  x.bot = L.tbot / kRADCN2;
+  x.ave = L.tave / kRADCN2;
+  x.rtop = 1. / x.top;
+  x.rbot = 1. / x.bot;
+  x.rave = 1. / x.ave;
+  return x;
+}
+// planck_d from RADCN1 V^3, XKT and 1/XKT
+__device__ __forceinline__ double planck_x(double V, double cv3, double XKT, double r) {
+  if (XKT <= 1.e-6) return 0.;
+  return cv3 / (exp(div_by(V, XKT, r)) - 1.);
+}
+
 // Layer terms at OD-grid point j of layer L, from its OD value `od`: TxA,
-// TxB, EmUp, EmDn (layerMerge_mode2 :1640-1762 with layerEmis).
-__device__ __forceinline__ void layer_terms_d(const RtSegLayer& L, int lin_in_tau, int64_t j, double od,
-                                              double out[4]) {
+// TxB, EmUp, EmDn (layerMerge_mode2 :1640-1762 with layerEmis).  *Blev, when
+// given: the Planck function at the layer's bottom (negative: not known), and,
+// on return, at its top.
+__device__ __forceinline__ void layer_terms_d(const RtSegLayer& L, const LayerXkt& X, int lin_in_tau, int64_t j,
+                                              double od, double out[4], double* Blev = nullptr) {
   const double v = L.v1 + (double)(j - 1) * L.dv_od;
-  double odA = od * L.scal_up;
-  odA = odA * 1.0;
-  double odB = od * L.scal_dn;
-  odB = odB * 1.0;
-  double TA = exp(-odA), TB = exp(-odB);
-  double XKTA_up = L.ttop / kRADCN2, XKTA_dn = L.tbot / kRADCN2, XKT = L.tave / kRADCN2;
-  double XKTB_up = L.tbot / kRADCN2, XKTB_dn = L.ttop / kRADCN2;
+  const double cv3 = kRADCN1 * v * v * v;
+  const double odA = od * L.scal_up, odB = od * L.scal_dn;
+  const double TA = exp(-odA), TB = exp(-odB);
+  const double absA = 1 - TA, absB = 1 - TB;
   double EU, ED;
-  {  // down: Ta = Tbot, Tb = Ttop over path B
-    double abso = 1 - TB;
-    double hlf = lin_in_tau ? hlf_d(odB) : 0.;
-    if (lin_in_tau == 0) ED = abso * planck_d(v, XKT);
-    else if (lin_in_tau == 1) {
-      double bba = planck_d(v, XKTA_dn), bb = planck_d(v, XKT);
-      ED = abso * (bba + 2 * (bb - bba) * hlf);
-    } else {
-      double bba = planck_d(v, XKTA_dn), bbb = planck_d(v, XKTB_dn);
-      ED = abso * (bba + (bbb - bba) * hlf);
-    }
-  }
-  if (lin_in_tau == 0) EU = ED;
-  else {  // up: Ta = Ttop, Tb = Tbot over path A
-    double abso = 1 - TA;
-    double hlf = hlf_d(odA);
+  if (lin_in_tau == 0) {
+    EU = ED = absB * planck_x(v, cv3, X.ave, X.rave);
+  } else {
+    // down: Ta = Tbot, Tb = Ttop over path B; up: Ta = Ttop, Tb = Tbot over path A
+    const double Bb = Blev && *Blev >= 0. ? *Blev : planck_x(v, cv3, X.bot, X.rbot);
+    const double Bt = planck_x(v, cv3, X.top, X.rtop);
+    if (Blev) *Blev = Bt;
+    const double hB = hlf_d(odB), hA = hlf_d(odA);
     if (lin_in_tau == 1) {
-      double bba = planck_d(v, XKTA_up), bb = planck_d(v, XKT);
-      EU = abso * (bba + 2 * (bb - bba) * hlf);
+      const double bb = planck_x(v, cv3, X.ave, X.rave);
+      ED = absB * (Bb + 2 * (bb - Bb) * hB);
+      EU = absA * (Bt + 2 * (bb - Bt) * hA);
     } else {
-      double bba = planck_d(v, XKTA_up), bbb = planck_d(v, XKTB_up);
-      EU = abso * (bba + (bbb - bba) * hlf);
+      ED = absB * (Bb + (Bt - Bb) * hB);
+      EU = absA * (Bt + (Bb - Bt) * hA);
     }
   }
   out[0] = TA;
@@ -259,10 +274,11 @@ __device__ __forceinline__ void layer_terms_f(const RtSegLayer& L, int lin_in_ta
 // the terms at OD-grid index j of layer L, with interpSpectrum's linear
 // extension by two points past either end
 template <bool Plain, typename Real>
-__device__ __forceinline__ void layer_terms_ext(const RtSegLayer& L, int lin_in_tau, int64_t j, Real t[4]) {
+__device__ __forceinline__ void layer_terms_ext(const RtSegLayer& L, const LayerXkt* X, int lin_in_tau, int64_t j,
+                                                Real t[4]) {
   const Real* od = reinterpret_cast<const Real*>(L.od);
   auto at = [&](int64_t k, Real o[4]) {
-    if constexpr (Plain) layer_terms_d(L, lin_in_tau, k, od[k - 1], o);
+    if constexpr (Plain) layer_terms_d(L, *X, lin_in_tau, k, od[k - 1], o);
     else layer_terms_f(L, lin_in_tau, k, od[k - 1], o);
   };
   if (j >= 1 && j <= L.n_od) {
@@ -380,7 +396,12 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_segment(const __grid_const
   __shared__ RtSegLayer sl[kRtSegMaxLayers];
   for (int k = threadIdx.x; k < a.nlay * (int)(sizeof(RtSegLayer) / 8); k += blockDim.x)
     reinterpret_cast<uint64_t*>(sl)[k] = reinterpret_cast<const uint64_t*>(a.lay)[k];
+  __shared__ LayerXkt sx[Plain ? kRtSegMaxLayers : 1];
   __syncthreads();
+  if constexpr (Plain) {
+    for (int k = threadIdx.x; k < a.nlay; k += blockDim.x) sx[k] = layer_xkt(sl[k]);
+    __syncthreads();
+  }
   const int64_t I0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * kRtPts + 1;
   if (I0 > a.n_out) return;
   const int np = (int)min((int64_t)kRtPts, a.n_out - I0 + 1);
@@ -392,11 +413,11 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_segment(const __grid_const
   }
   Real nxt[kRtPts];
   if (a.nlay > 0 && sl[0].ly.kind == 0) load_pts(reinterpret_cast<const Real*>(sl[0].od), I0, np, nxt);
-  float Bprev[kRtPts];  // mixed: the Planck function at the previous layer's top
+  Real Bprev[kRtPts];  // the Planck function at the previous layer's top (negative: not known)
   float vfp[kRtPts], cv3p[kRtPts];  // mixed: wavenumber and RADCN1 v^3 of the points (the run's grid)
 #pragma unroll
   for (int p = 0; p < kRtPts; ++p) {
-    Bprev[p] = -1.f;
+    Bprev[p] = -1;
     const float fi = (float)(int)(I0 + p - 1);
     vfp[p] = fmaf(fi, a.vr1, a.vr0);
     cv3p[p] = (float)kRADCN1 * vfp[p] * vfp[p] * vfp[p];
@@ -415,23 +436,24 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_segment(const __grid_const
       Real T[4];
       if (L.ly.kind == 0) {
         if constexpr (Plain) {
-          layer_terms_d(L, a.lin_in_tau, I, cur[p], T);
+          if (!L.bot_is_prev_top) Bprev[p] = -1.;
+          layer_terms_d(L, sx[l], a.lin_in_tau, I, cur[p], T, &Bprev[p]);
         } else {
           merge_lean(cur[p], L.scal_up_f, L.scal_dn_f, L.ka, L.kt, L.kb, vfp[p], cv3p[p], a.lin_in_tau, &Bprev[p],
                      L.bot_is_prev_top != 0 && Bprev[p] >= 0.f, &R[p], &F[p]);
           continue;
         }
       } else {
-        Bprev[p] = -1.f;
+        Bprev[p] = -1;
         const Stencil<Real> st = interp_stencil<Real>(L.ly, I);
         if (st.n == 1) {
-          layer_terms_ext<Plain>(L, a.lin_in_tau, st.i[0], T);
+          layer_terms_ext<Plain>(L, Plain ? &sx[l] : nullptr, a.lin_in_tau, st.i[0], T);
         } else {
 #pragma unroll
           for (int c = 0; c < 4; ++c) T[c] = 0;
           for (int k = 0; k < 4; ++k) {
             Real t[4];
-            layer_terms_ext<Plain>(L, a.lin_in_tau, st.i[k], t);
+            layer_terms_ext<Plain>(L, Plain ? &sx[l] : nullptr, a.lin_in_tau, st.i[k], t);
 #pragma unroll
             for (int c = 0; c < 4; ++c) T[c] += st.w[k] * t[c];
           }
