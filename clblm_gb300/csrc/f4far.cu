@@ -181,7 +181,8 @@ struct FarSumF {
       if (++pend == 8) flush();
     }
   }
-  __device__ __forceinline__ double total(int lane) {
+  template <bool Tile>
+  __device__ __forceinline__ double total(int lane, double) {
     flush();
     double v[16];
 #pragma unroll
@@ -190,10 +191,12 @@ struct FarSumF {
   }
 };
 
-// the same on the FP64 path
+// the same on the FP64 path.  The pedestals, parabolas in the node's offset
+// from m0, are summed by their coefficients: a node's term is then six
+// operations of the FP64 unit, which bounds the kernel, instead of ten.
 struct FarSumD {
-  double s[16];
-  __device__ __forceinline__ FarSumD() {
+  double s[16], p0, p1, p2;
+  __device__ __forceinline__ FarSumD() : p0(0.), p1(0.), p2(0.) {
 #pragma unroll
     for (int k = 0; k < 16; ++k) s[k] = 0.;
   }
@@ -203,15 +206,26 @@ struct FarSumD {
     for (int64_t i = i0 + first; i < i1; i += step) {
       const F4RecD d = recs[i];
       const double nfb0 = d.co2 ? -2. * d.fbnd : -d.fbnd, fb2 = d.co2 ? d.fbnd * rbnd2 : 0.;
+      const double x0 = fma((double)m0, dvr4, -d.xnui), t = fb2 * x0;
+      p0 += fma(t, x0, nfb0);
+      p1 += t;
+      p2 += fb2;
 #pragma unroll
       for (int k = 0; k < 16; ++k) {
         const double x = fma((double)(m0 + far_node(true, Tile, k)), dvr4, -d.xnui);
-        const double xx = x * x;
-        s[k] += fma(d.sil, rcp_d(d.al2 + xx), fma(xx, fb2, nfb0));
+        s[k] = fma(d.sil, rcp_d(fma(x, x, d.al2)), s[k]);
       }
     }
   }
-  __device__ __forceinline__ double total(int lane) { return lane_totals(s, lane); }
+  template <bool Tile>
+  __device__ __forceinline__ double total(int lane, double dvr4) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const double h = (double)far_node(true, Tile, k) * dvr4;
+      s[k] += fma(h, fma(h, p2, 2. * p1), p0);
+    }
+    return lane_totals(s, lane);
+  }
 };
 
 // a warp's 32 records in shared memory, mixed path: pairs of records, each
@@ -429,7 +443,7 @@ __global__ void __launch_bounds__(kFarThreads, Plain ? 4 : 6) k_f4_far(const __g
         s.template add<true>(recs, N2, E2, first, step, T0, dvr4p);
       }
     }
-    const double v = s.total(lane);
+    const double v = s.template total<true>(lane, P.dvr4);
     if (!(lane & 1)) nodeB[warp][lane >> 1] = v;
   }
   // no far range of the tile on a side: the leaf's far range is one
@@ -452,7 +466,7 @@ __global__ void __launch_bounds__(kFarThreads, Plain ? 4 : 6) k_f4_far(const __g
         range(E2, e2);
       }
     }
-    const double v = s.total(lane);
+    const double v = s.template total<false>(lane, P.dvr4);
     if (!(lane & 1)) nodeA[warp][lane >> 1] = v;
   }
   // the leaf's points
