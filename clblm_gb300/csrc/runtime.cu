@@ -207,7 +207,7 @@ struct clblm_handle {
   // the far-wing chain runs on a second stream, forked from and joined back
   // into `stream` within each OD batch
   cudaStream_t stream2 = nullptr, stream3 = nullptr;  // (3: the continuum and the radiation terms)
-  cudaEvent_t fork_ev = nullptr, join_ev = nullptr, join3_ev = nullptr;
+  cudaEvent_t fork_ev = nullptr, join_ev = nullptr, join3_ev = nullptr, map_ev = nullptr;
   int64_t acc_fnq = 0, acc_f4q = 0;
   double acc_ms_panel = 0., acc_ms_f4 = 0., acc_ms_line_chain = 0., acc_ms_f4_chain = 0., acc_ms_rt = 0.;
   int64_t acc_rt_bytes = 0;
@@ -896,13 +896,24 @@ InterpSpec interp_spec(double v1in, double dvin, int64_t nin, double v1out, doub
   return s;
 }
 
+// the handle's stream waits for the maps launched on the third one so far
+int join_maps(clblm_handle* h) {
+  CUDA_TRY(h, cudaEventRecord(h->map_ev, h->stream3));
+  CUDA_TRY(h, cudaStreamWaitEvent(h->stream, h->map_ev, 0));
+  return CLBLM_OK;
+}
+
 // For a general-ratio spec: the per-point (iIn, IP) map, built on the device
 // into `buf`.  interpSpectrum's outer loop restarts at J1 = INT((Vo - V1)/DVout
 // + 1.001), Vo = V1 + J2*DVout: every 2400 points while the rounding of Vo
 // stays below a thousandth of DVout, and then no table goes to the device (a
 // host wait in the middle of the call's launches); for finer grids the host
 // replays the loop.
-int build_interp_map(clblm_handle* h, InterpSpec* s, int64_t nout, DevBuf* buf) {
+// On the third stream it runs beside the optical depths (a map is a chain of
+// 2400 steps wherever a block has an undecided point: 126 us of a 100 cm-1
+// layer's 576), from behind the fork of the last run_od_batch, which follows
+// the buffer's last reader; on the handle's it keeps its place.
+int build_interp_map(clblm_handle* h, InterpSpec* s, int64_t nout, DevBuf* buf, cudaStream_t st) {
   if (s->kind == 0 || s->itype >= 0) return CLBLM_OK;
   const double V2out = s->v1 + (double)(nout - 1) * s->dvout;
   if (std::max(std::fabs(s->v1), std::fabs(V2out)) * 1.e-12 < s->dvout && s->dvout > 1.e-7) {
@@ -910,10 +921,10 @@ int build_interp_map(clblm_handle* h, InterpSpec* s, int64_t nout, DevBuf* buf) 
     CUDA_TRY(h, buf->ensure(sizeof(int2) * nout + 16 * (nb + 1) + 512));
     int2* map = buf->as<int2>();
     h->launches++;
-    k_interp_map<<<(unsigned)nb, kMapThreads, 0, h->stream>>>(*s, nullptr, nullptr, (int)nb, nout, map);
+    k_interp_map<<<(unsigned)nb, kMapThreads, 0, st>>>(*s, nullptr, nullptr, (int)nb, nout, map);
     CUDA_TRY(h, cudaGetLastError());
     s->map = map;
-    return CLBLM_OK;
+    return st == h->stream ? CLBLM_OK : join_maps(h);
   }
   std::vector<int64_t> j1;
   std::vector<double> vo;
@@ -935,14 +946,14 @@ int build_interp_map(clblm_handle* h, InterpSpec* s, int64_t nout, DevBuf* buf) 
   size_t off = ((sizeof(int2) * nout) + 255) & ~size_t(255);
   int64_t* dj1 = reinterpret_cast<int64_t*>(base + off);
   double* dvo = reinterpret_cast<double*>(base + off + 8 * (nb + 1));
-  CUDA_TRY(h, cudaMemcpyAsync(dj1, j1.data(), 8 * nb, cudaMemcpyHostToDevice, h->stream));
-  CUDA_TRY(h, cudaMemcpyAsync(dvo, vo.data(), 8 * nb, cudaMemcpyHostToDevice, h->stream));
+  CUDA_TRY(h, cudaMemcpyAsync(dj1, j1.data(), 8 * nb, cudaMemcpyHostToDevice, st));
+  CUDA_TRY(h, cudaMemcpyAsync(dvo, vo.data(), 8 * nb, cudaMemcpyHostToDevice, st));
   h->launches++;
-  k_interp_map<<<(unsigned)nb, kMapThreads, 0, h->stream>>>(*s, dj1, dvo, (int)nb, nout, map);
+  k_interp_map<<<(unsigned)nb, kMapThreads, 0, st>>>(*s, dj1, dvo, (int)nb, nout, map);
   CUDA_TRY(h, cudaGetLastError());
-  CUDA_TRY(h, cudaStreamSynchronize(h->stream));  // host block tables go out of scope
+  CUDA_TRY(h, cudaStreamSynchronize(st));  // host block tables go out of scope
   s->map = map;
-  return CLBLM_OK;
+  return st == h->stream ? CLBLM_OK : join_maps(h);
 }
 
 // ---- device pipeline for a batch of layers ----------------------------------
@@ -1769,7 +1780,8 @@ int clblm_gpu_create(const clblm_lines_t* lines, const clblm_cont_t* cont, int d
       cudaEventCreateWithFlags(&h->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&h->join_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaStreamCreateWithFlags(&h->stream3, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&h->join3_ev, cudaEventDisableTiming) != cudaSuccess) {
+      cudaEventCreateWithFlags(&h->join3_ev, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->map_ev, cudaEventDisableTiming) != cudaSuccess) {
     g_create_err = "cannot create the second stream";
     clblm_gpu_destroy(h);
     return CLBLM_ERR_CUDA;
@@ -1881,6 +1893,7 @@ int clblm_gpu_destroy(clblm_handle_t* h) {
   if (h->fork_ev) cudaEventDestroy(h->fork_ev);
   if (h->join_ev) cudaEventDestroy(h->join_ev);
   if (h->join3_ev) cudaEventDestroy(h->join3_ev);
+  if (h->map_ev) cudaEventDestroy(h->map_ev);
   if (h->stage_ev) cudaEventDestroy(h->stage_ev);
   h->stage.release();
   h->back.release();
@@ -2043,7 +2056,7 @@ int clblm_gpu_od(clblm_handle_t* h, const clblm_layer_t* layer, const clblm_grid
     dst = h->outbuf.as<double>();
   }
   InterpSpec s = interp_spec(P.v1, P.dv, P.nsamp, P.v1, hps[0].dv_out, n);
-  rc = build_interp_map(h, &s, n, &h->imap[0]);
+  rc = build_interp_map(h, &s, n, &h->imap[0], h->stream3);
   if (rc) return rc;
   const void* od = plain ? (const void*)(h->od.as<double>() + P.od_off) : (const void*)(h->od.as<float>() + P.od_off);
   h->launches++;
@@ -2294,7 +2307,7 @@ int clblm_gpu_rt_mode2(clblm_handle_t* h, const clblm_column_t* col, const clblm
     // the layer tables of this batch: each layer's grid, its map onto the
     // merge grid and the scalars of its terms
     h->rtseg_host.assign(count, RtSegLayer{});
-    int nlymap = 0;
+    int nlymap = 0, nrunmap = 0;
     for (int il = first; il < first + count; ++il) {
       const LayerPlan& P = rp.hps[il].P;
       RtSegLayer& L = h->rtseg_host[il - first];
@@ -2307,7 +2320,7 @@ int clblm_gpu_rt_mode2(clblm_handle_t* h, const clblm_column_t* col, const clblm
       L.ly = interp_spec(col->v1, odv, onn, col->v1, rp.grid_dv[il], rp.grid_n[il]);
       if (L.ly.kind != 0 && L.ly.itype < 0) {  // a coarser layer by a general ratio: its own map
         if ((int)h->rt_lymap.size() <= nlymap) h->rt_lymap.resize(nlymap + 1);
-        rc = build_interp_map(h, &L.ly, rp.grid_n[il], &h->rt_lymap[nlymap++]);
+        rc = build_interp_map(h, &L.ly, rp.grid_n[il], &h->rt_lymap[nlymap++], h->stream3);
         if (rc) return rc;
       }
       L.od = plain ? (const void*)(h->od.as<double>() + P.od_off) : (const void*)(h->od.as<float>() + P.od_off);
@@ -2353,8 +2366,13 @@ int clblm_gpu_rt_mode2(clblm_handle_t* h, const clblm_column_t* col, const clblm
       a.n_out = rp.grid_n[il];
       a.v1 = col->v1;
       a.mr = interp_spec(col->v1, in_dv, in_n, col->v1, rp.grid_dv[il], rp.grid_n[il]);
-      rc = build_interp_map(h, &a.mr, a.n_out, &h->imap[0]);
-      if (rc) return rc;
+      if (a.mr.kind != 0 && a.mr.itype < 0) {  // (a buffer each for the first few: the runs before read theirs)
+        const bool own = nrunmap++ < 4;
+        if (own && (int)h->rt_lymap.size() <= nlymap) h->rt_lymap.resize(nlymap + 1);
+        rc = build_interp_map(h, &a.mr, a.n_out, own ? &h->rt_lymap[nlymap++] : &h->imap[0],
+                              own ? h->stream3 : h->stream);
+        if (rc) return rc;
+      }
       a.rad_in = h->rt[cur * 2].p;
       a.refl_in = h->rt[cur * 2 + 1].p;
       a.rad_out = h->rt[(1 - cur) * 2].p;
@@ -3058,7 +3076,9 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
       rc = run_od_batch(h, hps, first, count, plain, true, ls, fs, ps);
       if (rc) return rc;
       h->launches += 2;
-      k_interp_map_jobs<<<dim3((unsigned)bmax, count), kMapThreads, 0, h->stream>>>(djobs, count);
+      k_interp_map_jobs<<<dim3((unsigned)bmax, count), kMapThreads, 0, h->stream3>>>(djobs, count);
+      rc = join_maps(h);
+      if (rc) return rc;
       const dim3 go((unsigned)((nlmax + kOdJobPoints - 1) / kOdJobPoints), count);
       if (plain) k_od_jobs<true><<<go, kOdJobThreads, 0, h->stream>>>(djobs, count, h->od.p, h->jod.p);
       else k_od_jobs<false><<<go, kOdJobThreads, 0, h->stream>>>(djobs, count, h->od.p, h->jod.p);
@@ -3492,7 +3512,9 @@ int batch_enqueue(clblm_handle* h, BatchPlan& bp, const clblm_profile_t* prof, c
     const int64_t nmax = c.nmax;
     const int bmax = c.bmax;
     h->launches += 2;
-    k_interp_map_jobs<<<dim3((unsigned)bmax, c.count), kMapThreads, 0, h->stream>>>(jobs, c.count);
+    k_interp_map_jobs<<<dim3((unsigned)bmax, c.count), kMapThreads, 0, h->stream3>>>(jobs, c.count);
+    rc = join_maps(h);
+    if (rc) return rc;
     if (plain)
       k_od_jobs<true><<<dim3((unsigned)((nmax + kOdJobPoints - 1) / kOdJobPoints), c.count), kOdJobThreads, 0,
                         h->stream>>>(jobs, c.count, h->od.p, h->jod.p);
