@@ -648,8 +648,9 @@ __device__ __forceinline__ void gather_plain(PanelSmem<true>& S, const PanelArgs
       const GridRec r = buf[k];
       if (g < r.g_lo || g > r.g_hi || (Cpl ? (r.q & ~kCplBit) : r.q) > qmax) continue;
       const GridRecD& d = S.wrecd[warp][k];
-      const double zf = fma((double)(g - r.g_lo + 1), d.zs, d.zfl);
-      const int iz = (int)(fabs(zf) + 1.5);
+      // (conversions in integer arithmetic: the FP64 unit bounds the pass)
+      const double zf = fma(i32_to_f64(g - r.g_lo + 1), d.zs, d.zfl);
+      const int iz = f64_to_i32_trunc(fabs(zf) + 1.5);
       if (iz > kNFMX) {
         atomicOr(a.err, 2);
         continue;
