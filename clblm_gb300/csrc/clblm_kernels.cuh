@@ -148,12 +148,12 @@ __global__ void k_f4_groups(int layer0, int64_t stride, const long long* vbits, 
                             const int* gnxt, const unsigned char* flags, int64_t tab_records, const int4* calls,
                             const int2* ncalls, int4* groups, int64_t* ngroups);
 constexpr int kGroupSumThreads = 256;
-__global__ void __launch_bounds__(kGroupSumThreads)
+__global__ void __launch_bounds__(kGroupSumThreads, 6)
     k_f4_groupsum(const LayerPlan* plans, int layer0, const F4Prep* prep, int64_t stride,
                               const int64_t* src, const int4* groups, const int64_t* ngroups, ShrunkLine* out);
 struct F4Rec;
 struct F4RecD;
-__global__ void __launch_bounds__(kSetupThreads, 3)
+__global__ void __launch_bounds__(kSetupThreads, 4)
     k_f4_lineinit(const LayerPlan* plans, int layer0, const ShrunkLine* sh, int64_t stride,
                               const int64_t* nsh, F4Rec* rec, F4RecD* recd, int64_t rstride, int64_t* nrec,
                               int64_t* nmirror, unsigned long long* stats, double* cpl);

@@ -2040,6 +2040,8 @@ __device__ __forceinline__ ShrunkLine shrunk_line(int k, bool mixed, double SUMV
 // per group take a thread per group, sorted by length: there are many of them,
 // and the FP64 unit, which takes as long for one lane as for 32, adds 32
 // groups' members at once.
+// Loads of scattered members and chains of additions: six CTAs of 40 registers
+// per SM hide them best (three of 83: 1.44 ms for 30 million lines, six: 0.83).
 constexpr int kGroupWarps = kGroupSumThreads / 32;
 // Launches of many lines do so at any length: a warp's group costs an addition
 // of the FP64 unit per line where 32 threads' groups cost three per 32 lines
@@ -2169,7 +2171,7 @@ __device__ __forceinline__ void group_sums_sorted(GroupShared& W, const F4Prep* 
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kGroupSumThreads)
+__global__ void __launch_bounds__(kGroupSumThreads, 6)
     k_f4_groupsum(const LayerPlan* __restrict__ plans, int layer0, const F4Prep* __restrict__ prep, int64_t stride,
                   const int64_t* __restrict__ src, const int4* __restrict__ groups,
                   const int64_t* __restrict__ ngroups, ShrunkLine* __restrict__ out) {
@@ -2360,7 +2362,7 @@ __device__ void f4_record(const LayerPlan& P, const ShrunkLine& L, double VNUI, 
   }
 }
 
-__global__ void __launch_bounds__(kSetupThreads, 3)
+__global__ void __launch_bounds__(kSetupThreads, 4)
     k_f4_lineinit(const LayerPlan* __restrict__ plans, int layer0, const ShrunkLine* __restrict__ sh,
                               int64_t stride, const int64_t* __restrict__ nsh, F4Rec* __restrict__ rec,
                               F4RecD* __restrict__ recd, int64_t rstride, int64_t* __restrict__ nrec,
