@@ -157,7 +157,7 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 }
 
 template <bool Plain>
-__global__ void __launch_bounds__(128) k_jac(JacArgs a) {
+__global__ void __launch_bounds__(128, Plain ? 1 : 8) k_jac(JacArgs a) {
   using Real = typename std::conditional<Plain, double, float>::type;
   int64_t iv = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int N2 = a.nlay;
