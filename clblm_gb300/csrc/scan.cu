@@ -27,7 +27,8 @@
 // points in M blocks of B, block b's point at t in [-1, 1] from its centre,
 //   exp(-2 pi i k n / N) = phase(k, b) exp(-i theta t),  theta = pi k / M,
 // and exp(-i theta t) = sum_p (-i theta)^p / p! t^p: 12 terms below 1e-16 for
-// theta < 0.2, so
+// theta < 0.2 (M >= 16 K), or 24 of them for theta < pi / 2 (M >= 2 K, where
+// 16 K leaves blocks of fewer than 32 points), so, of 12,
 //   k_scan_moments     sum_j x_j t_j^p of each block, p = 0 .. 11
 //   k_scan_fft<false>  their transforms of M points, two moments as one complex
 //   k_scan_low         the coefficients k < K from them, times the apodization,
@@ -230,19 +231,20 @@ __device__ __forceinline__ void scan_powers(int B, double (*T)[kScanPowers], int
 }
 
 // moments of a block of B points (even): the pairs (j, B-1-j), whose t are
-// opposite, over the kMomLanes lanes of a block; the FP64 unit bounds it (16
-// cycles an instruction: 17 a pair), so the powers of t come from a table and
+// opposite, over the kMomLanes lanes of a block; the FP64 unit bounds it (17
+// instructions a pair), so the powers of t come from a table and
 // a lane group is as small as the reduction's 16 values allow (lane q ends
-// with moments 2q and 2q+1): 77 -> 33 us on 2,000,000 points against a warp
+// with moments 2q and 2q+1, or four of 24): 77 -> 60 us on 2,000,000 points against a warp
 // per block and powers by multiplication.  The blocks past the data are
 // zeroed, and W gets exp(-2 pi i j / M) for the transforms.
+template <int Terms>
 __global__ void __launch_bounds__(kScanLowThreads)
     k_scan_moments(const double* __restrict__ s, int64_t off, int64_t ltotal, int boxed, int64_t ktotal, double fill,
                    double2* __restrict__ mom, int64_t nblk, int B, int64_t M, double2* __restrict__ W) {
-  constexpr int kMomLanes = 8;
-  __shared__ double T[kScanTerms / 2][kScanPowers];
+  constexpr int kMomLanes = 8, kSums = Terms <= 16 ? 16 : 32, kMine = kSums / kMomLanes;
+  __shared__ double T[Terms / 2][kScanPowers];
   const bool table = B / 2 <= kScanPowers;
-  if (table) scan_powers(B, T, kScanTerms / 2);
+  if (table) scan_powers(B, T, Terms / 2);
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthr = (int64_t)gridDim.x * blockDim.x;
   const int lane = threadIdx.x & (kMomLanes - 1);
   const int64_t n = boxed <= 1 ? ltotal : ktotal;
@@ -258,9 +260,9 @@ __global__ void __launch_bounds__(kScanLowThreads)
   const int64_t groups = (M * kMomLanes + 31) / 32 * (32 / kMomLanes);
   for (int64_t g = tid / kMomLanes; g < groups; g += nthr / kMomLanes) {
     const int64_t b = g < M ? g : M - 1;
-    double v[16];
+    double v[kSums];
 #pragma unroll
-    for (int p = 0; p < 16; ++p) v[p] = 0.;
+    for (int p = 0; p < kSums; ++p) v[p] = 0.;
     if (b < nblk) {
       const int64_t i0 = b * B;
       if (table) {
@@ -271,7 +273,7 @@ __global__ void __launch_bounds__(kScanLowThreads)
           v[0] += e;
           v[1] += o;
 #pragma unroll
-          for (int q = 1; q < kScanTerms / 2; ++q) {
+          for (int q = 1; q < Terms / 2; ++q) {
             v[2 * q] = fma(e, T[q][j], v[2 * q]);
             v[2 * q + 1] = fma(o, T[q][j], v[2 * q + 1]);
           }
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(kScanLowThreads)
           const double t = ((double)j - c) * rh, t2 = t * t;
           double e = x0 + x1, o = (x0 - x1) * t;
 #pragma unroll
-          for (int p = 0; p < kScanTerms; p += 2) {
+          for (int p = 0; p < Terms; p += 2) {
             v[p] += e;
             v[p + 1] += o;
             e *= t2;
@@ -291,18 +293,22 @@ __global__ void __launch_bounds__(kScanLowThreads)
         }
       }
     }
-    // totals over the lanes: lane l ends with those of v[2l], v[2l+1]
+    // totals over the lanes: lane l ends with those of v[kMine l ..]
 #pragma unroll
-    for (int h = 8; h >= 2; h >>= 1) {
-      const bool up = (lane & (h >> 1)) != 0;
+    for (int h = kSums / 2; h >= kMine; h >>= 1) {
+      const bool up = (lane & (h / kMine)) != 0;
 #pragma unroll
       for (int i = 0; i < h; ++i) {
         const double send = up ? v[i] : v[i + h];
         const double keep = up ? v[i + h] : v[i];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h >> 1);
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h / kMine);
       }
     }
-    if (lane < kScanTerms / 2) mom[(int64_t)lane * M + b] = make_double2(v[0], v[1]);
+#pragma unroll
+    for (int i = 0; i < kMine / 2; ++i) {
+      const int q = lane * (kMine / 2) + i;
+      if (q < Terms / 2) mom[(int64_t)q * M + b] = make_double2(v[2 * i], v[2 * i + 1]);
+    }
   }
   if (W)
     for (int64_t j = tid; j < M; j += nthr) {
@@ -325,7 +331,8 @@ __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -
 //   y[r + R c] = sum_j conj(w_C)^(j c) sum_{k = j mod C} conj(w_M)^(r k) Z[k].
 // Radix-4 Stockham passes (Stockham's autosort transform) in shared memory.
 // The 6 transforms of M = 32768 points were 255 us each way as 12 real ones of
-// a library with a CTA per transform (12 of 152 SMs); 192 CTAs take 13 us.
+// a library with a CTA per transform (12 of 152 SMs); 192 CTAs take 27 us
+// forward and 39 back (FP64 unit, and 40 SMs with a second CTA).
 // The parts' number is fixed, so that the sum over r stays 32 terms; above
 // kScanFftMaxC points a part, M is enough work for the library's transforms.
 template <bool Back>
@@ -403,11 +410,12 @@ __global__ void __launch_bounds__(kScanFftThreads)
 // to the coefficient w, and y_2q + i y_(2q+1) has the spectrum s (a - b) w at
 // k, s (a + b) conj(w) at -k.  R = kScanFftR parts (k_scan_fft), or 1 part (W
 // not read).
-__global__ void __launch_bounds__(32 * kScanTerms / 2)
+template <int Terms>
+__global__ void __launch_bounds__(32 * Terms / 2)
     k_scan_low(ScanArgs a, double fill_n, double scale, int64_t K, int64_t M, int R, const double2* __restrict__ X,
                const double2* __restrict__ W, double2* __restrict__ Z) {
   const double PI = 3.141592653589793;
-  __shared__ double2 part[kScanTerms / 2][kScanLowK], tot[kScanLowK];
+  __shared__ double2 part[Terms / 2][kScanLowK], tot[kScanLowK];
   const int q = threadIdx.x >> 5, lane = threadIdx.x & 31, kl = lane & (kScanLowK - 1);
   const int64_t k = (int64_t)blockIdx.x * kScanLowK + kl;
   const bool in = k < K;
@@ -449,7 +457,7 @@ __global__ void __launch_bounds__(32 * kScanTerms / 2)
   if (q == 0 && lane < kScanLowK && in) {
     double wr = 0., wi = 0.;
 #pragma unroll
-    for (int p = 0; p < kScanTerms / 2; ++p) {
+    for (int p = 0; p < Terms / 2; ++p) {
       wr += part[p][kl].x;
       wi += part[p][kl].y;
     }
@@ -478,8 +486,9 @@ __global__ void __launch_bounds__(32 * kScanTerms / 2)
 }
 
 // The scanned points [first, first + count): a warp per block, a lane per
-// pair of opposite points (13 FP64 instructions a pair bound it; 42 -> 27 us
+// pair of opposite points (13 FP64 instructions a pair bound it; 42 -> 33 us
 // with t from a table and the scale in the coefficients)
+template <int Terms>
 __global__ void __launch_bounds__(kScanLowThreads)
     k_scan_expand(const double2* __restrict__ y, int64_t M, int B, int64_t first, int64_t count,
                   double* __restrict__ out) {
@@ -491,14 +500,14 @@ __global__ void __launch_bounds__(kScanLowThreads)
   const int64_t b0 = first / B, b1 = (first + count - 1) / B;
   const double rh = 2. / (double)B, c = 0.5 * (double)(B - 1);
   for (int64_t b = b0 + (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b <= b1; b += warps) {
-    double2 Y[kScanTerms / 2];
+    double2 Y[Terms / 2];
 #pragma unroll
-    for (int q = 0; q < kScanTerms / 2; ++q) Y[q] = y[(int64_t)q * M + b];
+    for (int q = 0; q < Terms / 2; ++q) Y[q] = y[(int64_t)q * M + b];
     for (int j = lane; j < B / 2; j += 32) {
       const double t = table ? T[0][j] : ((double)j - c) * rh, t2 = table ? T[1][j] : t * t;
-      double e = Y[kScanTerms / 2 - 1].x, o = Y[kScanTerms / 2 - 1].y;
+      double e = Y[Terms / 2 - 1].x, o = Y[Terms / 2 - 1].y;
 #pragma unroll
-      for (int q = kScanTerms / 2 - 2; q >= 0; --q) {
+      for (int q = Terms / 2 - 2; q >= 0; --q) {
         e = fma(e, t2, Y[q].x);
         o = fma(o, t2, Y[q].y);
       }
@@ -510,6 +519,18 @@ __global__ void __launch_bounds__(kScanLowThreads)
   }
 }
 
+template __global__ void k_scan_moments<kScanTerms>(const double* __restrict__, int64_t, int64_t, int, int64_t, double,
+                                             double2* __restrict__, int64_t, int, int64_t, double2* __restrict__);
+template __global__ void k_scan_low<kScanTerms>(ScanArgs, double, double, int64_t, int64_t, int, const double2* __restrict__,
+                                         const double2* __restrict__, double2* __restrict__);
+template __global__ void k_scan_expand<kScanTerms>(const double2* __restrict__, int64_t, int, int64_t, int64_t,
+                                            double* __restrict__);
+template __global__ void k_scan_moments<kScanTermsWide>(const double* __restrict__, int64_t, int64_t, int, int64_t, double,
+                                             double2* __restrict__, int64_t, int, int64_t, double2* __restrict__);
+template __global__ void k_scan_low<kScanTermsWide>(ScanArgs, double, double, int64_t, int64_t, int, const double2* __restrict__,
+                                         const double2* __restrict__, double2* __restrict__);
+template __global__ void k_scan_expand<kScanTermsWide>(const double2* __restrict__, int64_t, int, int64_t, int64_t,
+                                            double* __restrict__);
 template __global__ void k_scan_fft<false>(const double2* __restrict__, double2* __restrict__, const double2* __restrict__,
                                           int64_t, int64_t, int);
 template __global__ void k_scan_fft<true>(const double2* __restrict__, double2* __restrict__, const double2* __restrict__,

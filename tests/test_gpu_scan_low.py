@@ -64,3 +64,15 @@ def test_data_ending_at_records_and_blocks(gpu_lib, n):
                                      (4300000, 2e-4, 0.2)])
 def test_transform_sizes(gpu_lib, n, dv, hw):
     _check(gpu_lib, n, dv, 5, hw, 1000.0 + 0.4 * dv * n, 1000.0 + 0.9 * dv * n, fill=0.5)
+
+
+# as many coefficients as a sixty-fourth of the points, and more: the wide form
+# (24 terms, blocks of 32 points and more) and the whole transform after it
+@pytest.mark.parametrize("fid", [3, 5])
+@pytest.mark.parametrize("hw", [0.30, 0.12, 0.082, 0.08, 0.05])
+def test_wide_form(gpu_lib, fid, hw):
+    _check(gpu_lib, 60000, 0.002, fid, hw, 1055.0, 1062.003, fill=0.5)
+
+
+def test_wide_form_of_many_points(gpu_lib):
+    _check(gpu_lib, 700000, 0.0015, 5, 0.4, 1300.0, 1800.0)
