@@ -21,8 +21,8 @@
 //
 // Mixed path: table look-ups, products and sums in FP32 with Kahan-
 // compensated accumulation; every table index is the reference's FP64 index
-// (an FP32 index whose argument is within 1e-3 of a rounding boundary is
-// recomputed in FP64).  Plain path: FP64 throughout.
+// (an FP32 index whose argument's error may reach across a rounding boundary
+// is formed again).  Plain path: FP64 throughout.
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -53,7 +53,7 @@ struct SumD {
 };
 
 // FP32 table index IZ = INT(|ZF| + 1.5) with ZF = ZFL + k*ZSLOPE.  When the
-// FP32 argument lies within 1e-3 of a rounding boundary it is redone in
+// FP32 argument may lie on the other side of a rounding boundary it is redone in
 // float-float (ZFL and ZSLOPE as hi + lo pairs, products and sums with their
 // exact errors, about 1e-8 absolute), and within 1e-7 of the boundary after
 // that, in FP64 with ZFL and ZSLOPE formed again from the line of the
