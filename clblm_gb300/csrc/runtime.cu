@@ -4190,8 +4190,11 @@ int clblm_gpu_fftscn(clblm_handle_t* h, const clblm_scan_t* scan, const double* 
                                                             nblk, B, M, own ? W : nullptr);
     CUDA_TRY(h, cudaGetLastError());
     if (own) {
-      CUDA_TRY(h, cudaFuncSetAttribute(k_scan_fft<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      CUDA_TRY(h, cudaFuncSetAttribute(k_scan_fft<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      // (the attribute is the kernel's, not the handle's: always the largest
+      // size, so that no thread's scan lowers it between another's and its launch)
+      constexpr int kSmemMax = (int)(sizeof(double2) * 3 * (size_t)kScanFftMaxC);
+      CUDA_TRY(h, cudaFuncSetAttribute(k_scan_fft<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
+      CUDA_TRY(h, cudaFuncSetAttribute(k_scan_fft<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
       k_scan_fft<false><<<parts, kScanFftThreads, smem, st>>>(Z, X, W, M, K, logC);
       CUDA_TRY(h, cudaGetLastError());
     } else {
