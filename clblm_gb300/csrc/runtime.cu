@@ -1417,47 +1417,61 @@ struct WsDims {
   }
 };
 
+// The layers of one batch: per line, per far-wing line and per panel its arrays
+// are as long as the largest layer's, times the layers.
+struct WsLayers {
+  int64_t ls = 1, fs = 1, ps = 1;  // the largest layer's
+  int64_t cnt = 0, odt = 0, r4t = 0, ctas = 0, blk = 0;
+  void add(const HostPlan& hp) {
+    const LayerPlan& P = hp.P;
+    ls = std::max<int64_t>(ls, P.line_hi - P.line_lo + 1);
+    fs = std::max<int64_t>(fs, P.f4_hi - P.f4_lo);
+    ps = std::max<int64_t>(ps, P.npanels);
+    cnt++;
+    odt += pad256(P.nsamp + 8) * P.nslice;
+    ctas += (int64_t)P.npanels * P.nslice;
+    r4t += pad256(P.nptr4 + 8);
+    blk += (int64_t)hp.blk_v1.size();
+  }
+  int64_t lstride() const { return pad256(ls); }
+  int64_t f4stride() const { return pad256(fs); }
+  WsDims dims() const {
+    const int64_t l = lstride(), f = f4stride();
+    WsDims d;
+    d.lsc = l * cnt;
+    d.fsc = f * cnt;
+    d.frecc = f4_records(f) * cnt;
+    d.f4aggc = (f + kF4Blk - 1) / kF4Blk * cnt;
+    d.psc = ps * cnt;
+    d.cnt = cnt;
+    d.odt = odt;
+    d.ctas = ctas;
+    d.r4t = r4t;
+    d.nblk4c = ((f + 1 + 1023) / 1024) * cnt;
+    d.smaxc = ((l + 1023) / 1024) * cnt;
+    d.raggc = 2 * 3 * cnt * ((l + kRecBlock - 1) / kRecBlock);
+    return d;
+  }
+};
+
 // Strides of the layers [first, first+count) and their offsets in the
 // per-batch buffers (OD, R4, ABSRB).
 WsDims batch_dims(std::vector<HostPlan>& hps, int first, int count, int64_t* lstride, int64_t* f4stride,
                   int64_t* pstride) {
-  int64_t ls = 1, fs = 1, ps = 1, odt = 0, r4t = 0, ctas = 0;
+  WsLayers w;
   for (int k = 0; k < count; ++k) {
     LayerPlan& P = hps[first + k].P;
-    ls = std::max<int64_t>(ls, P.line_hi - P.line_lo + 1);
-    fs = std::max<int64_t>(fs, P.f4_hi - P.f4_lo);
-    ps = std::max<int64_t>(ps, P.npanels);
-  }
-  ls = pad256(ls);
-  fs = pad256(fs);
-  for (int k = 0; k < count; ++k) {
-    LayerPlan& P = hps[first + k].P;
-    P.od_off = odt;
+    P.od_off = w.odt;
     P.od_pts = pad256(P.nsamp + 8);
-    odt += P.od_pts * P.nslice;
-    P.cta0 = ctas;
-    ctas += (int64_t)P.npanels * P.nslice;
-    P.r4_off = r4t;
-    r4t += pad256(P.nptr4 + 8);
+    P.cta0 = w.ctas;
+    P.r4_off = w.r4t;
     P.abs_off = (int64_t)k * (kNABSRB + 8);
+    w.add(hps[first + k]);
   }
-  WsDims d;
-  d.lsc = ls * count;
-  d.fsc = fs * count;
-  d.frecc = f4_records(fs) * count;
-  d.f4aggc = (fs + kF4Blk - 1) / kF4Blk * count;
-  d.psc = ps * count;
-  d.cnt = count;
-  d.odt = odt;
-  d.ctas = ctas;
-  d.r4t = r4t;
-  d.nblk4c = ((fs + 1 + 1023) / 1024) * count;
-  d.smaxc = ((ls + 1023) / 1024) * count;
-  d.raggc = 2 * 3 * count * ((ls + kRecBlock - 1) / kRecBlock);
-  *lstride = ls;
-  *f4stride = fs;
-  *pstride = ps;
-  return d;
+  *lstride = w.lstride();
+  *f4stride = w.f4stride();
+  *pstride = w.ps;
+  return w.dims();
 }
 
 // The parts of the tables' buffer for nL planned layers; returns its size.
@@ -1489,76 +1503,82 @@ size_t tab_layout(clblm_handle* h, int nL, int64_t vftt, int64_t blkt, int64_t i
   return off;
 }
 
-// Buffers of one OD batch (sized by d) and of all nL planned layers: the
+// The scratch buffers of one OD batch (sized by d; blkt: far-wing blocks of all
+// nL planned layers) and their bytes.  Nothing in them outlives the batch; the
+// tables' buffer and the pool of radiation-term segments, which do not grow
+// with the batch, stand apart.
+struct WsPart {
+  DevBuf* buf;
+  size_t bytes;
+};
+std::vector<WsPart> ws_parts(clblm_handle* h, const WsDims& d, int nL, int64_t blkt, bool plain) {
+  const size_t real = plain ? 8 : 4, cpl = h->has_cpl ? 1 : 0, n = (size_t)std::max(nL, 1);
+  const size_t lines = d.lsc, f4 = d.fsc, lay = d.cnt, f4recs = f4 + 4096 * lay, panels = d.psc;
+  // (FP64 records: the FP64 path only; DPTRAT and the lists of coupled records: coupled lists only)
+  return {{&h->linecpl, std::max<size_t>(cpl * sizeof(double) * lines, 256)},
+          {&h->f4cpl, std::max<size_t>(cpl * sizeof(double) * f4recs, 256)},
+          {&h->f4cpll, std::max<size_t>(cpl * sizeof(int64_t) * f4recs, 256)},
+          {&h->f4ncpl, sizeof(int64_t) * n},
+          {&h->prep, sizeof(LinePrep) * lines},
+          {&h->qpanel, sizeof(int) * lines},
+          {&h->rec, sizeof(GridRec) * lines * 3},
+          {&h->recd, plain ? sizeof(GridRecD) * lines * 3 : 256},
+          {&h->gpm, sizeof(int) * lines * 3},
+          {&h->reclo, sizeof(GridRecLo) * lines * 3},
+          {&h->gsm, sizeof(int) * lines * 3},
+          {&h->ragg, sizeof(int) * (size_t)d.raggc},
+          {&h->ranges, sizeof(int64_t) * 6 * panels},
+          {&h->od, real * (size_t)d.odt},
+          {&h->pwork, sizeof(int2) * (size_t)d.ctas},
+          {&h->psegn, sizeof(int) * panels},
+          {&h->psegs, sizeof(int) * kSegTab * panels},
+          {&h->psegv, sizeof(double2) * kSegTab * panels},
+          {&h->pxint, sizeof(XintPanel) * panels},
+          {&h->r4, real * (size_t)d.r4t},
+          {&h->absrb, sizeof(double) * (kNABSRB + 8) * lay},
+          {&h->blockmax, sizeof(int) * (size_t)d.smaxc},
+          {&h->f4prep, sizeof(F4Prep) * f4},
+          {&h->f4sh, sizeof(ShrunkLine) * f4},
+          {&h->f4blk, sizeof(int64_t) * (size_t)d.nblk4c},
+          {&h->f4ntot, sizeof(int64_t) * lay},
+          {&h->f4mask, sizeof(unsigned) * (f4 / 32 + lay)},
+          {&h->f4cidx, sizeof(int64_t) * (f4 + lay)},
+          {&h->f4vb, sizeof(long long) * f4},
+          {&h->f4lb, sizeof(long long) * f4},
+          {&h->f4src, sizeof(int64_t) * f4},
+          {&h->f4flag, f4},
+          {&h->f4nxt, sizeof(int) * f4},
+          {&h->f4cut, sizeof(int64_t) * lay},
+          {&h->f4grp, sizeof(int4) * f4},
+          {&h->f4tab, sizeof(unsigned) * kCallEnds * (size_t)d.frecc},
+          {&h->f4calls, sizeof(int4) * ((size_t)d.frecc + 2 * lay)},
+          {&h->f4ncall, sizeof(int2) * lay},
+          {&h->f4agg, sizeof(int) * 2 * (size_t)d.f4aggc},
+          {&h->f4rec, sizeof(F4Rec) * f4recs},
+          {&h->f4recd, plain ? sizeof(F4RecD) * f4recs : 256},
+          {&h->f4nrec, sizeof(int64_t) * n},
+          {&h->f4nmir, sizeof(int64_t) * n},
+          {&h->f4pm, sizeof(int) * f4recs},
+          {&h->f4sm, sizeof(int) * f4recs},
+          {&h->bfac, sizeof(double) * (kLIMOUT4 + 2) * (size_t)(blkt + 1)}};
+}
+
+// The buffers of one OD batch and the tables of all nL planned layers: the
 // first error, or success.
 cudaError_t ws_alloc(clblm_handle* h, const WsDims& d, int nL, int64_t vftt, int64_t blkt, int64_t isot,
                      bool plain) {
-  const size_t real = plain ? 8 : 4;
-  cudaError_t e = cudaSuccess;
-#define WS_ENSURE(x)                       \
-  do {                                     \
-    if ((e = (x)) != cudaSuccess) return e; \
-  } while (0)
-  WS_ENSURE(h->tabbuf.ensure(tab_layout(h, nL, vftt, blkt, isot)));
-  WS_ENSURE(h->linecpl.ensure(h->has_cpl ? sizeof(double) * d.lsc : 256));
-  WS_ENSURE(h->f4cpl.ensure(h->has_cpl ? sizeof(double) * (d.fsc + 4096 * d.cnt) : 256));
-  WS_ENSURE(h->f4cpll.ensure(h->has_cpl ? sizeof(int64_t) * (d.fsc + 4096 * d.cnt) : 256));
-  WS_ENSURE(h->f4ncpl.ensure(sizeof(int64_t) * std::max(nL, 1)));
-  WS_ENSURE(h->prep.ensure(sizeof(LinePrep) * d.lsc));
-  WS_ENSURE(h->qpanel.ensure(sizeof(int) * d.lsc));
-  WS_ENSURE(h->rec.ensure(sizeof(GridRec) * d.lsc * 3));
-  // FP64 records: the FP64 path only
-  WS_ENSURE(h->recd.ensure(plain ? sizeof(GridRecD) * d.lsc * 3 : 256));
-  WS_ENSURE(h->gpm.ensure(sizeof(int) * d.lsc * 3));
-  WS_ENSURE(h->reclo.ensure(sizeof(GridRecLo) * d.lsc * 3));
-  WS_ENSURE(h->gsm.ensure(sizeof(int) * d.lsc * 3));
-  WS_ENSURE(h->ragg.ensure(sizeof(int) * d.raggc));
-  WS_ENSURE(h->ranges.ensure(sizeof(int64_t) * 6 * d.psc));
-  WS_ENSURE(h->od.ensure(real * d.odt));
-  WS_ENSURE(h->pwork.ensure(sizeof(int2) * (size_t)d.ctas));
-  WS_ENSURE(h->psegn.ensure(sizeof(int) * d.psc));
-  WS_ENSURE(h->psegs.ensure(sizeof(int) * kSegTab * d.psc));
-  WS_ENSURE(h->psegv.ensure(sizeof(double2) * kSegTab * d.psc));
-  WS_ENSURE(h->pxint.ensure(sizeof(XintPanel) * d.psc));
-  WS_ENSURE(h->r4.ensure(real * d.r4t));
-  WS_ENSURE(h->absrb.ensure(sizeof(double) * (kNABSRB + 8) * d.cnt));
-  WS_ENSURE(h->blockmax.ensure(sizeof(int) * d.smaxc));
-  WS_ENSURE(h->f4prep.ensure(sizeof(F4Prep) * d.fsc));
-  WS_ENSURE(h->f4sh.ensure(sizeof(ShrunkLine) * d.fsc));
-  WS_ENSURE(h->f4blk.ensure(sizeof(int64_t) * d.nblk4c));
-  WS_ENSURE(h->f4ntot.ensure(sizeof(int64_t) * d.cnt));
-  WS_ENSURE(h->f4mask.ensure(sizeof(unsigned) * (d.fsc / 32 + d.cnt)));
-  WS_ENSURE(h->f4cidx.ensure(sizeof(int64_t) * (d.fsc + d.cnt)));
-  WS_ENSURE(h->f4vb.ensure(sizeof(long long) * d.fsc));
-  WS_ENSURE(h->f4lb.ensure(sizeof(long long) * d.fsc));
-  WS_ENSURE(h->f4src.ensure(sizeof(int64_t) * d.fsc));
-  WS_ENSURE(h->f4flag.ensure(d.fsc));
-  WS_ENSURE(h->f4nxt.ensure(sizeof(int) * d.fsc));
-  WS_ENSURE(h->f4cut.ensure(sizeof(int64_t) * d.cnt));
-  WS_ENSURE(h->f4grp.ensure(sizeof(int4) * d.fsc));
-  WS_ENSURE(h->f4tab.ensure(sizeof(unsigned) * kCallEnds * d.frecc));
-  WS_ENSURE(h->f4calls.ensure(sizeof(int4) * (d.frecc + 2 * d.cnt)));
-  WS_ENSURE(h->f4ncall.ensure(sizeof(int2) * d.cnt));
-  WS_ENSURE(h->f4agg.ensure(sizeof(int) * 2 * d.f4aggc));
-  WS_ENSURE(h->f4rec.ensure(sizeof(F4Rec) * (d.fsc + 4096 * d.cnt)));
-  WS_ENSURE(h->f4recd.ensure(plain ? sizeof(F4RecD) * (d.fsc + 4096 * d.cnt) : 256));
-  WS_ENSURE(h->f4nrec.ensure(sizeof(int64_t) * nL));
-  WS_ENSURE(h->f4nmir.ensure(sizeof(int64_t) * nL));
-  WS_ENSURE(h->f4pm.ensure(sizeof(int) * (d.fsc + 4096 * d.cnt)));
-  WS_ENSURE(h->f4sm.ensure(sizeof(int) * (d.fsc + 4096 * d.cnt)));
-  WS_ENSURE(h->segpool.ensure(kSegPoolBytes));
-  WS_ENSURE(h->bfac.ensure(sizeof(double) * (kLIMOUT4 + 2) * (blkt + 1)));
-#undef WS_ENSURE
+  cudaError_t e = h->tabbuf.ensure(tab_layout(h, nL, vftt, blkt, isot));
+  if (e == cudaSuccess) e = h->segpool.ensure(kSegPoolBytes);
+  for (const WsPart& p : ws_parts(h, d, nL, blkt, plain))
+    if (e == cudaSuccess) e = p.buf->ensure(p.bytes);
   return e;
 }
 
-// The buffers ws_alloc sizes: scratch of one batch, nothing in them outlives it.
+// The buffers that ws_alloc sizes.
 std::vector<DevBuf*> ws_buffers(clblm_handle* h) {
-  return {&h->prep,   &h->qpanel,   &h->rec,    &h->recd,   &h->gpm,    &h->reclo,
-          &h->gsm,    &h->ragg,   &h->ranges, &h->od,       &h->r4,     &h->absrb,  &h->blockmax, &h->f4prep, &h->f4sh, &h->f4mask, &h->f4blk, &h->f4ntot, &h->f4cidx,
-          &h->f4vb,   &h->f4lb,   &h->f4src,  &h->f4flag,   &h->f4nxt,  &h->f4cut,  &h->f4grp,  &h->f4rec,
-          &h->f4recd, &h->f4nrec, &h->f4nmir, &h->f4pm,     &h->f4sm,   &h->segpool, &h->bfac,   &h->linecpl, &h->f4cpl, &h->f4cpll,
-          &h->f4ncpl, &h->pwork,  &h->f4tab,  &h->f4calls,  &h->f4ncall, &h->f4agg, &h->psegn,  &h->psegs,  &h->psegv, &h->pxint, &h->tabbuf};
+  std::vector<DevBuf*> v = {&h->tabbuf, &h->segpool};
+  for (const WsPart& p : ws_parts(h, WsDims{}, 0, 0, false)) v.push_back(p.buf);
+  return v;
 }
 
 // Frees every work buffer of the handle (all but the line list, the shape
@@ -2716,12 +2736,14 @@ int jac_plan_block(clblm_handle* h, const clblm_rt_ctrl_t* ctrl, const clblm_jac
   return CLBLM_OK;
 }
 
+// Scratch, OD slabs and maps of the blocks whose ODs clblm_gpu_jac forms
+// together, and their ODs (three rows of CTAs each in the line bounds' grid)
+constexpr size_t kJacGroupBytes = (size_t)24 << 30;
+constexpr int kJacGroupJobs = 65535 / 3;
+
 // The blocks of noScattJacob (clblm_noScattJac.f90:206-232): V1B, V2B and
 // the block length, which is the first layer's OD length (:227-229); the next
 // block starts one DVout after the block's last point.
-// workspace, OD slabs and maps of the blocks whose ODs clblm_gpu_jac forms together
-constexpr size_t kJacGroupBytes = (size_t)24 << 30;
-
 struct JacBlock {
   double v1, v2;
   int64_t n;
@@ -2946,7 +2968,13 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
   for (size_t b = 0; b < blocks.size(); ++b)
     if (nlims[b] != blocks[b].n) return set_err(h, CLBLM_ERR_GRID, "Jacobian block length changed");
   const size_t budget = od_batch_budget(h);
-  size_t limit = std::min(budget, kJacGroupBytes);  // of a group of blocks; 0: one block at a time
+  size_t limit = std::min(budget, kJacGroupBytes);  // of the groups of blocks; 0: one block at a time
+  std::vector<size_t> most;                         // bytes of each buffer in any group so far
+  auto total_of = [](const std::vector<size_t>& v) {
+    size_t b = 0;
+    for (size_t x : v) b += x;
+    return b;
+  };
   for (size_t ib = 0; ib < blocks.size();) {
     // blocks [ib, ie): their ODs, OD slabs and maps within the limit
     std::vector<int64_t> jod_off, map_off;
@@ -2955,13 +2983,23 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
     std::vector<double> vo;
     int64_t jods = 0, maps = 0, nlmax = 0;
     int njob = 0, bmax = 0;
-    size_t ie = ib, bytes = 0;
+    size_t ie = ib;
+    WsLayers layers;
+    std::vector<size_t> taken;
     for (; ie < blocks.size(); ++ie) {
       const int64_t nlim = nlims[ie];
-      size_t w = real * (size_t)js.nvar * nl * nlim + 8 * plans[ie].size() * (size_t)nlim;
-      for (const HostPlan& hp : plans[ie]) w += od_job_bytes(hp.P, plain);
-      if (ie > ib && bytes + w > limit) break;
-      bytes += w;
+      // what the call's buffers take with this block in the group, not the sum
+      // of the blocks': one with many lines lengthens every job's arrays, and a
+      // buffer keeps the most that a group has needed
+      for (const HostPlan& hp : plans[ie]) layers.add(hp);
+      std::vector<size_t> need = {real * (size_t)(jods + (int64_t)js.nvar * nl * nlim),
+                                  sizeof(int2) * (size_t)(maps + (int64_t)plans[ie].size() * nlim)};
+      for (const WsPart& p : ws_parts(h, layers.dims(), (int)layers.cnt, layers.blk, plain)) need.push_back(p.bytes);
+      most.resize(need.size(), 0);
+      for (size_t k = 0; k < need.size(); ++k) need[k] = std::max(need[k], most[k]);
+      if (ie > ib && (limit == 0 || layers.cnt > kJacGroupJobs || total_of(need) > std::max(limit, total_of(most))))
+        break;
+      taken = need;
       jod_off.push_back(jods);
       map_off.push_back(maps);
       job0.push_back(njob);
@@ -2986,6 +3024,7 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
       nblk.push_back((int)j1.size() - blk0.back());
       bmax = std::max(bmax, nblk.back());
     }
+    most = taken;
     // the blocks' ODs on the uniform grid, [variant][layer][point] each
     {  // (out of memory: the batch scratch and the block buffers, dead here, are freed, then once more)
       auto alloc = [&]() -> cudaError_t {
