@@ -2975,6 +2975,11 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
     for (size_t x : v) b += x;
     return b;
   };
+  // between groups and before a group's first batch nothing in these is live
+  auto release_group = [&] {
+    for (DevBuf* b : ws_buffers(h)) b->release();
+    for (DevBuf* b : {&h->jod, &h->jmap, &h->jjobs, &h->jblk}) b->release();
+  };
   for (size_t ib = 0; ib < blocks.size();) {
     // blocks [ib, ie): their ODs, OD slabs and maps within the limit
     std::vector<int64_t> jod_off, map_off;
@@ -3026,7 +3031,7 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
     }
     most = taken;
     // the blocks' ODs on the uniform grid, [variant][layer][point] each
-    {  // (out of memory: the batch scratch and the block buffers, dead here, are freed, then once more)
+    {  // (out of memory: the batch scratch and the block buffers are freed, then once more)
       auto alloc = [&]() -> cudaError_t {
         cudaError_t e = h->jod.ensure(real * (size_t)jods);
         if (e == cudaSuccess) e = h->jmap.ensure(sizeof(int2) * (size_t)maps);
@@ -3037,11 +3042,11 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
       cudaError_t e = alloc();
       if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
-        for (DevBuf* b : ws_buffers(h)) b->release();
-        for (DevBuf* b : {&h->jod, &h->jmap, &h->jjobs}) b->release();
+        release_group();
         e = alloc();
-        if (e == cudaErrorMemoryAllocation && ie - ib > 1) {  // one block at a time, as little as there is
+        if (e == cudaErrorMemoryAllocation && limit != 0) {  // one block at a time, as little as there is
           cudaGetLastError();
+          release_group();
           limit = 0;
           continue;
         }
@@ -3071,8 +3076,11 @@ int jac_impl(clblm_handle_t* h, const clblm_column_t* col, const clblm_rt_ctrl_t
       }
       int64_t ls, fs, ps, odt;
       rc = prepare_batch(h, hps, first, count, plain, &ls, &fs, &ps, &odt);
-      if (rc == CLBLM_ERR_OOM && ie - ib > 1 && first == 0) {  // one block at a time, as little as there is
+      if (rc == CLBLM_ERR_OOM && limit != 0 && first == 0) {
+        // one block at a time, as little as there is: without the slabs and
+        // maps of the group, or of a larger group before it
         cudaGetLastError();
+        release_group();
         shrink = true;
         break;
       }

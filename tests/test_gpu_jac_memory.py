@@ -1,8 +1,9 @@
 """Device memory of clblm_gpu_jac, whose blocks of a wide window share the OD
 pipeline's launches in groups: a group keeps to its bound where one block has
 many more lines than the others (the pipeline's arrays are as long as the
-largest job's, times the jobs), and neither the groups nor several OD batches of
-a block change the result."""
+largest job's, times the jobs), a device with little memory left gets one block
+at a time, and neither the groups nor several OD batches of a block change the
+result."""
 import os
 
 import numpy as np
@@ -85,3 +86,40 @@ def test_groups_and_batches_do_not_change_the_result(gpu_lib, budget, precision)
     for gb in (0.15, 0.004):
         for k in KEYS:
             np.testing.assert_array_equal(got[gb][k], got[16.0][k], err_msg="%s at %g GB" % (k, gb))
+
+
+# the slabs and maps of all blocks still fit, then not even they
+@pytest.mark.parametrize("part", [1.0, 0.5])
+def test_little_memory_left(gpu_lib, budget, part):
+    import torch
+    v1, v2 = 700.0, 2300.0
+    col, prof, cont = _column(v1, v2)
+    lines = _lines(v1, v2, 2.0)
+    ctrl = T.rt_ctrl(precision=T.CLBLM_PREC_MIXED, grid_type=1)
+    h = gpu_lib.Handle(lines, cont)
+    want = h.jac(col, ctrl, prof)  # (the kernels are loaded and have their local memory)
+    h.close()
+    n = len(want["rad"])
+    h = gpu_lib.Handle(lines, cont)
+    out = {k: torch.zeros(((col.nlay + 1, n) if k in ("dtlev", "dqlev") else n), dtype=torch.float64, device="cuda")
+           for k in KEYS}
+    budget(8.0)  # the least that a call plans with whatever is free
+    # room for `part` of the OD slabs and maps of all blocks (16 and 32 bytes a
+    # layer and point, an eighth more for growth), and 0.15 GB
+    slabs = 48 * col.nlay * n * 9 // 8
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    fill = free - int(part * slabs) - int(0.15 * 2**30)
+    assert slabs > 2**30 and fill > 0
+    block = torch.empty(fill, dtype=torch.uint8, device="cuda")
+    try:
+        h.jac_device(col, ctrl, prof, out["rad"].data_ptr(), out["dtlev"].data_ptr(), out["dqlev"].data_ptr(),
+                     out["dtsfc"].data_ptr(), out["demis"].data_ptr(), n)
+        torch.cuda.synchronize()
+    finally:
+        del block
+        torch.cuda.empty_cache()
+        h.close()
+    for k in KEYS:
+        np.testing.assert_array_equal(out[k].cpu().numpy(), want[k], err_msg=k)
