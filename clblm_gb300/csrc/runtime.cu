@@ -52,8 +52,12 @@ struct DevBuf {
     g_buf_gen++;
     size_t want = n + n / 8 + 256;
     cudaError_t e = cudaMalloc(&p, want);
-    if (e == cudaSuccess) bytes = want;
-    else p = nullptr;
+    if (e == cudaSuccess) {
+      bytes = want;
+    } else {
+      p = nullptr;
+      cudaGetLastError();  // the status is returned: the next launch's check is not to find it
+    }
     return e;
   }
   void release() {
@@ -88,8 +92,12 @@ struct PinBuf {
     release();
     const size_t want = n + n / 4 + 4096;
     const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&p), want, cudaHostAllocDefault);
-    if (e == cudaSuccess) bytes = want;
-    else p = nullptr;
+    if (e == cudaSuccess) {
+      bytes = want;
+    } else {
+      p = nullptr;
+      cudaGetLastError();
+    }
     return e;
   }
   void release() {

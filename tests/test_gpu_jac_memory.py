@@ -123,3 +123,32 @@ def test_little_memory_left(gpu_lib, budget, part):
         h.close()
     for k in KEYS:
         np.testing.assert_array_equal(out[k].cpu().numpy(), want[k], err_msg=k)
+
+
+def test_call_after_an_out_of_memory_result(gpu_lib, budget):
+    """A call that returns out of memory leaves no error behind: neither the
+    next call of the handle nor another library's check finds it."""
+    import torch
+    col, prof, cont = _column(1000.0, 1004.0)
+    lines = _lines(1000.0, 1004.0, 60.0)
+    ctrl = T.rt_ctrl(precision=T.CLBLM_PREC_MIXED, grid_type=1)
+    h = gpu_lib.Handle(lines, cont)
+    want = h.jac(col, ctrl, prof)
+    h.close()
+    h = gpu_lib.Handle(lines, cont)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    block = torch.empty(free - int(0.1 * 2**30), dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(gpu_lib.ClblmError) as e:
+            h.jac(col, ctrl, prof)
+        assert e.value.code == T.CLBLM_ERR_OOM
+        torch.cuda.synchronize()
+    finally:
+        del block
+        torch.cuda.empty_cache()
+    got = h.jac(col, ctrl, prof)
+    h.close()
+    for k in KEYS:
+        np.testing.assert_array_equal(got[k], want[k], err_msg=k)
