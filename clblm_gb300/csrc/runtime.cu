@@ -1010,6 +1010,10 @@ size_t od_batch_budget(clblm_handle* h, size_t need = ~(size_t)0) {
   return b < lo ? lo : (b > hi ? hi : b);
 }
 
+// layers that the far-wing variants are timed on (the ODs of one block of a
+// 60-layer column's Jacobians, enough to fill the GPU)
+constexpr int kTuneLayers = 240;
+
 // The fastest of n launch variants on the work at hand: each variant runs once
 // to warm up and once timed on `st`.  The launches must be repeatable (they
 // do not write what they read).  While `st` is being captured into a graph
@@ -1239,20 +1243,24 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
       if (plain) k_f4_far<true><<<grid, kFarThreads, 0, st>>>(fa);
       else k_f4_far<false><<<grid, kFarThreads, 0, st>>>(fa);
     } else {
-      const dim3 grid((unsigned)((maxr4 + 2 + kF4Tile - 1) / kF4Tile), count);
-      auto f4 = [&](int v) {  // records per stage: 64, 128, 256
+      const unsigned tiles = (unsigned)((maxr4 + 2 + kF4Tile - 1) / kF4Tile);
+      auto f4 = [&](int v, int layers) {  // records per stage: 64, 128, 256
+        const dim3 grid(tiles, (unsigned)layers);
         if (v == 0) k_f4_conv<64><<<grid, kF4Threads, 0, st>>>(fa);
         else if (v == 1) k_f4_conv<128><<<grid, kF4Threads, 0, st>>>(fa);
         else k_f4_conv<256><<<grid, kF4Threads, 0, st>>>(fa);
       };
       int tv = h->tune.f4[0];
       if (tv < 0) {
-        int rc = tune_pick(h, st, 3, 2, f4, &h->tune.f4[0], &tv);
+        // (on some of the layers: six launches over the 3600 of a 60-layer 500
+        // cm-1 Jacobian were 57 ms beside a call of 71, over 240 they are 4)
+        const int some = std::min(count, kTuneLayers);
+        int rc = tune_pick(h, st, 3, 2, [&](int v) { f4(v, some); }, &h->tune.f4[0], &tv);
         if (rc) return rc;
       }
       h->launches++;
       CUDA_TRY(h, cudaEventRecord(h->ev[0], st));
-      f4(tv);
+      f4(tv, count);
     }
     if (h->has_cpl) {  // the coupled records' dispersion terms
       h->launches += 2;
