@@ -116,7 +116,7 @@ struct BatchGraph;
 // work; none of them changes a result (each variant computes every value
 // with the same operations in the same order).  -1: not chosen yet.
 struct Tuner {
-  int f4[2] = {-1, -1};   // k_f4_conv records per stage: 64 / 128 / 256 (index), per precision
+  int f4 = -1;            // k_f4_conv records per stage: 64 / 128 / 256 (index); the mixed path alone
   int rt[2] = {-1, -1};   // k_rt_segment threads per block: 128 / 256 / 512
   int jac[2] = {-1, -1};  // k_jac threads per block: 64 / 128
   bool on = true;         // CLBLM_AUTOTUNE=0: the defaults, no timing
@@ -1250,12 +1250,12 @@ int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int cou
         else if (v == 1) k_f4_conv<128><<<grid, kF4Threads, 0, st>>>(fa);
         else k_f4_conv<256><<<grid, kF4Threads, 0, st>>>(fa);
       };
-      int tv = h->tune.f4[0];
+      int tv = h->tune.f4;
       if (tv < 0) {
         // (on some of the layers: six launches over the 3600 of a 60-layer 500
         // cm-1 Jacobian were 57 ms beside a call of 71, over 240 they are 4)
         const int some = std::min(count, kTuneLayers);
-        int rc = tune_pick(h, st, 3, 2, [&](int v) { f4(v, some); }, &h->tune.f4[0], &tv);
+        int rc = tune_pick(h, st, 3, 2, [&](int v) { f4(v, some); }, &h->tune.f4, &tv);
         if (rc) return rc;
       }
       h->launches++;
@@ -1803,7 +1803,7 @@ int clblm_gpu_create(const clblm_lines_t* lines, const clblm_cont_t* cont, int d
   if (const char* e = std::getenv("CLBLM_F4_STAGE_RECORDS")) {
     const int v = std::atoi(e);
     for (int k = 0; k < 3; ++k)
-      if (kF4StageRecords[k] == v) h->tune.f4[0] = h->tune.f4[1] = k;
+      if (kF4StageRecords[k] == v) h->tune.f4 = k;
   }
   for (auto& e : h->ev) {
     if (cudaEventCreate(&e) != cudaSuccess) {
@@ -2171,8 +2171,9 @@ int clblm_gpu_od_stats(const clblm_handle_t* h, clblm_od_stats_t* stats) {
   if (!h || !stats) return CLBLM_ERR_ARG;
   *stats = h->last;
   const int p = h->last_plain ? 1 : 0;
-  // (a call without k_f4_conv leaves the choice open: its default shape)
-  stats->f4_stage_records = h->tune.f4[p] >= 0 ? kF4StageRecords[h->tune.f4[p]] : (h->last.launches > 0 ? kF4StageRecords[2] : 0);
+  // (calls without k_f4_conv leave the choice open: the default until it is made)
+  const int f4 = h->tune.f4 >= 0 ? h->tune.f4 : 2;
+  stats->f4_stage_records = h->tune.f4 >= 0 || h->last.launches > 0 ? kF4StageRecords[f4] : 0;
   stats->rt_threads = h->tune.rt[p] >= 0 ? kRtThreads[h->tune.rt[p]] : 0;
   stats->jac_threads = h->tune.jac[p] >= 0 ? kJacThreads[h->tune.jac[p]] : 0;
   return CLBLM_OK;

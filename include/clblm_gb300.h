@@ -227,7 +227,10 @@ typedef struct {
   double  ms_f4_chain;  /* batch start to the end of the far-wing chain (stream 2) */
   /* launch shapes the autotuner chose for the handle (0: not chosen yet); no
    * choice changes a result.  CLBLM_AUTOTUNE=0 in the environment keeps the
-   * defaults (256, 256, 128). */
+   * defaults (256, 256, 128).  The far-wing stages are those of the ODs of
+   * mixed Jacobian and batch calls, the first of which chooses; the other calls
+   * launch a kernel without stages, and after them the field holds the handle's
+   * size (chosen, set by CLBLM_F4_STAGE_RECORDS, or the default). */
   int32_t f4_stage_records; /* far-wing records per shared-memory stage     */
   int32_t rt_threads;       /* threads per block of the layer recurrence     */
   int32_t jac_threads;      /* threads per block of the Jacobian recurrence  */
