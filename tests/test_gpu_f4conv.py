@@ -1,5 +1,7 @@
 """k_f4_conv, which sums the far wings of mixed Jacobians' ODs record by record
-through shared-memory stages: no stage size changes a Jacobian by a bit."""
+through shared-memory stages: no stage size changes a Jacobian by a bit, and
+the mirror records of lines near 0 cm-1, which follow the direct ones through
+the stages, are the oracle's."""
 import os
 
 import numpy as np
@@ -44,3 +46,24 @@ def test_stage_size_does_not_change_a_jacobian(gpu_lib, mtckd, window):
     for stage in (64, 128, 256):
         for k in KEYS:
             np.testing.assert_array_equal(got[stage][k], got[0][k], err_msg="%s at %d records" % (k, stage))
+
+
+def test_mixed_jacobian_with_mirror_records(gpu_lib, oracle_mod):
+    """A mixed Jacobian below 25 cm-1, where the mirror records of the lines
+    near 0 follow the direct ones through k_f4_conv's stages (hundreds of them,
+    several stages): the far wings against the FP64 oracle's, at the
+    repository's tolerances for Jacobians."""
+    lines = synth.line_list(9000, 1.0, 70.0, seed=7, mols=synth.SEVEN)
+    _, col, _ = synth.config1(n_lines=10)
+    c = col.sub([20, 21]).with_window(3.0, 9.0)
+    prof = synth.jac_profile(col).sub(20, 2)
+    ctrl = T.rt_ctrl(precision=T.CLBLM_PREC_MIXED, grid_type=1, contnm_off=1)
+    h = gpu_lib.Handle(lines, None)
+    got = h.jac(c, ctrl, prof)
+    h.close()
+    want = oracle_mod.jac_mode2(oracle_mod.Session(), lines, c, ctrl, prof, None)
+    assert len(got["rad"]) == len(want["rad"]) and got["dv"] == want["dv"]
+    np.testing.assert_allclose(got["rad"], want["rad"], rtol=1e-4)
+    for k in ("dtlev", "dqlev", "dtsfc", "demis"):
+        scale = np.max(np.abs(want[k]), axis=-1, keepdims=True)
+        assert np.max(np.abs(got[k] - want[k]) / np.where(scale > 0, scale, 1.0)) <= 2e-3, k
