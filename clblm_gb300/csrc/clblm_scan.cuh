@@ -23,6 +23,7 @@ struct ScanArgs {
   double edge_v[kScanMaxEdges];
   int deconv;         // 1: divide by the pre-boxing's transform, Z / sin(Z)
   double deconv_a;    // its width parameter (the boxed DV)
+  double floor;       // k_scan_low: the apodization's value past the coefficients it forms
 };
 
 __global__ void k_scan_load(const double* s, int64_t off, int64_t ltotal, int M, int64_t ktotal, double fill,
@@ -49,10 +50,17 @@ template <int Terms>
 __global__ void __launch_bounds__(32 * Terms / 2)
     k_scan_low(ScanArgs a, double fill_n, double scale, int64_t K, int64_t M, int R, const double2* __restrict__ X,
                const double2* __restrict__ W, double2* __restrict__ Z);
-template <int Terms>
+// the data that k_scan_expand adds the apodization's floor of
+struct ScanFloor {
+  double floor, fill;
+  const double* s;
+  int64_t off, n;  // first point of the data in s; points (means) of them
+  int boxed;
+};
+template <int Terms, bool Floor>
 __global__ void __launch_bounds__(kScanLowThreads)
     k_scan_expand(const double2* __restrict__ y, int64_t M, int B, int64_t first, int64_t count,
-                  double* __restrict__ out);
+                  double* __restrict__ out, ScanFloor f);
 __global__ void k_scan_out(const double* y, int64_t first, int64_t count, double scale, double* out);
 
 }  // namespace clblm

@@ -4205,10 +4205,15 @@ int clblm_gpu_fftscn(clblm_handle_t* h, const clblm_scan_t* scan, const double* 
   };
   // An apodization that ends (functions 3 to 10 at 1/A; the Gaussian where its
   // floor e^-34 = 2e-15 begins) at a small part of the transform's path
-  // differences: the first K coefficients alone, through M-point transforms
+  // differences: the first K coefficients alone, through M-point transforms.
+  // The Gaussian's floor of the others is that of the data, added at the
+  // scanned points, but not where it is no constant (deconvolved: Z / sin(Z)
+  // grows past the first K) nor onto an output that lies over the data
   int64_t K = 0, M = 0;
   bool wide = false;
-  if (p.ivx == 1 && p.jfn >= 2 && p.jfn <= 10) {
+  const bool floored = p.jfn == 2;
+  const bool over = dscan < din + p.n1 - 1 + p.ltotal && din + p.n1 - 1 < dscan + p.ntotal;
+  if (p.ivx == 1 && p.jfn >= 2 && p.jfn <= 10 && !(floored && (p.deconv || over))) {
     const double end = p.jfn == 2 ? std::sqrt(17.) / (3.141592653589793 * p.A) : 1. / p.A;
     if (end / a.DX < 1.e9) K = (int64_t)(end / a.DX) + 3;
     for (int e = 0; e < a.nedge; ++e) K = std::max<int64_t>(K, a.edge_k[e] + 1);
@@ -4249,7 +4254,10 @@ int clblm_gpu_fftscn(clblm_handle_t* h, const clblm_scan_t* scan, const double* 
     h->launches += own ? 5 : 3;
     auto moments = wide ? k_scan_moments<kScanTermsWide> : k_scan_moments<kScanTerms>;
     auto coefs = wide ? k_scan_low<kScanTermsWide> : k_scan_low<kScanTerms>;
-    auto expand = wide ? k_scan_expand<kScanTermsWide> : k_scan_expand<kScanTerms>;
+    auto expand = wide ? (floored ? k_scan_expand<kScanTermsWide, true> : k_scan_expand<kScanTermsWide, false>)
+                       : (floored ? k_scan_expand<kScanTerms, true> : k_scan_expand<kScanTerms, false>);
+    a.floor = floored ? std::exp(-34.) : 0.;
+    const ScanFloor fl = {a.floor, scan->padding, din, p.n1 - 1, pts, p.M};
     moments<<<ctas(M / 4), kScanLowThreads, 0, st>>>(din, p.n1 - 1, p.ltotal, p.M, p.ktotal, scan->padding, Z,
                                                             nblk, B, M, own ? W : nullptr);
     CUDA_TRY(h, cudaGetLastError());
@@ -4279,7 +4287,7 @@ int clblm_gpu_fftscn(clblm_handle_t* h, const clblm_scan_t* scan, const double* 
                             reinterpret_cast<cufftDoubleComplex*>(X), CUFFT_INVERSE) != CUFFT_SUCCESS) {
       return set_err(h, CLBLM_ERR_CUDA, "FFTSCN: inverse transform");
     }
-    expand<<<ctas(p.ntotal / B + 2), kScanLowThreads, 0, st>>>(X, M, B, p.N1 - 1, p.ntotal, dscan);
+    expand<<<ctas(p.ntotal / B + 2), kScanLowThreads, 0, st>>>(X, M, B, p.N1 - 1, p.ntotal, dscan, fl);
     CUDA_TRY(h, cudaGetLastError());
   } else {
     // transform buffer: N reals, in place as N/2+1 complex

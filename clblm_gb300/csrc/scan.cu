@@ -38,6 +38,13 @@
 //   k_scan_expand      sum_p t^p Y_p(b) at the scanned points
 // The spectrum is read once and the scanned points written once; a 2^23-point
 // scan took 2.0 ms, nearly all of it in the transforms' passes over memory.
+// The Gaussian does not reach zero: its exponent stops at -34, so that every
+// coefficient past K keeps e^-34 = 1.7e-15 of itself.  The transforms carry the
+// Gaussian less that floor and k_scan_expand adds the floor times the data (the
+// Nyquist coefficient, which the reference drops, with them: below the rounding
+// of a transform): 790 -> 798 us for 2,000,000 points, 2070 -> 2140 us for
+// 7,000,000.  Deconvolved, where the floor is not a constant, the whole transform
+// serves.
 #include <cuda_runtime.h>
 
 #include "clblm_scan.cuh"
@@ -215,6 +222,14 @@ __global__ void k_scan_mulnum(const double2* __restrict__ H, int64_t nhalf, doub
   }
 }
 
+// point i of the data: the spectrum's own or, pre-boxed, the mean of `boxed`
+__device__ __forceinline__ double scan_point(const double* __restrict__ s, int64_t off, int boxed, int64_t i) {
+  if (boxed <= 1) return s[off + i];
+  double sum = 0.0;
+  for (int m = 0; m < boxed; ++m) sum = __dadd_rn(sum, s[off + i * boxed + m]);
+  return __ddiv_rn(sum, (double)boxed);
+}
+
 // t_j^(2q) of a block's lower half (q = 0: t itself) in shared memory
 __device__ __forceinline__ void scan_powers(int B, double (*T)[kScanPowers], int n) {
   const double rh = 2. / (double)B, c = 0.5 * (double)(B - 1);
@@ -250,10 +265,8 @@ __global__ void __launch_bounds__(kScanLowThreads)
   const int64_t n = boxed <= 1 ? ltotal : ktotal;
   auto value = [&](int64_t i) -> double {  // less FILL, which reaches k = 0 alone
     if (i >= n) return 0.;
-    if (boxed <= 1) return fill != 0. ? __dadd_rn(s[off + i], -fill) : s[off + i];
-    double sum = 0.0;
-    for (int m = 0; m < boxed; ++m) sum = __dadd_rn(sum, s[off + i * boxed + m]);
-    return __dadd_rn(__ddiv_rn(sum, (double)boxed), -fill);
+    const double x = scan_point(s, off, boxed, i);
+    return fill != 0. ? __dadd_rn(x, -fill) : x;
   };
   const double rh = 2. / (double)B, c = 0.5 * (double)(B - 1);
   // (whole warps: the last one's spare groups take block M - 1 again)
@@ -464,7 +477,7 @@ __global__ void __launch_bounds__(32 * Terms / 2)
     if (k == 0) wr += fill_n;
     const int64_t j = k / kScanHalf, kk = k - j * kScanHalf;
     const double xd = __dadd_rn(a.X0[j], __dmul_rn((double)kk, a.DX));
-    double h = apod(a.jfn, xd, a.A);
+    double h = apod(a.jfn, xd, a.A) - a.floor;  // (k_scan_expand adds the floor)
     for (int e = 0; e < a.nedge; ++e)
       if (k == a.edge_k[e]) h = a.edge_v[e];
     wr *= h;
@@ -487,11 +500,13 @@ __global__ void __launch_bounds__(32 * Terms / 2)
 
 // The scanned points [first, first + count): a warp per block, a lane per
 // pair of opposite points (13 FP64 instructions a pair bound it; 42 -> 33 us
-// with t from a table and the scale in the coefficients)
-template <int Terms>
+// with t from a table and the scale in the coefficients).  Floor: the
+// apodization's value at every coefficient that the transforms leave out, which
+// multiplies the data themselves (FILL past them).
+template <int Terms, bool Floor>
 __global__ void __launch_bounds__(kScanLowThreads)
     k_scan_expand(const double2* __restrict__ y, int64_t M, int B, int64_t first, int64_t count,
-                  double* __restrict__ out) {
+                  double* __restrict__ out, ScanFloor f) {
   __shared__ double T[2][kScanPowers];
   const bool table = B / 2 <= kScanPowers;
   if (table) scan_powers(B, T, 2);
@@ -513,8 +528,12 @@ __global__ void __launch_bounds__(kScanLowThreads)
       }
       o *= t;
       const int64_t i0 = b * B + j - first, i1 = b * B + B - 1 - j - first;
-      if (i0 >= 0 && i0 < count) out[i0] = e + o;
-      if (i1 >= 0 && i1 < count) out[i1] = e - o;
+      auto floor = [&](int64_t i) -> double {
+        if constexpr (!Floor) return 0.;
+        else return f.floor * (i + first < f.n ? scan_point(f.s, f.off, f.boxed, i + first) : f.fill);
+      };
+      if (i0 >= 0 && i0 < count) out[i0] = Floor ? e + o + floor(i0) : e + o;
+      if (i1 >= 0 && i1 < count) out[i1] = Floor ? e - o + floor(i1) : e - o;
     }
   }
 }
@@ -523,14 +542,18 @@ template __global__ void k_scan_moments<kScanTerms>(const double* __restrict__, 
                                              double2* __restrict__, int64_t, int, int64_t, double2* __restrict__);
 template __global__ void k_scan_low<kScanTerms>(ScanArgs, double, double, int64_t, int64_t, int, const double2* __restrict__,
                                          const double2* __restrict__, double2* __restrict__);
-template __global__ void k_scan_expand<kScanTerms>(const double2* __restrict__, int64_t, int, int64_t, int64_t,
-                                            double* __restrict__);
+template __global__ void k_scan_expand<kScanTerms, false>(const double2* __restrict__, int64_t, int, int64_t, int64_t,
+                                                   double* __restrict__, ScanFloor);
+template __global__ void k_scan_expand<kScanTerms, true>(const double2* __restrict__, int64_t, int, int64_t, int64_t,
+                                                   double* __restrict__, ScanFloor);
 template __global__ void k_scan_moments<kScanTermsWide>(const double* __restrict__, int64_t, int64_t, int, int64_t, double,
                                              double2* __restrict__, int64_t, int, int64_t, double2* __restrict__);
 template __global__ void k_scan_low<kScanTermsWide>(ScanArgs, double, double, int64_t, int64_t, int, const double2* __restrict__,
                                          const double2* __restrict__, double2* __restrict__);
-template __global__ void k_scan_expand<kScanTermsWide>(const double2* __restrict__, int64_t, int, int64_t, int64_t,
-                                            double* __restrict__);
+template __global__ void k_scan_expand<kScanTermsWide, false>(const double2* __restrict__, int64_t, int, int64_t, int64_t,
+                                                   double* __restrict__, ScanFloor);
+template __global__ void k_scan_expand<kScanTermsWide, true>(const double2* __restrict__, int64_t, int, int64_t, int64_t,
+                                                   double* __restrict__, ScanFloor);
 template __global__ void k_scan_fft<false>(const double2* __restrict__, double2* __restrict__, const double2* __restrict__,
                                           int64_t, int64_t, int);
 template __global__ void k_scan_fft<true>(const double2* __restrict__, double2* __restrict__, const double2* __restrict__,
