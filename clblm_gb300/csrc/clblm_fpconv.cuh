@@ -171,4 +171,17 @@ CLBLM_HD bool less_bits(double a, double b) {
 }
 CLBLM_HD bool zero_bits(double x) { return (fpc_bits(x) << 1) == 0; }
 
+#ifdef __CUDACC__
+// 1/x of a positive normal double: the hardware's approximation (PTX
+// rcp.approx.ftz.f64), then one step of the cubic iteration y (1 + e + e^2),
+// e = 1 - x y (Householder's method of order two): within a unit in the last
+// place
+__device__ __forceinline__ double rcp_d(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+#endif
+
 }  // namespace clblm

@@ -6,19 +6,18 @@
 // to either side, 976 at a 0.1 hPa layer, so a column's upper layers sum some
 // 6000 records at each point.  Away from the line a record's term
 // SIL / (AL2 + x^2) plus its pedestal (a parabola) is smooth on the scale of
-// its distance: on a leaf of 32 points it is a polynomial through NP of them
-// to 4e-8 (NP = 10, from 48 points away; mixed path, below its FP32 rounding)
-// or 4e-15 (NP = 16, from 64 away; FP64 path), and likewise on a tile of 128
-// points from four times those distances.  A CTA of four warps takes a tile, a
-// warp a leaf:
+// its distance: on a leaf of 32 points, and on a tile of 128 from four times
+// the distance, it is a polynomial through NP of them to the path's rounding
+// (clblm_f4nodes.cuh).  A CTA of four warps takes a tile, a warp a leaf:
 //   - records that keep DB away from the tile and reach all of it: at the
 //     tile's NP nodes, a record per lane, shared out among the warps;
 //   - the others that keep D away from the leaf and reach all of it: at the
 //     leaf's NP nodes, a record per lane;
 //   - the rest (near the leaf, or ending inside it): at its 32 points, one per
 //     lane, the records passing through shared memory.
-// With R = 976 that is 422 evaluations per unit of record density and point
-// instead of 1928.  Node sums are carried to the points in binary64.  The
+// With R = 976 that is 422 evaluations (FP64 path: 690) per unit of record
+// density and point instead of 1928.  Node sums are carried to the points
+// in binary64 (compensated on the FP64 path).  The
 // index ranges come from the running bounds of the records' centres (their
 // order is nearly that of their centres): searches, one per lane.
 //
@@ -31,6 +30,8 @@
 #include <type_traits>
 
 #include "clblm_common.cuh"
+#include "clblm_f4nodes.cuh"
+#include "clblm_fpconv.cuh"
 #include "clblm_kernels.cuh"
 #include "clblm_panel.cuh"
 
@@ -38,79 +39,16 @@ namespace clblm {
 
 namespace {
 
-constexpr int kLeaf = 32, kTileLeaves = kFarTile / kLeaf;
-static_assert(32 * kTileLeaves == kFarThreads, "a warp per leaf");
+constexpr int kLeaf = kFarLeaf, kTileLeaves = kFarTile / kLeaf;
+static_assert(kFarTile == kFarTilePts && 32 * kTileLeaves == kFarThreads, "a warp per leaf");
 
-template <bool Plain>
-struct Far;
-template <>
-struct Far<false> {
-  static constexpr int NP = 10, D = 48;
-};
-template <>
-struct Far<true> {
-  static constexpr int NP = 16, D = 64;
-};
-
-// nodes: the Chebyshev points of the leaf and of the tile, rounded to points
-__host__ __device__ constexpr int far_node(bool plain, bool tile, int k) {
-  constexpr int l10[10] = {0, 2, 5, 8, 13, 18, 23, 26, 29, 31};
-  constexpr int t10[10] = {1, 7, 19, 35, 54, 73, 92, 108, 120, 126};
-  constexpr int l16[16] = {0, 1, 2, 4, 6, 8, 11, 14, 17, 20, 23, 25, 27, 29, 30, 31};
-  constexpr int t16[16] = {0, 3, 7, 14, 23, 34, 45, 57, 70, 82, 93, 104, 113, 120, 124, 127};
-  return plain ? (tile ? t16[k] : l16[k]) : (tile ? t10[k] : l10[k]);
-}
-
-// weights of the NP nodes at each point (Lagrange)
-template <bool Plain>
-struct FarWeights {
-  double leaf[Far<Plain>::NP][kLeaf], tile[Far<Plain>::NP][kFarTile];
-};
-template <bool Plain>
-constexpr FarWeights<Plain> far_weights() {
-  constexpr int NP = Far<Plain>::NP;
-  FarWeights<Plain> w{};
-  for (int k = 0; k < NP; ++k) {
-    for (int i = 0; i < kLeaf; ++i) {
-      double v = 1.;
-      for (int j = 0; j < NP; ++j)
-        if (j != k)
-          v *= (double)(i - far_node(Plain, false, j)) / (double)(far_node(Plain, false, k) - far_node(Plain, false, j));
-      w.leaf[k][i] = v;
-    }
-    for (int i = 0; i < kFarTile; ++i) {
-      double v = 1.;
-      for (int j = 0; j < NP; ++j)
-        if (j != k)
-          v *= (double)(i - far_node(Plain, true, j)) / (double)(far_node(Plain, true, k) - far_node(Plain, true, j));
-      w.tile[k][i] = v;
-    }
-  }
-  return w;
-}
-__device__ const FarWeights<false> c_farw_mixed = far_weights<false>();
-__device__ const FarWeights<true> c_farw_plain = far_weights<true>();
-template <bool Plain>
-__device__ __forceinline__ double far_w(bool tile, int k, int i) {
-  if constexpr (Plain) return tile ? c_farw_plain.tile[k][i] : c_farw_plain.leaf[k][i];
-  else return tile ? c_farw_mixed.tile[k][i] : c_farw_mixed.leaf[k][i];
-}
+__device__ const FarWeights c_farw_mixed = far_weights();
+__device__ const FarPairs c_farw_plain = far_pairs();
 
 __device__ __forceinline__ float rcp_f(float x) {  // PTX rcp.approx: relative error < 2^-23
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
-}
-
-// 1/x of a positive normal double: the hardware's approximation (PTX
-// rcp.approx.ftz.f64), then one step of the cubic iteration y (1 + e + e^2),
-// e = 1 - x y (Householder's method of order two): within a unit in the last
-// place
-__device__ __forceinline__ double rcp_d(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
 }
 
 struct SumK {  // compensated FP32 sum
@@ -494,14 +432,25 @@ __global__ void __launch_bounds__(kFarThreads, Plain ? 4 : 6) k_f4_far(const __g
   // the reference's R4 is zero past NPTR4 (LBLF4Q :91-94)
   double v = 0.;
   if (m < P.nptr4) {
+    if constexpr (Plain) {
+      FarSum f;
 #pragma unroll
-    for (int k = 0; k < NP; ++k) {
-      const double b = (nodeB[0][k] + nodeB[1][k]) + (nodeB[2][k] + nodeB[3][k]);
-      v = fma(far_w<Plain>(true, k, kLeaf * warp + lane), b, v);
-      v = fma(far_w<Plain>(false, k, lane), nodeA[warp][k], v);
+      for (int k = 0; k < NP; ++k) {
+        const double b = (nodeB[0][k] + nodeB[1][k]) + (nodeB[2][k] + nodeB[3][k]);
+        f.add(c_farw_plain.tile[k][kLeaf * warp + lane], b);
+        f.add(c_farw_plain.leaf[k][lane], nodeA[warp][k]);
+      }
+      f.add(acc);
+      v = f.value();
+    } else {
+#pragma unroll
+      for (int k = 0; k < NP; ++k) {
+        const double b = (nodeB[0][k] + nodeB[1][k]) + (nodeB[2][k] + nodeB[3][k]);
+        v = fma(c_farw_mixed.tile[k][kLeaf * warp + lane], b, v);
+        v = fma(c_farw_mixed.leaf[k][lane], nodeA[warp][k], v);
+      }
+      v += acc.value();
     }
-    if constexpr (Plain) v += acc;
-    else v += acc.value();
   }
   R4[m] = (Real)v;
 }
