@@ -7,13 +7,13 @@
 //   mixed path   NP = 10, D = 48: 3.9e-8 of a term, below its FP32 rounding
 //   FP64 path    NP = 16, D = 80: 1.8e-16 of a term from the leaf, 3.1e-16 from
 //                the tile (D = 64: 3.5e-15 and 6.2e-15).  The weights of the
-//                polynomial (they add up to 1, their magnitudes to 3) stand as
-//                pairs of doubles and the sums over the nodes are compensated:
-//                in plain doubles those alone were 1.2e-15 of a term.  Against
-//                sums of the terms themselves, in record order, the error of a
-//                point is as large for one to five records (1.2e-16 rms) and a
-//                fifth of it for 300; the FP64 operations it takes are a
-//                thirtieth of the kernel's.
+//                polynomial (they add up to 1, their magnitudes to 3) are rounded
+//                once (factor by factor they were off by 3e-16 and 6e-16 of a
+//                term) and carry the sums' differences from one node's, a third
+//                of the rounding of the sums themselves.  Against the terms added
+//                at the point, in record order, the error of a point is 1.3e-16
+//                rms for one to five records (1.2e-16), 1.1e-16 for 30 (1.7e-16)
+//                and 1.0e-16 for 300 (4.9e-16).
 #pragma once
 
 #ifdef __CUDACC__
@@ -49,65 +49,51 @@ constexpr int far_node(bool plain, bool tile, int k) {
   return plain ? (tile ? t16[k] : l16[k]) : (tile ? t10[k] : l10[k]);
 }
 
-// weights of the NP nodes at each point (Lagrange), mixed path
-struct FarWeights {
-  double leaf[Far<false>::NP][kFarLeaf], tile[Far<false>::NP][kFarTilePts];
-};
-constexpr FarWeights far_weights() {
-  constexpr int NP = Far<false>::NP;
-  FarWeights w{};
-  for (int k = 0; k < NP; ++k) {
-    for (int i = 0; i < kFarLeaf; ++i) {
-      double v = 1.;
-      for (int j = 0; j < NP; ++j)
-        if (j != k)
-          v *= (double)(i - far_node(false, false, j)) /
-               (double)(far_node(false, false, k) - far_node(false, false, j));
-      w.leaf[k][i] = v;
-    }
-    for (int i = 0; i < kFarTilePts; ++i) {
-      double v = 1.;
-      for (int j = 0; j < NP; ++j)
-        if (j != k)
-          v *= (double)(i - far_node(false, true, j)) / (double)(far_node(false, true, k) - far_node(false, true, j));
-      w.tile[k][i] = v;
-    }
-  }
-  return w;
-}
-
-// the same, FP64 path, each the sum of two doubles
+// a * b as the sum of two doubles (Veltkamp's split, Dekker's product)
 struct FarPair {
   double hi, lo;
 };
-struct FarPairs {
-  FarPair leaf[Far<true>::NP][kFarLeaf], tile[Far<true>::NP][kFarTilePts];
-};
-// a * b as the sum of two doubles (Veltkamp's split, Dekker's product)
 constexpr FarPair far_product(double a, double b) {
   const double s = 134217729.;  // 2^27 + 1
   const double a1 = s * a - (s * a - a), a2 = a - a1, b1 = s * b - (s * b - b), b2 = b - b1, p = a * b;
   return {p, ((a1 * b1 - p) + a1 * b2 + a2 * b1) + a2 * b2};
 }
-constexpr FarPair far_pair(bool tile, int k, int i) {
-  // numerator and denominator exactly: products of 15 factors below 2^7
-  __int128 num = 1, den = 1;
-  for (int j = 0; j < Far<true>::NP; ++j)
-    if (j != k) {
-      num *= i - far_node(true, tile, j);
-      den *= far_node(true, tile, k) - far_node(true, tile, j);
-    }
-  const double nh = (double)num, nl = (double)(num - (__int128)nh);
-  const double dh = (double)den, dl = (double)(den - (__int128)dh);
-  const double q = nh / dh;
-  const FarPair p = far_product(q, dh);
-  return {q, ((nh - p.hi) - p.lo + nl - q * dl) / dh};
+// weight of node k at point i (Lagrange)
+template <bool Plain>
+constexpr double far_weight(bool tile, int k, int i) {
+  constexpr int NP = Far<Plain>::NP;
+  if (Plain) {
+    // numerator and denominator exactly (15 factors below 2^7), their quotient
+    // and its remainder
+    __int128 num = 1, den = 1;
+    for (int j = 0; j < NP; ++j)
+      if (j != k) {
+        num *= i - far_node(Plain, tile, j);
+        den *= far_node(Plain, tile, k) - far_node(Plain, tile, j);
+      }
+    const double nh = (double)num, nl = (double)(num - (__int128)nh);
+    const double dh = (double)den, dl = (double)(den - (__int128)dh);
+    const double q = nh / dh;
+    const FarPair p = far_product(q, dh);
+    return q + ((nh - p.hi) - p.lo + nl - q * dl) / dh;
+  }
+  double v = 1.;
+  for (int j = 0; j < NP; ++j)
+    if (j != k)
+      v *= (double)(i - far_node(Plain, tile, j)) /
+           (double)(far_node(Plain, tile, k) - far_node(Plain, tile, j));
+  return v;
 }
-constexpr FarPairs far_pairs() {
-  FarPairs w{};
-  for (int k = 0; k < Far<true>::NP; ++k) {
-    for (int i = 0; i < kFarLeaf; ++i) w.leaf[k][i] = far_pair(false, k, i);
-    for (int i = 0; i < kFarTilePts; ++i) w.tile[k][i] = far_pair(true, k, i);
+template <bool Plain>
+struct FarWeights {
+  double leaf[Far<Plain>::NP][kFarLeaf], tile[Far<Plain>::NP][kFarTilePts];
+};
+template <bool Plain>
+constexpr FarWeights<Plain> far_weights() {
+  FarWeights<Plain> w{};
+  for (int k = 0; k < Far<Plain>::NP; ++k) {
+    for (int i = 0; i < kFarLeaf; ++i) w.leaf[k][i] = far_weight<Plain>(false, k, i);
+    for (int i = 0; i < kFarTilePts; ++i) w.tile[k][i] = far_weight<Plain>(true, k, i);
   }
   return w;
 }
@@ -119,37 +105,17 @@ CLBLM_HD double far_fma(double a, double b, double c) {
   return std::fma(a, b, c);
 #endif
 }
-CLBLM_HD double far_mul(double a, double b) {
+CLBLM_HD double far_sub(double a, double b) {
 #ifdef __CUDA_ARCH__
-  return __dmul_rn(a, b);
+  return __dsub_rn(a, b);
 #else
-  return a * b;
-#endif
-}
-CLBLM_HD double far_add(double a, double b) {
-#ifdef __CUDA_ARCH__
-  return __dadd_rn(a, b);
-#else
-  return a + b;
+  return a - b;
 #endif
 }
 
-// sum of w_k v_k, the roundings of its products and additions kept beside it
-// (Knuth's two-sum; the dot product of Ogita, Rump and Oishi, SIAM J. Sci.
-// Comput. 26, 2005)
-struct FarSum {
-  double s = 0., c = 0.;
-  CLBLM_HD void add(double x) {
-    const double t = far_add(s, x), b = far_add(t, -s);
-    c = far_add(c, far_add(far_add(s, -far_add(t, -b)), far_add(x, -b)));
-    s = t;
-  }
-  CLBLM_HD void add(FarPair w, double v) {
-    const double p = far_mul(w.hi, v);
-    c = far_fma(w.lo, v, far_add(c, far_fma(w.hi, v, -p)));
-    add(p);
-  }
-  CLBLM_HD double value() const { return far_add(s, c); }
-};
+// FP64 path: s + w (v - ref) of a node's sum v, ref the sum of node kFarRef,
+// which the caller adds to the total
+constexpr int kFarRef = 8;
+CLBLM_HD double far_carry(double w, double v, double ref, double s) { return far_fma(w, far_sub(v, ref), s); }
 
 }  // namespace clblm

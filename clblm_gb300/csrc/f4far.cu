@@ -17,8 +17,7 @@
 //     lane, the records passing through shared memory.
 // With R = 976 that is 422 evaluations (FP64 path: 690) per unit of record
 // density and point instead of 1928.  Node sums are carried to the points
-// in binary64 (compensated on the FP64 path).  The
-// index ranges come from the running bounds of the records' centres (their
+// in binary64.  The index ranges come from the running bounds of the records' centres (their
 // order is nearly that of their centres): searches, one per lane.
 //
 // FP64: reference's terms, one division each (a reciprocal; the reference's
@@ -42,8 +41,8 @@ namespace {
 constexpr int kLeaf = kFarLeaf, kTileLeaves = kFarTile / kLeaf;
 static_assert(kFarTile == kFarTilePts && 32 * kTileLeaves == kFarThreads, "a warp per leaf");
 
-__device__ const FarWeights c_farw_mixed = far_weights();
-__device__ const FarPairs c_farw_plain = far_pairs();
+__device__ const FarWeights<false> c_farw_mixed = far_weights<false>();
+__device__ const FarWeights<true> c_farw_plain = far_weights<true>();
 
 __device__ __forceinline__ float rcp_f(float x) {  // PTX rcp.approx: relative error < 2^-23
   float r;
@@ -384,6 +383,7 @@ __global__ void __launch_bounds__(kFarThreads, Plain ? 4 : 6) k_f4_far(const __g
     const double v = s.template total<true>(lane, P.dvr4);
     if (!(lane & 1)) nodeB[warp][lane >> 1] = v;
   }
+  const bool tfar = E1 < N1 || N2 < E2;
   // no far range of the tile on a side: the leaf's far range is one
   if (!(E1 < N1)) E1 = N1 = n1;
   if (!(N2 < E2)) N2 = E2 = n2;
@@ -433,15 +433,22 @@ __global__ void __launch_bounds__(kFarThreads, Plain ? 4 : 6) k_f4_far(const __g
   double v = 0.;
   if (m < P.nptr4) {
     if constexpr (Plain) {
-      FarSum f;
+      // (far_carry; a tile or leaf without far records has nothing to carry)
+      double ref = 0.;
+      if (tfar) {
+        auto b = [&](int k) { return (nodeB[0][k] + nodeB[1][k]) + (nodeB[2][k] + nodeB[3][k]); };
+        const double r = b(kFarRef);
 #pragma unroll
-      for (int k = 0; k < NP; ++k) {
-        const double b = (nodeB[0][k] + nodeB[1][k]) + (nodeB[2][k] + nodeB[3][k]);
-        f.add(c_farw_plain.tile[k][kLeaf * warp + lane], b);
-        f.add(c_farw_plain.leaf[k][lane], nodeA[warp][k]);
+        for (int k = 0; k < NP; ++k) v = far_carry(c_farw_plain.tile[k][kLeaf * warp + lane], b(k), r, v);
+        ref = r;
       }
-      f.add(acc);
-      v = f.value();
+      if (fl || fr) {
+        const double r = nodeA[warp][kFarRef];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) v = far_carry(c_farw_plain.leaf[k][lane], nodeA[warp][k], r, v);
+        ref += r;
+      }
+      v = (v + ref) + acc;
     } else {
 #pragma unroll
       for (int k = 0; k < NP; ++k) {

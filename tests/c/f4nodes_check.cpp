@@ -1,7 +1,7 @@
-// Host check of the far wings' nodes (clblm_f4nodes.cuh): the FP64 path's
-// weights as pairs, the polynomial's own error at the least distance, the
-// compensated sum over the nodes, and sums of one to 300 records through nodes
-// against the same sums record by record, each to long double.
+// Host check of the far wings' nodes (clblm_f4nodes.cuh): the error of the
+// polynomial and its weights at the least distance, and sums of one to 300
+// records through nodes against the same sums record by record, each to long
+// double.
 #include <cmath>
 #include <cstdio>
 #include <random>
@@ -13,17 +13,16 @@ using namespace clblm;
 using L = long double;
 
 namespace {
-const FarWeights kMixed = far_weights();
-const FarPairs kPlain = far_pairs();
+const FarWeights<false> kMixed = far_weights<false>();
+const FarWeights<true> kPlain = far_weights<true>();
 int bad = 0;
 void hold(const char* what, L got, L bound) {
   printf("%s %.3Le (bound %.3Le)\n", what, got, bound);
   if (!(got <= bound)) bad++;
 }
-const FarPair& pair_of(bool tile, int k, int i) { return tile ? kPlain.tile[k][i] : kPlain.leaf[k][i]; }
 int points(bool tile) { return tile ? kFarTilePts : kFarLeaf; }
 
-// largest relative error of 1/x^2, x0 to either side, carried by the weights
+// largest relative error of 1/x^2, its pole to either side, carried by the weights
 L polynomial(bool plain, bool tile) {
   const int n = points(tile), NP = plain ? Far<true>::NP : Far<false>::NP;
   const L D = (plain ? Far<true>::D : Far<false>::D) * (tile ? 4 : 1);
@@ -33,9 +32,10 @@ L polynomial(bool plain, bool tile) {
       auto f = [&](int m) { return 1 / ((m - at) * (m - at)); };
       L s = 0;
       for (int k = 0; k < NP; ++k) {
-        const L w = plain ? (L)pair_of(tile, k, i).hi + (L)pair_of(tile, k, i).lo
-                          : (L)(tile ? kMixed.tile[k][i] : kMixed.leaf[k][i]);
-        s += w * f(far_node(plain, tile, k));
+        const double w = plain ? (tile ? kPlain.tile[k][i] : kPlain.leaf[k][i])
+                               : (tile ? kMixed.tile[k][i] : kMixed.leaf[k][i]);
+        const L ref = plain ? f(far_node(plain, tile, kFarRef)) : 0;
+        s += w * (f(far_node(plain, tile, k)) - ref) + (k == 0 ? ref : 0);
       }
       worst = std::fmax(worst, std::fabs(s / f(i) - 1));
     }
@@ -44,34 +44,16 @@ L polynomial(bool plain, bool tile) {
 }  // namespace
 
 int main() {
-  // the rounding of a double, 1.1e-16, is the FP64 path's measure, FP32's 6e-8 the mixed path's
+  // FP32's rounding is 6e-8 (mixed path), a double's 1.1e-16 (FP64 path: 1.8e-16
+  // and 3.1e-16 of the polynomial, and weights to half a unit, magnitudes adding
+  // up to 3, of differences up to 0.9 of the term)
   hold("mixed leaf", polynomial(false, false), 4.0e-8L);
   hold("mixed tile", polynomial(false, true), 4.0e-8L);
-  hold("fp64 leaf", polynomial(true, false), 2.0e-16L);
-  hold("fp64 tile", polynomial(true, true), 3.5e-16L);
+  hold("fp64 leaf", polynomial(true, false), 4.0e-16L);
+  hold("fp64 tile", polynomial(true, true), 5.5e-16L);
 
   std::mt19937_64 g(5);
   std::uniform_real_distribution<double> u(0., 1.);
-  // the sum over the nodes rounds once
-  L sum = 0;
-  for (int t = 0; t < 200; ++t) {
-    double v[2][16];
-    for (auto& r : v)
-      for (double& x : r) x = 1. + u(g);
-    for (int i = 0; i < kFarTilePts; ++i) {
-      FarSum s;
-      L e = 0;
-      for (int k = 0; k < 16; ++k)
-        for (int tile = 1; tile >= 0; --tile) {
-          const FarPair& w = pair_of(tile != 0, k, tile ? i : i % kFarLeaf);
-          s.add(w, v[tile][k]);
-          e += ((L)w.hi + (L)w.lo) * v[tile][k];
-        }
-      sum = std::fmax(sum, std::fabs(s.value() / e - 1));
-    }
-  }
-  hold("compensated sum", sum, 1.15e-16L);
-
   // records within R points of a tile, near records left out
   const int R = 976, T0 = 5000, D = Far<true>::D;
   const double step = 25. / R;
@@ -116,12 +98,11 @@ int main() {
           const double xd = std::fma((double)(T0 + i), step, -xn[q]);
           d += sil[q] / std::fma(xd, xd, al2[q]);
         }
-        FarSum s;
-        for (int k = 0; k < 16; ++k) {
-          s.add(kPlain.tile[k][i], vt[k]);
-          s.add(kPlain.leaf[k][i % kFarLeaf], vl[i / kFarLeaf][k]);
-        }
-        const L rn = s.value() / e - 1, rd = d / e - 1;
+        double s = 0.;
+        const double* a = vl[i / kFarLeaf];
+        for (int k = 0; k < 16; ++k) s = far_carry(kPlain.tile[k][i], vt[k], vt[kFarRef], s);
+        for (int k = 0; k < 16; ++k) s = far_carry(kPlain.leaf[k][i % kFarLeaf], a[k], a[kFarRef], s);
+        const L rn = (s + (vt[kFarRef] + a[kFarRef])) / e - 1, rd = d / e - 1;
         e_node += rn * rn;
         e_direct += rd * rd;
         cnt++;

@@ -1,6 +1,6 @@
 """The far wings' nodes (clblm_gb300/csrc/clblm_f4nodes.cuh): the error of the
-polynomial through them, of the sum over them, and of whole sums of records
-through them against those record by record: tests/c/f4nodes_check.cpp,
+polynomial through them and of whole sums of records through them against
+those record by record: tests/c/f4nodes_check.cpp,
 compiled for the host from the same header."""
 import shutil
 import subprocess
