@@ -124,7 +124,8 @@ __global__ void __launch_bounds__(kScanThreads)
                int64_t* cut);
 __global__ void __launch_bounds__(kScanThreads)
     k_f4_compact(const F4Prep* prep, const unsigned* mask, int64_t mstride, int64_t stride, const LayerPlan* plans,
-                 int layer0, const int64_t* blocksum, int nblk, int64_t* cidx, long long* vbits, long long* lbits, int64_t* src, unsigned char* flags,
+                 int layer0, const int64_t* blocksum, int nblk, int64_t* cidx, long long* vbits, long long* lbits,
+                 int64_t* src, unsigned char* flags,
                  int64_t* cut, int64_t* ntot);
 __global__ void k_f4_next(const long long* vbits, const long long* lbits, const int64_t* ntot, int64_t stride,
                           int* gnxt);

@@ -41,8 +41,9 @@ struct SegPool {
   double2* med_v;  // [kMedPoolSlots][kMaxSeg]
 };
 // bytes of the pool, next included
-constexpr size_t kSegPoolBytes = 256 + (sizeof(int) * (kSegSlot + 1) + 2 * sizeof(double) * kSegSlot) * (size_t)kSegPoolSlots +
-                                 (sizeof(int) + sizeof(double2)) * (size_t)kMaxSeg * kMedPoolSlots;
+constexpr size_t kSegPoolBytes =
+    256 + (sizeof(int) * (kSegSlot + 1) + 2 * sizeof(double) * kSegSlot) * (size_t)kSegPoolSlots +
+    (sizeof(int) + sizeof(double2)) * (size_t)kMaxSeg * kMedPoolSlots;
 
 struct PanelArgs {
   const LayerPlan* plans;

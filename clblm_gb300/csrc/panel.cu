@@ -285,8 +285,9 @@ __device__ __forceinline__ int seg_code(bool big, int slot) { return -2 - (2 * s
 // its second, the XINT set-up.  Past kSegTab segments they go to a slot of the
 // pool, and seg_n is the slot (seg_code) and seg_start[.. kSegTab] their
 // number; with no slot left seg_n is -1 and the far-wing pass forms them itself
-// (far infrared, 24 cm-1 panels: up to 800, 2 ms of that pass's CTA).  Both are chains of binary64 divisions and exponentials (a
-// segment takes about 3 us, the set-up 15): formed by one lane of the far-wing
+// (far infrared, 24 cm-1 panels: up to 800, 2 ms of that pass's CTA).  Both are
+// chains of binary64 divisions and exponentials (a segment takes about 3 us, the
+// set-up 15): formed by one lane of the far-wing
 // pass's CTA, the segments of a surface panel were two thirds of its 88 us,
 // and the set-up a third of the others' 43 us.
 __global__ void __launch_bounds__(64)
@@ -863,7 +864,8 @@ __global__ void __launch_bounds__(kPanelThreads, Plain ? (Part == kPanelWings ? 
   }
   if constexpr (kWings) {  // XINT set-up of the panel (k_panel_setup)
     const int* x = reinterpret_cast<const int*>(&a.xint[(int64_t)layer * a.panel_stride + p]);
-    for (int i = tid; i < (int)(sizeof(XintPanel) / sizeof(int)); i += kPanelThreads) reinterpret_cast<int*>(&S.X)[i] = x[i];
+    int* X = reinterpret_cast<int*>(&S.X);
+    for (int i = tid; i < (int)(sizeof(XintPanel) / sizeof(int)); i += kPanelThreads) X[i] = x[i];
   }
   __syncthreads();
   if constexpr (!Plain && kWings) {  // ABSRB of the panel as FP32
@@ -1561,9 +1563,10 @@ template __global__ void k_rsym<true>(const __grid_constant__ PanelArgs);
 // record, so the records per stage (CHUNK, a multiple of kF4Group, chosen by
 // the autotuner) do not change the result.
 //
-// Only the ODs of the mixed path's Jacobians come through here: they are
-// differenced (T + 1 K, Wtot * 1.01), which amplifies the last bits of a sum
-// formed another way by some thousands; k_f4_far, with a quarter of the
+// Only the ODs of the mixed path's Jacobians come through here: the viewing
+// path's, T + 1 K's and Wtot * 1.01's are differenced, which amplifies the last
+// bits of a sum formed another way by some thousands, and those of the molecule
+// alone, which are not, share their launch; k_f4_far, with a quarter of the
 // evaluations, serves every other call.
 
 // FP32 terms of far-wing record r at a thread's two points (packed FP32x2):

@@ -1397,9 +1397,10 @@ __global__ void __launch_bounds__(kScanThreads)
 // was 19 us of a layer's chain); the warps count with ballots.
 __global__ void __launch_bounds__(kScanThreads)
     k_f4_compact(const F4Prep* __restrict__ prep, const unsigned* __restrict__ mask, int64_t mstride, int64_t stride,
-                 const LayerPlan* __restrict__ plans, int layer0, const int64_t* __restrict__ blocksum, int nblk, int64_t* __restrict__ cidx,
-                 long long* __restrict__ vbits, long long* __restrict__ lbits, int64_t* __restrict__ src,
-                 unsigned char* __restrict__ flags, int64_t* __restrict__ cut, int64_t* __restrict__ ntot) {
+                 const LayerPlan* __restrict__ plans, int layer0, const int64_t* __restrict__ blocksum, int nblk,
+                 int64_t* __restrict__ cidx, long long* __restrict__ vbits, long long* __restrict__ lbits,
+                 int64_t* __restrict__ src, unsigned char* __restrict__ flags, int64_t* __restrict__ cut,
+                 int64_t* __restrict__ ntot) {
   constexpr int kWarps = kScanThreads / 32, kRows = kScanBlock / kScanThreads;
   __shared__ long long before[kWarps];
   __shared__ int total[kWarps];

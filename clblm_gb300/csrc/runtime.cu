@@ -181,13 +181,12 @@ struct clblm_handle {
   int nsm = 1;  // SMs of the device
   // every device buffer of the handle but the line list
   std::vector<DevBuf*> buffers() {
-    std::vector<DevBuf*> v = {&cont_self, &cont_for, &cont_texp, &cont_co2, &tabs,    &prep,    &qpanel,
-                              &rec,       &recd,     &ranges,    &od,      &r4,      &absrb,  &blockmax,  &f4prep,    &f4sh,    &f4rec,  &f4recd,  &f4nrec,
-                              &f4nmir,    &f4pm,     &f4sm,      &outbuf,  &bfac,     &f4mask,    &f4blk,     &f4ntot,  &f4cidx,  &f4vb,   &f4lb,    &f4src,
-                              &f4flag,    &f4cut,    &f4grp,     &f4nxt,   &ragg,    &segpool, &gpm,    &gsm,
-                              &reclo,     &jprof,    &jod,       &jmap,    &jjobs,   &jblk,    &jvjp,   &linecpl,   &f4cpl,    &f4cpll,    &f4ncpl,   &pwork,
-                              &f4tab,     &f4calls,  &f4ncall,  &f4agg,     &psegn,
-                              &psegs,     &psegv, &pxint, &tabbuf};
+    std::vector<DevBuf*> v = {&cont_self, &cont_for, &cont_texp, &cont_co2, &tabs, &tabbuf, &prep, &qpanel, &rec,
+                              &recd, &reclo, &gpm, &gsm, &ragg, &ranges, &blockmax, &linecpl, &pwork, &psegn, &psegs,
+                              &psegv, &pxint, &segpool, &od, &r4, &absrb, &bfac, &f4prep, &f4mask, &f4blk, &f4ntot,
+                              &f4cidx, &f4vb, &f4lb, &f4src, &f4flag, &f4cut, &f4nxt, &f4tab, &f4calls, &f4ncall,
+                              &f4grp, &f4sh, &f4rec, &f4recd, &f4nrec, &f4nmir, &f4agg, &f4pm, &f4sm, &f4cpl,
+                              &f4cpll, &f4ncpl, &jprof, &jod, &jmap, &jjobs, &jblk, &jvjp, &outbuf};
     for (auto& b : rt) v.push_back(&b);
     for (auto& b : imap) v.push_back(&b);
     v.push_back(&rtseg);
@@ -1082,7 +1081,8 @@ SegPool seg_pool(const clblm_handle* h) {
 
 // Runs the OD pipeline for `count` layers whose plans are already uploaded at
 // plans[first..]; OD of layer k lands at od + P.od_off (Real).
-// jac: the ODs of a Jacobian call (the mixed path keeps the order of their far-wing sums).
+// jac: the ODs of a Jacobian call (the mixed path keeps the order of their far-wing sums, of
+// the molecule alone too, which are not differenced but share the launch).
 int run_od_batch(clblm_handle* h, std::vector<HostPlan>& hps, int first, int count, bool plain, bool jac,
                  int64_t lstride, int64_t f4stride, int64_t pstride) {
   const LayerPlan* dplans = h->plans.as<const LayerPlan>();
@@ -4190,7 +4190,8 @@ int clblm_gpu_fftscn(clblm_handle_t* h, const clblm_scan_t* scan, const double* 
       cufftDestroy(h->scan_inv);
       h->scan_plans = false;
     }
-    if (len > (int64_t)1 << 30 || cufftPlan1d(&h->scan_fwd, (int)len, batch == 1 ? CUFFT_D2Z : CUFFT_Z2Z, batch) != CUFFT_SUCCESS)
+    if (len > (int64_t)1 << 30 ||
+        cufftPlan1d(&h->scan_fwd, (int)len, batch == 1 ? CUFFT_D2Z : CUFFT_Z2Z, batch) != CUFFT_SUCCESS)
       return set_err(h, CLBLM_ERR_OOM, "FFTSCN: no cuFFT plan for %lld points", (long long)len);
     if (cufftPlan1d(&h->scan_inv, (int)len, batch == 1 ? CUFFT_Z2D : CUFFT_Z2Z, batch) != CUFFT_SUCCESS) {
       cufftDestroy(h->scan_fwd);

@@ -538,26 +538,29 @@ __global__ void __launch_bounds__(kScanLowThreads)
   }
 }
 
-template __global__ void k_scan_moments<kScanTerms>(const double* __restrict__, int64_t, int64_t, int, int64_t, double,
-                                             double2* __restrict__, int64_t, int, int64_t, double2* __restrict__);
-template __global__ void k_scan_low<kScanTerms>(ScanArgs, double, double, int64_t, int64_t, int, const double2* __restrict__,
-                                         const double2* __restrict__, double2* __restrict__);
-template __global__ void k_scan_expand<kScanTerms, false>(const double2* __restrict__, int64_t, int, int64_t, int64_t,
-                                                   double* __restrict__, ScanFloor);
-template __global__ void k_scan_expand<kScanTerms, true>(const double2* __restrict__, int64_t, int, int64_t, int64_t,
-                                                   double* __restrict__, ScanFloor);
-template __global__ void k_scan_moments<kScanTermsWide>(const double* __restrict__, int64_t, int64_t, int, int64_t, double,
-                                             double2* __restrict__, int64_t, int, int64_t, double2* __restrict__);
-template __global__ void k_scan_low<kScanTermsWide>(ScanArgs, double, double, int64_t, int64_t, int, const double2* __restrict__,
-                                         const double2* __restrict__, double2* __restrict__);
-template __global__ void k_scan_expand<kScanTermsWide, false>(const double2* __restrict__, int64_t, int, int64_t, int64_t,
-                                                   double* __restrict__, ScanFloor);
-template __global__ void k_scan_expand<kScanTermsWide, true>(const double2* __restrict__, int64_t, int, int64_t, int64_t,
-                                                   double* __restrict__, ScanFloor);
-template __global__ void k_scan_fft<false>(const double2* __restrict__, double2* __restrict__, const double2* __restrict__,
-                                          int64_t, int64_t, int);
-template __global__ void k_scan_fft<true>(const double2* __restrict__, double2* __restrict__, const double2* __restrict__,
-                                          int64_t, int64_t, int);
+#define CLBLM_MOMENTS_ARGS                                                                              \
+  const double* __restrict__, int64_t, int64_t, int, int64_t, double, double2* __restrict__, int64_t, int, \
+      int64_t, double2* __restrict__
+#define CLBLM_LOW_ARGS                                                                                    \
+  ScanArgs, double, double, int64_t, int64_t, int, const double2* __restrict__, const double2* __restrict__, \
+      double2* __restrict__
+#define CLBLM_EXPAND_ARGS const double2* __restrict__, int64_t, int, int64_t, int64_t, double* __restrict__, ScanFloor
+#define CLBLM_SCANFFT_ARGS \
+  const double2* __restrict__, double2* __restrict__, const double2* __restrict__, int64_t, int64_t, int
+template __global__ void k_scan_moments<kScanTerms>(CLBLM_MOMENTS_ARGS);
+template __global__ void k_scan_moments<kScanTermsWide>(CLBLM_MOMENTS_ARGS);
+template __global__ void k_scan_low<kScanTerms>(CLBLM_LOW_ARGS);
+template __global__ void k_scan_low<kScanTermsWide>(CLBLM_LOW_ARGS);
+template __global__ void k_scan_expand<kScanTerms, false>(CLBLM_EXPAND_ARGS);
+template __global__ void k_scan_expand<kScanTerms, true>(CLBLM_EXPAND_ARGS);
+template __global__ void k_scan_expand<kScanTermsWide, false>(CLBLM_EXPAND_ARGS);
+template __global__ void k_scan_expand<kScanTermsWide, true>(CLBLM_EXPAND_ARGS);
+template __global__ void k_scan_fft<false>(CLBLM_SCANFFT_ARGS);
+template __global__ void k_scan_fft<true>(CLBLM_SCANFFT_ARGS);
+#undef CLBLM_MOMENTS_ARGS
+#undef CLBLM_LOW_ARGS
+#undef CLBLM_EXPAND_ARGS
+#undef CLBLM_SCANFFT_ARGS
 
 __global__ void k_scan_out(const double* __restrict__ y, int64_t first, int64_t count, double scale,
                            double* __restrict__ out) {
