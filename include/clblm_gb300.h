@@ -345,7 +345,14 @@ int clblm_gpu_jac_size(clblm_handle_t *h, const clblm_column_t *col,
  *   dr_dqlev   [(nlay+1)*npts]   dR/d ln q of each level for jac->jac_mol
  *   dr_dtskin  [npts]            dR/dTskin
  *   dr_demis   [npts]            dR/d emissivity
- * `cap` is the capacity of each spectrum (>= npts). */
+ * `cap` is the capacity of each spectrum (>= npts).
+ *
+ * Memory: the blocks' ODs are formed together, as many blocks as fit 24 GB of
+ * scratch, OD slabs and maps (or the OD budget, where that is less), one block
+ * at a time when the device has no room for more.  The handle keeps what it
+ * has allocated until it is destroyed.  CLBLM_OD_BUDGET_GB=<GB> in the
+ * environment sets the OD budget, and with it this bound, for programs that
+ * share the device's memory with others. */
 int clblm_gpu_jac(clblm_handle_t *h, const clblm_column_t *col,
                   const clblm_rt_ctrl_t *ctrl, const clblm_jac_t *jac,
                   double *rad, double *dr_dtlev, double *dr_dqlev,
