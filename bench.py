@@ -95,6 +95,20 @@ def load_traffic():
     return out
 
 
+def load_evaluated():
+    """Share of the reference's far-wing steps that k_f4_far evaluates on this
+    column (profiles/f4far_evaluations.md, line `k_f4_far mixed share`), or
+    None."""
+    try:
+        for line in (ROOT / "profiles" / "f4far_evaluations.md").read_text().splitlines():
+            f = line.split()
+            if f[:2] == ["k_f4_far", "mixed"]:
+                return float(f[2])
+    except (OSError, ValueError, IndexError):
+        pass
+    return None
+
+
 def roofline(work, kt, steps, ms_step, points):
     """Roofline of the dominant line-shape kernel: algorithmic FLOPs of one
     launch (the call's step counts) over its CUDA-event time on the library's
@@ -102,13 +116,15 @@ def roofline(work, kt, steps, ms_step, points):
     points) scales the measured DRAM bytes per point to the launch."""
     peak, mhz = fp32_peak_tflops()
     traffic = load_traffic()
+    share = load_evaluated()
+    f4_flop = FLOP_CNVF4Q * work["cnvf4q_steps"]
     kernels = {
-        "k_f4_far": (FLOP_CNVF4Q * work["cnvf4q_steps"], kt["ms_f4conv"] / steps, work["cnvf4q_steps"]),
-        "k_panel": (FLOP_CNVFNQ * work["cnvfnq_steps"], kt["ms_panel"] / steps, work["cnvfnq_steps"]),
+        "k_f4_far": (f4_flop * share if share is not None else None, kt["ms_f4conv"] / steps),
+        "k_panel": (FLOP_CNVFNQ * work["cnvfnq_steps"], kt["ms_panel"] / steps),
     }
     out = {}
-    for name, (flop, ms, nstep) in kernels.items():
-        ach = flop / (ms * 1e-3) / 1e12 if ms > 0 else None
+    for name, (flop, ms) in kernels.items():
+        ach = flop / (ms * 1e-3) / 1e12 if ms > 0 and flop is not None else None
         bpp = traffic.get(name)
         out[name] = {"bound": "fp32", "achieved": ach, "peak": peak, "unit": "TFLOP/s",
                      "frac": ach / peak if ach else None,
@@ -117,10 +133,13 @@ def roofline(work, kt, steps, ms_step, points):
                                         "(profiles/dram_traffic.txt) x this launch's points"
                                         if bpp is not None else None),
                      "ms_per_launch": ms, "share_of_step": ms / ms_step, "flop_per_launch": flop}
-    # the counted steps are the reference's, every record at every point it
-    # reaches; distant records are evaluated at nodes and interpolated
-    out["k_f4_far"]["flop_counted"] = ("the reference's steps; k_f4_far evaluates a quarter of them, so its pipes do "
-                                       "about a quarter of `achieved`")
+    # the call's counter holds the reference's steps, every record at every
+    # point it reaches; distant records are evaluated at nodes and interpolated
+    ms = out["k_f4_far"]["ms_per_launch"]
+    out["k_f4_far"]["flop_counted"] = "the evaluations made: evaluated_share of the reference's steps"
+    out["k_f4_far"]["evaluated_share"] = share
+    out["k_f4_far"]["evaluated_share_source"] = "counted once on this column (profiles/f4far_evaluations.md)"
+    out["k_f4_far"]["reference_steps_tflops"] = f4_flop / (ms * 1e-3) / 1e12 if ms > 0 else None
     if kt.get("ms_rt", 0) > 0 and work.get("rt_bytes", 0) > 0:
         # the layer recurrence (one launch per run of layers on one merge
         # grid): algorithmic bytes over its device time, against the measured
