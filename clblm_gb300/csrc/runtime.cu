@@ -2754,8 +2754,10 @@ int jac_plan_block(clblm_handle* h, const clblm_rt_ctrl_t* ctrl, const clblm_jac
 }
 
 // Scratch, OD slabs and maps of the blocks whose ODs clblm_gpu_jac forms
-// together, and their ODs (three rows of CTAs each in the line bounds' grid)
-constexpr size_t kJacGroupBytes = (size_t)24 << 30;
+// together, and their ODs (three rows of CTAs each in the line bounds' grid).
+// (At 24 GB the 25 blocks of a 60-layer 500 cm-1 call are three groups, 71.4 ms,
+// at 32 GB two, 70.9.)
+constexpr size_t kJacGroupBytes = (size_t)32 << 30;
 constexpr int kJacGroupJobs = 65535 / 3;
 
 // The blocks of noScattJacob (clblm_noScattJac.f90:206-232): V1B, V2B and

@@ -347,7 +347,7 @@ int clblm_gpu_jac_size(clblm_handle_t *h, const clblm_column_t *col,
  *   dr_demis   [npts]            dR/d emissivity
  * `cap` is the capacity of each spectrum (>= npts).
  *
- * Memory: the blocks' ODs are formed together, as many blocks as fit 24 GB of
+ * Memory: the blocks' ODs are formed together, as many blocks as fit 32 GB of
  * scratch, OD slabs and maps (or the OD budget, where that is less), one block
  * at a time when the device has no room for more.  The handle keeps what it
  * has allocated until it is destroyed.  CLBLM_OD_BUDGET_GB=<GB> in the
